@@ -1,71 +1,277 @@
 // True 32-bit matrix product for the check path: C[M,N] = A[M,K] W[N,K]^T (+ bias),
 // plain FMA in float, no tensor cores and no reduced-precision mode.  Each output
 // element sums its K products in index order, so a row's result does not depend
-// on how many other rows are in the batch.
+// on how many other rows are in the batch, nor on the tile the element falls into.
+//
+// A block of 16 x 16 threads computes TM * 16 rows x 128 columns, TM x 8 sums a thread, two columns an
+// instruction (fma.rn.f32x2 rounds each half as fmaf does).  Bound by the FMA pipe: per step of k a warp issues 4 TM
+// paired multiply-adds and reads TM + 8 floats a thread from shared memory, 8 of them as 16-byte loads.  Operands are
+// staged k-major, 16 of k at a time, the next piece's global loads in registers while this one is multiplied.
 #include "common.cuh"
 
-#define TILE_M 64
-#define TILE_N 64
+#define TILE_N 128
 #define TILE_K 16
+#define GEMM_THREADS 256
 
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ unsigned long long f32_pair(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f32_fma2(unsigned long long a, unsigned long long b,
+                                                       unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// VEC: K and lda are whole 4s and both bases lie on 16 bytes (16-byte loads along k)
+template <int TM, bool VEC>
+__global__ void __launch_bounds__(GEMM_THREADS, TM == 8 ? 2 : 3)
 gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
                 const float* __restrict__ bias, float* __restrict__ c, int M, int N, int K,
                 int lda, int ldc) {
-  __shared__ float a_s[TILE_K][TILE_M + 1];
-  __shared__ float w_s[TILE_K][TILE_N + 1];
+  constexpr int TILE_M = TM * 16;
+  constexpr int kAStride = TILE_M + 4, kWStride = TILE_N + 4;
+  // 16-byte pieces of k a thread loads a step
+  constexpr int kAPieces = (TILE_M * TILE_K / 4 + GEMM_THREADS - 1) / GEMM_THREADS;
+  constexpr int kWPieces = TILE_N * TILE_K / 4 / GEMM_THREADS;
+  __shared__ __align__(16) float a_s[2][TILE_K * kAStride];
+  __shared__ __align__(16) float w_s[2][TILE_K * kWStride];
   const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * TILE_N;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-  float acc[4][4];
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  unsigned long long acc[TM][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 
-  for (int k0 = 0; k0 < K; k0 += TILE_K) {
-    // 64 rows x 16 k = 1024 elements per operand, 4 per thread
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int idx = threadIdx.x + e * 256;
-      const int row = idx / TILE_K, kk = idx % TILE_K;
-      const int gk = k0 + kk;
-      a_s[kk][row] = (m0 + row < M && gk < K) ? a[(size_t)(m0 + row) * lda + gk] : 0.f;
-      w_s[kk][row] = (n0 + row < N && gk < K) ? w[(size_t)(n0 + row) * K + gk] : 0.f;
+  float4 a_r[kAPieces], w_r[kWPieces];
+  auto load4 = [&](const float* base, int row, int rows, int ld, int k) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < rows) {
+      const float* src = base + (size_t)row * ld + k;
+      if (VEC) {
+        if (k < K) v = *reinterpret_cast<const float4*>(src);
+      } else {
+        if (k < K) v.x = src[0];
+        if (k + 1 < K) v.y = src[1];
+        if (k + 2 < K) v.z = src[2];
+        if (k + 3 < K) v.w = src[3];
+      }
     }
-    __syncthreads();
+    return v;
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int e = 0; e < kAPieces; ++e) {
+      const int idx = threadIdx.x + e * GEMM_THREADS, row = idx / (TILE_K / 4);
+      if (TILE_M * TILE_K / 4 % GEMM_THREADS == 0 || row < TILE_M) a_r[e] = load4(a, m0 + row, M, lda, k0 + idx % (TILE_K / 4) * 4);
+    }
+#pragma unroll
+    for (int e = 0; e < kWPieces; ++e) {
+      const int idx = threadIdx.x + e * GEMM_THREADS;
+      w_r[e] = load4(w, n0 + idx / (TILE_K / 4), N, K, k0 + idx % (TILE_K / 4) * 4);
+    }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int e = 0; e < kAPieces; ++e) {
+      const int idx = threadIdx.x + e * GEMM_THREADS, row = idx / (TILE_K / 4);
+      float* to = &a_s[buf][idx % (TILE_K / 4) * 4 * kAStride + row];
+      if (TILE_M * TILE_K / 4 % GEMM_THREADS == 0 || row < TILE_M) {
+        to[0] = a_r[e].x; to[kAStride] = a_r[e].y; to[2 * kAStride] = a_r[e].z; to[3 * kAStride] = a_r[e].w;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kWPieces; ++e) {
+      const int idx = threadIdx.x + e * GEMM_THREADS;
+      float* to = &w_s[buf][idx % (TILE_K / 4) * 4 * kWStride + idx / (TILE_K / 4)];
+      to[0] = w_r[e].x; to[kWStride] = w_r[e].y; to[2 * kWStride] = w_r[e].z; to[3 * kWStride] = w_r[e].w;
+    }
+  };
+
+  fetch(0);
+  put(0);
+  __syncthreads();
+  const int steps = (K + TILE_K - 1) / TILE_K;
+  for (int s = 0; s < steps; ++s) {
+    const int buf = s & 1;
+    if (s + 1 < steps) fetch((s + 1) * TILE_K);
+    const float* a_b = &a_s[buf][ty * TM];
+    const float* w_b = &w_s[buf][tx * 4];
 #pragma unroll
     for (int kk = 0; kk < TILE_K; ++kk) {
-      float av[4], wv[4];
+      float av[TM];
+      if (TM % 4 == 0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = a_s[kk][ty * 4 + i];
+        for (int i = 0; i < TM; i += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(a_b + kk * kAStride + i);
+          av[i] = v.x; av[i + 1] = v.y; av[i + 2] = v.z; av[i + 3] = v.w;
+        }
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) wv[j] = w_s[kk][tx * 4 + j];
+        for (int i = 0; i < TM; ++i) av[i] = a_b[kk * kAStride + i];
+      }
+      // columns tx * 4 .. + 3 and 64 + tx * 4 .. + 3: neighbouring threads read neighbouring 16 bytes
+      const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(w_b + kk * kWStride);
+      const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(w_b + kk * kWStride + 64);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+      for (int i = 0; i < TM; ++i) {
+        const unsigned long long both = f32_pair(av[i], av[i]);
+        acc[i][0] = f32_fma2(both, lo.x, acc[i][0]);
+        acc[i][1] = f32_fma2(both, lo.y, acc[i][1]);
+        acc[i][2] = f32_fma2(both, hi.x, acc[i][2]);
+        acc[i][3] = f32_fma2(both, hi.y, acc[i][3]);
+      }
     }
+    if (s + 1 < steps) put(buf ^ 1);      // its last readers passed the barrier of the step before
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty * TM + i;
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) c[(size_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
+    for (int j = 0; j < 8; ++j) {
+      const int n = n0 + (j / 4) * 64 + tx * 4 + j % 4;
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][j / 2]));
+      if (n < N) c[(size_t)m * ldc + n] = (j % 2 ? hi : lo) + (bias ? bias[n] : 0.f);
     }
   }
+}
+
+template <int TM>
+static int launch_f32(const float* a, const float* w, const float* bias, float* c, int M, int N, int K, int lda, int ldc,
+                      bool vec, cudaStream_t stream) {
+  dim3 grid((N + TILE_N - 1) / TILE_N, (M + TM * 16 - 1) / (TM * 16));
+  if (grid.y > 65535) return TOKB200_BAD_SIZE;
+  if (vec) gemm_f32_kernel<TM, true><<<grid, GEMM_THREADS, 0, stream>>>(a, w, bias, c, M, N, K, lda, ldc);
+  else gemm_f32_kernel<TM, false><<<grid, GEMM_THREADS, 0, stream>>>(a, w, bias, c, M, N, K, lda, ldc);
+  return tokb200_launch_status();
+}
+
+// Few rows, or too few tiles of the kind above for the device: tiles of 4 R rows x 32 columns by 128 threads, a warp's
+// lanes are the columns and each warp keeps R rows (w + 4 i).  Bound by latency at these sizes: pieces of 32 of k come
+// through a ring of cp.async stages, so that several are on their way while one is multiplied.
+#define FEW_N 32
+#define FEW_K 32
+#define FEW_THREADS 128
+
+__device__ __forceinline__ void f32_copy16(float* dst, const float* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 16 : 0) : "memory");
+}
+
+template <int R, bool VEC>
+__global__ void __launch_bounds__(FEW_THREADS)
+gemm_f32_few_kernel(const float* __restrict__ a, const float* __restrict__ w,
+                    const float* __restrict__ bias, float* __restrict__ c, int M, int N, int K,
+                    int lda, int ldc) {
+  constexpr int kRows = 4 * R, kStages = R == 16 ? 3 : 4, kStride = FEW_K + 4;
+  __shared__ __align__(16) float a_s[kStages][kRows * kStride];
+  __shared__ __align__(16) float w_s[kStages][FEW_N * kStride];
+  const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * FEW_N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto piece = [&](float* to, const float* base, int row, int rows, int ld, int k) {
+    const bool in = row < rows && k < K;
+    const float* src = base + (in ? (size_t)row * ld + k : 0);
+    if (VEC) {
+      f32_copy16(to, src, in);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) to[i] = in && k + i < K ? src[i] : 0.f;
+    }
+  };
+  auto fetch = [&](int step) {
+    const int buf = step % kStages, k0 = step * FEW_K;
+#pragma unroll
+    for (int e = threadIdx.x; e < FEW_N * FEW_K / 4; e += FEW_THREADS)
+      piece(&w_s[buf][e / (FEW_K / 4) * kStride + e % (FEW_K / 4) * 4], w, n0 + e / (FEW_K / 4), N, K,
+            k0 + e % (FEW_K / 4) * 4);
+#pragma unroll
+    for (int e = threadIdx.x; e < kRows * FEW_K / 4; e += FEW_THREADS)
+      piece(&a_s[buf][e / (FEW_K / 4) * kStride + e % (FEW_K / 4) * 4], a, m0 + e / (FEW_K / 4), M, lda,
+            k0 + e % (FEW_K / 4) * 4);
+  };
+  float acc[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) acc[i] = 0.f;
+  const int steps = (K + FEW_K - 1) / FEW_K;
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    if (s < steps) fetch(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();                    // step s is in place, and everybody is done with the buffer fetched into next
+    if (s + kStages - 1 < steps) fetch(s + kStages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* w_b = &w_s[s % kStages][lane * kStride];
+    const float* a_b = &a_s[s % kStages][warp * kStride];
+#pragma unroll
+    for (int k = 0; k < FEW_K; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(w_b + k);
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 y = *reinterpret_cast<const float4*>(a_b + 4 * i * kStride + k);
+        acc[i] = fmaf(y.x, x.x, acc[i]);
+        acc[i] = fmaf(y.y, x.y, acc[i]);
+        acc[i] = fmaf(y.z, x.z, acc[i]);
+        acc[i] = fmaf(y.w, x.w, acc[i]);
+      }
+    }
+  }
+  const int n = n0 + lane;
+  if (n >= N) return;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int m = m0 + warp + 4 * i;
+    if (m < M) c[(size_t)m * ldc + n] = acc[i] + (bias ? bias[n] : 0.f);
+  }
+}
+
+template <int R>
+static int launch_f32_few(const float* a, const float* w, const float* bias, float* c, int M, int N, int K, int lda,
+                          int ldc, bool vec, cudaStream_t stream) {
+  dim3 grid((N + FEW_N - 1) / FEW_N, (M + 4 * R - 1) / (4 * R));
+  if (grid.y > 65535) return TOKB200_BAD_SIZE;
+  if (vec) gemm_f32_few_kernel<R, true><<<grid, FEW_THREADS, 0, stream>>>(a, w, bias, c, M, N, K, lda, ldc);
+  else gemm_f32_few_kernel<R, false><<<grid, FEW_THREADS, 0, stream>>>(a, w, bias, c, M, N, K, lda, ldc);
+  return tokb200_launch_status();
 }
 
 TOKB200_API int tokb200_gemm_f32(const float* a, const float* w, const float* bias, float* c,
                                  int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return TOKB200_OK;
   if (K <= 0 || lda < K || ldc < N) return TOKB200_BAD_SIZE;
-  const long long grid_y = (M + TILE_M - 1) / TILE_M;
-  if (grid_y > 65535) return TOKB200_BAD_SIZE;
-  dim3 grid((N + TILE_N - 1) / TILE_N, (unsigned)grid_y);
-  gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, w, bias, c, M, N, K, lda, ldc);
-  return tokb200_launch_status();
+  if (M > 64LL * 65535) return TOKB200_BAD_SIZE;
+  // Every form gives the same bits, so the choice is one of time alone: a round of one tile an SM takes as long as a
+  // tile's elements over the share of the FMA pipe that its form reaches (the divisors); the form with the least
+  // rounds x time wins, which is the largest tile where there are many and a small one where it fills the device.
+  struct Form { int rows, columns; float reach; };
+  static const Form forms[] = {{128, 128, 0.95f}, {64, 128, 0.85f}, {48, 128, 0.8f}, {64, 32, 0.6f}, {32, 32, 0.5f},
+                               {16, 32, 0.4f}, {4, 32, 0.25f}};
+  const long long sms = 148;
+  int best = 0;
+  double least = 0.;
+  for (int i = 0; i < (int)(sizeof(forms) / sizeof(forms[0])); ++i) {
+    const long long down = (M + forms[i].rows - 1) / forms[i].rows;
+    const long long tiles = down * ((N + forms[i].columns - 1) / forms[i].columns);
+    if (down > 65535) continue;
+    const double time = (double)((tiles + sms - 1) / sms) * forms[i].rows * forms[i].columns / forms[i].reach;
+    if (i == 0 || time < least) { best = i; least = time; }
+  }
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && ((((uintptr_t)a) | ((uintptr_t)w)) & 15) == 0;
+  switch (best) {
+    case 0: return launch_f32<8>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 1: return launch_f32<4>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 2: return launch_f32<3>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 3: return launch_f32_few<16>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 4: return launch_f32_few<8>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 5: return launch_f32_few<4>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    default: return launch_f32_few<1>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+  }
 }

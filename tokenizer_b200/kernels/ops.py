@@ -350,6 +350,22 @@ def paged_attention_generic(q, k_pool, v_pool, out, block_table, row_req, pos, n
         "paged_attention")
 
 
+def paged_attention_f32_tiles_supported(nh: int, nkv: int, d: int) -> bool:
+    return d in (64, 128) and nh % nkv == 0
+
+
+def paged_attention_f32_tiles(q, k_pool, v_pool, out, block_table, row_req, pos, tiles, n_tiles, nh, nkv, d, page, scale,
+                              sink: Optional[torch.Tensor] = None, softcap: Optional[float] = None) -> None:
+    """`paged_attention_generic` in 32-bit for rows that see every key up to their own, bit for bit, tile by tile:
+    `tiles` is int32 [n, 2], (first row, rows <= 64) of consecutive rows of one request."""
+    if q.dtype != torch.float32 or not paged_attention_f32_tiles_supported(nh, nkv, d):
+        raise ValueError("paged_attention_f32_tiles: float32 heads of 64 or 128 lanes in whole groups")
+    _check(_lib("attention_generic").tokb200_paged_attention_f32_tiles(
+        _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table), _i(block_table.shape[1]), _ptr(row_req),
+        _ptr(pos), _ptr(tiles), _i(n_tiles), _i(nh), _i(nkv), _i(d), _i(page), _f(scale), _sink(sink, nh),
+        _f(softcap or 0.0), _stream()), "paged_attention_f32_tiles")
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
              out: torch.Tensor) -> None:
     """out[M,N] = a[M,K] w[N,K]^T (+ bias), true 32-bit."""

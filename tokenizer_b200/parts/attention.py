@@ -200,6 +200,13 @@ class PagedAttention:
                 self.window, self.scale, sink=sink, chunk=self.chunk, softcap=self.softcap,
                 keep_first=self.keep_first)
             return
+        if q.dtype == torch.float32 and tiles is not None and ctx.max_q_len > 1 and self.window is None and \
+                self.chunk is None and ops.paged_attention_f32_tiles_supported(self.nh, self.nkv, self.d):
+            # portions in 32-bit: the kernel below's bits, a chunk's keys read once a tile of rows
+            ops.paged_attention_f32_tiles(
+                q, k_pool, v_pool, out, group.block_table, ctx.row_req, ctx.pos, tiles[0], tiles[1], self.nh, self.nkv,
+                self.d, group.page_size, self.scale, sink=sink, softcap=self.softcap)
+            return
         ops.paged_attention_generic(
             q, k_pool, v_pool, out, group.block_table, ctx.row_req, ctx.pos,
             self.nh, self.nkv, self.d, group.page_size, self.window, self.scale, sink=sink, chunk=self.chunk, softcap=self.softcap,
