@@ -1,0 +1,91 @@
+"""The delta rules in chunks against the same rule token by token in 64 bits: portions of one token to several chunks and
+their remainders, continued portions (a matrix and kept inputs that are not zero), idle rows, decays next to one, next to
+zero and mixed by channel, heads of fewer than 128 lanes, values of 16 to 128, taps other than four."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from tokenizer_b200.kernels import ops as o
+    return o
+
+
+def rule(proj, decay_in, p, by_channel, conv_w, a_log, dt_bias, kept, S, scale):
+    """One request in float64: `proj` [n, channels + heads], `decay_in` [n, heads (* dim)]; returns o and moves S."""
+    groups, heads, dim, vdim, taps = p
+    n, channels = proj.shape[0], 2 * groups * dim + heads * vdim
+    x = torch.cat([kept, proj[:, :channels]])
+    y = sum(x[j:j + n] * conv_w[:, j] for j in range(taps))
+    y = y * torch.sigmoid(y)
+    q, k, v = torch.split(y, [groups * dim, groups * dim, heads * vdim], dim=1)
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+    q = unit(q.reshape(n, groups, dim)).repeat_interleave(heads // groups, 1) * scale
+    k = unit(k.reshape(n, groups, dim)).repeat_interleave(heads // groups, 1)
+    v, beta = v.reshape(n, heads, vdim), torch.sigmoid(proj[:, channels:channels + heads])
+    rate, soft = torch.exp(a_log), torch.nn.functional.softplus(decay_in + dt_bias)
+    g = torch.exp(-rate[:, None] * soft.view(n, heads, dim)) if by_channel else \
+        torch.exp(-rate * soft)[..., None].expand(n, heads, dim)
+    o = torch.empty(n, heads, vdim, dtype=torch.float64)
+    for t in range(n):
+        S.mul_(g[t][:, :, None])
+        u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S.add_(k[t][:, :, None] * u[:, None, :])
+        o[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return o.reshape(n, -1), x[x.shape[0] - (taps - 1):]
+
+
+@pytest.mark.parametrize("by_channel", [False, True])
+@pytest.mark.parametrize("groups,heads,dim,vdim,taps,shift", [
+    (1, 2, 128, 128, 4, -3.0), (2, 2, 128, 64, 4, 3.0), (1, 3, 72, 48, 2, 0.0), (2, 4, 100, 16, 1, -6.0)])
+def test_against_the_rule(by_channel, groups, heads, dim, vdim, taps, shift):
+    o = ops()
+    assert o.delta_chunks_supported(dim, vdim)
+    lengths = [[1, 33, 0, 64, 95, 32], [31, 2, 40, 1, 0, 70]]          # two portions a request, some of them empty
+    n_req, channels = len(lengths[0]), 2 * groups * dim + heads * vdim
+    g = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    conv_w, a_log = rnd(channels, taps) * 0.5, rnd(heads) * 0.5
+    dt_bias = rnd(heads * (dim if by_channel else 1)) * 2.0 + shift       # decays spread around the shift's
+    off = heads * vdim * 128
+    size = -(-(off + (taps - 1) * channels) // 4) * 4
+    state = torch.zeros(n_req, size)
+    matrices = rnd(n_req, heads, dim, vdim) * 0.3
+    state[:, :off] = torch.nn.functional.pad(matrices.transpose(2, 3), (0, 128 - dim)).reshape(n_req, -1)
+    kept = [rnd(taps - 1, channels) for _ in range(n_req)]
+    for r in range(n_req):
+        state[r, off:off + (taps - 1) * channels] = kept[r].reshape(-1)
+    S, kept = [m.double() for m in matrices], [k.double() for k in kept]
+    slots = torch.randperm(n_req, generator=g)
+    dev = torch.empty(n_req, size, device=DEV)
+    dev[slots.to(DEV)] = state.to(DEV)
+    for portion in lengths:
+        starts = [0]
+        for n in portion:
+            starts.append(starts[-1] + n)
+        rows = starts[-1] + 5                                             # idle rows behind the last request
+        proj = rnd(rows, channels + heads + 8 + heads)
+        width = heads * (dim if by_channel else 1)
+        decay = rnd(rows, width + 4) if by_channel else proj
+        at = 0 if by_channel else channels + heads + 8
+        out = torch.full((rows, heads * vdim), 9.0, device=DEV)
+        d_proj = proj.to(DEV)
+        o.delta_chunks(d_proj, 0, channels, decay.to(DEV) if by_channel else d_proj, at, by_channel, groups, heads, dim, vdim,
+                       taps, conv_w.to(DEV), a_log.to(DEV), dt_bias.to(DEV), dev, off,
+                       torch.tensor(starts, dtype=torch.int32, device=DEV), slots.int().to(DEV), out)
+        got, got_state = out.cpu().double(), dev[slots.to(DEV)].cpu().double()
+        assert bool((got[starts[-1]:] == 9.0).all())
+        for r, n in enumerate(portion):
+            span = slice(starts[r], starts[r + 1])
+            if n:
+                want, kept[r] = rule(proj[span].double(), decay[span, at:at + width].double(), (groups, heads, dim, vdim, taps),
+                                     by_channel, conv_w.double(), a_log.double(), dt_bias.double(), kept[r], S[r], dim ** -0.5)
+                # 32-bit sums of 128 products, a chain of three chunks at most: some tens of 2^-24 of the largest value
+                assert float((got[span] - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+            m = got_state[r, :off].view(heads, vdim, 128)
+            assert bool((m[..., dim:] == 0).all())
+            assert float((m[..., :dim].transpose(1, 2) - S[r]).abs().max()) < 1e-5 * max(1.0, float(S[r].abs().max()))
+            if taps > 1:
+                assert torch.equal(got_state[r, off:off + (taps - 1) * channels], kept[r].reshape(-1))

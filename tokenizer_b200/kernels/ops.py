@@ -1304,6 +1304,43 @@ def cdr_record(dim: int, vdim: int) -> int:
     return int(_lib("channel_delta").tokb200_cdr_record(_i(dim), _i(vdim)))
 
 
+# ---- the delta rules in chunks of 32 tokens (`csrc/delta_chunks.cu`) ----
+def delta_chunks_supported(dim: int, vdim: int) -> bool:
+    return bool(_lib("delta_chunks").tokb200_delta_chunks_supported(_i(dim), _i(vdim)))
+
+
+def delta_chunks(proj: torch.Tensor, qkv_at: int, b_at: int, decay: torch.Tensor, decay_at: int, by_channel: bool,
+                 groups: int, heads: int, dim: int, vdim: int, taps: int, conv_w, a_log, dt_bias, state: torch.Tensor,
+                 conv_off: int, q_start, state_slot, o_out: torch.Tensor) -> None:
+    """The delta rule over every request's rows, in chunks: short convolution + silu of q, k, v (`proj`'s columns
+    qkv_at ..), unit vectors, beta = sigmoid(proj[b_at ..]), decays exp(-exp(a_log) softplus(decay[decay_at ..] + dt_bias))
+    (one a head and key channel with `by_channel`, else one a head, from the same product as q, k and v), the recurrence,
+    `o_out` float32 [T, heads * vdim].  The matrices in `state` ([heads, vdim, 128] at the start of a slot) and the kept
+    inputs behind them move on."""
+    channels, n = 2 * groups * dim + heads * vdim, proj.shape[0]
+    per_head = dim if by_channel else 1
+    if state.dtype != torch.float32 or state.dim() != 2 or conv_w.numel() != channels * taps or \
+            conv_off + (taps - 1) * channels > state.shape[1] or max(qkv_at + channels, b_at + heads) > proj.shape[1] or \
+            decay.shape[0] != n or decay_at + heads * per_head > decay.shape[1] or a_log.numel() != heads or \
+            dt_bias.numel() != heads * per_head or heads * vdim * 128 > state.shape[1] or \
+            decay.dtype != (torch.float32 if by_channel else proj.dtype) or \
+            o_out.dtype != torch.float32 or tuple(o_out.shape) != (n, heads * vdim):
+        raise ValueError("delta_chunks: sizes of the products, the state, the taps or the output disagree")
+    requests, lib = q_start.shape[0] - 1, _lib("delta_chunks")
+    lib.tokb200_delta_chunk_floats.restype = ctypes.c_longlong
+    floats = lib.tokb200_delta_chunk_floats(_i(n), _i(requests), _i(heads), _i(vdim))
+    records = torch.empty(floats, dtype=torch.float32, device=proj.device)
+    _check(lib.tokb200_delta_chunk_prepare(
+        _sliced_ptr(proj), _i(_tag(proj)), _i(_ld(proj)), _i(qkv_at), _i(b_at), _sliced_ptr(decay), _i(_ld(decay)),
+        _i(decay_at), _i(int(by_channel)), _i(groups), _i(heads), _i(dim), _i(vdim), _i(taps), _ptr(conv_w), _ptr(a_log),
+        _ptr(dt_bias), _ptr(state), _ll(state.shape[1]), _i(conv_off), _ptr(q_start), _ptr(state_slot), _i(n), _i(requests),
+        _ptr(records), _stream()), "delta_chunk_prepare")
+    short_conv_state(proj, qkv_at, channels, taps, state, conv_off, q_start, state_slot)
+    _check(lib.tokb200_delta_chunk_scan(
+        _ptr(records), _i(heads), _i(dim), _i(vdim), _ptr(state), _ll(state.shape[1]), _ptr(q_start), _ptr(state_slot),
+        _i(requests), _ptr(o_out), _stream()), "delta_chunk_scan")
+
+
 def cdr_records(n_rows: int, n_requests: int, heads: int, dim: int, vdim: int, device) -> torch.Tensor:
     """Room for a step's records: every request's portion is cut into runs of four rows."""
     return torch.empty((n_rows // CDR_RUN + n_requests, heads, cdr_record(dim, vdim)), dtype=torch.float32, device=device)

@@ -23,6 +23,7 @@ def all_variants():
         ("layer_norm.cu", (), ()),
         ("delta_rule.cu", (), ()),
         ("channel_delta.cu", (), ()),
+        ("delta_chunks.cu", (), ()),
         ("dynamic_tanh.cu", (), ()),
         ("rotary_store.cu", (), ()),
         ("moe.cu", (), ()),

@@ -114,6 +114,16 @@ def stacked_rows(weights, multiple: int = 8):
     return torch.cat(weights, dim=0)
 
 
+# A step whose longest portion has this many tokens runs the delta rules in chunks (bfloat16 models, heads that
+# `ops.delta_chunks_supported` takes)
+DELTA_CHUNKS_FROM = 32
+
+
+def _delta_chunks(runtime, dim: int, vdim: int) -> bool:
+    """A float32 model keeps the token-by-token forms: its rows' bits do not depend on how a prompt was cut."""
+    return runtime.dtype == torch.bfloat16 and ops.delta_chunks_supported(dim, vdim)
+
+
 class GatedDeltaNet:
     """The gated delta rule: per head a matrix state S (dim x vdim, float32) that every token
     decays, corrects along its key and reads along its query:
@@ -171,9 +181,12 @@ class GatedDeltaNet:
         # a slot: [heads, vdim, dim_padded] and behind it [taps - 1, channels], in whole 4s of floats
         self.conv_off = self.heads * self.vdim * self.dim_padded
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
+        self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
 
     def shape_key(self, q_lens):
         longest = max(q_lens)
+        if self.chunked and longest >= DELTA_CHUNKS_FROM:
+            return "delta_chunks"
         return "delta1" if longest == 1 else "delta" if longest < 32 else "delta32"      # the kernels' choices
 
     def input_stack(self):
@@ -199,15 +212,21 @@ class GatedDeltaNet:
                          self.conv_w, self.a_log, self.dt_bias, self.gain, out_scale, self.eps, cache.state,
                          self.conv_off, ctx.row_req, ctx.q_start, ctx.state_slot, y)
             return self.out.forward(y, partials_ok=True)
+        o = torch.empty((n, h * self.vdim), dtype=torch.float32, device=proj.device)
+        y = self.runtime.empty(n, h * self.vdim)
+        if self.chunked and ctx.max_q_len >= DELTA_CHUNKS_FROM:
+            ops.delta_chunks(proj, at, at + c, proj, at + c + h, False, self.groups, h, self.dim, self.vdim, self.taps,
+                             self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
+                             ctx.state_slot, o)
+            ops.gdn_out_norm(o, proj, at + c + 2 * h, self.gain, out_scale, self.eps, y, h, self.vdim, ctx.row_req)
+            return self.out.forward(y, partials_ok=True)
         qkv = torch.empty((n, c), dtype=torch.float32, device=proj.device)
         bg = torch.empty((n, 2 * h + self.groups), dtype=torch.float32, device=proj.device)
         ops.gdn_prepare(proj, at, at + c, at + c + h, self.groups, h, self.dim, self.vdim, self.taps, self.conv_w,
                         self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.row_req, ctx.q_start,
                         ctx.state_slot, qkv, bg)
-        o = torch.empty((n, h * self.vdim), dtype=torch.float32, device=proj.device)
         ops.gdn_scan(qkv, bg, self.groups, h, self.dim, self.vdim, cache.state, ctx.q_start, ctx.state_slot, o,
                      longest=ctx.max_q_len)
-        y = self.runtime.empty(n, h * self.vdim)
         ops.gdn_out_norm(o, proj, at + c + 2 * h, self.gain, out_scale, self.eps, y, h, self.vdim, ctx.row_req)
         return self.out.forward(y, partials_ok=True)
 
@@ -288,9 +307,12 @@ class ChannelDeltaNet:
         # a slot: [heads, vdim, dim_padded] and behind it [taps - 1, channels], in whole 4s of floats
         self.conv_off = self.heads * self.vdim * self.dim_padded
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
+        self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
 
     def shape_key(self, q_lens):
-        return "channel_delta1" if max(q_lens) == 1 else "channel_delta"      # the kernels' choice
+        longest = max(q_lens)                                                # the kernels' choice
+        return "channel_delta1" if longest == 1 else \
+            "delta_chunks" if self.chunked and longest >= DELTA_CHUNKS_FROM else "channel_delta"
 
     def cache_need(self):
         return CacheNeed(state=StateNeed((self.state_floats,)))
@@ -321,11 +343,18 @@ class ChannelDeltaNet:
                                      ctx.state_slot)
             return self.out.forward(y, partials_ok=True)
         pre = self._second_products(proj)
+        o = torch.empty((n, heads * self.vdim), dtype=torch.float32, device=proj.device)
+        if self.chunked and ctx.max_q_len >= DELTA_CHUNKS_FROM:
+            ops.delta_chunks(proj, 0, self.b_at, pre, 0, True, self.groups, heads, self.dim, self.vdim, self.taps,
+                             self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
+                             ctx.state_slot, o)
+            ops.gdn_out_norm(o, pre, heads * self.dim, self.gain, 1.0, self.eps, y, heads, self.vdim, ctx.row_req,
+                             gate_kind="sigmoid")
+            return self.out.forward(y, partials_ok=True)
         records = ops.cdr_records(n, ctx.q_start.shape[0] - 1, heads, self.dim, self.vdim, proj.device)
         ops.cdr_prepare(proj, 0, self.b_at, pre, self.groups, heads, self.dim, self.vdim, self.taps, self.conv_w, self.a_log,
                         self.dt_bias, cache.state, self.conv_off, ctx.q_start, ctx.state_slot, records)
         ops.short_conv_state(proj, 0, self.channels, self.taps, cache.state, self.conv_off, ctx.q_start, ctx.state_slot)
-        o = torch.empty((n, heads * self.vdim), dtype=torch.float32, device=proj.device)
         ops.cdr_scan(records, heads, self.dim, self.vdim, cache.state, ctx.q_start, ctx.state_slot, o)
         ops.gdn_out_norm(o, pre, heads * self.dim, self.gain, 1.0, self.eps, y, heads, self.vdim, ctx.row_req,
                          gate_kind="sigmoid")
