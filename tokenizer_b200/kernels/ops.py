@@ -826,9 +826,11 @@ def attention_tcgen05_supported(nh: int, nkv: int, d: int) -> bool:
 
 def attention_tcgen05(q, k_pool, v_pool, out, block_table, row_req, pos, tiles, n_tiles, nh, nkv, d,
                       page, window, scale, sink: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
-                      softcap: Optional[float] = None, keep_first: int = 0) -> None:
+                      softcap: Optional[float] = None, keep_first: int = 0, split: Optional[bool] = None) -> None:
     """Attention for portions of prompts on tcgen05 (bfloat16, head size 64 or 128).
-    `tiles` is int32 [n, 2]: (first row, rows <= 128) of consecutive rows of one request."""
+    `tiles` is int32 [n, 2]: (first row, rows <= 128) of consecutive rows of one request.  `split`: a block
+    takes one head and cuts its keys in two (True) or two heads of a key/value head (False); None: by the
+    amount of work."""
     if q.dtype != torch.bfloat16:
         raise ValueError("attention_tcgen05 is the bfloat16 kernel")
     if not attention_tcgen05_supported(nh, nkv, d):
@@ -836,9 +838,10 @@ def attention_tcgen05(q, k_pool, v_pool, out, block_table, row_req, pos, tiles, 
     lib = _load("attention_tcgen05.cu", defines=(f"HEAD_DIM={d}",))
     _check(lib.tokb200_attention_tcgen05(
         _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
-        _i(block_table.shape[1]), _ptr(row_req), _ptr(pos), _ptr(tiles), _i(n_tiles), _i(nh),
-        _i(nkv), _i(d), _i(page), _i(-1 if window is None else int(window)), _i(0 if chunk is None else int(chunk)), _i(int(keep_first)), _f(scale), _sink(sink, nh),
-        _f(softcap or 0.0), _stream()), "attention_tcgen05")
+        _i(block_table.shape[1]), _ptr(row_req), _ptr(pos), _ptr(tiles), _i(n_tiles), _i(q.numel() // (nh * d)),
+        _i(k_pool.numel() // (nkv * d)), _i(nh), _i(nkv), _i(d), _i(page), _i(-1 if window is None else int(window)),
+        _i(0 if chunk is None else int(chunk)), _i(int(keep_first)), _f(scale), _sink(sink, nh),
+        _f(softcap or 0.0), _i(-1 if split is None else int(split)), _stream()), "attention_tcgen05")
 
 
 def attention_tcgen05_check(d: int) -> None:
