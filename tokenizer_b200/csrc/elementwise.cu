@@ -275,10 +275,51 @@ __global__ void residual_add_kernel(float* __restrict__ x, const TD* __restrict_
   }
 }
 
+// The same, eight elements a thread with 16-byte loads (n a multiple of 8, aligned bases), the planes added in index
+// order.  Bound by memory: one element a thread and turn kept too few bytes in
+// flight (bfloat16 delta, us before / now: 8,192 x 3,584 81 / 40, 2,048 x 2,048 12.7 / 6.9).
+template <typename TD>
+__global__ void __launch_bounds__(256)
+residual_add8_kernel(float* __restrict__ x, const TD* __restrict__ delta, size_t n, int n_partials) {
+  pdl_wait();
+  pdl_launch();
+  const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  if (i >= n) return;
+  float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
+#pragma unroll 4
+  for (int s = 0; s < n_partials; ++s) {
+    if (sizeof(TD) == 2) {
+      const uint4 d = *reinterpret_cast<const uint4*>(delta + (size_t)s * n + i);
+      const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d);
+      const float2 d0 = __bfloat1622float2(d2[0]), d1 = __bfloat1622float2(d2[1]), d3 = __bfloat1622float2(d2[2]),
+                   d4 = __bfloat1622float2(d2[3]);
+      a.x += d0.x; a.y += d0.y; a.z += d1.x; a.w += d1.y;
+      b.x += d3.x; b.y += d3.y; b.z += d4.x; b.w += d4.y;
+    } else {
+      const float* src = reinterpret_cast<const float*>(delta) + (size_t)s * n + i;
+      const float4 d = *reinterpret_cast<const float4*>(src), e = *reinterpret_cast<const float4*>(src + 4);
+      a.x += d.x; a.y += d.y; a.z += d.z; a.w += d.w;
+      b.x += e.x; b.y += e.y; b.z += e.z; b.w += e.w;
+    }
+  }
+  *reinterpret_cast<float4*>(x + i) = a;
+  *reinterpret_cast<float4*>(x + i + 4) = b;
+}
+
 TOKB200_API int tokb200_residual_add(float* x, const void* delta, int delta_dtype, int n_partials,
                                      long long n, cudaStream_t stream) {
   if (n <= 0) return TOKB200_OK;
   if (n_partials < 1) return TOKB200_BAD_SIZE;
+  // fewer elements than a device of 148 SMs has threads at a block each: one element a thread, and more blocks, is faster
+  if (n >= 8 * 256 * 148 && n % 8 == 0 && n / 2048 < 0x7fffffff && ((((uintptr_t)x) | ((uintptr_t)delta)) & 15) == 0) {
+    const dim3 grid((unsigned)((n + 2047) / 2048));
+    if (delta_dtype == TOKB200_F32)
+      return launch_dependent(residual_add8_kernel<float>, grid, dim3(256), 0, stream, x, (const float*)delta, (size_t)n,
+                              n_partials);
+    if (delta_dtype == TOKB200_BF16)
+      return launch_dependent(residual_add8_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, x,
+                              (const __nv_bfloat16*)delta, (size_t)n, n_partials);
+  }
   const int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
   if (delta_dtype == TOKB200_F32)
     residual_add_kernel<float><<<blocks, 256, 0, stream>>>(x, (const float*)delta, (size_t)n, n_partials);
