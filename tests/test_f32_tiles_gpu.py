@@ -28,6 +28,18 @@ def test_product_rows_do_not_depend_on_the_batch(M, N, K):
     assert torch.equal(few, out[:, :min(N, 40)])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (5, 33, 7), (64, 128, 16), (129, 257, 100), (300, 130, 36)])
+def test_every_form_of_the_product_gives_the_same_bits(M, N, K):
+    o = ops()
+    a, w, bias = rnd(M, K, seed=4), rnd(N, K, seed=5), rnd(N, seed=6)
+    outs = [torch.full((M, N), 9.0, device=DEV) for _ in range(6)]
+    for form, out in enumerate(outs):
+        o.gemm_f32(a, w, bias, out, form=form)
+    assert all(torch.equal(out, outs[0]) for out in outs)
+    with pytest.raises(Exception):
+        o.gemm_f32(a, w, bias, outs[0], form=6)
+
+
 @pytest.mark.parametrize("nh,nkv,d,page,sink,softcap", [
     (4, 2, 64, 16, False, None), (3, 1, 128, 5, True, None), (2, 2, 64, 64, True, 20.0), (7, 1, 64, 16, False, None)])
 def test_attention_tiles_give_the_bits_of_single_rows(nh, nkv, d, page, sink, softcap):

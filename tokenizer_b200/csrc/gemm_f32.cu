@@ -3,27 +3,15 @@
 // element sums its K products in index order, so a row's result does not depend
 // on how many other rows are in the batch, nor on the tile the element falls into.
 //
-// A block of 16 x 16 threads computes TM * 16 rows x 128 columns, TM x 8 sums a thread, two columns an
-// instruction (fma.rn.f32x2 rounds each half as fmaf does).  Bound by the FMA pipe: per step of k a warp issues 4 TM
-// paired multiply-adds and reads TM + 8 floats a thread from shared memory, 8 of them as 16-byte loads.  Operands are
-// staged k-major, 16 of k at a time, the next piece's global loads in registers while this one is multiplied.
+// A block of 16 x 16 threads computes TM * 16 rows x 128 columns, TM x 8 sums a thread.  Bound by the FMA pipe: per step
+// of k a thread reads TM numbers of A and 8 of W, by 16-byte loads and a step ahead of their use, for 8 TM multiply-adds
+// (paired ones, fma.rn.f32x2, measured half as fast).  Operands are staged k-major, 16 of k at a time, the next piece's
+// global loads in registers while this one is multiplied.
 #include "common.cuh"
 
 #define TILE_N 128
 #define TILE_K 16
 #define GEMM_THREADS 256
-
-__device__ __forceinline__ unsigned long long f32_pair(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f32_fma2(unsigned long long a, unsigned long long b,
-                                                       unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 // VEC: K and lda are whole 4s and both bases lie on 16 bytes (16-byte loads along k)
 template <int TM, bool VEC>
@@ -40,11 +28,11 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
   __shared__ __align__(16) float w_s[2][TILE_K * kWStride];
   const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * TILE_N;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  unsigned long long acc[TM][4];
+  float acc[TM][8];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
 
   float4 a_r[kAPieces], w_r[kWPieces];
   auto load4 = [&](const float* base, int row, int rows, int ld, int k) {
@@ -100,30 +88,29 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
     if (s + 1 < steps) fetch((s + 1) * TILE_K);
     const float* a_b = &a_s[buf][ty * TM];
     const float* w_b = &w_s[buf][tx * 4];
+    // a step of k's operands: TM of A, and columns tx * 4 .. + 3 and 64 + tx * 4 .. + 3 of W (neighbouring threads read
+    // neighbouring 16 bytes)
+    float av[2][TM], wv[2][8];
+    auto operands = [&](int kk, int to) {
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(a_b + kk * kAStride + i);
+        av[to][i] = v.x; av[to][i + 1] = v.y; av[to][i + 2] = v.z; av[to][i + 3] = v.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(w_b + kk * kWStride + j * 16);
+        wv[to][j] = v.x; wv[to][j + 1] = v.y; wv[to][j + 2] = v.z; wv[to][j + 3] = v.w;
+      }
+    };
+    operands(0, 0);
 #pragma unroll
     for (int kk = 0; kk < TILE_K; ++kk) {
-      float av[TM];
-      if (TM % 4 == 0) {
+      if (kk + 1 < TILE_K) operands(kk + 1, (kk + 1) & 1);
 #pragma unroll
-        for (int i = 0; i < TM; i += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(a_b + kk * kAStride + i);
-          av[i] = v.x; av[i + 1] = v.y; av[i + 2] = v.z; av[i + 3] = v.w;
-        }
-      } else {
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int i = 0; i < TM; ++i) av[i] = a_b[kk * kAStride + i];
-      }
-      // columns tx * 4 .. + 3 and 64 + tx * 4 .. + 3: neighbouring threads read neighbouring 16 bytes
-      const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(w_b + kk * kWStride);
-      const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(w_b + kk * kWStride + 64);
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        const unsigned long long both = f32_pair(av[i], av[i]);
-        acc[i][0] = f32_fma2(both, lo.x, acc[i][0]);
-        acc[i][1] = f32_fma2(both, lo.y, acc[i][1]);
-        acc[i][2] = f32_fma2(both, hi.x, acc[i][2]);
-        acc[i][3] = f32_fma2(both, hi.y, acc[i][3]);
-      }
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[kk & 1][i], wv[kk & 1][j], acc[i][j]);
     }
     if (s + 1 < steps) put(buf ^ 1);      // its last readers passed the barrier of the step before
     __syncthreads();
@@ -135,9 +122,7 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int n = n0 + (j / 4) * 64 + tx * 4 + j % 4;
-      float lo, hi;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][j / 2]));
-      if (n < N) c[(size_t)m * ldc + n] = (j % 2 ? hi : lo) + (bias ? bias[n] : 0.f);
+      if (n < N) c[(size_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
     }
   }
 }
@@ -243,35 +228,37 @@ static int launch_f32_few(const float* a, const float* w, const float* bias, flo
   return tokb200_launch_status();
 }
 
+// `form`: the tile, an index into `forms` below; -1: by the rule.
 TOKB200_API int tokb200_gemm_f32(const float* a, const float* w, const float* bias, float* c,
-                                 int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+                                 int M, int N, int K, int lda, int ldc, int form, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return TOKB200_OK;
   if (K <= 0 || lda < K || ldc < N) return TOKB200_BAD_SIZE;
   if (M > 64LL * 65535) return TOKB200_BAD_SIZE;
-  // Every form gives the same bits, so the choice is one of time alone: a round of one tile an SM takes as long as a
-  // tile's elements over the share of the FMA pipe that its form reaches (the divisors); the form with the least
-  // rounds x time wins, which is the largest tile where there are many and a small one where it fills the device.
-  struct Form { int rows, columns; float reach; };
-  static const Form forms[] = {{128, 128, 0.95f}, {64, 128, 0.85f}, {48, 128, 0.8f}, {64, 32, 0.6f}, {32, 32, 0.5f},
-                               {16, 32, 0.4f}, {4, 32, 0.25f}};
+  // Every form gives the same bits, so the choice is one of time alone: measured, a lone tile on an SM takes `first`
+  // cycles a step of k and every further one `more` (at 777 rows, us of forms 0 1 3: 9,728 x 896 343 / 371 / 536, 896 x
+  // 4,864 506 / 367 / 292, 1,152 x 896 97 / 72 / 77); the form with the least time for the SM that gets the most wins.
+  struct Form { int rows, columns; float first, more; };
+  static const Form forms[] = {{128, 128, 191.f, 180.f}, {64, 128, 136.f, 108.f}, {64, 32, 53.f, 35.f}, {32, 32, 30.f, 21.f},
+                               {16, 32, 24.f, 12.f}, {4, 32, 15.6f, 7.3f}};
   const long long sms = 148;
-  int best = 0;
+  int best = -1;
   double least = 0.;
   for (int i = 0; i < (int)(sizeof(forms) / sizeof(forms[0])); ++i) {
     const long long down = (M + forms[i].rows - 1) / forms[i].rows;
     const long long tiles = down * ((N + forms[i].columns - 1) / forms[i].columns);
     if (down > 65535) continue;
-    const double time = (double)((tiles + sms - 1) / sms) * forms[i].rows * forms[i].columns / forms[i].reach;
-    if (i == 0 || time < least) { best = i; least = time; }
+    const double time = forms[i].first + (double)((tiles + sms - 1) / sms - 1) * forms[i].more;
+    if (best < 0 || time < least) { best = i; least = time; }
   }
+  if (form >= (int)(sizeof(forms) / sizeof(forms[0]))) return TOKB200_BAD_SIZE;
+  if (form >= 0) best = form;
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ((((uintptr_t)a) | ((uintptr_t)w)) & 15) == 0;
   switch (best) {
     case 0: return launch_f32<8>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
     case 1: return launch_f32<4>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
-    case 2: return launch_f32<3>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
-    case 3: return launch_f32_few<16>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
-    case 4: return launch_f32_few<8>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
-    case 5: return launch_f32_few<4>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 2: return launch_f32_few<16>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 3: return launch_f32_few<8>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
+    case 4: return launch_f32_few<4>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
     default: return launch_f32_few<1>(a, w, bias, c, M, N, K, lda, ldc, vec, stream);
   }
 }

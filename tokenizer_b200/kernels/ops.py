@@ -367,8 +367,8 @@ def paged_attention_f32_tiles(q, k_pool, v_pool, out, block_table, row_req, pos,
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
-             out: torch.Tensor) -> None:
-    """out[M,N] = a[M,K] w[N,K]^T (+ bias), true 32-bit."""
+             out: torch.Tensor, form: Optional[int] = None) -> None:
+    """out[M,N] = a[M,K] w[N,K]^T (+ bias), true 32-bit.  `form`: the tile (all give the same bits); None: by size."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N):
@@ -377,8 +377,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
         if t.dtype != torch.float32:
             raise ValueError("gemm_f32 takes float32")
     _check(_lib("gemm_f32").tokb200_gemm_f32(
-        _ptr(a), _ptr(w), _ptr(bias), _ptr(out), _i(M), _i(N), _i(K), _i(K), _i(N), _stream()),
-        "gemm_f32")
+        _ptr(a), _ptr(w), _ptr(bias), _ptr(out), _i(M), _i(N), _i(K), _i(K), _i(N),
+        _i(-1 if form is None else int(form)), _stream()), "gemm_f32")
 
 
 def sample(logits: torch.Tensor, temperature: Optional[torch.Tensor],
