@@ -188,22 +188,38 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
         dst[t * kDcStride + l] = upto * src[(e + t) * kDcStride + l];
       }
     }
-    {                                                   // pairs inside the eight: warp w takes token e + w as the key
-      const int s = e + warp;
-      float4 p = reinterpret_cast<const float4*>(k_s + s * kDcStride)[lane];
-#pragma unroll 1
-      for (int t = s; t < e + 8; ++t) {
-        const float4 kt = reinterpret_cast<const float4*>(k_s + t * kDcStride)[lane];
-        const float4 qt = reinterpret_cast<const float4*>(q_s + t * kDcStride)[lane];
-        if (t > s) {
-          const float4 g = reinterpret_cast<const float4*>(g_s + t * kDcStride)[lane];
-          p.x *= g.x; p.y *= g.y; p.z *= g.z; p.w *= g.w;
+    {
+      // pairs inside the eight: warp w takes token e + w as the key and all eight tokens as the other, those before it
+      // with nothing; the sixteen sums cross the lanes together, in 8 + 4 + 2 + 1 exchanges and a last one
+      float sums[16];
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const float4 kt = reinterpret_cast<const float4*>(k_s + (e + t) * kDcStride)[lane];
+        const float4 qt = reinterpret_cast<const float4*>(q_s + (e + t) * kDcStride)[lane];
+        const float4 g = reinterpret_cast<const float4*>(g_s + (e + t) * kDcStride)[lane];
+        if (t == warp) p = kt;
+        else { p.x *= g.x; p.y *= g.y; p.z *= g.z; p.w *= g.w; }
+        sums[t] = fmaf(p.x, kt.x, p.y * kt.y) + fmaf(p.z, kt.z, p.w * kt.w);
+        sums[8 + t] = fmaf(p.x, qt.x, p.y * qt.y) + fmaf(p.z, qt.z, p.w * qt.w);
+      }
+#pragma unroll
+      for (int width = 8; width > 0; width >>= 1) {        // lanes with the bit keep the upper half of what is left
+        const bool upper = lane & (2 * width);
+#pragma unroll
+        for (int i = 0; i < width; ++i) {
+          const float got = __shfl_xor_sync(0xffffffffu, upper ? sums[i] : sums[i + width], 2 * width);
+          sums[i] = (upper ? sums[i + width] : sums[i]) + got;
         }
-        const float kk = warp_sum(fmaf(p.x, kt.x, p.y * kt.y) + fmaf(p.z, kt.z, p.w * kt.w));
-        const float qk = warp_sum(fmaf(p.x, qt.x, p.y * qt.y) + fmaf(p.z, qt.z, p.w * qt.w));
-        if (lane == 0) {
-          if (t > s) a_s[t * kDcPairs + s] = kk * beta_s[t];
-          m_s[t * kDcPairs + s] = qk;
+      }
+      sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], 1);
+      // lanes 2 i, 2 i + 1 hold sum i: keys with token i, then queries
+      const int t = (lane >> 1) & 7;
+      if (!(lane & 1)) {
+        if (lane < 16) {
+          if (t > warp) a_s[(e + t) * kDcPairs + e + warp] = sums[0] * beta_s[e + t];
+        } else if (t >= warp) {
+          m_s[(e + t) * kDcPairs + e + warp] = sums[0];
         }
       }
     }

@@ -115,8 +115,12 @@ def stacked_rows(weights, multiple: int = 8):
 
 
 # A step whose longest portion has this many tokens runs the delta rules in chunks (bfloat16 models, heads that
-# `ops.delta_chunks_supported` takes)
-DELTA_CHUNKS_FROM = 32
+# `ops.delta_chunks_supported` takes).  Chunks cost more arithmetic and save a chain of tokens: with one decay a head, 16
+# heads, us of the token-by-token form / chunks: 32 tokens 31 / 34, four requests of 48 68 / 58, 64 tokens 43 / 37.  With a
+# decay a channel the other form walks four tokens a step and fills the device sooner: 256 tokens 68 / 58, eight requests
+# of 256 253 / 316, 512 tokens 125 / 81, four of 512 348 / 331.
+DELTA_CHUNKS_FROM = 48
+CHANNEL_DELTA_CHUNKS_FROM = 512
 
 
 def _delta_chunks(runtime, dim: int, vdim: int) -> bool:
@@ -312,7 +316,7 @@ class ChannelDeltaNet:
     def shape_key(self, q_lens):
         longest = max(q_lens)                                                # the kernels' choice
         return "channel_delta1" if longest == 1 else \
-            "delta_chunks" if self.chunked and longest >= DELTA_CHUNKS_FROM else "channel_delta"
+            "delta_chunks" if self.chunked and longest >= CHANNEL_DELTA_CHUNKS_FROM else "channel_delta"
 
     def cache_need(self):
         return CacheNeed(state=StateNeed((self.state_floats,)))
@@ -344,7 +348,7 @@ class ChannelDeltaNet:
             return self.out.forward(y, partials_ok=True)
         pre = self._second_products(proj)
         o = torch.empty((n, heads * self.vdim), dtype=torch.float32, device=proj.device)
-        if self.chunked and ctx.max_q_len >= DELTA_CHUNKS_FROM:
+        if self.chunked and ctx.max_q_len >= CHANNEL_DELTA_CHUNKS_FROM:
             ops.delta_chunks(proj, 0, self.b_at, pre, 0, True, self.groups, heads, self.dim, self.vdim, self.taps,
                              self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
                              ctx.state_slot, o)
