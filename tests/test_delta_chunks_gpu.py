@@ -1,6 +1,6 @@
 """The delta rules in chunks against the same rule token by token in 64 bits: portions of one token to several chunks and
 their remainders, continued portions (a matrix and kept inputs that are not zero), idle rows, decays next to one, next to
-zero and mixed by channel, heads of fewer than 128 lanes, values of 16 to 128, taps other than four."""
+zero and mixed by channel, heads of fewer than 128 lanes, values of 16 to 128, taps other than four, both widths of a block."""
 import pytest
 import torch
 
@@ -37,10 +37,10 @@ def rule(proj, decay_in, p, by_channel, conv_w, a_log, dt_bias, kept, S, scale):
     return o.reshape(n, -1), x[x.shape[0] - (taps - 1):]
 
 
-@pytest.mark.parametrize("by_channel", [False, True])
+@pytest.mark.parametrize("by_channel,columns", [(False, 0), (True, 16), (False, 32), (True, 32)])
 @pytest.mark.parametrize("groups,heads,dim,vdim,taps,shift", [
     (1, 2, 128, 128, 4, -3.0), (2, 2, 128, 64, 4, 3.0), (1, 3, 72, 48, 2, 0.0), (2, 4, 100, 16, 1, -6.0)])
-def test_against_the_rule(by_channel, groups, heads, dim, vdim, taps, shift):
+def test_against_the_rule(by_channel, columns, groups, heads, dim, vdim, taps, shift):
     o = ops()
     assert o.delta_chunks_supported(dim, vdim)
     lengths = [[1, 33, 0, 64, 95, 32], [31, 2, 40, 1, 0, 70]]          # two portions a request, some of them empty
@@ -74,7 +74,8 @@ def test_against_the_rule(by_channel, groups, heads, dim, vdim, taps, shift):
         d_proj = proj.to(DEV)
         o.delta_chunks(d_proj, 0, channels, decay.to(DEV) if by_channel else d_proj, at, by_channel, groups, heads, dim, vdim,
                        taps, conv_w.to(DEV), a_log.to(DEV), dt_bias.to(DEV), dev, off,
-                       torch.tensor(starts, dtype=torch.int32, device=DEV), slots.int().to(DEV), out)
+                       torch.tensor(starts, dtype=torch.int32, device=DEV), slots.int().to(DEV), out,
+                       columns=columns)
         got, got_state = out.cpu().double(), dev[slots.to(DEV)].cpu().double()
         assert bool((got[starts[-1]:] == 9.0).all())
         for r, n in enumerate(portion):

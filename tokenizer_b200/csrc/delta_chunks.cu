@@ -11,12 +11,18 @@
 //
 //   delta_chunk_prepare   a block a (chunk, head): the short convolution over time with silu (its inputs straight from
 //                         the stacked product, and from the kept inputs in front of a portion), unit vectors, decays,
-//                         then A, M, W, U0 and the scaled queries and keys as one record.  The sums between tokens of
-//                         unlike eighths of a chunk are plain products of rows that were scaled up to the eighth's edge;
-//                         inside an eighth the decays are multiplied in key by key
-//   delta_chunk_scan      a block a (16 columns of a head's matrix, request): the chunks one after another.  The 64 x
-//                         128 rows of W and G q meet the columns in 4 x 4 register tiles, k cut over four pairs of warps;
-//                         the next chunk's record is on its way (cp.async) while this one is worked through
+//                         then A, M, W, U0 and the scaled queries and keys as one record.  Pairs of tokens in different
+//                         halves of 32, 16 or 8 tokens are plain products of rows that were decayed to and from the
+//                         middle; inside four the decays are multiplied in key by key
+//   delta_chunk_scan      a block a (16 or 32 columns of a head's matrix, request): the chunks one after another.  The 64
+//                         x 128 rows of W and G q meet the columns in 8 x 4 or 8 x 8 register tiles, k cut over the eight
+//                         warps; the next chunk's record is on its way (cp.async) while this one is worked through
+//
+// Both are bound by reads of shared memory: a register tile of R x C costs R + C cycles of the 128 bytes a cycle that come
+// back, and R C / 4 of the multiply-adds.  So tiles are as large as the threads allow, and a row of A is read once for
+// two columns.  Measured (16 heads of 128 x 128, both kernels and the kept inputs between them, us; before: tiles of 4 x 4,
+// pairs eight tokens at a time): a prompt of 2,048 tokens 294 -> 266 with one decay a head and 328 -> 283 with one a
+// channel, four prompts of 5,100 in all 763 -> 557, eight of 256 316 -> 252.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).
@@ -24,7 +30,7 @@
 
 #define DC_TOKENS 32
 #define DC_DIM 128                        // lanes of a key, zeros behind the head's own
-#define DC_COLS 16                        // columns of a scan block
+#define DC_COLS 16                        // columns of a narrow scan block (wide ones: 32)
 #define DC_MAX_TAPS 16
 #define DC_PREPARE_THREADS 256
 #define DC_SCAN_THREADS 256
@@ -54,6 +60,28 @@ struct DeltaChunkArgs {
   int groups, heads, dim, vdim, taps, conv_off, n_requests;
 };
 
+// N sums of every lane over LANES neighbouring lanes, all N together: lanes give away the half of their sums that the
+// other side of the exchange keeps.  N >= LANES: lane i of the LANES ends with sums i N / LANES .. in front; N < LANES: with
+// sum i N / LANES (rounded down) in front.
+template <int N, int LANES, int KEEP>
+__device__ __forceinline__ void dc_exchange(float (&sums)[KEEP], int lane) {
+  if constexpr (LANES > 1) {
+    if constexpr (N > 1) {
+      const bool upper = lane & (LANES / 2);
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? sums[i] : sums[i + N / 2], LANES / 2);
+        sums[i] = (upper ? sums[i + N / 2] : sums[i]) + got;
+      }
+      dc_exchange<N / 2, LANES / 2>(sums, lane);
+    } else {
+      sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], LANES / 2);
+      dc_exchange<1, LANES / 2>(sums, lane);
+    }
+  }
+}
+template <int V> struct dc_int { static constexpr int value = V; };
+
 // T: type of proj (and of `decay` where it is one a head: the same product's columns)
 template <typename T, bool BY_CHANNEL>
 __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_kernel(const DeltaChunkArgs a) {
@@ -61,9 +89,9 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   float* q_s = dc_raw;                                  // [32][132] each
   float* k_s = q_s + DC_TOKENS * kDcStride;
   float* g_s = k_s + DC_TOKENS * kDcStride;
-  float* r_s = g_s + DC_TOKENS * kDcStride;             // keys decayed up to the next eighth's edge
-  float* l_s = r_s + DC_TOKENS * kDcStride;             // an eighth's keys, then its queries, decayed from its edge on
-  float* a_s = l_s + 16 * kDcStride;                    // [32][36]
+  float* l_s = g_s + DC_TOKENS * kDcStride;             // keys, then queries, of upper halves, decayed from the edge on
+  float* r_s = l_s + DC_TOKENS * kDcStride;             // keys of lower halves, decayed up to the edge
+  float* a_s = r_s + 16 * kDcStride;                    // [32][36]
   float* m_s = a_s + DC_TOKENS * kDcPairs;              // [32][36]
   float* beta_s = m_s + DC_TOKENS * kDcPairs;           // [32]
   const int place = blockIdx.x, h = blockIdx.y;
@@ -87,74 +115,90 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   const T* proj = static_cast<const T*>(a.proj);
   float* rec = a.records + ((size_t)place * a.heads + h) * (size_t)(kDcU + DC_TOKENS * a.vdim);
 
-  // ---- convolution and silu: a channel a thread, down the chunk's tokens ----
-  auto convolve = [&](int ch, float (&y)[DC_TOKENS]) {
-    const T* in = proj + a.qkv_at + ch;
-    const float* w = a.conv_w + (size_t)ch * a.taps;
-    // an input `back` places before the portion's start is the kept one that many from the end
-    auto input = [&](int at) {
-      return at >= 0 ? to_float(in[(size_t)(start + at) * a.ld]) : kept[(size_t)(a.taps - 1 + at) * channels + ch];
-    };
-    if (a.taps == 4) {
-      const float w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-      float x0 = input(at0 - 3), x1 = input(at0 - 2), x2 = input(at0 - 1);
-#pragma unroll
-      for (int t = 0; t < DC_TOKENS; ++t) y[t] = t < n_here ? to_float(in[(size_t)(t0 + t) * a.ld]) : 0.f;
-#pragma unroll
-      for (int t = 0; t < DC_TOKENS; ++t) {
-        const float x3 = y[t];
-        const float v = fmaf(w3, x3, fmaf(w2, x2, fmaf(w1, x1, w0 * x0)));
-        y[t] = t < n_here ? v * dc_sigmoid(v) : 0.f;
-        x0 = x1; x1 = x2; x2 = x3;
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < DC_TOKENS; ++t) {
-        float v = 0.f;
-        if (t < n_here)
-          for (int j = 0; j < a.taps; ++j) v = fmaf(w[j], input(at0 + t - (a.taps - 1 - j)), v);
-        y[t] = v * dc_sigmoid(v);
-      }
-    }
+  const int l = threadIdx.x & (DC_DIM - 1), half = threadIdx.x / DC_DIM;
+  // ---- convolution and silu, a channel a thread: threads 0 .. 127 take q and the first half of k's tokens, the others v
+  // (kept in registers) and the second half; all inputs are asked for before the first is used ----
+  float col[DC_TOKENS], key[DC_TOKENS / 2], pre[DC_TOKENS / 2];
+  const int a_lanes = half ? a.vdim : a.dim;
+  const int a_ch = half ? 2 * a.groups * a.dim + h * a.vdim + l : group * a.dim + l, k_ch = (a.groups + group) * a.dim + l;
+  const int k0 = half * (DC_TOKENS / 2);
+  // an input `back` places before the portion's start is the kept one that many from the end
+  auto input = [&](int ch, int at) {
+    return at >= 0 ? to_float(proj[(size_t)(start + at) * a.ld + a.qkv_at + ch]) : kept[(size_t)(a.taps - 1 + at) * channels + ch];
   };
-  float col[DC_TOKENS];                                 // threads 128 ..: a column of v, later of U0; below: of W
-  if (threadIdx.x < DC_DIM) {
-    const int l = threadIdx.x;
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-      float* dst = which ? k_s : q_s;
-      if (l < a.dim) {
-        convolve((which ? a.groups + group : group) * a.dim + l, col);
-      } else {
+  if (BY_CHANNEL) {
+    const float* raw = static_cast<const float*>(a.decay) + a.decay_at + h * a.dim + l;
 #pragma unroll
-        for (int t = 0; t < DC_TOKENS; ++t) col[t] = 0.f;
-      }
+    for (int i = 0; i < DC_TOKENS / 2; ++i)
+      pre[i] = half + 2 * i < n_here && l < a.dim ? raw[(size_t)(t0 + half + 2 * i) * a.decay_ld] : 0.f;
+  } else {
+    const T* raw = static_cast<const T*>(a.decay) + a.decay_at + h;
 #pragma unroll
-      for (int t = 0; t < DC_TOKENS; ++t) dst[t * kDcStride + l] = col[t];
+    for (int i = 0; i < 4; ++i) pre[i] = warp + 8 * i < n_here ? to_float(raw[(size_t)(t0 + warp + 8 * i) * a.decay_ld]) : 0.f;
+  }
+  auto silu = [](float v) { return v * dc_sigmoid(v); };
+  if (a.taps == 4) {
+    const T* a_in = proj + a.qkv_at + a_ch;
+    const T* k_in = proj + a.qkv_at + k_ch;
+    float ax[3], kx[3], aw[4], kw[4];
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) col[t] = t < n_here && l < a_lanes ? to_float(a_in[(size_t)(t0 + t) * a.ld]) : 0.f;
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS / 2; ++t) key[t] = k0 + t < n_here && l < a.dim ? to_float(k_in[(size_t)(t0 + k0 + t) * a.ld]) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      ax[j] = l < a_lanes ? input(a_ch, at0 - 3 + j) : 0.f;
+      kx[j] = k0 < n_here && l < a.dim ? input(k_ch, at0 + k0 - 3 + j) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      aw[j] = l < a_lanes ? a.conv_w[(size_t)a_ch * 4 + j] : 0.f;
+      kw[j] = l < a.dim ? a.conv_w[(size_t)k_ch * 4 + j] : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) {
+      const float x = col[t], v = fmaf(aw[3], x, fmaf(aw[2], ax[2], fmaf(aw[1], ax[1], aw[0] * ax[0])));
+      col[t] = t < n_here ? silu(v) : 0.f;
+      ax[0] = ax[1]; ax[1] = ax[2]; ax[2] = x;
+    }
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS / 2; ++t) {
+      const float x = key[t], v = fmaf(kw[3], x, fmaf(kw[2], kx[2], fmaf(kw[1], kx[1], kw[0] * kx[0])));
+      key[t] = k0 + t < n_here ? silu(v) : 0.f;
+      kx[0] = kx[1]; kx[1] = kx[2]; kx[2] = x;
     }
   } else {
-    const int j = threadIdx.x - DC_DIM;
-    if (j < a.vdim) {
-      convolve(2 * a.groups * a.dim + h * a.vdim + j, col);
-    } else {
+    auto sum = [&](int ch, int t) {
+      float v = 0.f;
+      for (int j = 0; j < a.taps; ++j) v = fmaf(a.conv_w[(size_t)ch * a.taps + j], input(ch, at0 + t - (a.taps - 1 - j)), v);
+      return silu(v);
+    };
 #pragma unroll
-      for (int t = 0; t < DC_TOKENS; ++t) col[t] = 0.f;
-    }
+    for (int t = 0; t < DC_TOKENS; ++t) col[t] = t < n_here && l < a_lanes ? sum(a_ch, t) : 0.f;
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS / 2; ++t) key[t] = k0 + t < n_here && l < a.dim ? sum(k_ch, k0 + t) : 0.f;
   }
+  if (!half) {
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) q_s[t * kDcStride + l] = col[t];
+  }
+#pragma unroll
+  for (int t = 0; t < DC_TOKENS / 2; ++t) k_s[(k0 + t) * kDcStride + l] = key[t];
   // ---- decays and beta; A and M start as zeros ----
   {
     const float rate = expf(a.a_log[h]);
     if (BY_CHANNEL) {
-      const float* pre = static_cast<const float*>(a.decay) + a.decay_at + h * a.dim;
-      for (int i = threadIdx.x; i < DC_TOKENS * DC_DIM; i += DC_PREPARE_THREADS) {
-        const int t = i / DC_DIM, l = i % DC_DIM;
-        g_s[t * kDcStride + l] = t < n_here && l < a.dim
-            ? expf(-rate * dc_softplus(pre[(size_t)(t0 + t) * a.decay_ld + l] + a.dt_bias[h * a.dim + l])) : 1.f;
+      const float shift = l < a.dim ? a.dt_bias[h * a.dim + l] : 0.f;
+#pragma unroll
+      for (int i = 0; i < DC_TOKENS / 2; ++i) {
+        const int t = half + 2 * i;
+        g_s[t * kDcStride + l] = t < n_here && l < a.dim ? expf(-rate * dc_softplus(pre[i] + shift)) : 1.f;
       }
     } else {
-      const T* pre = static_cast<const T*>(a.decay) + a.decay_at + h;
-      for (int t = warp; t < DC_TOKENS; t += DC_PREPARE_THREADS / 32) {
-        const float g = t < n_here ? expf(-rate * dc_softplus(to_float(pre[(size_t)(t0 + t) * a.decay_ld]) + a.dt_bias[h])) : 1.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = warp + 8 * i;
+        const float g = t < n_here ? expf(-rate * dc_softplus(pre[i] + a.dt_bias[h])) : 1.f;
         *reinterpret_cast<float4*>(g_s + t * kDcStride + lane * 4) = make_float4(g, g, g, g);
       }
     }
@@ -164,163 +208,212 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   }
   __syncthreads();
   // ---- unit vectors: a warp a row, four lanes of it a thread ----
-  for (int row = warp; row < 2 * DC_TOKENS; row += DC_PREPARE_THREADS / 32) {
-    const bool key = row >= DC_TOKENS;
-    float4* at = reinterpret_cast<float4*>((key ? k_s : q_s) + (row % DC_TOKENS) * kDcStride) + lane;
+#pragma unroll
+  for (int i = 0; i < 2 * DC_TOKENS; i += DC_PREPARE_THREADS / 32) {
+    const bool of_k = i >= DC_TOKENS;
+    float4* at = reinterpret_cast<float4*>((of_k ? k_s : q_s) + (i % DC_TOKENS + warp) * kDcStride) + lane;
     float4 v = *at;
-    const float unit = 1.0f / sqrtf(warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) + 1e-6f) * (key ? 1.f : a.q_scale);
+    const float unit = 1.0f / sqrtf(warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) + 1e-6f) * (of_k ? 1.f : a.q_scale);
     v.x *= unit; v.y *= unit; v.z *= unit; v.w *= unit;
     *at = v;
-    if (key) reinterpret_cast<float4*>(r_s + (row % DC_TOKENS) * kDcStride)[lane] = v;
   }
   __syncthreads();
-  // ---- A and M, eight tokens' rows at a time ----
-#pragma unroll 1
-  for (int e = 0; e < DC_TOKENS; e += 8) {
-    {                                                   // the eight's rows, decayed from its first token on
-      const int l = threadIdx.x & (DC_DIM - 1);
-      const float* src = threadIdx.x < DC_DIM ? k_s : q_s;
-      float* dst = l_s + (threadIdx.x < DC_DIM ? 0 : 8) * kDcStride;
-      float upto = 1.f;
+  // ---- A and M: pairs whose tokens a block of 2 w tokens' middle parts, w = 16, 8, 4, as products of rows that were
+  // decayed to and from that middle; 4 x 4 pairs of both matrices a thread over a share of the lanes ----
+  auto level = [&](auto width) {
+    constexpr int w = decltype(width)::value;
+    // token `i` of the 16 in lower halves; + w: its like in the upper half
+    auto token = [](int i) { return (i / w) * 2 * w + i % w; };
+    if (!half) {
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        upto *= g_s[(e + t) * kDcStride + l];
-        dst[t * kDcStride + l] = upto * src[(e + t) * kDcStride + l];
-      }
-    }
-    {
-      // pairs inside the eight: warp w takes token e + w as the key and all eight tokens as the other, those before it
-      // with nothing; the sixteen sums cross the lanes together, in 8 + 4 + 2 + 1 exchanges and a last one
-      float sums[16];
-      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 16; i += w) {
+        float upto = 1.f;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float4 kt = reinterpret_cast<const float4*>(k_s + (e + t) * kDcStride)[lane];
-        const float4 qt = reinterpret_cast<const float4*>(q_s + (e + t) * kDcStride)[lane];
-        const float4 g = reinterpret_cast<const float4*>(g_s + (e + t) * kDcStride)[lane];
-        if (t == warp) p = kt;
-        else { p.x *= g.x; p.y *= g.y; p.z *= g.z; p.w *= g.w; }
-        sums[t] = fmaf(p.x, kt.x, p.y * kt.y) + fmaf(p.z, kt.z, p.w * kt.w);
-        sums[8 + t] = fmaf(p.x, qt.x, p.y * qt.y) + fmaf(p.z, qt.z, p.w * qt.w);
-      }
-#pragma unroll
-      for (int width = 8; width > 0; width >>= 1) {        // lanes with the bit keep the upper half of what is left
-        const bool upper = lane & (2 * width);
-#pragma unroll
-        for (int i = 0; i < width; ++i) {
-          const float got = __shfl_xor_sync(0xffffffffu, upper ? sums[i] : sums[i + width], 2 * width);
-          sums[i] = (upper ? sums[i + width] : sums[i]) + got;
+        for (int j = i; j < i + w; ++j) {
+          const int t = token(j) + w;
+          upto *= g_s[t * kDcStride + l];
+          l_s[j * kDcStride + l] = upto * k_s[t * kDcStride + l];
+          l_s[(16 + j) * kDcStride + l] = upto * q_s[t * kDcStride + l];
         }
       }
-      sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], 1);
-      // lanes 2 i, 2 i + 1 hold sum i: keys with token i, then queries
-      const int t = (lane >> 1) & 7;
-      if (!(lane & 1)) {
-        if (lane < 16) {
-          if (t > warp) a_s[(e + t) * kDcPairs + e + warp] = sums[0] * beta_s[e + t];
-        } else if (t >= warp) {
-          m_s[(e + t) * kDcPairs + e + warp] = sums[0];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; i += w) {
+        float behind = 1.f;
+#pragma unroll
+        for (int j = i + w - 1; j >= i; --j) {
+          const int t = token(j);
+          r_s[j * kDcStride + l] = behind * k_s[t * kDcStride + l];
+          behind *= g_s[t * kDcStride + l];
         }
       }
     }
     __syncthreads();
-    {                                                   // the eight against every token before it
-      const int t = lane & 7, s = warp * 4 + (lane >> 3);
-      if (s < e) {
-        const float* kl = l_s + t * kDcStride;
-        const float* ql = kl + 8 * kDcStride;
-        const float* rs = r_s + s * kDcStride;
-        float kk[2] = {0.f, 0.f}, qk[2] = {0.f, 0.f};
-#pragma unroll 4
-        for (int l = 0; l < DC_DIM; l += 4) {
-          const float4 x = *reinterpret_cast<const float4*>(kl + l), y = *reinterpret_cast<const float4*>(ql + l);
-          const float4 z = *reinterpret_cast<const float4*>(rs + l);
-          kk[0] = fmaf(x.x, z.x, kk[0]); kk[1] = fmaf(x.y, z.y, kk[1]);
-          kk[0] = fmaf(x.z, z.z, kk[0]); kk[1] = fmaf(x.w, z.w, kk[1]);
-          qk[0] = fmaf(y.x, z.x, qk[0]); qk[1] = fmaf(y.y, z.y, qk[1]);
-          qk[0] = fmaf(y.z, z.z, qk[0]); qk[1] = fmaf(y.w, z.w, qk[1]);
-        }
-        a_s[(e + t) * kDcPairs + s] = (kk[0] + kk[1]) * beta_s[e + t];
-        m_s[(e + t) * kDcPairs + s] = qk[0] + qk[1];
-      }
-    }
-    __syncthreads();
-    {                                                   // the keys so far, decayed over this eight
-      const int l = threadIdx.x & (DC_DIM - 1), half = threadIdx.x / DC_DIM;
-      float behind = 1.f;
+    constexpr int kAcross = w / 4, kTiles = 16 / w * kAcross * kAcross, kLanes = w == 16 ? 16 : 32;
+    const int tile = threadIdx.x / kLanes, slice = threadIdx.x % kLanes;
+    if (tile < kTiles) {                                // whole warps
+      const int t4 = tile / (kAcross * kAcross) * w + tile / kAcross % kAcross * 4;      // rows of l_s, of r_s
+      const int s4 = tile / (kAcross * kAcross) * w + tile % kAcross * 4;
+      float sums[32];
 #pragma unroll
-      for (int t = 7; t >= 0; --t) {
-        if ((t & 1) == half) r_s[(e + t) * kDcStride + l] *= behind;
-        behind *= g_s[(e + t) * kDcStride + l];
+      for (int i = 0; i < 32; ++i) sums[i] = 0.f;
+#pragma unroll
+      for (int c = 0; c < DC_DIM; c += kLanes * 4) {
+        float4 z[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) z[j] = *reinterpret_cast<const float4*>(r_s + (s4 + j) * kDcStride + c + slice * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {                   // four keys, four queries
+          const float4 x = *reinterpret_cast<const float4*>(l_s + (i / 4 * 16 + t4 + i % 4) * kDcStride + c + slice * 4);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float& v = sums[i * 4 + j];
+            v = fmaf(x.x, z[j].x, v); v = fmaf(x.y, z[j].y, v);
+            v = fmaf(x.z, z[j].z, v); v = fmaf(x.w, z[j].w, v);
+          }
+        }
       }
-      for (int s = half; s < e; s += 2) r_s[s * kDcStride + l] *= behind;
+      dc_exchange<32, kLanes>(sums, lane);
+#pragma unroll
+      for (int e = 0; e < 32 / kLanes; ++e) {
+        const int i = slice * (32 / kLanes) + e;        // the sum this lane holds
+        const int t = token(t4 + i / 4 % 4) + w, s = token(s4 + i % 4);
+        if (i < 16) a_s[t * kDcPairs + s] = sums[e] * beta_s[t];
+        else m_s[t * kDcPairs + s] = sums[e];
+      }
     }
-    __syncthreads();
+  };
+  level(dc_int<16>());
+  __syncthreads();
+  level(dc_int<8>());
+  __syncthreads();
+  level(dc_int<4>());
+  {
+    // pairs inside four tokens, a warp the four: token s's key decayed on from token to token
+    const int e = warp * 4;
+    float4 k[4], q[4], g[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      k[i] = reinterpret_cast<const float4*>(k_s + (e + i) * kDcStride)[lane];
+      q[i] = reinterpret_cast<const float4*>(q_s + (e + i) * kDcStride)[lane];
+      g[i] = reinterpret_cast<const float4*>(g_s + (e + i) * kDcStride)[lane];
+    }
+    float sums[16];                                     // of (t, s): the query's for s <= t at 4 t + s, the key's for s < t at 4 s + t
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      float4 p = k[s];
+#pragma unroll
+      for (int t = s; t < 4; ++t) {
+        if (t > s) {
+          p.x *= g[t].x; p.y *= g[t].y; p.z *= g[t].z; p.w *= g[t].w;
+          sums[4 * s + t] = fmaf(p.x, k[t].x, p.y * k[t].y) + fmaf(p.z, k[t].z, p.w * k[t].w);
+        }
+        sums[4 * t + s] = fmaf(p.x, q[t].x, p.y * q[t].y) + fmaf(p.z, q[t].z, p.w * q[t].w);
+      }
+    }
+    dc_exchange<16, 32>(sums, lane);
+    const int i = lane >> 1, x = i >> 2, y = i & 3;
+    if (!(lane & 1)) {
+      if (y <= x) m_s[(e + x) * kDcPairs + e + y] = sums[0];
+      else a_s[(e + y) * kDcPairs + e + x] = sums[0] * beta_s[e + y];
+    }
   }
-  // ---- (I + A) W = beta G k and (I + A) U0 = beta v, a column a thread; the scaled queries on the way ----
-  if (threadIdx.x < DC_DIM) {
-    float upto = 1.f;
+  __syncthreads();
+  // ---- (I + A) W = beta G k and (I + A) U0 = beta v, a column of both a thread of the first half (a row of A is read
+  // once for the two); the second half writes the scaled queries and keys and M meanwhile ----
+  if (half) {
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) l_s[t * kDcStride + l] = col[t];
+  }
+  __syncthreads();
+  if (!half) {
+    float other[DC_TOKENS], upto = 1.f;
 #pragma unroll
     for (int t = 0; t < DC_TOKENS; ++t) {
-      upto *= g_s[t * kDcStride + threadIdx.x];
-      rec[kDcQ + t * DC_DIM + threadIdx.x] = upto * q_s[t * kDcStride + threadIdx.x];
-      col[t] = beta_s[t] * (upto * k_s[t * kDcStride + threadIdx.x]);
+      const float beta = beta_s[t];
+      upto *= g_s[t * kDcStride + l];
+      col[t] = beta * (upto * k_s[t * kDcStride + l]);
+      other[t] = beta * l_s[t * kDcStride + l];
     }
-    rec[kDcG + threadIdx.x] = upto;
+#pragma unroll
+    for (int t = 1; t < DC_TOKENS; ++t) {
+      float sum[2] = {0.f, 0.f}, more[2] = {0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < t; s += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a_s + t * kDcPairs + s);
+        sum[0] = fmaf(x.x, col[s], sum[0]); more[0] = fmaf(x.x, other[s], more[0]);
+        if (s + 1 < t) { sum[1] = fmaf(x.y, col[s + 1], sum[1]); more[1] = fmaf(x.y, other[s + 1], more[1]); }
+        if (s + 2 < t) { sum[0] = fmaf(x.z, col[s + 2], sum[0]); more[0] = fmaf(x.z, other[s + 2], more[0]); }
+        if (s + 3 < t) { sum[1] = fmaf(x.w, col[s + 3], sum[1]); more[1] = fmaf(x.w, other[s + 3], more[1]); }
+      }
+      col[t] -= sum[0] + sum[1];
+      other[t] -= more[0] + more[1];
+    }
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) rec[t * DC_DIM + l] = col[t];
+    if (l < a.vdim) {
+#pragma unroll
+      for (int t = 0; t < DC_TOKENS; ++t) rec[kDcU + t * a.vdim + l] = other[t];
+    }
   } else {
+    float upto = 1.f, behind = 1.f;
 #pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) col[t] *= beta_s[t];
-  }
-#pragma unroll
-  for (int t = 1; t < DC_TOKENS; ++t) {
-    float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int s = 0; s < t; s += 4) {
-      const float4 x = *reinterpret_cast<const float4*>(a_s + t * kDcPairs + s);
-      sum[0] = fmaf(x.x, col[s], sum[0]);
-      if (s + 1 < t) sum[1] = fmaf(x.y, col[s + 1], sum[1]);
-      if (s + 2 < t) sum[2] = fmaf(x.z, col[s + 2], sum[2]);
-      if (s + 3 < t) sum[3] = fmaf(x.w, col[s + 3], sum[3]);
+    for (int t = 0; t < DC_TOKENS; ++t) {
+      upto *= g_s[t * kDcStride + l];
+      rec[kDcQ + t * DC_DIM + l] = upto * q_s[t * kDcStride + l];
     }
-    col[t] -= (sum[0] + sum[1]) + (sum[2] + sum[3]);
-  }
-  if (threadIdx.x < DC_DIM) {
+    rec[kDcG + l] = upto;
 #pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) rec[t * DC_DIM + threadIdx.x] = col[t];
-  } else if (threadIdx.x - DC_DIM < a.vdim) {
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) rec[kDcU + t * a.vdim + threadIdx.x - DC_DIM] = col[t];
+    for (int t = DC_TOKENS - 1; t >= 0; --t) {
+      rec[kDcK + t * DC_DIM + l] = behind * k_s[t * kDcStride + l];
+      behind *= g_s[t * kDcStride + l];
+    }
+    for (int i = l; i < DC_TOKENS * DC_TOKENS; i += DC_DIM) rec[kDcM + i] = m_s[i / DC_TOKENS * kDcPairs + i % DC_TOKENS];
   }
-  for (int i = threadIdx.x; i < DC_TOKENS * DC_DIM / 4; i += DC_PREPARE_THREADS) {
-    const int t = i / (DC_DIM / 4), l = i % (DC_DIM / 4) * 4;
-    *reinterpret_cast<float4*>(rec + kDcK + t * DC_DIM + l) = *reinterpret_cast<const float4*>(r_s + t * kDcStride + l);
-  }
-  for (int i = threadIdx.x; i < DC_TOKENS * DC_TOKENS; i += DC_PREPARE_THREADS)
-    rec[kDcM + i] = m_s[i / DC_TOKENS * kDcPairs + i % DC_TOKENS];
 }
 constexpr int kDcPrepareSmem = (4 * DC_TOKENS * kDcStride + 16 * kDcStride + 2 * DC_TOKENS * kDcPairs + DC_TOKENS) * 4;
 
 // ---- the chunks one after another --------------------------------------------------------------------------------
-// a stage, in floats: W and G q (64 x 132), decayed k (32 x 128), M (32 x 36), G_31 (128), U0 (32 x 16)
+// a stage, in floats: W and G q (64 x 132), decayed k (32 x 128), M (32 x 36), G_31 (128), U0 (32 x COLS)
 constexpr int kDsK = 2 * DC_TOKENS * kDcStride, kDsM = kDsK + DC_TOKENS * DC_DIM, kDsG = kDsM + DC_TOKENS * kDcPairs,
-              kDsU = kDsG + DC_DIM, kDsStage = kDsU + DC_TOKENS * DC_COLS;
-// behind the two stages: the columns of S [128][16], the four partial sums [4][64][16], U [32][16]
-constexpr int kDsFloats = 2 * kDsStage + DC_DIM * DC_COLS + 4 * 2 * DC_TOKENS * DC_COLS + DC_TOKENS * DC_COLS;
+              kDsU = kDsG + DC_DIM;
+// behind the two stages: the columns of S [128][COLS], the eight partial sums [8][64][COLS], U [32][COLS]
+template <int COLS> constexpr int dc_scan_floats() {
+  return 2 * (kDsU + DC_TOKENS * COLS) + DC_DIM * COLS + 8 * 2 * DC_TOKENS * COLS + DC_TOKENS * COLS;
+}
+
+// two or four neighbouring floats in one access
+__device__ __forceinline__ void dc_load(float (&v)[2], const float* p) {
+  const float2 a = *reinterpret_cast<const float2*>(p);
+  v[0] = a.x; v[1] = a.y;
+}
+__device__ __forceinline__ void dc_load(float (&v)[4], const float* p) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void dc_store(float* p, const float (&v)[2]) { *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]); }
+__device__ __forceinline__ void dc_store(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
 
 __device__ __forceinline__ void dc_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
 
+template <int COLS>
 __global__ void __launch_bounds__(DC_SCAN_THREADS, 1)
 delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, float* __restrict__ state,
                         long long state_stride, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                         float* __restrict__ o_out) {
+  constexpr int kStage = kDsU + DC_TOKENS * COLS;
+  constexpr int kOwn = COLS / 8;                         // columns of S a thread
+  constexpr int kRows = COLS / 16;                       // rows of W or G q a thread adds up, four columns of each
   extern __shared__ __align__(16) float ds_raw[];
-  float* s_s = ds_raw + 2 * kDsStage;
-  float* part_s = s_s + DC_DIM * DC_COLS;
-  float* u_s = part_s + 4 * 2 * DC_TOKENS * DC_COLS;
-  const int r = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * DC_COLS;
+  float* s_s = ds_raw + 2 * kStage;
+  float* part_s = s_s + DC_DIM * COLS;
+  float* u_s = part_s + 8 * 2 * DC_TOKENS * COLS;
+  const int r = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
   const int first = q_start[r], n = q_start[r + 1] - first;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_wait();
@@ -332,126 +425,152 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
   auto fetch = [&](int c) {
     if (c < chunks) {
       const float* src = base + (size_t)c * heads * record;
-      float* dst = ds_raw + (c & 1) * kDsStage;
-      for (int i = threadIdx.x; i < 2 * DC_TOKENS * DC_DIM / 4; i += DC_SCAN_THREADS)
+      float* dst = ds_raw + (c & 1) * kStage;
+#pragma unroll
+      for (int j = 0; j < 2 * DC_TOKENS * DC_DIM / 4; j += DC_SCAN_THREADS) {
+        const int i = j + threadIdx.x;
         dc_copy16(dst + i / (DC_DIM / 4) * kDcStride + i % (DC_DIM / 4) * 4, src + i * 4);
-      for (int i = threadIdx.x; i < DC_TOKENS * DC_DIM / 4; i += DC_SCAN_THREADS)
-        dc_copy16(dst + kDsK + i * 4, src + kDcK + i * 4);
+      }
+#pragma unroll
+      for (int j = 0; j < DC_TOKENS * DC_DIM / 4; j += DC_SCAN_THREADS)
+        dc_copy16(dst + kDsK + (j + threadIdx.x) * 4, src + kDcK + (j + threadIdx.x) * 4);
       dc_copy16(dst + kDsM + threadIdx.x / (DC_TOKENS / 4) * kDcPairs + threadIdx.x % (DC_TOKENS / 4) * 4,
                 src + kDcM + threadIdx.x * 4);
       if (threadIdx.x < DC_DIM / 4) dc_copy16(dst + kDsG + threadIdx.x * 4, src + kDcG + threadIdx.x * 4);
-      if (threadIdx.x >= 128) {
-        const int i = threadIdx.x - 128, t = i / (DC_COLS / 4), l = i % (DC_COLS / 4) * 4;
-        dc_copy16(dst + kDsU + t * DC_COLS + l, src + kDcU + t * vdim + col0 + l);
+      if ((int)threadIdx.x >= DC_SCAN_THREADS - DC_TOKENS * COLS / 4) {
+        const int i = threadIdx.x - (DC_SCAN_THREADS - DC_TOKENS * COLS / 4), t = i / (COLS / 4), l = i % (COLS / 4) * 4;
+        dc_copy16(dst + kDsU + t * COLS + l, src + kDcU + t * vdim + col0 + l);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  static_assert(DC_SCAN_THREADS == DC_TOKENS * DC_TOKENS / 4 && DC_TOKENS * DC_COLS / 4 == 128, "a copy a thread");
+  static_assert(DC_SCAN_THREADS == DC_TOKENS * DC_TOKENS / 4 && DC_TOKENS * COLS / 4 <= DC_SCAN_THREADS, "a copy a thread");
   fetch(0);
-  // this thread's share of the matrix: rows row .. + 3 of columns 2 pair, 2 pair + 1
-  const int row = ((warp & 3) * 8 + lane / 4) * 4, pair = (warp >> 2) * 4 + lane % 4;
-  float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + 2 * pair) * DC_DIM + row;
-  float S[4][2];
+  // this thread's share of the matrix: rows row .. + 3 of columns own .. + kOwn - 1
+  const int row = ((warp & 3) * 8 + lane / 4) * 4, own = ((warp >> 2) * 4 + lane % 4) * kOwn;
+  float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + own) * DC_DIM + row;
+  float S[4][kOwn];
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
+  for (int j = 0; j < kOwn; ++j) {
     const float4 v = *reinterpret_cast<const float4*>(mine + j * DC_DIM);
     S[0][j] = v.x; S[1][j] = v.y; S[2][j] = v.z; S[3][j] = v.w;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    *reinterpret_cast<float2*>(s_s + (row + i) * DC_COLS + 2 * pair) = make_float2(S[i][0], S[i][1]);
+  for (int i = 0; i < 4; ++i) dc_store(s_s + (row + i) * COLS + own, S[i]);
 
   for (int c = 0; c < chunks; ++c) {
-    const float* stage = ds_raw + (c & 1) * kDsStage;
+    const float* stage = ds_raw + (c & 1) * kStage;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                     // the record and the matrix are in place
     fetch(c + 1);                                        // into the stage that the chunk before has left
     {
-      // rows of W (even warps) and of G q (odd ones) times the columns: lanes k0 .. k0 + 31, rows group + 8 i
-      const int k0 = (warp >> 1) * 32, group = lane >> 2, cols = (lane & 3) * 4;
-      const float* x_s = stage + ((warp & 1) * DC_TOKENS + group) * kDcStride;
-      float acc[4][4];
+      // the 64 rows of W and G q times the columns, lanes k0 .. k0 + 15 a warp: rows group + 8 i, columns cols .. + 3
+      // and, of 32, cols + 16 .. + 19
+      constexpr int kWide = COLS / 16;
+      const int k0 = warp * 16, group = lane >> 2, cols = (lane & 3) * 4;
+      const float* x_s = stage + group * kDcStride;
+      float acc[8][4 * kWide];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 4 * kWide; ++j) acc[i][j] = 0.f;
 #pragma unroll
-      for (int k = k0; k < k0 + 32; k += 4) {
-        float4 x[4];
+      for (int k = k0; k < k0 + 16; k += 4) {
+        float4 x[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(x_s + i * 8 * kDcStride + k);
+        for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(x_s + i * 8 * kDcStride + k);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const float4 y = *reinterpret_cast<const float4*>(s_s + (k + kk) * DC_COLS + cols);
+        for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float v = kk == 0 ? x[i].x : kk == 1 ? x[i].y : kk == 2 ? x[i].z : x[i].w;
-            acc[i][0] = fmaf(v, y.x, acc[i][0]);
-            acc[i][1] = fmaf(v, y.y, acc[i][1]);
-            acc[i][2] = fmaf(v, y.z, acc[i][2]);
-            acc[i][3] = fmaf(v, y.w, acc[i][3]);
+          for (int e = 0; e < kWide; ++e) {
+            const float4 y = *reinterpret_cast<const float4*>(s_s + (k + kk) * COLS + e * 16 + cols);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float v = kk == 0 ? x[i].x : kk == 1 ? x[i].y : kk == 2 ? x[i].z : x[i].w;
+              acc[i][4 * e] = fmaf(v, y.x, acc[i][4 * e]);
+              acc[i][4 * e + 1] = fmaf(v, y.y, acc[i][4 * e + 1]);
+              acc[i][4 * e + 2] = fmaf(v, y.z, acc[i][4 * e + 2]);
+              acc[i][4 * e + 3] = fmaf(v, y.w, acc[i][4 * e + 3]);
+            }
           }
-        }
       }
-      float* to = part_s + (((warp >> 1) * 2 + (warp & 1)) * DC_TOKENS + group) * DC_COLS + cols;
+      float* to = part_s + (warp * 2 * DC_TOKENS + group) * COLS + cols;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float4*>(to + i * 8 * DC_COLS) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < kWide; ++e)
+          *reinterpret_cast<float4*>(to + i * 8 * COLS + e * 16) =
+              make_float4(acc[i][4 * e], acc[i][4 * e + 1], acc[i][4 * e + 2], acc[i][4 * e + 3]);
     }
     __syncthreads();
-    // a row (of W for the first half of the threads, of G q for the second) and four columns a thread
-    const int t = (threadIdx.x >> 2) & (DC_TOKENS - 1), cols = (threadIdx.x & 3) * 4;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    // kRows rows (of W for the first half of the threads, of G q for the second) of four columns a thread
+    const bool second = threadIdx.x >= 128;
+    const int t = (threadIdx.x & 127) / (COLS / 4), cols = threadIdx.x % (COLS / 4) * 4;
+    float4 sum[kRows];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 v = *reinterpret_cast<const float4*>(part_s + (i * 2 * DC_TOKENS + (threadIdx.x >> 2)) * DC_COLS + cols);
-      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-    }
-    if (threadIdx.x < 128) {
-      const float4 v = *reinterpret_cast<const float4*>(stage + kDsU + t * DC_COLS + cols);
-      *reinterpret_cast<float4*>(u_s + t * DC_COLS + cols) = make_float4(v.x - sum.x, v.y - sum.y, v.z - sum.z, v.w - sum.w);
+    for (int e = 0; e < kRows; ++e) {
+      sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(
+            part_s + ((i * 2 + second) * DC_TOKENS + t + e * (DC_TOKENS / kRows)) * COLS + cols);
+        sum[e].x += v.x; sum[e].y += v.y; sum[e].z += v.z; sum[e].w += v.w;
+      }
+      if (!second) {
+        const int at = (t + e * (DC_TOKENS / kRows)) * COLS + cols;
+        const float4 v = *reinterpret_cast<const float4*>(stage + kDsU + at);
+        *reinterpret_cast<float4*>(u_s + at) = make_float4(v.x - sum[e].x, v.y - sum[e].y, v.z - sum[e].z, v.w - sum[e].w);
+      }
     }
     __syncthreads();
-    if (threadIdx.x >= 128) {
+    if (second) {
       const float* m_row = stage + kDsM + t * kDcPairs;          // zeros behind the diagonal
 #pragma unroll 4
       for (int s = 0; s < DC_TOKENS; s += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(m_row + s);
+        float4 x[kRows];
+#pragma unroll
+        for (int e = 0; e < kRows; ++e) x[e] = *reinterpret_cast<const float4*>(m_row + e * (DC_TOKENS / kRows) * kDcPairs + s);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 u = *reinterpret_cast<const float4*>(u_s + (s + i) * DC_COLS + cols);
-          const float v = i == 0 ? x.x : i == 1 ? x.y : i == 2 ? x.z : x.w;
-          sum.x = fmaf(v, u.x, sum.x); sum.y = fmaf(v, u.y, sum.y);
-          sum.z = fmaf(v, u.z, sum.z); sum.w = fmaf(v, u.w, sum.w);
+          const float4 u = *reinterpret_cast<const float4*>(u_s + (s + i) * COLS + cols);
+#pragma unroll
+          for (int e = 0; e < kRows; ++e) {
+            const float v = i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w;
+            sum[e].x = fmaf(v, u.x, sum[e].x); sum[e].y = fmaf(v, u.y, sum[e].y);
+            sum[e].z = fmaf(v, u.z, sum[e].z); sum[e].w = fmaf(v, u.w, sum[e].w);
+          }
         }
       }
-      const int token = c * DC_TOKENS + t;
-      if (token < n)
-        *reinterpret_cast<float4*>(o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + cols) = sum;
+#pragma unroll
+      for (int e = 0; e < kRows; ++e) {
+        const int token = c * DC_TOKENS + t + e * (DC_TOKENS / kRows);
+        if (token < n)
+          *reinterpret_cast<float4*>(o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + cols) = sum[e];
+      }
     }
     // the matrix moves on by the chunk
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float g = stage[kDsG + row + i];
-      S[i][0] *= g;
-      S[i][1] *= g;
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j) S[i][j] *= g;
     }
 #pragma unroll 8
     for (int s = 0; s < DC_TOKENS; ++s) {
       const float4 k = *reinterpret_cast<const float4*>(stage + kDsK + s * DC_DIM + row);
-      const float2 u = *reinterpret_cast<const float2*>(u_s + s * DC_COLS + 2 * pair);
-      S[0][0] = fmaf(k.x, u.x, S[0][0]); S[0][1] = fmaf(k.x, u.y, S[0][1]);
-      S[1][0] = fmaf(k.y, u.x, S[1][0]); S[1][1] = fmaf(k.y, u.y, S[1][1]);
-      S[2][0] = fmaf(k.z, u.x, S[2][0]); S[2][1] = fmaf(k.z, u.y, S[2][1]);
-      S[3][0] = fmaf(k.w, u.x, S[3][0]); S[3][1] = fmaf(k.w, u.y, S[3][1]);
+      float u[kOwn];
+      dc_load(u, u_s + s * COLS + own);
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j) {
+        S[0][j] = fmaf(k.x, u[j], S[0][j]); S[1][j] = fmaf(k.y, u[j], S[1][j]);
+        S[2][j] = fmaf(k.z, u[j], S[2][j]); S[3][j] = fmaf(k.w, u[j], S[3][j]);
+      }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      *reinterpret_cast<float2*>(s_s + (row + i) * DC_COLS + 2 * pair) = make_float2(S[i][0], S[i][1]);
+    for (int i = 0; i < 4; ++i) dc_store(s_s + (row + i) * COLS + own, S[i]);
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+  for (int j = 0; j < kOwn; ++j)
     *reinterpret_cast<float4*>(mine + j * DC_DIM) = make_float4(S[0][j], S[1][j], S[2][j], S[3][j]);
 }
 
@@ -510,17 +629,31 @@ TOKB200_API int tokb200_delta_chunk_prepare(const void* proj, int proj_dtype, in
   return TOKB200_BAD_DTYPE;
 }
 
+template <int COLS>
+static int dc_scan(const float* records, int heads, int vdim, float* state, long long state_stride, const int* q_start,
+                   const int* state_slot, int n_requests, float* o_out, cudaStream_t stream) {
+  constexpr int bytes = dc_scan_floats<COLS>() * (int)sizeof(float);
+  static bool done[64] = {};
+  const int status = dc_allow(delta_chunk_scan_kernel<COLS>, bytes, done);
+  if (status != TOKB200_OK) return status;
+  return launch_dependent(delta_chunk_scan_kernel<COLS>, dim3(vdim / COLS, heads, n_requests), dim3(DC_SCAN_THREADS),
+                          (size_t)bytes, stream, records, heads, vdim, state, state_stride, q_start, state_slot, o_out);
+}
+
+// `columns`: of a block, 16 or 32; 0: by the number of blocks.
 TOKB200_API int tokb200_delta_chunk_scan(const float* records, int heads, int dim, int vdim, float* state,
                                          long long state_stride, const int* q_start, const int* state_slot,
-                                         int n_requests, float* o_out, cudaStream_t stream) {
+                                         int n_requests, float* o_out, int columns, cudaStream_t stream) {
   if (n_requests <= 0) return TOKB200_OK;
   if (heads <= 0 || heads > 65535 || n_requests > 65535 || !tokb200_delta_chunks_supported(dim, vdim))
     return TOKB200_BAD_SIZE;
   if ((((uintptr_t)records | (uintptr_t)state | (uintptr_t)o_out) & 15) || state_stride % 4) return TOKB200_BAD_ALIGNMENT;
-  constexpr int bytes = kDsFloats * (int)sizeof(float);
-  static bool done[64] = {};
-  const int status = dc_allow(delta_chunk_scan_kernel, bytes, done);
-  if (status != TOKB200_OK) return status;
-  return launch_dependent(delta_chunk_scan_kernel, dim3(vdim / DC_COLS, heads, n_requests), dim3(DC_SCAN_THREADS),
-                          (size_t)bytes, stream, records, heads, vdim, state, state_stride, q_start, state_slot, o_out);
+  // Wide blocks do a column's work in less (5,900 cycles a chunk of 32 columns against 4,900 of 16) but are half as many:
+  // taken where narrow ones would need a second turn on 148 SMs (us, narrow / wide: 16 heads of one request 266 / 366, of
+  // four 270 / 236, 32 heads of one request 268 / 234).
+  const bool wide = columns ? columns == 32 : (long long)vdim / DC_COLS * heads * n_requests > 148;
+  if (columns && columns != 16 && columns != 32) return TOKB200_BAD_SIZE;
+  if (wide && vdim % 32 == 0)
+    return dc_scan<32>(records, heads, vdim, state, state_stride, q_start, state_slot, n_requests, o_out, stream);
+  return dc_scan<16>(records, heads, vdim, state, state_stride, q_start, state_slot, n_requests, o_out, stream);
 }

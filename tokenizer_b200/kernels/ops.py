@@ -1314,11 +1314,12 @@ def delta_chunks_supported(dim: int, vdim: int) -> bool:
 
 def delta_chunks(proj: torch.Tensor, qkv_at: int, b_at: int, decay: torch.Tensor, decay_at: int, by_channel: bool,
                  groups: int, heads: int, dim: int, vdim: int, taps: int, conv_w, a_log, dt_bias, state: torch.Tensor,
-                 conv_off: int, q_start, state_slot, o_out: torch.Tensor) -> None:
+                 conv_off: int, q_start, state_slot, o_out: torch.Tensor, columns: int = 0) -> None:
     """The delta rule over every request's rows, in chunks: short convolution + silu of q, k, v (`proj`'s columns
     qkv_at ..), unit vectors, beta = sigmoid(proj[b_at ..]), decays exp(-exp(a_log) softplus(decay[decay_at ..] + dt_bias))
     (one a head and key channel with `by_channel`, else one a head, from the same product as q, k and v), the recurrence,
-    `o_out` float32 [T, heads * vdim].  The matrices in `state` ([heads, vdim, 128] at the start of a slot) and the kept
+    `o_out` float32 [T, heads * vdim].  `columns` of a head's matrix a block of the scan: 16, 32 or, with 0, by the number
+    of blocks.  The matrices in `state` ([heads, vdim, 128] at the start of a slot) and the kept
     inputs behind them move on."""
     channels, n = 2 * groups * dim + heads * vdim, proj.shape[0]
     per_head = dim if by_channel else 1
@@ -1341,7 +1342,7 @@ def delta_chunks(proj: torch.Tensor, qkv_at: int, b_at: int, decay: torch.Tensor
     short_conv_state(proj, qkv_at, channels, taps, state, conv_off, q_start, state_slot)
     _check(lib.tokb200_delta_chunk_scan(
         _ptr(records), _i(heads), _i(dim), _i(vdim), _ptr(state), _ll(state.shape[1]), _ptr(q_start), _ptr(state_slot),
-        _i(requests), _ptr(o_out), _stream()), "delta_chunk_scan")
+        _i(requests), _ptr(o_out), _i(columns), _stream()), "delta_chunk_scan")
 
 
 def cdr_records(n_rows: int, n_requests: int, heads: int, dim: int, vdim: int, device) -> torch.Tensor:

@@ -116,11 +116,11 @@ def stacked_rows(weights, multiple: int = 8):
 
 # A step whose longest portion has this many tokens runs the delta rules in chunks (bfloat16 models, heads that
 # `ops.delta_chunks_supported` takes).  Chunks cost more arithmetic and save a chain of tokens: with one decay a head, 16
-# heads, us of the token-by-token form / chunks: 32 tokens 31 / 34, four requests of 48 68 / 58, 64 tokens 43 / 37.  With a
-# decay a channel the other form walks four tokens a step and fills the device sooner: 256 tokens 68 / 58, eight requests
-# of 256 253 / 316, 512 tokens 125 / 81, four of 512 348 / 331.
-DELTA_CHUNKS_FROM = 48
-CHANNEL_DELTA_CHUNKS_FROM = 512
+# heads, us of the token-by-token form / chunks: 32 tokens 31 / 28, four requests of 48 70 / 43, 64 tokens 43 / 30.  With a
+# decay a channel the other form walks four tokens a step and fills the device sooner: 64 tokens 28 / 33, two requests of
+# 100 44 / 44, 128 tokens 43 / 39, eight requests of 128 129 / 126, 512 tokens 130 / 72.
+DELTA_CHUNKS_FROM = 32
+CHANNEL_DELTA_CHUNKS_FROM = 128
 
 
 def _delta_chunks(runtime, dim: int, vdim: int) -> bool:
