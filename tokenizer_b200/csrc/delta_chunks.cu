@@ -20,9 +20,10 @@
 //
 // Both are bound by reads of shared memory: a register tile of R x C costs R + C cycles of the 128 bytes a cycle that come
 // back, and R C / 4 of the multiply-adds.  So tiles are as large as the threads allow, and a row of A is read once for
-// two columns.  Measured (16 heads of 128 x 128, both kernels and the kept inputs between them, us; before: tiles of 4 x 4,
-// pairs eight tokens at a time): a prompt of 2,048 tokens 294 -> 266 with one decay a head and 328 -> 283 with one a
-// channel, four prompts of 5,100 in all 763 -> 557, eight of 256 316 -> 252.
+// two columns, and half of a scan block's threads own the whole matrix (4 x 4 or 8 x 4 of it each).  Measured (16 heads of
+// 128 x 128, both kernels and the kept inputs between them, us; before: tiles of 4 x 4, pairs eight tokens at a time): a
+// prompt of 2,048 tokens 294 -> 254 with one decay a head and 328 -> 272 with one a channel, four prompts of 5,100 in all
+// 763 -> 537, eight of 256 316 -> 247.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).
@@ -382,18 +383,8 @@ template <int COLS> constexpr int dc_scan_floats() {
   return 2 * (kDsU + DC_TOKENS * COLS) + DC_DIM * COLS + 8 * 2 * DC_TOKENS * COLS + DC_TOKENS * COLS;
 }
 
-// two or four neighbouring floats in one access
-__device__ __forceinline__ void dc_load(float (&v)[2], const float* p) {
-  const float2 a = *reinterpret_cast<const float2*>(p);
-  v[0] = a.x; v[1] = a.y;
-}
-__device__ __forceinline__ void dc_load(float (&v)[4], const float* p) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void dc_store(float* p, const float (&v)[2]) { *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]); }
-__device__ __forceinline__ void dc_store(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+__device__ __forceinline__ void dc_add(float4& a, float v, const float4& b) {
+  a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
 }
 
 __device__ __forceinline__ void dc_copy16(float* dst, const float* src) {
@@ -407,7 +398,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
                         long long state_stride, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                         float* __restrict__ o_out) {
   constexpr int kStage = kDsU + DC_TOKENS * COLS;
-  constexpr int kOwn = COLS / 8;                         // columns of S a thread
+  constexpr int kOwn = COLS / 4;                         // rows of S a thread of the first half, four columns of each
   constexpr int kRows = COLS / 16;                       // rows of W or G q a thread adds up, four columns of each
   extern __shared__ __align__(16) float ds_raw[];
   float* s_s = ds_raw + 2 * kStage;
@@ -446,17 +437,25 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
   };
   static_assert(DC_SCAN_THREADS == DC_TOKENS * DC_TOKENS / 4 && DC_TOKENS * COLS / 4 <= DC_SCAN_THREADS, "a copy a thread");
   fetch(0);
-  // this thread's share of the matrix: rows row .. + 3 of columns own .. + kOwn - 1
-  const int row = ((warp & 3) * 8 + lane / 4) * 4, own = ((warp >> 2) * 4 + lane % 4) * kOwn;
+  // threads 0 .. 127: rows row .. + kOwn - 1 of columns own .. + 3 of the matrix
+  const bool owner = threadIdx.x < 128;
+  const int row = (threadIdx.x & 127) / (COLS / 4) * kOwn, own = threadIdx.x % (COLS / 4) * 4;
   float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + own) * DC_DIM + row;
-  float S[4][kOwn];
+  float4 S[kOwn];
+  if (owner) {
 #pragma unroll
-  for (int j = 0; j < kOwn; ++j) {
-    const float4 v = *reinterpret_cast<const float4*>(mine + j * DC_DIM);
-    S[0][j] = v.x; S[1][j] = v.y; S[2][j] = v.z; S[3][j] = v.w;
+    for (int e = 0; e < kOwn; e += 4) {
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(mine + j * DC_DIM + e);
+      S[e] = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+      S[e + 1] = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+      S[e + 2] = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
+      S[e + 3] = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
+    }
+#pragma unroll
+    for (int i = 0; i < kOwn; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * COLS + own) = S[i];
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) dc_store(s_s + (row + i) * COLS + own, S[i]);
 
   for (int c = 0; c < chunks; ++c) {
     const float* stage = ds_raw + (c & 1) * kStage;
@@ -504,7 +503,6 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
     }
     __syncthreads();
     // kRows rows (of W for the first half of the threads, of G q for the second) of four columns a thread
-    const bool second = threadIdx.x >= 128;
     const int t = (threadIdx.x & 127) / (COLS / 4), cols = threadIdx.x % (COLS / 4) * 4;
     float4 sum[kRows];
 #pragma unroll
@@ -513,17 +511,17 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float4 v = *reinterpret_cast<const float4*>(
-            part_s + ((i * 2 + second) * DC_TOKENS + t + e * (DC_TOKENS / kRows)) * COLS + cols);
+            part_s + ((i * 2 + !owner) * DC_TOKENS + t + e * (DC_TOKENS / kRows)) * COLS + cols);
         sum[e].x += v.x; sum[e].y += v.y; sum[e].z += v.z; sum[e].w += v.w;
       }
-      if (!second) {
+      if (owner) {
         const int at = (t + e * (DC_TOKENS / kRows)) * COLS + cols;
         const float4 v = *reinterpret_cast<const float4*>(stage + kDsU + at);
         *reinterpret_cast<float4*>(u_s + at) = make_float4(v.x - sum[e].x, v.y - sum[e].y, v.z - sum[e].z, v.w - sum[e].w);
       }
     }
     __syncthreads();
-    if (second) {
+    if (!owner) {
       const float* m_row = stage + kDsM + t * kDcPairs;          // zeros behind the diagonal
 #pragma unroll 4
       for (int s = 0; s < DC_TOKENS; s += 4) {
@@ -534,11 +532,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
         for (int i = 0; i < 4; ++i) {
           const float4 u = *reinterpret_cast<const float4*>(u_s + (s + i) * COLS + cols);
 #pragma unroll
-          for (int e = 0; e < kRows; ++e) {
-            const float v = i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w;
-            sum[e].x = fmaf(v, u.x, sum[e].x); sum[e].y = fmaf(v, u.y, sum[e].y);
-            sum[e].z = fmaf(v, u.z, sum[e].z); sum[e].w = fmaf(v, u.w, sum[e].w);
-          }
+          for (int e = 0; e < kRows; ++e) dc_add(sum[e], i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w, u);
         }
       }
 #pragma unroll
@@ -547,31 +541,36 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
         if (token < n)
           *reinterpret_cast<float4*>(o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + cols) = sum[e];
       }
-    }
-    // the matrix moves on by the chunk
+    } else {
+      // the matrix moves on by the chunk
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float g = stage[kDsG + row + i];
-#pragma unroll
-      for (int j = 0; j < kOwn; ++j) S[i][j] *= g;
-    }
-#pragma unroll 8
-    for (int s = 0; s < DC_TOKENS; ++s) {
-      const float4 k = *reinterpret_cast<const float4*>(stage + kDsK + s * DC_DIM + row);
-      float u[kOwn];
-      dc_load(u, u_s + s * COLS + own);
-#pragma unroll
-      for (int j = 0; j < kOwn; ++j) {
-        S[0][j] = fmaf(k.x, u[j], S[0][j]); S[1][j] = fmaf(k.y, u[j], S[1][j]);
-        S[2][j] = fmaf(k.z, u[j], S[2][j]); S[3][j] = fmaf(k.w, u[j], S[3][j]);
+      for (int i = 0; i < kOwn; ++i) {
+        const float g = stage[kDsG + row + i];
+        S[i] = make_float4(S[i].x * g, S[i].y * g, S[i].z * g, S[i].w * g);
       }
+#pragma unroll 8
+      for (int s = 0; s < DC_TOKENS; ++s) {
+        const float4 u = *reinterpret_cast<const float4*>(u_s + s * COLS + own);
+#pragma unroll
+        for (int e = 0; e < kOwn; e += 4) {
+          const float4 k = *reinterpret_cast<const float4*>(stage + kDsK + s * DC_DIM + row + e);
+          dc_add(S[e], k.x, u); dc_add(S[e + 1], k.y, u); dc_add(S[e + 2], k.z, u); dc_add(S[e + 3], k.w, u);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kOwn; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * COLS + own) = S[i];
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dc_store(s_s + (row + i) * COLS + own, S[i]);
   }
+  if (owner) {
 #pragma unroll
-  for (int j = 0; j < kOwn; ++j)
-    *reinterpret_cast<float4*>(mine + j * DC_DIM) = make_float4(S[0][j], S[1][j], S[2][j], S[3][j]);
+    for (int e = 0; e < kOwn; e += 4) {
+      const float4* v = S + e;
+      *reinterpret_cast<float4*>(mine + e) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+      *reinterpret_cast<float4*>(mine + DC_DIM + e) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+      *reinterpret_cast<float4*>(mine + 2 * DC_DIM + e) = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
+      *reinterpret_cast<float4*>(mine + 3 * DC_DIM + e) = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
+    }
+  }
 }
 
 // ---- launchers ---------------------------------------------------------------------------------------------------
@@ -648,9 +647,9 @@ TOKB200_API int tokb200_delta_chunk_scan(const float* records, int heads, int di
   if (heads <= 0 || heads > 65535 || n_requests > 65535 || !tokb200_delta_chunks_supported(dim, vdim))
     return TOKB200_BAD_SIZE;
   if ((((uintptr_t)records | (uintptr_t)state | (uintptr_t)o_out) & 15) || state_stride % 4) return TOKB200_BAD_ALIGNMENT;
-  // Wide blocks do a column's work in less (5,900 cycles a chunk of 32 columns against 4,900 of 16) but are half as many:
-  // taken where narrow ones would need a second turn on 148 SMs (us, narrow / wide: 16 heads of one request 266 / 366, of
-  // four 270 / 236, 32 heads of one request 268 / 234).
+  // Wide blocks do a column's work in less time but are half as many: taken where narrow ones would need a second turn on
+  // 148 SMs (us, narrow / wide: 16 heads of one request of 2,048 tokens 254 / 353, of four of 512 260 / 228, 32 heads of one
+  // of 1,024 257 / 227).
   const bool wide = columns ? columns == 32 : (long long)vdim / DC_COLS * heads * n_requests > 148;
   if (columns && columns != 16 && columns != 32) return TOKB200_BAD_SIZE;
   if (wide && vdim % 32 == 0)

@@ -114,13 +114,21 @@ def stacked_rows(weights, multiple: int = 8):
     return torch.cat(weights, dim=0)
 
 
-# A step whose longest portion has this many tokens runs the delta rules in chunks (bfloat16 models, heads that
-# `ops.delta_chunks_supported` takes).  Chunks cost more arithmetic and save a chain of tokens: with one decay a head, 16
-# heads, us of the token-by-token form / chunks: 32 tokens 31 / 28, four requests of 48 70 / 43, 64 tokens 43 / 30.  With a
-# decay a channel the other form walks four tokens a step and fills the device sooner: 64 tokens 28 / 33, two requests of
-# 100 44 / 44, 128 tokens 43 / 39, eight requests of 128 129 / 126, 512 tokens 130 / 72.
+# Steps whose longest portion has fewer tokens never run the delta rules in chunks: with a decay a channel a lone prompt of
+# 64 tokens takes 28 us token by token (four a step) and 32 in chunks, 128 tokens 43 / 38; with one a head 32 tokens 32 / 27.
 DELTA_CHUNKS_FROM = 32
 CHANNEL_DELTA_CHUNKS_FROM = 128
+
+
+def _chunks_pay(q_lens, heads: int, chain: float, work: float) -> bool:
+    """Whether chunks of 32 tokens are the faster form of a delta rule for portions of these lengths.  Chunks cost 0.22 us
+    a chunk and head whatever is in it (a lone token too) and never wait for a chain; token by token a step takes `chain`
+    us a token of its longest portion, or `work` us a token and head once the device is full.  Measured for heads of 128 x
+    128, one decay a head / one a channel, us token by token -> in chunks, 16 heads: 2,048 tokens 772 -> 254 / 558 -> 272;
+    512 and 15 single ones 231 -> 114 / 199 -> 124; 512 and 63 single ones 248 -> 309 / 171 -> 320 (not taken); 128 x 4 and
+    8 x 28 154 -> 185 / 116 -> 195 (not taken); eight of 512 with one a channel 494 -> 441."""
+    chunks = sum((n + 31) // 32 for n in q_lens)
+    return 20.0 + 0.22 * heads * chunks <= 18.0 + max(chain * max(q_lens), work * heads * sum(q_lens))
 
 
 def _delta_chunks(runtime, dim: int, vdim: int) -> bool:
@@ -187,9 +195,12 @@ class GatedDeltaNet:
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
         self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
 
+    def _in_chunks(self, q_lens) -> bool:
+        return self.chunked and max(q_lens, default=0) >= DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.34, 0.0115)
+
     def shape_key(self, q_lens):
         longest = max(q_lens)
-        if self.chunked and longest >= DELTA_CHUNKS_FROM:
+        if self._in_chunks(q_lens):
             return "delta_chunks"
         return "delta1" if longest == 1 else "delta" if longest < 32 else "delta32"      # the kernels' choices
 
@@ -218,7 +229,7 @@ class GatedDeltaNet:
             return self.out.forward(y, partials_ok=True)
         o = torch.empty((n, h * self.vdim), dtype=torch.float32, device=proj.device)
         y = self.runtime.empty(n, h * self.vdim)
-        if self.chunked and ctx.max_q_len >= DELTA_CHUNKS_FROM:
+        if self._in_chunks(ctx.q_lens):
             ops.delta_chunks(proj, at, at + c, proj, at + c + h, False, self.groups, h, self.dim, self.vdim, self.taps,
                              self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
                              ctx.state_slot, o)
@@ -313,10 +324,11 @@ class ChannelDeltaNet:
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
         self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
 
-    def shape_key(self, q_lens):
-        longest = max(q_lens)                                                # the kernels' choice
-        return "channel_delta1" if longest == 1 else \
-            "delta_chunks" if self.chunked and longest >= CHANNEL_DELTA_CHUNKS_FROM else "channel_delta"
+    def _in_chunks(self, q_lens) -> bool:
+        return self.chunked and max(q_lens, default=0) >= CHANNEL_DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.26, 0.0077)
+
+    def shape_key(self, q_lens):                                             # the kernels' choice
+        return "channel_delta1" if max(q_lens) == 1 else "delta_chunks" if self._in_chunks(q_lens) else "channel_delta"
 
     def cache_need(self):
         return CacheNeed(state=StateNeed((self.state_floats,)))
@@ -348,7 +360,7 @@ class ChannelDeltaNet:
             return self.out.forward(y, partials_ok=True)
         pre = self._second_products(proj)
         o = torch.empty((n, heads * self.vdim), dtype=torch.float32, device=proj.device)
-        if self.chunked and ctx.max_q_len >= CHANNEL_DELTA_CHUNKS_FROM:
+        if self._in_chunks(ctx.q_lens):
             ops.delta_chunks(proj, 0, self.b_at, pre, 0, True, self.groups, heads, self.dim, self.vdim, self.taps,
                              self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
                              ctx.state_slot, o)
