@@ -1,0 +1,54 @@
+"""The state-space recurrence in chunks against the same recurrence token by token in 64 bits: portions of one token to
+several chunks and their remainders, continued portions, idle rows, empty requests, decays next to one and next to zero,
+states of fewer than 128 lanes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("heads,groups,vdim,n_state,shift,dtype", [
+    (4, 2, 64, 128, -3.0, torch.float32), (3, 1, 32, 72, 3.0, torch.float32), (2, 2, 96, 100, 0.0, torch.bfloat16)])
+def test_against_the_recurrence(heads, groups, vdim, n_state, shift, dtype):
+    from tokenizer_b200.kernels import ops as o
+    assert o.ssd_chunks_supported(vdim, n_state)
+    lengths = [[1, 33, 0, 64, 95, 32], [31, 2, 40, 1, 0, 70]]
+    n_req, inner, share = len(lengths[0]), heads * vdim, heads // groups
+    g = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    dt_bias, a_log, skip = rnd(heads) + shift, rnd(heads) * 0.5, rnd(heads)
+    S = [rnd(heads, n_state, vdim) * 0.3 for _ in range(n_req)]
+    size = -(-(inner * n_state + 12) // 4) * 4
+    slots = torch.randperm(n_req, generator=g)
+    dev = torch.full((n_req, size), 7.0, device=DEV)
+    for r in range(n_req):
+        dev[slots[r], :inner * n_state] = S[r].transpose(1, 2).reshape(-1).to(DEV)
+    S = [s.double() for s in S]
+    for portion in lengths:
+        starts = [0]
+        for n in portion:
+            starts.append(starts[-1] + n)
+        rows = starts[-1] + 3
+        xbc, proj = rnd(rows, inner + 2 * groups * n_state), rnd(rows, heads + 11).to(dtype)
+        y = torch.full((rows, inner), 9.0, device=DEV)
+        o.ssd_chunks(xbc.to(DEV), proj.to(DEV), 11, dt_bias.to(DEV), a_log.to(DEV), skip.to(DEV), heads, groups, vdim, n_state,
+                     dev, torch.tensor(starts, dtype=torch.int32, device=DEV), slots.int().to(DEV), y)
+        got, got_state = y.cpu().double(), dev[slots.to(DEV)].cpu().double()
+        assert bool((got[starts[-1]:] == 9.0).all())
+        dt = torch.nn.functional.softplus(proj[:, 11:].double() + dt_bias.double())
+        keep = torch.exp(-torch.exp(a_log.double()) * dt)
+        x = xbc[:, :inner].double().view(rows, heads, vdim)
+        b, c = (t.reshape(rows, groups, n_state).double().repeat_interleave(share, 1)
+                for t in torch.split(xbc[:, inner:], groups * n_state, dim=1))
+        for r, n in enumerate(portion):
+            want = torch.empty(n, heads, vdim, dtype=torch.float64)
+            for i, t in enumerate(range(starts[r], starts[r + 1])):
+                S[r] = keep[t][:, None, None] * S[r] + (dt[t][:, None] * b[t])[:, :, None] * x[t][:, None, :]
+                want[i] = torch.einsum("hnv,hn->hv", S[r], c[t]) + skip.double()[:, None] * x[t]
+            # 32-bit sums of 128 products, a chain of three chunks at most: some tens of 2^-24 of the largest value
+            if n:
+                assert float((got[starts[r]:starts[r + 1]] - want.reshape(n, -1)).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+            m = got_state[r, :inner * n_state].view(heads, vdim, n_state).transpose(1, 2)
+            assert float((m - S[r]).abs().max()) < 1e-5 * max(1.0, float(S[r].abs().max()))
+        assert bool((got_state[:, inner * n_state:] == 7.0).all())

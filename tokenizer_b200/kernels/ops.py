@@ -1667,6 +1667,29 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_at: int, dt_bias, a_lo
         counter.launches += 1
 
 
+def ssd_chunks_supported(vdim: int, n_state: int) -> bool:
+    return bool(_lib("ssd_chunks").tokb200_ssd_chunks_supported(_i(vdim), _i(n_state)))
+
+
+def ssd_chunks(xbc: torch.Tensor, proj: torch.Tensor, dt_at: int, dt_bias, a_log, skip, heads: int, groups: int, vdim: int,
+               n_state: int, state: torch.Tensor, q_start, state_slot, y: torch.Tensor) -> None:
+    """`mamba2_scan` in chunks of 32 tokens (the same sums in another order), for portions of prompts."""
+    n, requests = xbc.shape[0], q_start.shape[0] - 1
+    if xbc.dtype != torch.float32 or y.dtype != torch.float32 or tuple(y.shape) != (n, heads * vdim) or \
+            xbc.shape[1] != heads * vdim + 2 * groups * n_state or state.dtype != torch.float32 or state.dim() != 2 or \
+            heads * vdim * n_state > state.shape[1] or dt_at + heads > proj.shape[1] or proj.shape[0] != n or \
+            any(v.dtype != torch.float32 or v.numel() != heads for v in (dt_bias, a_log, skip)):
+        raise ValueError("ssd_chunks: sizes of the inputs, the state or the output disagree")
+    lib = _lib("ssd_chunks")
+    lib.tokb200_ssd_chunk_floats.restype = ctypes.c_longlong
+    records = torch.empty(lib.tokb200_ssd_chunk_floats(_i(n), _i(requests), _i(heads)), dtype=torch.float32, device=xbc.device)
+    _check(lib.tokb200_ssd_chunks(
+        _ptr(xbc), _i(xbc.shape[1]), _sliced_ptr(proj), _i(_tag(proj)), _i(_ld(proj)), _i(dt_at), _ptr(dt_bias), _ptr(a_log),
+        _ptr(skip), _i(heads), _i(groups), _i(vdim), _i(n_state), _ptr(state), _ll(state.shape[1]), _ptr(q_start),
+        _ptr(state_slot), _i(n), _i(requests), _ptr(y), _ptr(records), _stream()), "ssd_chunks")
+    counter.launches += 1
+
+
 def mamba2_out_norm(y: torch.Tensor, proj: torch.Tensor, z_at: int, gain: torch.Tensor, eps: float, parts: int,
                     row_req, out: torch.Tensor) -> None:
     """out = (y * silu(proj[:, z_at ..])) divided by its root mean square inside each of `parts` equal parts of

@@ -29,6 +29,7 @@ def all_variants():
         ("moe.cu", (), ()),
         ("short_conv.cu", (), ()),
         ("mamba2.cu", (), ()),
+        ("ssd_chunks.cu", (), ()),
         ("mlstm.cu", (), ()),
         ("mlstm_chunks.cu", (), ()),
         ("streams.cu", (), ()),

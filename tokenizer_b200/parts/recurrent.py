@@ -377,6 +377,10 @@ class ChannelDeltaNet:
         return self.out.forward(y, partials_ok=True)
 
 
+# A step whose longest portion has this many tokens may run the state-space recurrence in chunks
+SSD_CHUNKS_FROM = 128
+
+
 class Mamba2:
     """The selective state-space mixer with a scalar decay a head (Mamba-2).  With inner = heads * vdim,
     N = `state` lanes and G = `groups`: the input product W_in h is [z: inner | x: inner | B: G N | C: G N |
@@ -432,12 +436,27 @@ class Mamba2:
         # a slot: [heads, vdim, N] and behind it [taps - 1, channels], in whole 4s of floats
         self.conv_off = self.heads * self.vdim * self.n
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
+        # a float32 model keeps the token-by-token form, as with the delta rules
+        self.chunked = runtime.dtype == torch.bfloat16 and ops.ssd_chunks_supported(self.vdim, self.n)
 
     def cache_need(self):
         return CacheNeed(state=StateNeed((self.state_floats,)))
 
-    def shape_key(self, q_lens):
-        return "ssm1" if max(q_lens) == 1 else "ssm"
+    def _in_chunks(self, q_lens) -> bool:
+        """Chunks of 32 tokens are cut over blocks of 32 columns, one a multiprocessor at a time, and are the faster form
+        where portions of length fill one or two turns of them; the token-by-token form cuts finer (few columns) and packs
+        better (many).  us token by token / in chunks, heads of 64 x 128: 64 heads, 2,048 tokens 307 / 214, two prompts of
+        1,905 and 1,096 412 / 312, 128 tokens 32 / 24, 40 tokens 13 / 18; 48 heads, 1,024 tokens 128 / 111; 32 heads, 2,048
+        tokens 175 / 203; 128 heads, 1,024 tokens 247 / 210, 128 tokens 44 / 52; 64 heads, four of 512 215 / 220."""
+        if not self.chunked or max(q_lens, default=0) < SSD_CHUNKS_FROM:
+            return False
+        columns = self.heads * self.vdim // 32
+        blocks = columns * sum(n >= SSD_CHUNKS_FROM // 2 for n in q_lens)
+        return 96 <= blocks <= 296 and max(q_lens) >= SSD_CHUNKS_FROM * (1 if blocks <= 148 else 2) and \
+            columns * len(q_lens) <= 592                              # portions of a few tokens take turns, too
+
+    def shape_key(self, q_lens):                                             # the kernels' choice
+        return "ssm1" if max(q_lens) == 1 else "ssm_chunks" if self._in_chunks(q_lens) else "ssm"
 
     def streamed_weights(self):
         return [self.inputs.weight, self.out.weight]
@@ -453,8 +472,9 @@ class Mamba2:
             ops.short_conv_state(proj, self.inner, self.channels, self.taps, cache.state, self.conv_off, ctx.q_start,
                                  ctx.state_slot)
         y = torch.empty((n, self.inner), dtype=torch.float32, device=proj.device)
-        ops.mamba2_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.a_log, self.skip, self.heads,
-                        self.groups, self.vdim, self.n, cache.state, ctx.q_start, ctx.state_slot, y)
+        scan = ops.ssd_chunks if self._in_chunks(ctx.q_lens) else ops.mamba2_scan
+        scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.a_log, self.skip, self.heads, self.groups, self.vdim,
+             self.n, cache.state, ctx.q_start, ctx.state_slot, y)
         gated = self.runtime.empty(n, self.inner)
         ops.mamba2_out_norm(y, proj, 0, self.gain, self.eps, self.norm_groups, ctx.row_req, gated)
         return self.out.forward(gated, partials_ok=True)
