@@ -1,0 +1,49 @@
+"""The rules that pick a kernel by a step's portions, on the measured sides of their lines, and that a captured step's key
+tells apart what they tell apart."""
+from types import SimpleNamespace
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from tokenizer_b200.parts import attention, recurrent
+
+
+def delta(kind, heads, chunked=True):
+    part = kind.__new__(kind)
+    part.heads, part.chunked = heads, chunked
+    return part
+
+
+@pytest.mark.parametrize("q_lens,by_head,by_channel", [
+    ([2048], True, True), ([512] + [1] * 15, True, True), ([512] + [1] * 63, False, False), ([31], False, False),
+    ([64], True, False), ([128] * 4 + [8] * 28, False, False), ([512] * 8, True, True), ([1], False, False), ([], False, False)])
+def test_delta_rules(q_lens, by_head, by_channel):
+    for kind, want in ((recurrent.GatedDeltaNet, by_head), (recurrent.ChannelDeltaNet, by_channel)):
+        assert delta(kind, 16)._in_chunks(q_lens) is want
+        assert not delta(kind, 16, chunked=False)._in_chunks(q_lens)
+        if q_lens:
+            assert (delta(kind, 16).shape_key(q_lens) == "delta_chunks") is want
+
+
+@pytest.mark.parametrize("heads,q_lens,want", [
+    (64, [2048], True), (64, [1905, 1096], True), (64, [128], True), (64, [127], False), (128, [255], False), (128, [1024], True),
+    (32, [2048], False), (48, [1024], True), (64, [512] * 4, False), (64, [2048] + [1] * 15, False), (64, [400, 1, 1, 1], True),
+    (64, [1], False)])
+def test_state_space_rule(heads, q_lens, want):
+    part = delta(recurrent.Mamba2, heads)
+    part.vdim = 64
+    assert part._in_chunks(q_lens) is want and (part.shape_key(q_lens) == "ssm_chunks") is want
+
+
+@pytest.mark.parametrize("longest,tokens,reach,d,want", [
+    (128, 128, 128, 64, True), (384, 384, 512, 64, True), (385, 385, 512, 64, False), (256, 1024, 256, 64, True),
+    (256, 1152, 256, 64, False), (200, 256, 1024, 64, False), (128, 128, 128, 128, False)])
+def test_short_portions_of_near_keys(monkeypatch, longest, tokens, reach, d, want):
+    monkeypatch.setattr(attention.ops, "prefill_attention_supported", lambda *a: True)
+    part = attention.PagedAttention()
+    part.nh, part.nkv, part.d = 14, 2, d
+    ctx = SimpleNamespace(max_q_len=longest, n_tokens=tokens)
+    group = SimpleNamespace(block_table=torch.empty(1, reach // 16), page_size=16)
+    assert part._near(ctx, group, (None, 1)) is want and part._near(ctx, group, None) is False
+    assert (part.shape_key([longest]) == "middle") is (longest < attention._WIDE_ALWAYS)

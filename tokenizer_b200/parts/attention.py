@@ -127,6 +127,14 @@ _SPLIT_MIXED = os.environ.get("TOKB200_MIXED", "split") != "tiles"
 # portions from this length on go to the tcgen05 kernel (shorter ones would leave most of a
 # 128-row tile empty)
 _WIDE_FROM = 96
+# ... but where heads have 64 lanes, no portion of a small step has _WIDE_ALWAYS tokens and no key lies further back than
+# _NEAR, the mma.sync kernel is the faster one inside a model: it starts while its predecessor still runs, which the
+# tcgen05 kernel must not, and there is little work to make up for that (24 layers of 14 heads over 2, us a step, mma.sync /
+# tcgen05: one portion of 128 tokens 1,071 / 1,185, of 256 1,099 / 1,147, of 384 1,276 / 1,319, of 512 1,352 / 1,356, of 768
+# 1,713 / 1,477; four of 128 1,172 / 1,282, five of 200 1,510 / 1,530, three of 500 2,032 / 1,961)
+_WIDE_ALWAYS = 385
+_NEAR = 512
+_SMALL_STEP = 1024
 
 
 class PagedAttention:
@@ -152,9 +160,16 @@ class PagedAttention:
         longest = max(q_lens) if q_lens else 0
         if longest == 1:
             return "single"
-        kind = "wide" if longest >= _WIDE_FROM else "tiles"
+        kind = "wide" if longest >= _WIDE_ALWAYS else "middle" if longest >= _WIDE_FROM else "tiles"
         # portions with single tokens beside them launch the decoding kernel too
         return kind + "+1" if min(q_lens) == 1 else kind
+
+    def _near(self, ctx, group, tiles) -> bool:
+        """Whether portions that the tcgen05 kernel could take are faster on the mma.sync kernel: by sizes that a captured
+        step's key holds (its rows, its tables' widths, the lengths' kind)."""
+        return self.d == 64 and ctx.max_q_len < _WIDE_ALWAYS and ctx.n_tokens <= _SMALL_STEP and tiles is not None and \
+            group.block_table.shape[1] * group.page_size <= _NEAR and \
+            ops.prefill_attention_supported(self.nh, self.nkv, self.d)
 
     def attend(self, q, out, ctx, group, cache):
         """Choose the kernel by precision and by the shape of the batch.  A group that keeps one
@@ -183,7 +198,7 @@ class PagedAttention:
                 keep_first=self.keep_first)
             wide, tiles = ctx.views[_LONG_WIDE_TILES.key], ctx.views[_LONG_TILES.key]
         if _PROMPT_KERNEL == "tcgen05" and q.dtype == torch.bfloat16 and \
-                wide is not None and ctx.max_q_len >= _WIDE_FROM and \
+                wide is not None and ctx.max_q_len >= _WIDE_FROM and not self._near(ctx, group, tiles) and \
                 ops.attention_tcgen05_supported(self.nh, self.nkv, self.d):
             # long portions on the tcgen05 kernel (128-row tiles, scores in tensor memory)
             ops.attention_tcgen05(

@@ -193,7 +193,9 @@ class GatedDeltaNet:
         # a slot: [heads, vdim, dim_padded] and behind it [taps - 1, channels], in whole 4s of floats
         self.conv_off = self.heads * self.vdim * self.dim_padded
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
-        self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
+        # who asks for a form of the scan gets it
+        self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim) and \
+            not {"TOKB200_GDN_SCAN", "TOKB200_GDN_ROWS"} & set(os.environ)
 
     def _in_chunks(self, q_lens) -> bool:
         return self.chunked and max(q_lens, default=0) >= DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.34, 0.0115)
@@ -436,8 +438,9 @@ class Mamba2:
         # a slot: [heads, vdim, N] and behind it [taps - 1, channels], in whole 4s of floats
         self.conv_off = self.heads * self.vdim * self.n
         self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
-        # a float32 model keeps the token-by-token form, as with the delta rules
-        self.chunked = runtime.dtype == torch.bfloat16 and ops.ssd_chunks_supported(self.vdim, self.n)
+        # a float32 model keeps the token-by-token form, as with the delta rules, and so does who asks for its segments
+        self.chunked = runtime.dtype == torch.bfloat16 and ops.ssd_chunks_supported(self.vdim, self.n) and \
+            "TOKB200_M2_SEGMENTS" not in os.environ
 
     def cache_need(self):
         return CacheNeed(state=StateNeed((self.state_floats,)))
