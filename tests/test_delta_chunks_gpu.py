@@ -90,3 +90,38 @@ def test_against_the_rule(by_channel, columns, groups, heads, dim, vdim, taps, s
             assert float((m[..., :dim].transpose(1, 2) - S[r]).abs().max()) < 1e-5 * max(1.0, float(S[r].abs().max()))
             if taps > 1:
                 assert torch.equal(got_state[r, off:off + (taps - 1) * channels], kept[r].reshape(-1))
+
+
+@pytest.mark.parametrize("by_channel,columns", [(False, 16), (False, 32), (True, 16), (True, 32)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [1, 17, 30, 45])
+def test_a_token_changes_nothing_before_it(by_channel, columns, value, at):
+    """An infinity or NaN in a token's values or key leaves the rows in front of it in the same chunk as they are, bit for bit."""
+    o = ops()
+    groups, heads, dim, vdim, n = 1, 2, 128, 32, 50
+    channels = 2 * dim + heads * vdim
+    g = torch.Generator().manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    conv_w, a_log, dt_bias = rnd(channels, 1), rnd(heads), rnd(heads * (dim if by_channel else 1))      # one tap: a token's own
+    proj = rnd(n, channels + 2 * heads)
+    decay = rnd(n, heads * dim) if by_channel else proj
+    first = rnd(1, heads * vdim * 128)
+    q_start = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+
+    def run(proj):
+        out, state = torch.empty(n, heads * vdim, device=DEV), first.clone()
+        o.delta_chunks(proj, 0, channels, decay if by_channel else proj, 0 if by_channel else channels + heads, by_channel,
+                       groups, heads, dim, vdim, 1, conv_w, a_log, dt_bias, state, heads * vdim * 128, q_start,
+                       torch.zeros(1, dtype=torch.int32, device=DEV), out, columns=columns)
+        return out
+    want = run(proj)
+    assert torch.isfinite(want).all()
+    for column in (2 * dim + 3, dim + 5):                     # a value of the first head, a lane of the key
+        bad = proj.clone()
+        bad[at, column] = value
+        got = run(bad)
+        assert torch.equal(got[:at], want[:at])
+        assert not torch.isfinite(got[at:]).all()
+        if column >= 2 * dim:                                 # a value's column meets no other
+            others = [c for c in range(heads * vdim) if c != column - 2 * dim]
+            assert torch.equal(got[:, others], want[:, others])

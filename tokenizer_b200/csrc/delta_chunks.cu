@@ -522,17 +522,22 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
     }
     __syncthreads();
     if (!owner) {
-      const float* m_row = stage + kDsM + t * kDcPairs;          // zeros behind the diagonal
-#pragma unroll 4
+      // what comes behind a row's own token is left out, not added with weight 0: an infinity or a NaN there is not this row's
+      constexpr int kApart = DC_TOKENS / kRows;
+      const float* m_row = stage + kDsM + t * kDcPairs;
+#pragma unroll
       for (int s = 0; s < DC_TOKENS; s += 4) {
         float4 x[kRows];
 #pragma unroll
-        for (int e = 0; e < kRows; ++e) x[e] = *reinterpret_cast<const float4*>(m_row + e * (DC_TOKENS / kRows) * kDcPairs + s);
+        for (int e = 0; e < kRows; ++e)
+          if (s < (e + 1) * kApart) x[e] = *reinterpret_cast<const float4*>(m_row + e * kApart * kDcPairs + s);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float4 u = *reinterpret_cast<const float4*>(u_s + (s + i) * COLS + cols);
 #pragma unroll
-          for (int e = 0; e < kRows; ++e) dc_add(sum[e], i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w, u);
+          for (int e = 0; e < kRows; ++e)
+            if (s + i < (e + 1) * kApart && (s + i <= e * kApart || s + i <= t + e * kApart))
+              dc_add(sum[e], i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w, u);
         }
       }
 #pragma unroll
