@@ -52,3 +52,37 @@ def test_against_the_recurrence(heads, groups, vdim, n_state, shift, dtype):
             m = got_state[r, :inner * n_state].view(heads, vdim, n_state).transpose(1, 2)
             assert float((m - S[r]).abs().max()) < 1e-5 * max(1.0, float(S[r].abs().max()))
         assert bool((got_state[:, inner * n_state:] == 7.0).all())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [1, 15, 17, 30, 45])
+def test_a_token_changes_nothing_before_it(value, at):
+    """An infinity or NaN in a token's x, B, C or step leaves the rows in front of it in the same chunk as they are, bit for
+    bit."""
+    from tokenizer_b200.kernels import ops as o
+    heads, groups, vdim, n_state, n = 2, 1, 32, 128, 50
+    inner = heads * vdim
+    g = torch.Generator().manual_seed(12)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    dt_bias, a_log, skip, first = rnd(heads), rnd(heads), rnd(heads), rnd(1, inner * n_state)
+    xbc, proj = rnd(n, inner + 2 * groups * n_state), rnd(n, heads)
+
+    def run(xbc, proj):
+        y, state = torch.empty(n, inner, device=DEV), first.clone()
+        o.ssd_chunks(xbc, proj, 0, dt_bias, a_log, skip, heads, groups, vdim, n_state, state,
+                     torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV), y)
+        return y
+    want = run(xbc, proj)
+    assert torch.isfinite(want).all()
+    for column in (3, inner + 7, inner + n_state + 9, -1):    # x, B, C, the step
+        bad, bad_proj = xbc.clone(), proj.clone()
+        if column < 0:
+            bad_proj[at, 0] = value
+        else:
+            bad[at, column] = value
+        got = run(bad, bad_proj)
+        assert torch.equal(got[:at], want[:at])
+        assert not torch.isfinite(got[at:]).all()
+        if column == 3:                                       # a column of x meets no other
+            others = [c for c in range(inner) if c != 3]
+            assert torch.equal(got[:, others], want[:, others])

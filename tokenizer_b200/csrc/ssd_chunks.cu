@@ -118,6 +118,8 @@ constexpr int kSsB = SC_TOKENS * kScStride, kSsM = kSsB + SC_TOKENS * SC_DIM, kS
 // behind the two stages: the columns of S [128][32], the eight partial sums [8][32][32], the weighted x [32][32]
 constexpr int kSsBytes = (2 * kSsStage + SC_DIM * SC_COLS + 8 * SC_TOKENS * SC_COLS + SC_TOKENS * SC_COLS) * 4;
 
+template <bool V> struct sc_bool { static constexpr bool value = V; };
+
 __device__ __forceinline__ void sc_add(float4& a, float v, const float4& b) {
   a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
 }
@@ -192,10 +194,12 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                     // the chunk and the matrix are in place
     fetch(c + 1);                                        // into the stage that the chunk before has left
+    float zero;
     {
       const float w = stage[kSsR + t];
       const float4 x = *reinterpret_cast<const float4*>(stage + kSsX + threadIdx.x * 4);
       *reinterpret_cast<float4*>(u_s + threadIdx.x * 4) = make_float4(w * x.x, w * x.y, w * x.z, w * x.w);
+      zero = fmaf(x.x, 0.f, x.y * 0.f) + fmaf(x.z, 0.f, x.w * 0.f);      // a NaN where one of them is no number
     }
     {
       // the rows of C times the columns, lanes k0 .. k0 + 7 a half warp: rows group + 4 i, columns cols .. + 3 and
@@ -238,7 +242,7 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
         *reinterpret_cast<float4*>(to + 16) = make_float4(v[4], v[5], v[6], v[7]);
       }
     }
-    __syncthreads();
+    const bool wild = __syncthreads_or(!(zero == 0.f));      // the chunk's x holds infinities or NaN
     if (owner) {
       // the matrix moves on by the chunk
       const float all = stage[kSsG + SC_TOKENS - 1];
@@ -267,18 +271,25 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
           sum[e].x += v.x; sum[e].y += v.y; sum[e].z += v.z; sum[e].w += v.w;
         }
       }
+      // M is 0 behind a row's own token; where an infinity or a NaN stands there it is left out, not added with weight 0
+      auto rows = [&](auto all) {
 #pragma unroll
-      for (int s = 0; s < SC_TOKENS; s += 4) {
-        float4 m[2];                                     // zeros behind a row's own token
+        for (int s = 0; s < SC_TOKENS; s += 4) {
+          float4 m[2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) m[e] = *reinterpret_cast<const float4*>(stage + kSsM + at[e] * kScPairs + s);
+          for (int e = 0; e < 2; ++e) m[e] = *reinterpret_cast<const float4*>(stage + kSsM + at[e] * kScPairs + s);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = *reinterpret_cast<const float4*>(stage + kSsX + (s + i) * SC_COLS + c4);
+          for (int i = 0; i < 4; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(stage + kSsX + (s + i) * SC_COLS + c4);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) sc_add(acc[e], i == 0 ? m[e].x : i == 1 ? m[e].y : i == 2 ? m[e].z : m[e].w, x);
+            for (int e = 0; e < 2; ++e)
+              if (decltype(all)::value || s + i <= at[e])
+                sc_add(acc[e], i == 0 ? m[e].x : i == 1 ? m[e].y : i == 2 ? m[e].z : m[e].w, x);
+          }
         }
-      }
+      };
+      if (wild) rows(sc_bool<false>());
+      else rows(sc_bool<true>());
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int token = c * SC_TOKENS + at[e];
