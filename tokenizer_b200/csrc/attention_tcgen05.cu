@@ -26,8 +26,8 @@
 //     memory as bfloat16.  The accumulator stays in tensor memory over the whole walk; the reference maximum
 //     follows the true one lazily: only when the maximum has grown by more than 2^8 since it was set are the
 //     sum and the accumulator rescaled, which happens a few times per row; probabilities stay below 2^8.
-// Measured (28 heads over 4 of 128 lanes, one prompt, us): 8,192 tokens 1,547 -> 555 (311 -> 867 TFLOP/s), 2,048 126 ->
-// 56; 14 heads over 2 of 64: 346 -> 229 and 36.8 -> 29.1.  The form before it took one tile and one head a block, and its
+// Measured (28 heads over 4 of 128 lanes, one prompt, us): 8,192 tokens 1,547 -> 547 (311 -> 880 TFLOP/s), 2,048 126 ->
+// 58; 14 heads over 2 of 64: 346 -> 223 and 36.8 -> 27.3.  The form before it took one tile and one head a block, and its
 // loader waited for a block's copies before it asked for the next.  What bounds it now: a step of the two lanes takes
 // 5,000 cycles at 128 lanes, of which the tensor core 2,300 and each lane's softmax 1,900 (the exponentials alone 1,024 of
 // MUFU), the rest the hand-offs between them; scores asked for while the softmax still runs (probabilities through shared
@@ -69,7 +69,19 @@ constexpr int kHalfKeys = FA_KEYS / 2;            // of a block, that a softmax 
 __device__ int fa_error_flag = 0;
 
 
+// shared memory: q of the two lanes | ring of key and value tiles (each a whole number of 16 KB sub-tiles), then
+// what a row's threads tell one another, then the barriers
+constexpr int kTileBytes = kDBlocks * kSubTile;
+constexpr int kStatBytes = 2 * 2 * FA_ROWS * 4;
+constexpr int kBarBytes = (2 * FA_BUFFERS + 7) * 8 + 8;     // the barriers, where tensor memory lies, whether a wait ran out
+constexpr int kFaSmem = 2 * kTileBytes + FA_BUFFERS * kTileBytes + kStatBytes + kBarBytes;
+static_assert(kFaSmem > 116 * 1024 && kFaSmem <= 227 * 1024, "one block an SM: it takes all of tensor memory");
+
+extern __shared__ __align__(1024) unsigned char fa_raw[];      // swizzle atoms: 1024-byte aligned
+
 __device__ __forceinline__ unsigned fa_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// the word that a wait that ran out sets
+__device__ __forceinline__ unsigned fa_gave_up_at() { return fa_smem(fa_raw) + (unsigned)(kFaSmem - 4); }
 __device__ __forceinline__ void fa_mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(fa_smem(bar)), "r"(count));
 }
@@ -81,6 +93,12 @@ __device__ __forceinline__ bool fa_mbar_wait(unsigned long long* bar, unsigned p
   // the thread sleeps in hardware until the phase completes or the hint runs out, so
   // waiting warps do not take issue slots from working ones
   const unsigned suspend_ns = 20000u;
+  // Unrolled, and with the report of a wait that ran out at each of its two dozen places, this loop made half of the
+  // kernel's 115 KB of code.  Behind a layer's other kernels that code starts cold, and its misses stand in a row: one
+  // portion of 128 tokens behind 256 MB of other traffic took 16.1 us (14 heads of 64) and 17.3 (12 of 128), and 9.3 and
+  // 11.8 with this, loops of the loaders kept as loops and the block's start in the order it has now; 2,048 tokens 36.4 ->
+  // 28.1 and 36.7 -> 32.3.
+#pragma unroll 1
   for (unsigned spin = 0; spin < FA_WAIT_LIMIT; ++spin) {
     unsigned done;
     asm volatile(
@@ -90,8 +108,7 @@ __device__ __forceinline__ bool fa_mbar_wait(unsigned long long* bar, unsigned p
         : "=r"(done) : "r"(addr), "r"(parity), "r"(suspend_ns) : "memory");
     if (done) return true;
   }
-  atomicExch(&fa_error_flag, 1);
-  tokb200_report_error(TOKB200_LIB_ATTENTION_TCGEN05, 1);
+  asm volatile("st.shared.u32 [%0], 1;" ::"r"(fa_gave_up_at()) : "memory");      // reported at the block's end
   return false;
 }
 // byte offset of element (row, 16-byte piece c) in a [rows x 64] bfloat16 tile with 128-byte swizzle
@@ -216,14 +233,6 @@ __device__ __forceinline__ void fa_tma(void* dst, const CUtensorMap* map, unsign
       ::"r"(fa_smem(dst)), "l"(map), "r"(fa_smem(bar)), "r"(x), "r"(y) : "memory");
 }
 
-// shared memory: q of the two lanes | ring of key and value tiles (each a whole number of 16 KB sub-tiles), then
-// what a row's threads tell one another, then the barriers
-constexpr int kTileBytes = kDBlocks * kSubTile;
-constexpr int kStatBytes = 2 * 2 * FA_ROWS * 4;
-constexpr int kBarBytes = (2 * FA_BUFFERS + 7) * 8 + 8;     // the barriers, and where tensor memory lies
-constexpr int kFaSmem = 2 * kTileBytes + FA_BUFFERS * kTileBytes + kStatBytes + kBarBytes;
-static_assert(kFaSmem > 116 * 1024 && kFaSmem <= 227 * 1024, "one block an SM: it takes all of tensor memory");
-
 template <bool CAPPED>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -234,7 +243,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                          const int* __restrict__ tiles, int n_tiles, int nh, int nkv, int page, int run,
                          int pool_rows, int split_all, int window, int chunk, int keep_first, float scale_log2,
                          const float* __restrict__ sink, float cap_in, float cap_out) {
-  extern __shared__ __align__(1024) unsigned char fa_raw[];      // swizzle atoms: 1024-byte aligned
   unsigned char* q_s = fa_raw;                                   // lane 0, lane 1
   unsigned char* ring = q_s + 2 * kTileBytes;
   float* stat_s = reinterpret_cast<float*>(ring + FA_BUFFERS * kTileBytes);   // [lane][half][row]
@@ -255,32 +263,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int h0 = split_all ? blockIdx.x : kvh * group + (blockIdx.x % pairs) * 2;
   const bool split = split_all || h0 + 1 == (kvh + 1) * group;     // a group's odd head is split
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = tiles[2 * tile], n_rows = tiles[2 * tile + 1];
-  const int r_id = row_req[row0];
-  // uniform over the block; a misaligned base (never seen) is reported instead of used
-  const bool aligned = (fa_smem(fa_raw) & 1023u) == 0;
-  if (!aligned && threadIdx.x == 0) {
-    atomicExch(&fa_error_flag, 2);
-    tokb200_report_error(TOKB200_LIB_ATTENTION_TCGEN05, 2);
-  }
-  const bool live = aligned && tile < n_tiles && r_id >= 0 && n_rows > 0;
-  const int pos0 = live ? pos[row0] : 0;
-  const int pos_last = pos0 + n_rows - 1;
-  const int lo_first = first_visible_key(pos0, window, chunk);
-  const int lo_last = first_visible_key(pos_last, window, chunk);
-  const int kb_first = lo_first / FA_KEYS * FA_KEYS;
-  // blocks of kept keys that lie before the first block of the window
-  const int n_kept = min((keep_first + FA_KEYS - 1) / FA_KEYS, kb_first / FA_KEYS);
-  const int n_blocks = live ? n_kept + (pos_last - kb_first) / FA_KEYS + 1 : 0;
-  auto first_of = [&](int b) { return b < n_kept ? b * FA_KEYS : kb_first + (b - n_kept) * FA_KEYS; };
-  // what a lane walks: its step b is block `block_of(lane, b)`
-  auto steps_of = [&](int l) { return split ? (n_blocks + 1 - l) / 2 : n_blocks; };
-  auto block_of = [&](int l, int b) { return split ? 2 * b + l : b; };
-  // the ring's sequence of tiles: K0 V0 K1 V1 ... side by side, K0 K1 V0 K2 V1 K3 ... split (in the order of their
-  // use; a split walk's place for the keys behind the last block stays empty, nothing comes behind it in its buffer)
-  auto k_place = [&](int b) { return split ? (b < 2 ? b : 2 * b - 1) : 2 * b; };
-  auto v_place = [&](int b) { return split ? 2 * b + 2 : 2 * b + 1; };
-  const int* table = block_table + (size_t)(live ? r_id : 0) * table_stride;
+  // What needs nothing of the step comes first: the trips to memory for the step's rows, one behind the other, then lie
+  // beside the maps' way into the SM and the claim on tensor memory, not in front of them.
   constexpr int kMmaWarp = FA_SOFTMAX_WARPS + FA_LOADER_WARPS;
   const bool by_tma = run > 0;            // runs of keys inside one page, 8 to 128 of them
 
@@ -297,6 +281,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       fa_mbar_init(&pv_done[i], 1);
     }
     fa_mbar_init(q_full, 1);
+    tmem_slot[1] = 0;                            // no wait has run out
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) {
@@ -304,6 +289,35 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                  ::"r"(fa_smem(tmem_slot)), "r"((unsigned)kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  const int row0 = tiles[2 * tile], n_rows = tiles[2 * tile + 1];
+  const int r_id = row_req[row0], pos_row0 = pos[row0];
+  // uniform over the block; a misaligned base (never seen) is reported instead of used
+  const bool aligned = (fa_smem(fa_raw) & 1023u) == 0;
+  if (!aligned && threadIdx.x == 0) {
+    atomicExch(&fa_error_flag, 2);
+    tokb200_report_error(TOKB200_LIB_ATTENTION_TCGEN05, 2);
+  }
+  const bool live = aligned && tile < n_tiles && r_id >= 0 && n_rows > 0;
+  const int pos0 = live ? pos_row0 : 0;
+  const int pos_last = pos0 + n_rows - 1;
+  const int lo_first = first_visible_key(pos0, window, chunk);
+  const int lo_last = first_visible_key(pos_last, window, chunk);
+  const int kb_first = lo_first / FA_KEYS * FA_KEYS;
+  // blocks of kept keys that lie before the first block of the window
+  const int n_kept = min((keep_first + FA_KEYS - 1) / FA_KEYS, kb_first / FA_KEYS);
+  const int n_blocks = live ? n_kept + (pos_last - kb_first) / FA_KEYS + 1 : 0;
+  auto first_of = [&](int b) { return b < n_kept ? b * FA_KEYS : kb_first + (b - n_kept) * FA_KEYS; };
+  // what a lane walks: its step b is block `block_of(lane, b)`
+  auto steps_of = [&](int l) { return split ? (n_blocks + 1 - l) / 2 : n_blocks; };
+  auto block_of = [&](int l, int b) { return split ? 2 * b + l : b; };
+  // the ring's sequence of tiles: K0 V0 K1 V1 ... side by side, K0 K1 V0 K2 V1 K3 ... split (in the order of their
+  // use; a split walk's place for the keys behind the last block stays empty, nothing comes behind it in its buffer)
+  auto k_place = [&](int b) { return split ? (b < 2 ? b : 2 * b - 1) : 2 * b; };
+  auto v_place = [&](int b) { return split ? 2 * b + 2 : 2 * b + 1; };
+  // and back: whether a place holds values, and of which block (n_blocks or more: it stays empty)
+  auto of_values = [&](int n) { return split ? n >= 2 && n % 2 == 0 : n % 2 == 1; };
+  auto block_at = [&](int n) { return !split ? n / 2 : n < 2 ? n : n % 2 == 0 ? n / 2 - 1 : (n + 1) / 2; };
+  const int* table = block_table + (size_t)(live ? r_id : 0) * table_stride;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -334,8 +348,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       struct Place { int b, y; bool values, some, all; };
       auto locate = [&](int n) {
         Place at;
-        at.values = split ? (n >= 2 && n % 2 == 0) : n % 2 == 1;
-        at.b = split ? (n < 2 ? n : at.values ? n / 2 - 1 : (n + 1) / 2) : n / 2;
+        at.values = of_values(n);
+        at.b = block_at(n);
         at.y = pool_rows;
         at.some = at.all = false;
         if (n < n_places && at.b < n_blocks && lane < runs) {
@@ -348,6 +362,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       };
       int n = loader;
       Place next = locate(n);
+#pragma unroll 1
       for (; n < n_places; n += FA_LOADER_WARPS) {
         const Place at = next;
         next = locate(n + FA_LOADER_WARPS);
@@ -357,9 +372,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         unsigned char* dst = ring + buf * kTileBytes;
         const unsigned mixed = __ballot_sync(0xffffffffu, at.values && at.some && !at.all);
         if (mixed) {                                     // values seen in part: zeros for the others
+#pragma unroll 1
           for (unsigned left = mixed; left; left &= left - 1) {
             const int i = __ffs(left) - 1;
             const int row = __shfl_sync(0xffffffffu, at.y, i), first = first_of(at.b) + i * run;
+#pragma unroll 1
             for (int e = lane; e < run * (HEAD_DIM / 8); e += 32) {
               const int t = e / (HEAD_DIM / 8), c = e % (HEAD_DIM / 8);
               uint4 piece = make_uint4(0u, 0u, 0u, 0u);
@@ -384,6 +401,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       // every copy has landed before the block gives its shared memory back, whatever became of its readers (the places
       // that nothing came behind in their buffers)
       const int end = min(n, n_places);
+#pragma unroll 1
       for (int i = loader; i < end; i += FA_LOADER_WARPS)
         if (i >= end - FA_BUFFERS && locate(i).b < n_blocks)
           fa_mbar_wait(&full[i % FA_BUFFERS], (i / FA_BUFFERS) & 1);
@@ -651,6 +669,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   pdl_launch();
+  if (threadIdx.x == 0 && tmem_slot[1] != 0) {
+    atomicExch(&fa_error_flag, 1);
+    tokb200_report_error(TOKB200_LIB_ATTENTION_TCGEN05, 1);
+  }
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
