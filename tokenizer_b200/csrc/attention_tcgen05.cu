@@ -224,6 +224,9 @@ __device__ __forceinline__ float fa_exp2(float x) {
   return y;
 }
 
+__device__ __forceinline__ void fa_copy16(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(fa_smem(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void fa_expect(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fa_smem(bar)), "r"(bytes) : "memory");
 }
@@ -406,38 +409,71 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         if (i >= end - FA_BUFFERS && locate(i).b < n_blocks)
           fa_mbar_wait(&full[i % FA_BUFFERS], (i / FA_BUFFERS) & 1);
     } else {
-      // pages of other sizes: a row's 16-byte pieces by plain loads, eight of them in flight a thread
-      constexpr int kPieces = FA_KEYS * (HEAD_DIM / 8), kStep = FA_LOADER_WARPS * 32;
-      static_assert(kPieces % (8 * kStep) == 0, "whole rounds of eight");
+      // Pages of other sizes: each warp copies half of every tile's rows (cp.async, 16 bytes a lane, a row's lanes side by
+      // side), kLag places on their way at a time; before a place is asked for, the one kLag before it is waited for and
+      // announced.  Plain loads, whose values a thread had to hold, kept 8 of them in flight a thread (2,048 tokens, cold
+      // caches, us, plain loads / now / pages of 16 by TMA: pages of 20 keys, 28 heads of 128 211 / 70 / 59, 14 of 64 114 / 38
+      // / 28; pages of 5 keys 223 / 70 and 127 / 38).  A place that is not announced yet is never one that the release of a
+      // buffer still waits for: kLag < the buffers (side by side a place is read out only when the one behind it has been
+      // announced too).
+      constexpr int kLag = HEAD_DIM == 64 ? 4 : 3, kRowPieces = HEAD_DIM / 8, kRowsAtOnce = 32 / kRowPieces;
+      static_assert(kLag < FA_BUFFERS, "a buffer's release may wait for the place behind it");
+      // a place's block, and of this lane's two keys of the warp's half their pages (-1: not seen) and places in them
+      struct Copy { int b, page_at[2], in_page[2]; };
+      auto look_up = [&](int n) {
+        Copy at;
+        at.b = n < n_places ? block_at(n) : n_blocks;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int key = first_of(at.b) + loader * 64 + i * 32 + lane;
+          at.in_page[i] = key % page;
+          at.page_at[i] = at.b < n_blocks && visible(key) ? table[key / page] : -1;
+        }
+        return at;
+      };
+      auto announce = [&](int n) {                       // this thread's copies of place n have landed
+        if (block_at(n) < n_blocks) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) fa_mbar_arrive(&full[n % FA_BUFFERS]);
+        }
+      };
+      bool ok = true;
+      Copy next = look_up(0);
+#pragma unroll 1
       for (int n = 0; n < n_places; ++n) {
-        const bool values = split ? (n >= 2 && n % 2 == 0) : n % 2 == 1;
-        const int b = split ? (n < 2 ? n : values ? n / 2 - 1 : (n + 1) / 2) : n / 2;
-        if (b >= n_blocks) continue;
-        const int buf = n % FA_BUFFERS, use = n / FA_BUFFERS;
-        if (use > 0 && !__all_sync(0xffffffffu, fa_mbar_wait(&empty[buf], (use - 1) & 1))) break;
-        unsigned char* dst = ring + buf * kTileBytes;
-        const __nv_bfloat16* pool = values ? v_pool : k_pool;
-        for (int e0 = loader * 32 + lane; e0 < kPieces; e0 += 8 * kStep) {
-          uint4 piece[8];
+        const Copy at = next;
+        next = look_up(n + 1);
+        if (n >= kLag) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kLag - 1) : "memory");
+          announce(n - kLag);
+        }
+        if (at.b < n_blocks) {
+          const int buf = n % FA_BUFFERS, use = n / FA_BUFFERS;
+          if (use > 0 && !__all_sync(0xffffffffu, fa_mbar_wait(&empty[buf], (use - 1) & 1))) { ok = false; break; }
+          unsigned char* dst = ring + buf * kTileBytes;
+          const int c = lane % kRowPieces;
+          const unsigned char* pool =
+              reinterpret_cast<const unsigned char*>((of_values(n) ? v_pool : k_pool) + kvh * HEAD_DIM + c * 8);
+          const unsigned row_bytes = (unsigned)nkv * HEAD_DIM * 2;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int e = e0 + i * kStep, t = e / (HEAD_DIM / 8), c = e % (HEAD_DIM / 8);
-            const int key = first_of(b) + t;
-            piece[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (visible(key))
-              piece[i] = *reinterpret_cast<const uint4*>(
-                  pool + ((size_t)(table[key / page] * page + key % page) * nkv + kvh) * HEAD_DIM + c * 8);
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int e = e0 + i * kStep, t = e / (HEAD_DIM / 8), c = e % (HEAD_DIM / 8);
-            *reinterpret_cast<uint4*>(dst + (c / 8) * kSubTile + swz(t, c % 8)) = piece[i];
+          for (int half = 0; half < 2; ++half) {
+            const int mine = at.page_at[half] < 0 ? -1 : at.page_at[half] * page + at.in_page[half];
+#pragma unroll 8
+            for (int i = 0; i < 32; i += kRowsAtOnce) {
+              const int t = half * 32 + i + lane / kRowPieces;              // of the warp's half of the tile
+              const int row = __shfl_sync(0xffffffffu, mine, t % 32);
+              fa_copy16(dst + (c / 8) * kSubTile + swz(loader * 64 + t, c % 8),
+                        pool + (size_t)(unsigned)(row < 0 ? 0 : row) * row_bytes, row >= 0);
+            }
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) fa_mbar_arrive(&full[buf]);
+        asm volatile("cp.async.commit_group;" ::: "memory");
       }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (ok)
+#pragma unroll 1
+        for (int n = max(0, n_places - kLag); n < n_places; ++n) announce(n);
       if (loader == 0) fa_mbar_wait(q_full, 0);          // q's copies are TMA's all the same
     }
   } else if (live && warp == kMmaWarp) {
