@@ -47,3 +47,23 @@ def test_short_portions_of_near_keys(monkeypatch, longest, tokens, reach, d, wan
     group = SimpleNamespace(block_table=torch.empty(1, reach // 16), page_size=16)
     assert part._near(ctx, group, (None, 1)) is want and part._near(ctx, group, None) is False
     assert (part.shape_key([longest]) == "middle") is (longest < attention._WIDE_ALWAYS)
+
+
+def heads_of(nh, nkv, d=64, window=None, chunk=None):
+    part = attention.PagedAttention()
+    part.nh, part.nkv, part.d, part.window, part.chunk = nh, nkv, d, window, chunk
+    return part
+
+
+@pytest.mark.parametrize("nh,nkv,q_lens,window,cut", [
+    (14, 2, [512], None, True), (14, 2, [2048], None, True), (14, 2, [384] * 4, None, False), (14, 2, [500] * 3, None, False),
+    (14, 2, [700] * 2, None, True), (14, 2, [2048], 256, False), (14, 2, [480] + [1] * 31, None, True), (32, 8, [640], None, True),
+    (32, 8, [500] * 2, None, False), (32, 8, [1536], None, False), (28, 4, [200] * 5, None, True), (28, 4, [2048], None, False),
+    (4, 4, [4096], None, True)])
+def test_where_keys_are_cut(nh, nkv, q_lens, window, cut):
+    part = heads_of(nh, nkv, window=window)
+    assert part._cut_keys(q_lens) is cut
+    # a captured step's key tells the two apart, in whatever order the requests come
+    assert part.shape_key(q_lens).endswith("two heads a block" + ("+1" if 1 in q_lens else "")) is not cut
+    assert part.shape_key(q_lens) == part.shape_key(q_lens[::-1])
+    assert part.shape_key([n for n in q_lens if n > 1]).endswith("two heads a block") is not cut

@@ -757,8 +757,7 @@ static int fa_map(CUtensorMap* map, const void* base, long long rows, long long 
 }
 
 // tiles: [n_tiles][2] = (first row, rows) of consecutive rows of one request, rows <= 128.  `q_rows`, `pool_rows`: rows
-// of q and of the pools.  `split`: 1 cuts every head's key blocks over the two lanes, 0 puts heads side by side, -1:
-// by the rule below.
+// of q and of the pools.  `split`: 1 cuts every head's key blocks over the two lanes, 0 puts heads side by side.
 TOKB200_API int tokb200_attention_tcgen05(
     const void* q, const void* k_pool, const void* v_pool, void* out, const int* block_table,
     int table_stride, const int* row_req, const int* pos, const int* tiles, int n_tiles, int q_rows, int pool_rows,
@@ -770,7 +769,6 @@ TOKB200_API int tokb200_attention_tcgen05(
   if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15)
     return TOKB200_BAD_ALIGNMENT;
   static bool configured[64] = {};
-  static int sms[64] = {};
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return TOKB200_BAD_SIZE;
   if (!configured[device]) {
@@ -778,7 +776,6 @@ TOKB200_API int tokb200_attention_tcgen05(
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kFaSmem);
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(attention_tcgen05_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFaSmem);
-    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
     if (err != cudaSuccess) return (int)err;
     configured[device] = true;
   }
@@ -792,10 +789,6 @@ TOKB200_API int tokb200_attention_tcgen05(
   if (status == TOKB200_OK) status = fa_map(&map_v, v_pool, pool_rows, (long long)nkv * HEAD_DIM, run ? run : 8);
   if (status != TOKB200_OK) return status;
   const int pairs = nkv * ((nh / nkv + 1) / 2);
-  // With fewer pairs of heads than SMs the halves of a head fill the device better; with more, sharing a block's
-  // keys and values counts (us split / side by side, 12 to 28 heads of 128: 128 pairs 41 / 49, 30 / 31 and
-  // 46 / 49; 256 pairs 81 / 56, 51 / 37 and 143 / 88; 14 heads of 64: 128 pairs 33 / 41, 256 pairs 102 / 71)
-  if (split < 0) split = (long long)pairs * n_tiles < sms[device];
   dim3 grid(split ? nh : pairs, n_tiles);
   // This kernel starts strictly after its predecessor.  Started early (its blocks allocating tensor
   // memory and waiting while the rotary kernel before it still runs), with the product after it

@@ -824,24 +824,45 @@ def attention_tcgen05_supported(nh: int, nkv: int, d: int) -> bool:
     return d in (64, 128) and nh % nkv == 0
 
 
+def attention_tcgen05_split(nh: int, nkv: int, tiles: int, walk: int, sms: int = 148) -> bool:
+    """Whether the tcgen05 attention cuts each head's keys over the two lanes of a block (nh * tiles blocks) instead of
+    giving a block two heads (about half as many blocks, each of which walks as many pairs of 128 keys as the other form
+    in two).  `tiles`: of 128 rows that the step really has; `walk`: the keys that its longest tile sees.
+    A block owns its SM, so what counts is how often the SMs are filled: the cut halves where that is no more often than
+    with two heads a block, and where it is (twice instead of once), when the longest walk is at least five blocks of keys,
+    which then outweighs a second start.  us, cut / two heads, behind cold caches: 14 heads over 2 of 64: one portion of 512
+    12.3 / 16.9 (56 blocks), 1,536 20.6 / 32.6 (168), four of 384 17.5 / 16.0 (168), three of 500 17.5 / 17.7 (168), two of 700
+    18.0 / 20.5 (168), sixteen of 128 18.2 / 13.0 (224); 32 over 8 of 64: 640 15.9 / 18.6 (160), two of 500 19.9 / 17.6 (256),
+    1,024 23.3 / 25.2 (256), 1,536 39.3 / 32.8 (384 against 192); 28 over 4 of 128: 768 24.4 / 27.9 (168), four of 256 24.6 /
+    19.5 (224), five of 200 24.2 / 28.3 (280 against 160), 2,048 70 / 59 (448 against 256); 16 over 4 of 128: two of 700 25.4 /
+    26.0 (192), three of 500 24.1 / 22.6 (192)."""
+    fills = -(-nh * tiles // sms)
+    pairs = nkv * ((nh // nkv + 1) // 2)
+    with_two = -(-pairs * tiles // sms)
+    return fills <= with_two or (fills == 2 and walk > 4 * 128)
+
+
 def attention_tcgen05(q, k_pool, v_pool, out, block_table, row_req, pos, tiles, n_tiles, nh, nkv, d,
                       page, window, scale, sink: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
                       softcap: Optional[float] = None, keep_first: int = 0, split: Optional[bool] = None) -> None:
     """Attention for portions of prompts on tcgen05 (bfloat16, head size 64 or 128).
     `tiles` is int32 [n, 2]: (first row, rows <= 128) of consecutive rows of one request.  `split`: a block
-    takes one head and cuts its keys in two (True) or two heads of a key/value head (False); None: by the
-    amount of work."""
+    takes one head and cuts its keys in two (True) or two heads of a key/value head (False); None: by
+    `attention_tcgen05_split`, all tiles taken for live ones and the tables for the longest walk."""
     if q.dtype != torch.bfloat16:
         raise ValueError("attention_tcgen05 is the bfloat16 kernel")
     if not attention_tcgen05_supported(nh, nkv, d):
         raise ValueError(f"attention_tcgen05: head size {d} is not taken (64 or 128)")
+    if split is None:
+        reach = block_table.shape[1] * page
+        split = attention_tcgen05_split(nh, nkv, n_tiles, reach if window is None else min(reach, int(window) + 128))
     lib = _load("attention_tcgen05.cu", defines=(f"HEAD_DIM={d}",))
     _check(lib.tokb200_attention_tcgen05(
         _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
         _i(block_table.shape[1]), _ptr(row_req), _ptr(pos), _ptr(tiles), _i(n_tiles), _i(q.numel() // (nh * d)),
         _i(k_pool.numel() // (nkv * d)), _i(nh), _i(nkv), _i(d), _i(page), _i(-1 if window is None else int(window)),
         _i(0 if chunk is None else int(chunk)), _i(int(keep_first)), _f(scale), _sink(sink, nh),
-        _f(softcap or 0.0), _i(-1 if split is None else int(split)), _stream()), "attention_tcgen05")
+        _f(softcap or 0.0), _i(int(split)), _stream()), "attention_tcgen05")
 
 
 def attention_tcgen05_check(d: int) -> None:

@@ -147,6 +147,7 @@ class PagedAttention:
 
     graph_safe = True   # launches depend on device-side metadata only
     sink = None
+    window = None       # n: a key is hidden when key + n < query
     chunk = None        # n: keys are seen inside chunks of n positions counted from 0
     keep_first = 0      # a sequence's first keys, seen whatever the window or the chunk says
     softcap = None      # c: a score s counts as c * tanh(s / c)
@@ -161,8 +162,19 @@ class PagedAttention:
         if longest == 1:
             return "single"
         kind = "wide" if longest >= _WIDE_ALWAYS else "middle" if longest >= _WIDE_FROM else "tiles"
+        if longest >= _WIDE_FROM and not self._cut_keys(q_lens):
+            kind += ", two heads a block"
         # portions with single tokens beside them launch the decoding kernel too
         return kind + "+1" if min(q_lens) == 1 else kind
+
+    def _cut_keys(self, q_lens) -> bool:
+        """Whether the tcgen05 kernel cuts a head's keys over a block's two lanes (`ops.attention_tcgen05_split`): by the
+        tiles that the step's portions have, not by the tiles a padded step has room for, and by what both an eager and a
+        replayed step of these portions know, so that they round alike."""
+        portions = [n for n in q_lens if n > 1 or not _SPLIT_MIXED] or list(q_lens)
+        walk = min([max(portions)] + ([self.window + ops.WIDE_TILE_ROWS] if self.window is not None else []) +
+                   ([self.chunk] if self.chunk else []))
+        return ops.attention_tcgen05_split(self.nh, self.nkv, sum(-(-n // ops.WIDE_TILE_ROWS) for n in portions), walk)
 
     def _near(self, ctx, group, tiles) -> bool:
         """Whether portions that the tcgen05 kernel could take are faster on the mma.sync kernel: by sizes that a captured
@@ -205,7 +217,7 @@ class PagedAttention:
                 q, k_pool, v_pool, out, group.block_table, ctx.row_req, ctx.pos,
                 wide[0], wide[1], self.nh, self.nkv, self.d, group.page_size,
                 self.window, self.scale, sink=sink, chunk=self.chunk, softcap=self.softcap,
-                keep_first=self.keep_first)
+                keep_first=self.keep_first, split=self._cut_keys(ctx.q_lens))
             return
         if q.dtype == torch.bfloat16 and tiles is not None and \
                 ops.prefill_attention_supported(self.nh, self.nkv, self.d):
