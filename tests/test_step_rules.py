@@ -67,3 +67,13 @@ def test_where_keys_are_cut(nh, nkv, q_lens, window, cut):
     assert part.shape_key(q_lens).endswith("two heads a block" + ("+1" if 1 in q_lens else "")) is not cut
     assert part.shape_key(q_lens) == part.shape_key(q_lens[::-1])
     assert part.shape_key([n for n in q_lens if n > 1]).endswith("two heads a block") is not cut
+
+
+@pytest.mark.parametrize("nh,nkv,tokens,reach,want", [
+    (14, 2, 1024, 256, True), (32, 8, 256, 256, True), (32, 8, 384, 512, False), (32, 8, 512, 256, False), (64, 8, 128, 128, True),
+    (64, 8, 256, 256, False)])
+def test_near_keys_of_many_heads(monkeypatch, nh, nkv, tokens, reach, want):
+    monkeypatch.setattr(attention.ops, "prefill_attention_supported", lambda *a: True)
+    ctx = SimpleNamespace(max_q_len=96, n_tokens=tokens)
+    group = SimpleNamespace(block_table=torch.empty(1, reach // 16), page_size=16)
+    assert heads_of(nh, nkv)._near(ctx, group, (None, 1)) is want

@@ -127,14 +127,17 @@ _SPLIT_MIXED = os.environ.get("TOKB200_MIXED", "split") != "tiles"
 # portions from this length on go to the tcgen05 kernel (shorter ones would leave most of a
 # 128-row tile empty)
 _WIDE_FROM = 96
-# ... but where heads have 64 lanes, no portion of a small step has _WIDE_ALWAYS tokens and no key lies further back than
-# _NEAR, the mma.sync kernel is the faster one inside a model: it starts while its predecessor still runs, which the
-# tcgen05 kernel must not, and there is little work to make up for that (24 layers of 14 heads over 2, us a step, mma.sync /
-# tcgen05: one portion of 128 tokens 1,071 / 1,185, of 256 1,099 / 1,147, of 384 1,276 / 1,319, of 512 1,352 / 1,356, of 768
-# 1,713 / 1,477; four of 128 1,172 / 1,282, five of 200 1,510 / 1,530, three of 500 2,032 / 1,961)
+# ... but where heads have 64 lanes, no portion of a small step has _WIDE_ALWAYS tokens, no key lies further back than
+# _NEAR and there is little work (heads times rows times keys in reach), the mma.sync kernel is the faster one inside a
+# model or as fast: it starts while its predecessor still runs, which the tcgen05 kernel must not.  us a layer of a
+# captured step, mma.sync / tcgen05: 14 heads over 2, one portion of 128 tokens 44.5 / 47.2, of 256 46.0 / 46.7, of 384 53.2
+# / 52.9, of 512 56.7 / 54.5; four of 128 49.2 / 51.8, five of 200 63.4 / 62.2, eight of 128 59.8 / 60.8; 32 heads over 8,
+# 128 65.1 / 67.4, 256 66.0 / 65.7, 384 82.8 / 78.8.  The kernels alone behind cold caches: 32 heads over 8, 256 9.1 / 9.6,
+# 384 15.5 / 11.3, four of 256 17.1 / 14.1; 64 over 8, 128 6.6 / 8.9, 192 9.7 / 9.5, 256 11.9 / 10.0
 _WIDE_ALWAYS = 385
 _NEAR = 512
 _SMALL_STEP = 1024
+_NEAR_WORK = 14 * 1024 * 256
 
 
 class PagedAttention:
@@ -179,8 +182,9 @@ class PagedAttention:
     def _near(self, ctx, group, tiles) -> bool:
         """Whether portions that the tcgen05 kernel could take are faster on the mma.sync kernel: by sizes that a captured
         step's key holds (its rows, its tables' widths, the lengths' kind)."""
+        reach = group.block_table.shape[1] * group.page_size
         return self.d == 64 and ctx.max_q_len < _WIDE_ALWAYS and ctx.n_tokens <= _SMALL_STEP and tiles is not None and \
-            group.block_table.shape[1] * group.page_size <= _NEAR and \
+            reach <= _NEAR and self.nh * ctx.n_tokens * min(reach, _WIDE_ALWAYS - 1) <= _NEAR_WORK and \
             ops.prefill_attention_supported(self.nh, self.nkv, self.d)
 
     def attend(self, q, out, ctx, group, cache):
