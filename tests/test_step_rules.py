@@ -49,6 +49,21 @@ def test_short_portions_of_near_keys(monkeypatch, longest, tokens, reach, d, wan
     assert (part.shape_key([longest]) == "middle") is (longest < attention._WIDE_ALWAYS)
 
 
+@pytest.mark.parametrize("heads,q_lens,want", [(4, [32], False), (4, [48], False), (4, [64], True), (8, [32], True)])
+def test_delta_rule_of_few_heads(heads, q_lens, want):
+    part = delta(recurrent.GatedDeltaNet, heads)
+    assert part._in_chunks(q_lens) is want and (part.shape_key(q_lens) == "delta_chunks") is want
+
+
+@pytest.mark.parametrize("heads,vdim,q_lens,want", [
+    (8, 128, [128] * 16, False), (16, 64, [128] * 16, False), (16, 128, [128] * 16, True), (16, 32, [128] * 16, True),
+    (4, 128, [128] * 16, True), (16, 16, [128] * 16, True), (8, 128, [512] * 8, True), (16, 128, [128], True)])
+def test_channel_delta_rule_of_short_portions(heads, vdim, q_lens, want):
+    part = delta(recurrent.ChannelDeltaNet, heads)
+    part.vdim = vdim
+    assert part._in_chunks(q_lens) is want and (part.shape_key(q_lens) == "delta_chunks") is want
+
+
 def heads_of(nh, nkv, d=64, window=None, chunk=None):
     part = attention.PagedAttention()
     part.nh, part.nkv, part.d, part.window, part.chunk = nh, nkv, d, window, chunk

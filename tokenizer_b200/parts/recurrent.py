@@ -118,17 +118,34 @@ def stacked_rows(weights, multiple: int = 8):
 # 64 tokens takes 28 us token by token (four a step) and 32 in chunks, 128 tokens 43 / 38; with one a head 32 tokens 32 / 27.
 DELTA_CHUNKS_FROM = 32
 CHANNEL_DELTA_CHUNKS_FROM = 128
+# with one decay a head and fewer heads than this, twice the length: a layer of 4 heads takes 35.8 us token by token for a
+# prompt of 32 tokens, 43.2 for 48 and 49.3 for 64, in chunks 39.1, 44.2 and 44.5; of 8 heads 45.1 and 44.3 for 32
+DELTA_CHUNKS_HEADS = 8
 
 
 def _chunks_pay(q_lens, heads: int, chain: float, work: float) -> bool:
     """Whether chunks of 32 tokens are the faster form of a delta rule for portions of these lengths.  Chunks cost 0.22 us
-    a chunk and head whatever is in it (a lone token too) and never wait for a chain; token by token a step takes `chain`
-    us a token of its longest portion, or `work` us a token and head once the device is full.  Measured for heads of 128 x
-    128, one decay a head / one a channel, us token by token -> in chunks, 16 heads: 2,048 tokens 772 -> 254 / 558 -> 272;
-    512 and 15 single ones 231 -> 114 / 199 -> 124; 512 and 63 single ones 248 -> 309 / 171 -> 320 (not taken); 128 x 4 and
-    8 x 28 154 -> 185 / 116 -> 195 (not taken); eight of 512 with one a channel 494 -> 441."""
+    a chunk and head whatever is in it (a lone token too); their chain, some 2.6 us a chunk of the longest portion, is a
+    quarter of the one token by token and never decides.  Token by token a step takes `chain` us a token of its longest
+    portion, or `work` us a token and head once the device is full.  Fitted to heads of 128 x 128, one decay a head / one a
+    channel, us token by token -> in chunks, 16 heads: 2,048 tokens 772 -> 254 / 558 -> 272; 512 and 15 single ones 231 ->
+    114 / 199 -> 124; 512 and 63 single ones 248 -> 309 / 171 -> 320 (not taken); 128 x 4 and 8 x 28 154 -> 185 / 116 -> 195
+    (not taken); eight of 512 with one a channel 494 -> 441.  Values of fewer lanes make both forms cheaper, and the choice
+    stays right: a layer of 16 heads of 128 x 16, us, eight of 512 394 -> 282 / 470 -> 312, sixteen of 128 174 -> 167 / 223
+    -> 186, one of 128 73 -> 48 / 56 -> 54; of 128 x 64 sixteen of 128 295 -> 227 / 236 -> 245, which `_full_turns` is for."""
     chunks = sum((n + 31) // 32 for n in q_lens)
     return 20.0 + 0.22 * heads * chunks <= 18.0 + max(chain * max(q_lens), work * heads * sum(q_lens))
+
+
+def _full_turns(n_requests: int, heads: int, vdim: int) -> bool:
+    """Whether the blocks of a chunk scan (32 columns of a head's matrix of one request each, one a multiprocessor) fill
+    their last turn on 148 multiprocessors at least half.  With a decay a channel and portions of fewer than 256 tokens, where
+    the two forms are close, an empty last turn is what makes chunks the slower one: sixteen portions of 128, us a layer
+    token by token / in chunks: 512 blocks (3.46 turns) 8 heads of 128 x 128 180 / 191, 16 of 128 x 64 236 / 245, 16 of 72 x
+    64 225 / 236; 1,024 blocks (6.92) 318 / 311; 256 (1.73) 16 heads of 128 x 32 227 / 202, 4 of 128 x 128 144 / 115.  Values
+    that are no whole 32s take blocks of 16 columns, whose turns are short: 32 heads of 128 x 16 339 / 312."""
+    turns = vdim // 32 * heads * n_requests / 148.0
+    return vdim % 32 != 0 or turns <= 1.0 or turns % 1.0 >= 0.5
 
 
 def _delta_chunks(runtime, dim: int, vdim: int) -> bool:
@@ -198,7 +215,8 @@ class GatedDeltaNet:
             not {"TOKB200_GDN_SCAN", "TOKB200_GDN_ROWS"} & set(os.environ)
 
     def _in_chunks(self, q_lens) -> bool:
-        return self.chunked and max(q_lens, default=0) >= DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.34, 0.0115)
+        least = DELTA_CHUNKS_FROM * (1 if self.heads >= DELTA_CHUNKS_HEADS else 2)
+        return self.chunked and max(q_lens, default=0) >= least and _chunks_pay(q_lens, self.heads, 0.34, 0.0115)
 
     def shape_key(self, q_lens):
         longest = max(q_lens)
@@ -327,7 +345,9 @@ class ChannelDeltaNet:
         self.chunked = self.dim_padded == 128 and _delta_chunks(runtime, self.dim, self.vdim)
 
     def _in_chunks(self, q_lens) -> bool:
-        return self.chunked and max(q_lens, default=0) >= CHANNEL_DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.26, 0.0077)
+        longest = max(q_lens, default=0)
+        return self.chunked and longest >= CHANNEL_DELTA_CHUNKS_FROM and _chunks_pay(q_lens, self.heads, 0.26, 0.0077) and \
+            (longest >= 2 * CHANNEL_DELTA_CHUNKS_FROM or _full_turns(len(q_lens), self.heads, self.vdim))
 
     def shape_key(self, q_lens):                                             # the kernels' choice
         return "channel_delta1" if max(q_lens) == 1 else "delta_chunks" if self._in_chunks(q_lens) else "channel_delta"
