@@ -133,8 +133,9 @@ TOKB200_API int tokb200_paged_attention_generic(
 // heads of 64 or 128 lanes.  A block takes a tile and a query head: a chunk's 128 keys and values are staged in shared
 // memory once for the tile's rows instead of being read by every row.  256 threads, 16 x 16: thread (ty, tx) keeps rows
 // 4 ty .. + 3, in the first product keys tx + 16 i (a warp sum's butterfly over 32 keys is then one addition inside the
-// thread and four exchanges), in the second lanes 4 tx .. of the head.  Bound by the FMA pipe, with K of the next chunk
-// on its way during the second product and V during the first.
+// thread and four exchanges), in the second lanes 4 tx .. of the head, with K of the next chunk on its way during the second
+// product and V during the first.  A block an SM, so eight warps: neither pipe is full (777 tokens, 14 heads of 64: FMA 32 %,
+// shared memory 40 %), warps wait for shared memory and for results, and 182 blocks leave most of a second turn empty.
 #define ATT_TILE_ROWS 64
 
 __device__ __forceinline__ void att_copy16(float* dst, const float* src, bool in) {

@@ -18,9 +18,12 @@
 //                         x 128 rows of W and G q meet the columns in 8 x 4 or 8 x 8 register tiles, k cut over the eight
 //                         warps; the next chunk's record is on its way (cp.async) while this one is worked through
 //
-// Both are bound by reads of shared memory: a register tile of R x C costs R + C cycles of the 128 bytes a cycle that come
-// back, and R C / 4 of the multiply-adds.  So tiles are as large as the threads allow, and a row of A is read once for
-// two columns, and half of a scan block's threads own the whole matrix (4 x 4 or 8 x 4 of it each).  Measured (16 heads of
+// The scan is bound by reads of shared memory (counters: the pipe that brings them back busy 62 % of the time, the FMA
+// pipe 36 %): a register tile of R x C costs R + C cycles of the 128 bytes a cycle that come back, and R C / 4 of the
+// multiply-adds.  So tiles are as large as the threads allow, a row of A is read once for two columns, and half of a scan
+// block's threads own the whole matrix (4 x 4 or 8 x 4 of it each).  The prepare kernel waits for instructions most (more
+// than a quarter of its warps' time: a block runs its long unrolled code once), then for registers and shared memory; that
+// pipe is busy 36 % there.  Measured (16 heads of
 // 128 x 128, both kernels and the kept inputs between them, us; before: tiles of 4 x 4, pairs eight tokens at a time): a
 // prompt of 2,048 tokens 294 -> 254 with one decay a head and 328 -> 272 with one a channel, four prompts of 5,100 in all
 // 763 -> 537, eight of 256 316 -> 247.

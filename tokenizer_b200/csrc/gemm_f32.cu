@@ -3,9 +3,10 @@
 // element sums its K products in index order, so a row's result does not depend
 // on how many other rows are in the batch, nor on the tile the element falls into.
 //
-// A block of 16 x 16 threads computes TM * 16 rows x 128 columns, TM x 8 sums a thread.  Bound by the FMA pipe: per step
-// of k a thread reads TM numbers of A and 8 of W, by 16-byte loads and a step ahead of their use, for 8 TM multiply-adds
-// (paired ones, fma.rn.f32x2, measured half as fast).  Operands are staged k-major, 16 of k at a time, the next piece's
+// A block of 16 x 16 threads computes TM * 16 rows x 128 columns, TM x 8 sums a thread.  Per step of k a thread reads TM
+// numbers of A and 8 of W, by 16-byte loads and a step ahead of their use, for 8 TM multiply-adds (paired ones,
+// fma.rn.f32x2, measured half as fast).  Bound by issue: four of five slots are taken, the FMA pipe and the pipe of shared
+// memory are busy 70 % of the time each (counters, 777 x 9,728 x 896, tiles of 128 rows).  Operands are staged k-major, 16 of k at a time, the next piece's
 // global loads in registers while this one is multiplied.
 #include "common.cuh"
 
@@ -138,8 +139,9 @@ static int launch_f32(const float* a, const float* w, const float* bias, float* 
 }
 
 // Few rows, or too few tiles of the kind above for the device: tiles of 4 R rows x 32 columns by 128 threads, a warp's
-// lanes are the columns and each warp keeps R rows (w + 4 i).  Bound by latency at these sizes: pieces of 32 of k come
-// through a ring of cp.async stages, so that several are on their way while one is multiplied.
+// lanes are the columns and each warp keeps R rows (w + 4 i).  With few rows bound by latency: pieces of 32 of k come
+// through a ring of cp.async stages, so that several are on their way while one is multiplied.  With many bound by reads of
+// shared memory (its pipe busy 90 % at 777 x 896 x 4,864 in tiles of 32 rows, the FMA pipe 36 %).
 #define FEW_N 32
 #define FEW_K 32
 #define FEW_THREADS 128

@@ -27,7 +27,7 @@ from .linear import Linear
 _position_tables = {}
 
 # Which kernel takes long prompt portions in bfloat16: the tcgen05 kernel (128-row
-# tiles, scores and outputs in tensor memory; 45 us on 2,048 tokens of 14 heads) or,
+# tiles, scores and outputs in tensor memory; 27 us on 2,048 tokens of 14 heads) or,
 # with TOKB200_ATTENTION=mma, the mma.sync kernel (64-row tiles; 73 us), which also
 # takes the short portions and the head sizes the first does not.
 _PROMPT_KERNEL = os.environ.get("TOKB200_ATTENTION", "tcgen05")
