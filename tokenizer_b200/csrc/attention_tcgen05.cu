@@ -795,7 +795,8 @@ TOKB200_API int tokb200_attention_tcgen05(
   // started early as well, about one step in a hundred of some 1,800 prompt tokens came out with
   // a few rows wrong (bitwise comparison of repeated identical steps; never with either of the
   // two early starts taken away, nor with this kernel alone or between two products).  The cause
-  // has not been found; the early start saved about two microseconds a layer.
+  // has not been found; the early start saved about two microseconds a layer.  All of that was seen with the
+  // kernel's form of one tile and head a block; this one has not been started early.
   return launch_ordered(false, softcap > 0.f ? attention_tcgen05_kernel<true> : attention_tcgen05_kernel<false>, grid,
                         dim3(FA_THREADS), (size_t)kFaSmem, stream, map_q, map_k,
                         map_v, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out,
