@@ -5,6 +5,7 @@ refuses.  There is no CPU path: a tensor that is not on a GPU is an error."""
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -135,7 +136,7 @@ class scratch_scope:
 # loaded; the host reads the word (plain memory, no CUDA call) wherever it has just
 # synchronised with the device, and raises.
 _LIBRARY_NAMES = {1: "gemm_tcgen05", 2: "attention_tcgen05", 3: "ffn_small_m", 4: "linear_stream",
-                  5: "layer_small_m"}
+                  5: "layer_small_m", 6: "gemm_f32_tcgen05"}
 _REASONS = {1: "a wait on a shared-memory barrier ran out", 2: "a wait between blocks ran out"}
 _error_word = None          # (ctypes int at the host address, device address)
 _registered = {}            # id(library handle) -> handle: libraries that know the word
@@ -191,7 +192,7 @@ def raise_if_error(where: str = "") -> None:
     for lib in _registered.values():          # clear the per-library flags too
         for name in ("tokb200_gemm_tcgen05_error", "tokb200_attention_tcgen05_error",
                      "tokb200_ffn_small_m_error", "tokb200_linear_stream_error",
-                     "tokb200_layer_small_m_error"):
+                     "tokb200_layer_small_m_error", "tokb200_gemm_f32_tcgen05_error"):
             try:
                 getattr(lib, name)()
             except AttributeError:
@@ -366,9 +367,36 @@ def paged_attention_f32_tiles(q, k_pool, v_pool, out, block_table, row_req, pos,
         _f(softcap or 0.0), _stream()), "paged_attention_f32_tiles")
 
 
+@functools.lru_cache(maxsize=4096)
+def gemm_f32_tcgen05_plan(M: int, N: int, K: int):
+    """(tile, whether the groups of k go to different blocks, how many groups) for a product of these sizes."""
+    tile, split, groups = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+    status = _lib("gemm_f32_tcgen05").tokb200_gemm_f32_tcgen05_plan(_i(M), _i(N), _i(K), ctypes.byref(tile),
+                                                                    ctypes.byref(split), ctypes.byref(groups))
+    if status != 0:
+        raise ValueError("gemm_f32_tcgen05: " + _STATUS_TEXT.get(status, str(status)))
+    return tile.value, split.value, groups.value
+
+
+def gemm_f32_tcgen05(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+                     tile: Optional[int] = None, split: Optional[bool] = None) -> None:
+    """The product of `gemm_f32` on the tensor cores, its operands as exact sums of three bfloat16 numbers; K a multiple of 4.
+    `tile` and `split` (None: by size) change no bit."""
+    M, K = a.shape
+    N = w.shape[0]
+    planned, cut, groups = gemm_f32_tcgen05_plan(M, N, K)
+    tile, split = planned if tile is None else tile, cut if split is None else split
+    partials = torch.empty((groups, M, N), dtype=torch.float32, device=a.device) if split and groups > 1 else None
+    _check(_lib("gemm_f32_tcgen05").tokb200_gemm_f32_tcgen05(
+        _ptr(a), _ptr(w), _ptr(bias), _ptr(out), _ptr(partials), _i(M), _i(N), _i(K), _i(tile), _i(1 if split else 0),
+        _stream()), "gemm_f32_tcgen05")
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
              out: torch.Tensor, form: Optional[int] = None) -> None:
-    """out[M,N] = a[M,K] w[N,K]^T (+ bias), true 32-bit.  `form`: the tile (all give the same bits); None: by size."""
+    """out[M,N] = a[M,K] w[N,K]^T (+ bias), true 32-bit; a row's bits do not depend on the batch.  `form`: a tile of the
+    kernel of multiply-adds (all give the same bits); None: the tensor cores where k is long enough (a rule on K and the
+    operands' alignment alone, so that a row meets the same kernel in every batch), else that kernel's tile by size."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N):
@@ -376,6 +404,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
     for t in (a, w, out):
         if t.dtype != torch.float32:
             raise ValueError("gemm_f32 takes float32")
+    if form is None and K >= 768 and K % 4 == 0 and M > 0 and N > 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0:
+        gemm_f32_tcgen05(a, w, bias, out)
+        return
     _check(_lib("gemm_f32").tokb200_gemm_f32(
         _ptr(a), _ptr(w), _ptr(bias), _ptr(out), _i(M), _i(N), _i(K), _i(K), _i(N),
         _i(-1 if form is None else int(form)), _stream()), "gemm_f32")

@@ -10,6 +10,7 @@ def all_variants():
         ("elementwise.cu", (), ()),
         ("attention_generic.cu", (), ()),
         ("gemm_f32.cu", (), ()),
+        ("gemm_f32_tcgen05.cu", (), ()),
         ("sampling.cu", (), ()),
         ("linear_small_m.cu", (), ()),
         ("gemm_tcgen05.cu", (), ()),
