@@ -26,10 +26,10 @@
 //     memory as bfloat16.  The accumulator stays in tensor memory over the whole walk; the reference maximum
 //     follows the true one lazily: only when the maximum has grown by more than 2^8 since it was set are the
 //     sum and the accumulator rescaled, which happens a few times per row; probabilities stay below 2^8.
-// Measured (28 heads over 4 of 128 lanes, one prompt, us): 8,192 tokens 1,547 -> 547 (311 -> 880 TFLOP/s), 2,048 126 ->
-// 58; 14 heads over 2 of 64: 346 -> 223 and 36.8 -> 27.3.  The form before it took one tile and one head a block, and its
+// Measured (28 heads over 4 of 128 lanes, one prompt, us): 8,192 tokens 1,547 -> 456 (311 -> 1,054 TFLOP/s), 2,048 126 ->
+// 47; 14 heads over 2 of 64: 346 -> 198 and 36.8 -> 24.7.  The form before it took one tile and one head a block, and its
 // loader waited for a block's copies before it asked for the next.  What bounds it now: a step of the two lanes takes
-// 5,000 cycles at 128 lanes, of which the tensor core 2,300 and each lane's softmax 1,900 (the exponentials alone 1,024 of
+// 4,200 cycles at 128 lanes, of which the tensor core 2,300 and each lane's softmax 1,900 (the exponentials alone 1,024 of
 // MUFU), the rest the hand-offs between them; scores asked for while the softmax still runs (probabilities through shared
 // memory at 128 lanes) measured slower, 590 us: both lanes' softmaxes then run at once and slow one another.
 // Everything but q, k, v, p and the output is 32-bit.  Every wait is bounded; when one runs out an error flag
@@ -265,7 +265,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int kvh = split_all ? blockIdx.x / group : blockIdx.x / pairs;
   const int h0 = split_all ? blockIdx.x : kvh * group + (blockIdx.x % pairs) * 2;
   const bool split = split_all || h0 + 1 == (kvh + 1) * group;     // a group's odd head is split
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // through a shuffle, so that the compiler can see it is the same for the whole warp: the roles are then no divergent
+  // branches and may keep such values in uniform registers (28 heads of 128, 8,192
+  // tokens: 548 -> 456 us, 2,048: 58 -> 47; 14 heads of 64, 2,048 tokens: 27.6 -> 24.7)
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // What needs nothing of the step comes first: the trips to memory for the step's rows, one behind the other, then lie
   // beside the maps' way into the SM and the claim on tensor memory, not in front of them.
   constexpr int kMmaWarp = FA_SOFTMAX_WARPS + FA_LOADER_WARPS;
@@ -324,7 +327,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_base = *tmem_slot;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();
 
   if (live && warp >= FA_SOFTMAX_WARPS && warp < kMmaWarp) {
