@@ -367,6 +367,16 @@ struct QkvEpilogue {
   int nh, nkv, d;
 };
 
+// A product over groups of rows (routed experts): what stands in a unit of work says where its rows, its piece of the
+// weight and its output lie.  `units` and their number are on the device, written by the kernel that sorts the rows.
+struct GroupedWork {
+  const int4* units;            // gate/up: first row, first gate row of W, first output column, output columns that count;
+                                // down: first row, first column of W, first output column, blocks of 64 of k
+  const int* count;
+  int up_at;                    // gate/up: W's row of a gate row's up row lies this far behind it
+  const float* share;           // gate/up: what a row's output is multiplied by
+};
+
 // GATED: the weight rows come in blocks of 256 = 128 "gate" rows followed by the 128
 // "up" rows of the same outputs; the epilogue writes silu(gate) * up, 128 columns a
 // tile, and the 2 N wide product never goes to memory.
@@ -374,13 +384,15 @@ struct QkvEpilogue {
 // q and k by each row's position (half-split pairs (j, j + d/2), the whole head) and writes q to
 // its matrix (TMA store) and k and v to the rows' cache slots, so the stacked product never goes
 // to memory.  Tiles of 128 columns hold whole heads (d = 64 or 128) of one kind.
-template <int BLOCK_N, int STAGES, bool OUT_F32, bool GATED, bool QKV = false, bool PAIR = false>
+// GROUPED (pairs alone): CTA 0 loads a unit's gate rows and CTA 1 its up rows, which lie apart in the stacked weight; of the
+// down product (32-bit output) a unit's k is its expert's lanes.
+template <int BLOCK_N, int STAGES, bool OUT_F32, bool GATED, bool QKV = false, bool PAIR = false, bool GROUPED = false>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
                                const __grid_constant__ CUtensorMap map_w,
                                const __grid_constant__ CUtensorMap map_out,
                                const float* __restrict__ bias, int M, int N, int K, int k_splits,
-                               const QkvEpilogue qkv) {
+                               const QkvEpilogue qkv, const GroupedWork grouped) {
   static_assert(!QKV || (BLOCK_N == 128 && !OUT_F32 && !GATED), "the QKV epilogue works on 128-column bfloat16 tiles");
   // k_splits > 1 (32-bit output only): a unit of work is (tile, piece of k); the output is
   // [k_splits, M, N] partial sums that the consumer adds in index order, written through a
@@ -388,6 +400,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
   using S = TcPersistentSmem<BLOCK_N, STAGES, OUT_F32, GATED, PAIR>;
   static_assert(!GATED || (BLOCK_N == 256 && !OUT_F32), "the gated epilogue pairs two halves of a 256 tile");
   static_assert(!PAIR || !QKV, "the QKV epilogue has no pair form");
+  static_assert(!GROUPED || (PAIR && GATED != OUT_F32), "groups of rows: the gated and the 32-bit product of pairs");
   // PAIR: the grid is clusters of two CTAs; a tile has 256 rows, of which this CTA owns 128
   constexpr int kTileM = PAIR ? 2 * TC_BLOCK_M : TC_BLOCK_M;
   const int rank = PAIR ? (int)cluster_rank() : 0;
@@ -409,7 +422,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
   const int total_tiles = m_tiles * n_tiles;
   const int k_blocks = (K + TC_BLOCK_K - 1) / TC_BLOCK_K;
   const int kb_per_split = (k_blocks + k_splits - 1) / k_splits;
-  const int total_units = total_tiles * k_splits;
+  int total_units = total_tiles * k_splits;
 
   if (threadIdx.x == 0) {
     // PAIR: the loads of both CTAs count on CTA 0's "full"; a commit arrives on "empty" and
@@ -435,16 +448,20 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem_base = *tmem_slot;
   pdl_wait();
+  if (GROUPED) total_units = *grouped.count;
 
   if (warp == 0) {
     if (lane == 0) {
       int it = 0;                                   // k blocks issued so far, over all tiles
       bool ok = true;
       for (int unit = worker; ok && unit < total_units; unit += workers) {
-        const int tile = unit % total_tiles, split = unit / total_tiles;
-        const int m0 = (tile % m_tiles) * kTileM + rank * TC_BLOCK_M;
-        const int n0 = (tile / m_tiles) * BLOCK_N + (PAIR ? rank * (BLOCK_N / 2) : 0);
-        const int kb_end = min(k_blocks, (split + 1) * kb_per_split);
+        const int4 what = GROUPED ? grouped.units[unit] : int4();
+        const int tile = GROUPED ? 0 : unit % total_tiles, split = GROUPED ? 0 : unit / total_tiles;
+        const int m0 = GROUPED ? what.x + rank * TC_BLOCK_M : (tile % m_tiles) * kTileM + rank * TC_BLOCK_M;
+        const int n0 = GROUPED ? (GATED ? what.y + rank * grouped.up_at : what.z + rank * (BLOCK_N / 2))
+                               : (tile / m_tiles) * BLOCK_N + (PAIR ? rank * (BLOCK_N / 2) : 0);
+        const int w_k0 = GROUPED && !GATED ? what.y : 0;
+        const int kb_end = GROUPED ? (GATED ? k_blocks : what.w) : min(k_blocks, (split + 1) * kb_per_split);
         for (int kb = split * kb_per_split; kb < kb_end; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1)) { ok = false; break; }   // fresh barriers pass
@@ -453,7 +470,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
             if (rank == 0) mbar_expect_tx(&full[s], 2 * S::kStage);      // the bytes of both CTAs
             const unsigned bar = leader_address(&full[s]);
             tma_load_2d_pair(a_tile, &map_x, bar, kb * TC_BLOCK_K, m0);
-            tma_load_2d_pair(a_tile + S::kABytes, &map_w, bar, kb * TC_BLOCK_K, n0);
+            tma_load_2d_pair(a_tile + S::kABytes, &map_w, bar, w_k0 + kb * TC_BLOCK_K, n0);
           } else {
             mbar_expect_tx(&full[s], S::kStage);
             tma_load_2d(a_tile, &map_x, &full[s], kb * TC_BLOCK_K, m0);
@@ -469,8 +486,9 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
       int it = 0, round = 0;
       bool ok = true;
       for (int unit = worker; ok && unit < total_units; unit += workers, ++round) {
-        const int split = unit / total_tiles;
-        const int kb_begin = split * kb_per_split, kb_end = min(k_blocks, kb_begin + kb_per_split);
+        const int split = GROUPED ? 0 : unit / total_tiles;
+        const int kb_begin = split * kb_per_split;
+        const int kb_end = GROUPED ? (GATED ? k_blocks : grouped.units[unit].w) : min(k_blocks, kb_begin + kb_per_split);
         const int buf = round & 1;
         // the epilogue (of both CTAs) has drained it
         if (!(PAIR ? mbar_wait_cluster(&acc_empty[buf], ((round >> 1) & 1) ^ 1)
@@ -504,8 +522,11 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
     const bool issuer = warp == 2 && lane == 0;     // the thread that issues the TMA stores
     int round = 0;
     for (int unit = worker; unit < total_units; unit += workers, ++round) {
-      const int tile = unit % total_tiles, split = unit / total_tiles;
-      const int m0 = (tile % m_tiles) * kTileM + rank * TC_BLOCK_M, n0 = (tile / m_tiles) * BLOCK_N;
+      const int4 what = GROUPED ? grouped.units[unit] : int4();
+      const int tile = GROUPED ? 0 : unit % total_tiles, split = GROUPED ? 0 : unit / total_tiles;
+      const int m0 = GROUPED ? what.x + rank * TC_BLOCK_M : (tile % m_tiles) * kTileM + rank * TC_BLOCK_M;
+      const int n0 = GROUPED ? (GATED ? 2 * what.z : what.z) : (tile / m_tiles) * BLOCK_N;
+      const float share = GROUPED && GATED ? grouped.share[m0 + r] : 1.f;
       const int buf = round & 1;
       if (!mbar_wait(&acc_full[buf], (round >> 1) & 1)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -613,7 +634,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
               const bool silu = qkv.activation == TOKB200_ACT_SILU;     // uniform over the grid
               const float a0 = silu ? __fdividef(g0, 1.0f + __expf(-g0)) : gate_activation(qkv.activation, g0);
               const float a1 = silu ? __fdividef(g1, 1.0f + __expf(-g1)) : gate_activation(qkv.activation, g1);
-              __nv_bfloat162 pair = __floats2bfloat162_rn(a0 * u0, a1 * u1);
+              __nv_bfloat162 pair = GROUPED ? __floats2bfloat162_rn(a0 * u0 * share, a1 * u1 * share)
+                                            : __floats2bfloat162_rn(a0 * u0, a1 * u1);
               ow[e] = *reinterpret_cast<unsigned*>(&pair);
             }
             *reinterpret_cast<uint4*>(slab + (((piece0 + j) ^ (r & 7)) << 4)) = o;
@@ -675,7 +697,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
         if (GATED) {   // the tile's 128 output columns start at n0 / 2
 #pragma unroll 1
           for (int sl = 0; sl < 2; ++sl)
-            if (n0 / 2 + sl * 64 < N / 2)
+            if (GROUPED ? sl * 64 < what.w : n0 / 2 + sl * 64 < N / 2)
               tma_store_2d(&map_out, staging + sl * S::kSlabBytes, n0 / 2 + sl * 64, m0);
         } else if (!QKV || n0 < qkv.nh * qkv.d) {
 #pragma unroll 1
@@ -765,14 +787,16 @@ static int make_out_map(CUtensorMap* map, void* base, long long M, long long N, 
   return r == CUDA_SUCCESS ? TOKB200_OK : TOKB200_BAD_ALIGNMENT;
 }
 
-template <int BLOCK_N, int STAGES, bool OUT_F32, bool GATED = false, bool QKV = false, bool PAIR = false>
+// `grouped`: M rows of x, N rows of W and K its columns; x's rows are `x_k` wide (0: K), the output's `out_n` (0: by N)
+template <int BLOCK_N, int STAGES, bool OUT_F32, bool GATED = false, bool QKV = false, bool PAIR = false, bool GROUPED = false>
 static int launch_tc_persistent(const void* x, const void* w, const float* bias, void* out, int M, int N,
                                 int K, cudaStream_t stream, int k_splits = 1,
-                                const QkvEpilogue* qkv_in = nullptr, int activation = TOKB200_ACT_NONE) {
+                                const QkvEpilogue* qkv_in = nullptr, int activation = TOKB200_ACT_NONE,
+                                const GroupedWork* grouped_in = nullptr, int x_k = 0, int out_n = 0) {
   using S = TcPersistentSmem<BLOCK_N, STAGES, OUT_F32, GATED, PAIR>;
   static_assert(S::kTotal <= 227 * 1024, "shared memory of one CTA");
   CUtensorMap map_x, map_w, map_out;
-  int status = make_map(&map_x, x, M, K, TC_BLOCK_M);
+  int status = make_map(&map_x, x, M, x_k ? x_k : K, TC_BLOCK_M);
   if (status != TOKB200_OK) return status;
   status = make_map(&map_w, w, N, K, PAIR ? BLOCK_N / 2 : BLOCK_N);      // a pair's CTA loads half the rows
   if (status != TOKB200_OK) return status;
@@ -780,13 +804,15 @@ static int launch_tc_persistent(const void* x, const void* w, const float* bias,
   QkvEpilogue qkv = {};
   if (QKV) qkv = *qkv_in;
   qkv.activation = activation;
-  status = make_out_map(&map_out, out, M, GATED ? N / 2 : (QKV ? (long long)qkv.nh * qkv.d : N), OUT_F32, k_splits);
+  GroupedWork grouped = {};
+  if (GROUPED) grouped = *grouped_in;
+  status = make_out_map(&map_out, out, M, out_n ? out_n : GATED ? N / 2 : (QKV ? (long long)qkv.nh * qkv.d : N), OUT_F32, k_splits);
   if (status != TOKB200_OK) return status;
   static bool configured[64] = {};
   static int sm_count[64] = {};
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return TOKB200_BAD_SIZE;
-  auto kernel = gemm_tcgen05_persistent_kernel<BLOCK_N, STAGES, OUT_F32, GATED, QKV, PAIR>;
+  auto kernel = gemm_tcgen05_persistent_kernel<BLOCK_N, STAGES, OUT_F32, GATED, QKV, PAIR, GROUPED>;
   if (!configured[device]) {
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (err != cudaSuccess) return (int)err;
@@ -795,11 +821,12 @@ static int launch_tc_persistent(const void* x, const void* w, const float* bias,
     configured[device] = true;
   }
   const int tile_m = PAIR ? 2 * TC_BLOCK_M : TC_BLOCK_M;
-  const int tiles = ((M + tile_m - 1) / tile_m) * ((N + BLOCK_N - 1) / BLOCK_N) * k_splits;
+  // grouped: how many units there are only the device knows, every pair comes
+  const int tiles = GROUPED ? 1 << 30 : ((M + tile_m - 1) / tile_m) * ((N + BLOCK_N - 1) / BLOCK_N) * k_splits;
   if (!PAIR) {
     dim3 grid(tiles < sm_count[device] ? tiles : sm_count[device]);
     return launch_dependent(kernel, grid, dim3(TC_THREADS), (size_t)S::kTotal, stream, map_x, map_w, map_out,
-                            bias, M, N, K, k_splits, qkv);
+                            bias, M, N, K, k_splits, qkv, grouped);
   }
   // clusters of two CTAs, one cluster per pair of SMs at most
   const int pairs = sm_count[device] / 2;
@@ -821,7 +848,7 @@ static int launch_tc_persistent(const void* x, const void* w, const float* bias,
   attribute[1].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 2;
-  cudaError_t err = cudaLaunchKernelEx(&config, kernel, map_x, map_w, map_out, bias, M, N, K, k_splits, qkv);
+  cudaError_t err = cudaLaunchKernelEx(&config, kernel, map_x, map_w, map_out, bias, M, N, K, k_splits, qkv, grouped);
   return err == cudaSuccess ? TOKB200_OK : (int)err;
 }
 
@@ -936,6 +963,31 @@ TOKB200_API int tokb200_gemm_tcgen05_pair(const void* x, const void* w, const fl
       return launch_tc_persistent<128, 6, false, false, false, true>(x, w, bias, out, M, N, K, stream, 1, nullptr, activation);
     default: return TOKB200_BAD_SIZE;
   }
+}
+
+// The two products of routed experts over rows sorted by expert (see moe.cu for the units).
+// gate/up: act[rows, width] = share * f(x Wg^T) * (x Wu^T), w [2 inner, hidden] with the up rows `inner` behind the gate rows.
+TOKB200_API int tokb200_gemm_tcgen05_grouped_gated(const void* x, const void* w, void* act, const int* units, const int* count,
+                                                   const float* share, int rows, int inner, int hidden, int width,
+                                                   int activation, cudaStream_t stream) {
+  if (rows <= 0) return TOKB200_OK;
+  if (rows % 256 || inner <= 0 || hidden <= 0 || hidden % 8 || width <= 0 || width % 8 || activation < 0 ||
+      activation >= TOKB200_ACT_COUNT)
+    return TOKB200_BAD_SIZE;
+  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)act | (uintptr_t)units) & 15) return TOKB200_BAD_ALIGNMENT;
+  const GroupedWork work = {(const int4*)units, count, inner, share};
+  return launch_tc_persistent<256, 6, false, true, false, true, true>(x, w, nullptr, act, rows, 2 * inner, hidden, stream, 1,
+                                                                      nullptr, activation, &work, 0, width);
+}
+// down: out[rows, hidden] (32-bit) = act[rows, width] W^T over the unit's lanes, w [hidden, inner].
+TOKB200_API int tokb200_gemm_tcgen05_grouped_down(const void* act, const void* w, void* out, const int* units, const int* count,
+                                                  int rows, int inner, int hidden, int width, cudaStream_t stream) {
+  if (rows <= 0) return TOKB200_OK;
+  if (rows % 256 || inner <= 0 || inner % 8 || hidden <= 0 || hidden % 4 || width <= 0 || width % 8) return TOKB200_BAD_SIZE;
+  if (((uintptr_t)act | (uintptr_t)w | (uintptr_t)out | (uintptr_t)units) & 15) return TOKB200_BAD_ALIGNMENT;
+  const GroupedWork work = {(const int4*)units, count, 0, nullptr};
+  return launch_tc_persistent<256, 5, true, false, false, true, true>(act, w, nullptr, out, rows, hidden, inner, stream, 1,
+                                                                      nullptr, TOKB200_ACT_NONE, &work, width);
 }
 
 // out[M, N/2] = act(x Wg^T) * (x Wu^T) where w [N, K] holds, for every 128 outputs,

@@ -361,3 +361,219 @@ TOKB200_API int tokb200_moe_gate(const void* gu, const float* share, void* out, 
                             on_input, share_ld);
   return TOKB200_BAD_DTYPE;
 }
+
+// ---- a prompt's rows sorted by expert --------------------------------------------------------------------------------
+// The dense form above computes every expert for every token: experts / top times the arithmetic, at the rate of one large
+// product.  From some hundred rows on the chosen rows alone are worth their sorting (rows in whole tiles of 256 a group, the
+// shared expert's group, all tokens, first):
+//   moe_rank      a block an expert: its tokens in order, and every token's place among them
+//   moe_gather    the rows' copies group by group, their shares, and the units of work of the two products
+//                 (`GroupedWork` in gemm_tcgen05.cu)
+//   moe_combine   a token's rows of the down product, added up in 32-bit in the order of the experts, the shared one first
+// 2,048 tokens x 2,048, two of eight experts of 1,408 lanes and a shared one of 2,816 (us): products and gate 249 -> 135 with
+// the three kernels in it.
+#define MOE_GROUP_ROWS 256
+#define MOE_GROUPED_EXPERTS 128
+
+struct MoeSort {
+  const float* share;       // [T, share_ld]; not chosen: 0
+  int share_ld, tokens, experts, ff, shared, hidden;
+  int* count;               // [experts]
+  int* list;                // [experts, T]: an expert's tokens
+  int* rank;                // [experts, T]: a token's place among them, or -1
+  int* first;               // [experts + 1]: a group's first row (experts: the shared one's)
+  int* totals;              // units of the gate/up and of the down product
+  int4* gate_units;
+  int4* down_units;
+};
+
+__global__ void __launch_bounds__(1024) moe_rank_kernel(const MoeSort a) {
+  __shared__ int warps_s[33];
+  const int e = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_launch();
+  int before = 0;
+  for (int t0 = 0; t0 < a.tokens; t0 += 1024) {
+    const int t = t0 + threadIdx.x;
+    const bool chosen = t < a.tokens && !(a.share[(size_t)t * a.share_ld + e] == 0.f);
+    const unsigned votes = __ballot_sync(0xffffffffu, chosen);
+    __syncthreads();
+    if (lane == 0) warps_s[warp] = __popc(votes);
+    __syncthreads();
+    int mine = 0, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int n = warps_s[w];
+      mine += w < warp ? n : 0;
+      all += n;
+    }
+    const int place = before + mine + __popc(votes & ((1u << lane) - 1u));
+    if (t < a.tokens) a.rank[(size_t)e * a.tokens + t] = chosen ? place : -1;
+    if (chosen) a.list[(size_t)e * a.tokens + place] = t;
+    before += all;
+  }
+  if (threadIdx.x == 0) a.count[e] = before;
+}
+
+// A warp a row; block 0 writes the units too.
+__global__ void __launch_bounds__(256) moe_gather_kernel(const MoeSort a, const uint4* __restrict__ h, uint4* __restrict__ x,
+                                                         float* __restrict__ row_share, int max_rows) {
+  __shared__ int first_s[MOE_GROUPED_EXPERTS + 2], count_s[MOE_GROUPED_EXPERTS + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_launch();
+  for (int e = threadIdx.x; e < a.experts; e += blockDim.x) count_s[e] = a.count[e];
+  __syncthreads();
+  // group 0 is the shared expert's (none: no rows), group 1 + e expert e's
+  if (warp == 0) {
+    int at = a.shared ? (a.tokens + MOE_GROUP_ROWS - 1) / MOE_GROUP_ROWS : 0;
+    if (lane == 0) first_s[0] = 0;
+    for (int e0 = 0; e0 < a.experts; e0 += 32) {
+      const int tiles = e0 + lane < a.experts ? (count_s[e0 + lane] + MOE_GROUP_ROWS - 1) / MOE_GROUP_ROWS : 0;
+      int sum = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int got = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += got;
+      }
+      // never behind the buffers' end, whatever the shares hold
+      if (e0 + lane < a.experts) first_s[1 + e0 + lane] = min((at + sum - tiles) * MOE_GROUP_ROWS, max_rows);
+      at += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) first_s[1 + a.experts] = min(at * MOE_GROUP_ROWS, max_rows);
+  }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    for (int e = threadIdx.x; e <= a.experts; e += blockDim.x) a.first[e] = first_s[e < a.experts ? 1 + e : 0];
+    int gate_at = 0, down_at = 0;
+    const int down_columns = (a.hidden + 255) / 256;
+    for (int g = 0; g <= a.experts; ++g) {
+      const int tiles = (first_s[g + 1] - first_s[g]) / MOE_GROUP_ROWS, width = g == 0 ? a.shared : a.ff;
+      const int lanes = g == 0 ? a.experts * a.ff : (g - 1) * a.ff, columns = (width + 127) / 128;
+      for (int i = threadIdx.x; i < tiles * columns; i += blockDim.x) {
+        const int c = i / tiles * 128;
+        a.gate_units[gate_at + i] = make_int4(first_s[g] + i % tiles * MOE_GROUP_ROWS, lanes + c, c, min(128, width - c));
+      }
+      for (int i = threadIdx.x; i < tiles * down_columns; i += blockDim.x)
+        a.down_units[down_at + i] = make_int4(first_s[g] + i % tiles * MOE_GROUP_ROWS, lanes, i / tiles * 256, width / 64);
+      gate_at += tiles * columns;
+      down_at += tiles * down_columns;
+    }
+    if (threadIdx.x == 0) { a.totals[0] = gate_at; a.totals[1] = down_at; }
+  }
+  const int row = blockIdx.x * 8 + warp;
+  if (row >= max_rows || row >= first_s[a.experts + 1]) return;
+  int g = 0;                                              // the group whose rows lie around this one: the last that begins at or before it
+  for (int e0 = 0; e0 < a.experts; e0 += 32)
+    g += __popc(__ballot_sync(0xffffffffu, e0 + lane < a.experts && first_s[1 + e0 + lane] <= row));
+  // groups without rows begin where the next one does and are never the last
+  const int at = row - first_s[g];
+  if (at >= (g == 0 ? a.tokens : count_s[g - 1])) {      // behind a group's last row: nobody reads what becomes of it
+    if (lane == 0) row_share[row] = 0.f;
+    return;
+  }
+  const int t = g == 0 ? at : a.list[(size_t)(g - 1) * a.tokens + at];
+  const int pieces = a.hidden / 8;
+  for (int i = lane; i < pieces; i += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if (i + 32 * j < pieces) v[j] = h[(size_t)t * pieces + i + 32 * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if (i + 32 * j < pieces) x[(size_t)row * pieces + i + 32 * j] = v[j];
+  }
+  if (lane == 0) row_share[row] = a.share[(size_t)t * a.share_ld + (g == 0 ? a.experts : g - 1)];
+}
+
+// A block a token, four columns a thread at a time.
+__global__ void __launch_bounds__(256) moe_combine_kernel(const MoeSort a, const float* __restrict__ rows,
+                                                          __nv_bfloat16* __restrict__ out, int max_rows) {
+  __shared__ int from_s[MOE_GROUPED_EXPERTS + 1];
+  __shared__ int n_s;
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_launch();
+  if (threadIdx.x < 32) {
+    int n = a.shared ? 1 : 0;
+    if (a.shared && lane == 0) from_s[0] = a.first[a.experts] + t;
+    for (int e0 = 0; e0 < a.experts; e0 += 32) {
+      const int place = e0 + lane < a.experts ? a.rank[(size_t)(e0 + lane) * a.tokens + t] : -1;
+      const unsigned votes = __ballot_sync(0xffffffffu, place >= 0);
+      if (place >= 0) from_s[n + __popc(votes & ((1u << lane) - 1u))] = min(a.first[e0 + lane] + place, max_rows - 1);
+      n += __popc(votes);
+    }
+    if (lane == 0) n_s = n;
+  }
+  __syncthreads();
+  const int n = n_s;
+  for (int c = threadIdx.x * 4; c < a.hidden; c += 1024) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(rows + (size_t)from_s[i] * a.hidden + c);
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(sum.x, sum.y), __floats2bfloat162_rn(sum.z, sum.w)};
+    *reinterpret_cast<uint2*>(out + (size_t)t * a.hidden + c) = *reinterpret_cast<uint2*>(o);
+  }
+}
+
+// Rows that `tokens` tokens of `top` experts each can take, whole tiles a group.
+static long long moe_grouped_rows(int tokens, int experts, int top, int shared) {
+  const long long tile = MOE_GROUP_ROWS, groups = experts < (long long)tokens * top ? experts : (long long)tokens * top;
+  return ((long long)tokens * top / tile + groups + (shared ? (tokens + tile - 1) / tile : 0)) * tile;
+}
+static MoeSort moe_sort_args(const float* share, int share_ld, int tokens, int experts, int top, int ff, int shared, int hidden,
+                             int* scratch) {
+  const long long tiles = moe_grouped_rows(tokens, experts, top, shared) / MOE_GROUP_ROWS;
+  const int widest = ff > shared ? ff : shared;
+  MoeSort a = {share, share_ld, tokens, experts, ff, shared, hidden};
+  a.gate_units = (int4*)scratch;                          // on 16 bytes, as the scratch is
+  a.down_units = a.gate_units + tiles * ((widest + 127) / 128);
+  a.totals = (int*)(a.down_units + tiles * ((hidden + 255) / 256));
+  a.count = a.totals + 4;
+  a.first = a.count + experts;
+  a.list = a.first + experts + 1;
+  a.rank = a.list + (long long)experts * tokens;
+  return a;
+}
+static bool moe_sort_takes(int tokens, int experts, int top, int ff, int shared, int hidden) {
+  return tokens > 0 && experts > 0 && experts <= MOE_GROUPED_EXPERTS && top > 0 && top <= experts && ff > 0 && ff % 64 == 0 &&
+         shared >= 0 && shared % 64 == 0 && hidden > 0 && hidden % 8 == 0 &&
+         moe_grouped_rows(tokens, experts, top, shared) <= 128LL * 65535;
+}
+
+// Sizes of the buffers of the sorted form: rows, ints of scratch, where in it the units of the two products and their
+// numbers lie (in ints).
+TOKB200_API int tokb200_moe_sort_sizes(int tokens, int experts, int top, int ff, int shared, int hidden, long long* rows,
+                                       long long* ints, long long* gate_at, long long* down_at, long long* totals_at) {
+  if (!moe_sort_takes(tokens, experts, top, ff, shared, hidden)) return TOKB200_BAD_SIZE;
+  *rows = moe_grouped_rows(tokens, experts, top, shared);
+  int* const zero = nullptr;
+  const MoeSort a = moe_sort_args(nullptr, 0, tokens, experts, top, ff, shared, hidden, zero);
+  auto at = [&](const void* p) { return (long long)((uintptr_t)p / sizeof(int)); };
+  *gate_at = at(a.gate_units);
+  *down_at = at(a.down_units);
+  *totals_at = at(a.totals);
+  *ints = at(a.rank) + (long long)experts * tokens;
+  return TOKB200_OK;
+}
+
+TOKB200_API int tokb200_moe_sort(const void* h, const float* share, int share_ld, int tokens, int experts, int top, int ff,
+                                 int shared, int hidden, int* scratch, void* x, float* row_share, cudaStream_t stream) {
+  if (!moe_sort_takes(tokens, experts, top, ff, shared, hidden) || share_ld < experts + (shared ? 1 : 0)) return TOKB200_BAD_SIZE;
+  if (((uintptr_t)h | (uintptr_t)scratch | (uintptr_t)x) & 15) return TOKB200_BAD_ALIGNMENT;
+  const MoeSort a = moe_sort_args(share, share_ld, tokens, experts, top, ff, shared, hidden, scratch);
+  const int status = launch_dependent(moe_rank_kernel, dim3(experts), dim3(1024), 0, stream, a);
+  if (status != TOKB200_OK) return status;
+  const int rows = (int)moe_grouped_rows(tokens, experts, top, shared);
+  return launch_dependent(moe_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, a, (const uint4*)h, (uint4*)x,
+                          row_share, rows);
+}
+
+TOKB200_API int tokb200_moe_combine(const float* rows, int tokens, int experts, int top, int ff, int shared, int hidden,
+                                    int* scratch, void* out, cudaStream_t stream) {
+  if (!moe_sort_takes(tokens, experts, top, ff, shared, hidden)) return TOKB200_BAD_SIZE;
+  if (((uintptr_t)rows | (uintptr_t)scratch | (uintptr_t)out) & 15) return TOKB200_BAD_ALIGNMENT;
+  const MoeSort a = moe_sort_args(nullptr, 0, tokens, experts, top, ff, shared, hidden, scratch);
+  return launch_dependent(moe_combine_kernel, dim3(tokens), dim3(256), 0, stream, a, rows, (__nv_bfloat16*)out,
+                          (int)moe_grouped_rows(tokens, experts, top, shared));
+}

@@ -1600,6 +1600,69 @@ def moe_gate(gu: torch.Tensor, share: torch.Tensor, out: torch.Tensor, experts: 
            "moe_gate")
 
 
+@functools.lru_cache(maxsize=1024)
+def _moe_sort_sizes(tokens: int, experts: int, top: int, ff: int, shared: int, hidden: int):
+    sizes = [ctypes.c_longlong(0) for _ in range(5)]
+    status = _lib("moe").tokb200_moe_sort_sizes(_i(tokens), _i(experts), _i(top), _i(ff), _i(shared), _i(hidden),
+                                                *[ctypes.byref(n) for n in sizes])
+    return None if status != 0 else tuple(n.value for n in sizes)
+
+
+def moe_grouped_supported(tokens: int, experts: int, top: int, ff: int, shared: int, hidden: int, activation: str) -> bool:
+    """Whether `moe_grouped` takes these sizes: up to 128 experts, inner sizes in whole 64s, an activation of `ACTIVATIONS`."""
+    return activation in ACTIVATIONS and _moe_sort_sizes(tokens, experts, top, ff, shared, hidden) is not None
+
+
+def moe_grouped_pays(tokens: int, experts: int, top: int, ff: int, shared: int, hidden: int) -> bool:
+    """Whether sorted rows take less time than every expert's lanes for every token, by the sizes: the arithmetic at 1,450
+    TFLOP/s and a sixth more for the gate's pass, against 1,150 TFLOP/s over whole tiles of 256 rows (half a tile empty a
+    group) and 45 us, which are the sorting, the adding up and products too small to fill the device.  Measured, dense /
+    sorted us: two of eight experts of 1,408 lanes, one shared of 2,816, hidden 2,048: 400 tokens 77 / 78, 800 117 / 89,
+    2,048 254 / 147; half of these sizes: 800 44 / 44, 1,200 58 / 60, 2,048 80 / 65; eight of 64 of 512, hidden 1,024: 400
+    98 / 110, 600 130 / 111; four of 32 of 256: 800 47 / 55, 1,200 63 / 57; six of eight of 1,408: 1,200 136 / 131, 5,100
+    543 / 460."""
+    dense = 6.0 * tokens * (experts * ff + shared) * hidden / 1450e6
+    rows = max(tokens * top + 128 * experts, 256 * experts)
+    chosen = 6.0 * hidden * (rows * ff + -(-tokens // 256) * 256 * shared) / 1150e6
+    return 1.15 * dense + 15.0 > chosen + 45.0
+
+
+def moe_grouped(h: torch.Tensor, share: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, experts: int, top: int,
+                ff: int, shared: int, activation: str) -> torch.Tensor:
+    """The routed experts' feed-forward (and a shared one's of `shared` lanes) over the rows that chose them: bfloat16 `h`
+    [T, hidden], `share` float32 [T, experts (+ 1) or more] (not chosen: 0; at most `top` others a token), the stacked
+    weights `gate_up` [2 inner, hidden] and `down` [hidden, inner], lanes as `moe_gate` orders them.  Returns bfloat16
+    [T, hidden], the sum over the experts in 32-bit."""
+    n, hidden = h.shape
+    inner = experts * ff + shared
+    if h.dtype != torch.bfloat16 or gate_up.dtype != torch.bfloat16 or down.dtype != torch.bfloat16 or \
+            tuple(gate_up.shape) != (2 * inner, hidden) or tuple(down.shape) != (hidden, inner) or \
+            share.dtype != torch.float32 or share.shape[0] != n or share.shape[1] < experts + int(shared > 0):
+        raise ValueError("moe_grouped: bfloat16 rows and stacked weights, shares float32 [T, experts (+ 1) or more]")
+    if not moe_grouped_supported(n, experts, top, ff, shared, hidden, activation):
+        raise ValueError("moe_grouped: up to 128 experts, inner sizes in whole 64s, one of " + ", ".join(ACTIVATIONS))
+    rows, ints, gate_at, down_at, totals_at = _moe_sort_sizes(n, experts, top, ff, shared, hidden)
+    width = max(ff, shared)
+    scratch = torch.empty(ints, dtype=torch.int32, device=h.device)
+    x = torch.empty((rows, hidden), dtype=torch.bfloat16, device=h.device)
+    row_share = torch.empty(rows, dtype=torch.float32, device=h.device)
+    act = torch.empty((rows, width), dtype=torch.bfloat16, device=h.device)
+    sums = torch.empty((rows, hidden), dtype=torch.float32, device=h.device)
+    out = torch.empty((n, hidden), dtype=torch.bfloat16, device=h.device)
+    at = lambda place: ctypes.c_void_p(scratch.data_ptr() + 4 * place)
+    sizes = (_i(n), _i(experts), _i(top), _i(ff), _i(shared), _i(hidden))
+    _check(_lib("moe").tokb200_moe_sort(_ptr(h), _ptr(share), _i(share.shape[1]), *sizes, _ptr(scratch), _ptr(x),
+                                        _ptr(row_share), _stream()), "moe_sort")
+    _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_grouped_gated(
+        _ptr(x), _ptr(gate_up), _ptr(act), at(gate_at), at(totals_at), _ptr(row_share), _i(rows), _i(inner), _i(hidden),
+        _i(width), _i(ACTIVATIONS[activation]), _stream()), "gemm_tcgen05_grouped_gated")
+    _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_grouped_down(
+        _ptr(act), _ptr(down), _ptr(sums), at(down_at), at(totals_at + 1), _i(rows), _i(inner), _i(hidden), _i(width),
+        _stream()), "gemm_tcgen05_grouped_down")
+    _check(_lib("moe").tokb200_moe_combine(_ptr(sums), *sizes, _ptr(scratch), _ptr(out), _stream()), "moe_combine")
+    return out
+
+
 # ---- a short convolution across steps; a layer whose sublayers share one norm; learned positions ----
 CONV_ACTIVATIONS = {None: 0, "silu": 1}
 

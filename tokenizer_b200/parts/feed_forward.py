@@ -169,7 +169,8 @@ class RoutedMLP:
     choose (`csrc/moe.cu`); the down product over all lanes is the weighted sum of the chosen
     experts' outputs.  Nothing depends on values read back to the host, so a step can be captured.
     It costs experts / top times the routed experts' arithmetic: what a model of few experts pays
-    for products of full size instead of a product per expert over gathered rows.
+    for products of full size.  Steps of many rows sort them by expert instead and compute the chosen
+    lanes alone (`ops.moe_grouped`; where that pays: `ops.moe_grouped_pays`).
 
     Parameters beyond the sizes: `score` ("softmax_of_chosen" as above; "sigmoid": scores
     s = sigmoid(z), the choice made on s + `<prefix>.correction` (with `correction`) among the experts
@@ -249,6 +250,13 @@ class RoutedMLP:
     def streamed_weights(self):
         return [self.gate_up.weight, self.down.weight]
 
+    def _grouped(self, n, h):
+        """Whether the rows are sorted by expert: what the kernels take, and where it pays."""
+        if h.dtype != torch.bfloat16 or self.share_on != "output" or self.identity or \
+                not ops.moe_grouped_pays(n, self.experts, self.top, self.ff, self.shared, h.shape[1]):
+            return False
+        return ops.moe_grouped_supported(n, self.experts, self.top, self.ff, self.shared, h.shape[1], self.activation)
+
     def forward(self, h):
         n = h.shape[0]
         columns = self.experts + (1 if self.shared else 0) + (1 if self.identity else 0)
@@ -256,6 +264,9 @@ class RoutedMLP:
         ops.moe_route(h, self.router, self.experts, self.top, self.shared_mode, share, score=self.score,
                       correction=self.correction, groups=self.groups, keep=self.group_keep, scale=self.route_scale,
                       identity=self.identity, group_worth=self.group_worth, renormalize=self.renormalize)
+        if self._grouped(n, h):
+            return ops.moe_grouped(h, share, self.gate_up.weight, self.down.weight, self.experts, self.top, self.ff,
+                                   self.shared, self.activation)
         act = self.runtime.empty(n, self.inner)
         ops.moe_gate(self.gate_up.forward(h), share, act, self.experts, self.ff, bool(self.shared), self.activation,
                      limit=self.limit, shared_limit=self.shared_limit, alpha=self.alpha,
