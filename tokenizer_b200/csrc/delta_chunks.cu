@@ -31,18 +31,18 @@
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).
 #include "common.cuh"
+#include "exact_mma.cuh"
 
 #define DC_TOKENS 32
 #define DC_DIM 128                        // lanes of a key, zeros behind the head's own
 #define DC_COLS 16                        // columns of a narrow scan block (wide ones: 32)
 #define DC_MAX_TAPS 16
 #define DC_PREPARE_THREADS 256
-#define DC_SCAN_THREADS 256
 constexpr int kDcStride = DC_DIM + 4;     // of rows that several lanes read at once, 16 bytes each
 constexpr int kDcPairs = DC_TOKENS + 4;   // of A's and M's rows
-// a record, in floats: W, G q, decayed k (32 x 128 each), M (32 x 32), G_31 (128), U0 (32 x vdim)
-constexpr int kDcQ = DC_TOKENS * DC_DIM, kDcK = 2 * kDcQ, kDcM = 3 * kDcQ, kDcG = kDcM + DC_TOKENS * DC_TOKENS,
-              kDcU = kDcG + DC_DIM;
+// a record, in floats: W over G q (64 x 128), then decayed k (32 x 128), as pieces in the order in which a lane of a product
+// takes them ([16 channels][tile][piece][lane] of 16 bytes, see exact_mma.cuh); M (32 x 32), G_31 (128), U0 (32 x vdim)
+constexpr int kDcK = 8 * 4 * 3 * 128, kDcM = kDcK + 8 * 2 * 3 * 128, kDcG = kDcM + DC_TOKENS * DC_TOKENS, kDcU = kDcG + DC_DIM;
 
 __device__ __forceinline__ float dc_sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float dc_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
@@ -330,8 +330,9 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
     for (int t = 0; t < DC_TOKENS; ++t) l_s[t * kDcStride + l] = col[t];
   }
   __syncthreads();
+  float other[DC_TOKENS];
   if (!half) {
-    float other[DC_TOKENS], upto = 1.f;
+    float upto = 1.f;
 #pragma unroll
     for (int t = 0; t < DC_TOKENS; ++t) {
       const float beta = beta_s[t];
@@ -339,6 +340,9 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
       col[t] = beta * (upto * k_s[t * kDcStride + l]);
       other[t] = beta * l_s[t * kDcStride + l];
     }
+  }
+  __syncthreads();                                       // the keys' rows are read
+  if (!half) {
 #pragma unroll
     for (int t = 1; t < DC_TOKENS; ++t) {
       float sum[2] = {0.f, 0.f}, more[2] = {0.f, 0.f};
@@ -354,7 +358,7 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
       other[t] -= more[0] + more[1];
     }
 #pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) rec[t * DC_DIM + l] = col[t];
+    for (int t = 0; t < DC_TOKENS; ++t) l_s[t * kDcStride + l] = col[t];
     if (l < a.vdim) {
 #pragma unroll
       for (int t = 0; t < DC_TOKENS; ++t) rec[kDcU + t * a.vdim + l] = other[t];
@@ -364,220 +368,265 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
 #pragma unroll
     for (int t = 0; t < DC_TOKENS; ++t) {
       upto *= g_s[t * kDcStride + l];
-      rec[kDcQ + t * DC_DIM + l] = upto * q_s[t * kDcStride + l];
+      q_s[t * kDcStride + l] *= upto;
     }
     rec[kDcG + l] = upto;
 #pragma unroll
     for (int t = DC_TOKENS - 1; t >= 0; --t) {
-      rec[kDcK + t * DC_DIM + l] = behind * k_s[t * kDcStride + l];
+      k_s[t * kDcStride + l] *= behind;
       behind *= g_s[t * kDcStride + l];
     }
     for (int i = l; i < DC_TOKENS * DC_TOKENS; i += DC_DIM) rec[kDcM + i] = m_s[i / DC_TOKENS * kDcPairs + i % DC_TOKENS];
+  }
+  __syncthreads();
+  // ---- W, G q and the decayed keys in pieces, six tiles a warp: channels 16 w on, of 16 rows or of 16 tokens ----
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int e = 0; e < 6; ++e) {
+    unsigned p[3][4];
+    uint4* to;
+    if (e < 4) {
+      const float* from = (e < 2 ? l_s : q_s) + ((e & 1) * 16 + g) * kDcStride + warp * 16 + 2 * c;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 v = *reinterpret_cast<const float2*>(from + (i & 1) * 8 * kDcStride + (i >> 1) * 8);
+        xm_cut(v.x, v.y, p[0][i], p[1][i], p[2][i]);
+      }
+      to = reinterpret_cast<uint4*>(rec) + (warp * 4 + e) * 3 * 32 + lane;
+    } else {
+      const float* from = k_s + ((e - 4) * 16 + 2 * c) * kDcStride + warp * 16 + g;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float* at = from + (i & 1) * 8 * kDcStride + (i >> 1) * 8;
+        xm_cut(at[0], at[kDcStride], p[0][i], p[1][i], p[2][i]);
+      }
+      to = reinterpret_cast<uint4*>(rec + kDcK) + (warp * 2 + e - 4) * 3 * 32 + lane;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) to[q * 32] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
   }
 }
 constexpr int kDcPrepareSmem = (4 * DC_TOKENS * kDcStride + 16 * kDcStride + 2 * DC_TOKENS * kDcPairs + DC_TOKENS) * 4;
 
 // ---- the chunks one after another --------------------------------------------------------------------------------
-// a stage, in floats: W and G q (64 x 132), decayed k (32 x 128), M (32 x 36), G_31 (128), U0 (32 x COLS)
-constexpr int kDsK = 2 * DC_TOKENS * kDcStride, kDsM = kDsK + DC_TOKENS * DC_DIM, kDsG = kDsM + DC_TOKENS * kDcPairs,
-              kDsU = kDsG + DC_DIM;
-// behind the two stages: the columns of S [128][COLS], the eight partial sums [8][64][COLS], U [32][COLS]
-template <int COLS> constexpr int dc_scan_floats() {
-  return 2 * (kDsU + DC_TOKENS * COLS) + DC_DIM * COLS + 8 * 2 * DC_TOKENS * COLS + DC_TOKENS * COLS;
-}
-
-__device__ __forceinline__ void dc_add(float4& a, float v, const float4& b) {
-  a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
-}
-
-__device__ __forceinline__ void dc_copy16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
+// The products run on the tensor cores with their operands in exact pieces (exact_mma.cuh).
+//   warps 0 .. 7    channels 16 w .. + 15 of the block's columns of S, transposed, in the layout of a product's result, which
+//                   is that of the next product's second operand.  W and G q times S over their channels, the eight partial
+//                   sums through shared memory, U; then S = G S + K^T U
+//   warps 8 .. 11   bring the next chunk's M, G_31 and U0 (cp.async), and finish G q S + M U: plain multiply-adds over the
+//                   tokens up to a row's own (an infinity or a NaN behind it is not this row's)
+// A chunk of 16 columns takes 3,300 cycles (4,900 with multiply-adds, whose reads of shared memory bounded it): the tensor
+// pipe's own 1,150, and the two meetings of all warps, whose sums and cuts lie one behind the other.  us, a scan of 16 heads
+// of 128 x 128: one prompt of 2,048 tokens 162 -> 112, four of 5,100 in all 322 -> 245.  Pieces straight from memory to
+// registers a chunk ahead instead of two chunks ahead through shared memory: 128; 32-bit records, cut by the helping warps: 216.
+#define DT_THREADS 384
+#define DT_HELPERS 128
+#define DT_PITCH 40                       // floats between columns of U: no two lanes of a load on one bank
+// a stage, in floats: M (32 x 36), G_31 (128), U0 (32 x COLS)
+constexpr int kDtG = DC_TOKENS * kDcPairs, kDtU = kDtG + DC_DIM;
+constexpr int kDtPieces = kDcM * 4;       // bytes of a record's pieces
+template <int COLS> struct DtShape {
+  static constexpr int kStage = kDtU + DC_TOKENS * COLS;
+  static constexpr int kPart = 3 * kStage;                                  // [8][64][16] partial sums
+  static constexpr int kUs = kPart + 8 * 64 * 16;                           // [2][COLS][DT_PITCH]
+  static constexpr int kOs = kUs + 2 * COLS * DT_PITCH;                     // [2][32][COLS + 4]
+  static constexpr int kRing = kOs + 2 * DC_TOKENS * (COLS + 4);            // [2] chunks' pieces, a lane's places in eighteens
+  static constexpr int kSmem = kRing * 4 + 2 * kDtPieces;
+};
 
 template <int COLS>
-__global__ void __launch_bounds__(DC_SCAN_THREADS, 1)
+__global__ void __launch_bounds__(DT_THREADS, 1)
 delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, float* __restrict__ state,
                         long long state_stride, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                         float* __restrict__ o_out) {
-  constexpr int kStage = kDsU + DC_TOKENS * COLS;
-  constexpr int kOwn = COLS / 4;                         // rows of S a thread of the first half, four columns of each
-  constexpr int kRows = COLS / 16;                       // rows of W or G q a thread adds up, four columns of each
-  extern __shared__ __align__(16) float ds_raw[];
-  float* s_s = ds_raw + 2 * kStage;
-  float* part_s = s_s + DC_DIM * COLS;
-  float* u_s = part_s + 8 * 2 * DC_TOKENS * COLS;
+  using S = DtShape<COLS>;
+  constexpr int kHalves = COLS / 16;
+  extern __shared__ __align__(16) float dt_raw[];
+  float* part_s = dt_raw + S::kPart;
   const int r = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
   const int first = q_start[r], n = q_start[r + 1] - first;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp's number through a shuffle: the compiler sees that the roles do not diverge
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int g = lane >> 2, c = lane & 3;                 // of a product's layout: row (or column) and pair
   pdl_wait();
   pdl_launch();
   if (n <= 0) return;
   const int chunks = (n + DC_TOKENS - 1) / DC_TOKENS;
   const size_t record = (size_t)(kDcU + DC_TOKENS * vdim);
   const float* base = records + ((size_t)(first / DC_TOKENS + r) * heads + h) * record;
-  auto fetch = [&](int c) {
-    if (c < chunks) {
-      const float* src = base + (size_t)c * heads * record;
-      float* dst = ds_raw + (c & 1) * kStage;
-#pragma unroll
-      for (int j = 0; j < 2 * DC_TOKENS * DC_DIM / 4; j += DC_SCAN_THREADS) {
-        const int i = j + threadIdx.x;
-        dc_copy16(dst + i / (DC_DIM / 4) * kDcStride + i % (DC_DIM / 4) * 4, src + i * 4);
-      }
-#pragma unroll
-      for (int j = 0; j < DC_TOKENS * DC_DIM / 4; j += DC_SCAN_THREADS)
-        dc_copy16(dst + kDsK + (j + threadIdx.x) * 4, src + kDcK + (j + threadIdx.x) * 4);
-      dc_copy16(dst + kDsM + threadIdx.x / (DC_TOKENS / 4) * kDcPairs + threadIdx.x % (DC_TOKENS / 4) * 4,
-                src + kDcM + threadIdx.x * 4);
-      if (threadIdx.x < DC_DIM / 4) dc_copy16(dst + kDsG + threadIdx.x * 4, src + kDcG + threadIdx.x * 4);
-      if ((int)threadIdx.x >= DC_SCAN_THREADS - DC_TOKENS * COLS / 4) {
-        const int i = threadIdx.x - (DC_SCAN_THREADS - DC_TOKENS * COLS / 4), t = i / (COLS / 4), l = i % (COLS / 4) * 4;
-        dc_copy16(dst + kDsU + t * COLS + l, src + kDcU + t * vdim + col0 + l);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  static_assert(DC_SCAN_THREADS == DC_TOKENS * DC_TOKENS / 4 && DC_TOKENS * COLS / 4 <= DC_SCAN_THREADS, "a copy a thread");
-  fetch(0);
-  // threads 0 .. 127: rows row .. + kOwn - 1 of columns own .. + 3 of the matrix
-  const bool owner = threadIdx.x < 128;
-  const int row = (threadIdx.x & 127) / (COLS / 4) * kOwn, own = threadIdx.x % (COLS / 4) * 4;
-  float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + own) * DC_DIM + row;
-  float4 S[kOwn];
-  if (owner) {
-#pragma unroll
-    for (int e = 0; e < kOwn; e += 4) {
-      float4 v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(mine + j * DC_DIM + e);
-      S[e] = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-      S[e + 1] = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-      S[e + 2] = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
-      S[e + 3] = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
-    }
-#pragma unroll
-    for (int i = 0; i < kOwn; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * COLS + own) = S[i];
-  }
 
-  for (int c = 0; c < chunks; ++c) {
-    const float* stage = ds_raw + (c & 1) * kStage;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                     // the record and the matrix are in place
-    fetch(c + 1);                                        // into the stage that the chunk before has left
-    {
-      // the 64 rows of W and G q times the columns, lanes k0 .. k0 + 15 a warp: rows group + 8 i, columns cols .. + 3
-      // and, of 32, cols + 16 .. + 19
-      constexpr int kWide = COLS / 16;
-      const int k0 = warp * 16, group = lane >> 2, cols = (lane & 3) * 4;
-      const float* x_s = stage + group * kDcStride;
-      float acc[8][4 * kWide];
+  if (warp < 8) {
+    float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + g) * DC_DIM + warp * 16 + 2 * c;
+    float s[kHalves][2][4];                              // columns g and g + 8 of a half, channels 8 j + 2 c, + 1
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+    for (int e = 0; e < kHalves; ++e)
 #pragma unroll
-        for (int j = 0; j < 4 * kWide; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int k = k0; k < k0 + 16; k += 4) {
-        float4 x[8];
+        for (int i = 0; i < 4; i += 2)
+          *reinterpret_cast<float2*>(&s[e][j][i]) = *reinterpret_cast<const float2*>(mine + (e * 16 + i * 4) * DC_DIM + j * 8);
+    // The pieces of a record that a lane takes are its own alone: copied two chunks ahead to places of shared memory that no
+    // other thread touches.
+    const unsigned ring = (unsigned)__cvta_generic_to_shared(dt_raw + S::kRing) + (warp * 18 * 32 + lane) * 16;
+    auto fetch = [&](int chunk) {
+      if (chunk < chunks) {
+        const float* src = base + (size_t)chunk * heads * record + lane * 4;
+        const unsigned to = ring + (chunk & 1) * kDtPieces;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(x_s + i * 8 * kDcStride + k);
+        for (int i = 0; i < 18; ++i) {
+          const float* from = i < 12 ? src + (warp * 12 + i) * 128 : src + kDcK + (warp * 6 + i - 12) * 128;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * 512), "l"(from) : "memory");
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto piece = [&](int chunk, int i, unsigned (&v)[4]) {
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                   : "r"(ring + (chunk & 1) * kDtPieces + i * 512) : "memory");
+    };
+    fetch(0);
+    fetch(1);
+    __syncthreads();                                     // the first stage is in place
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      const float* stage = dt_raw + chunk % 3 * S::kStage;
+      float* u_s = dt_raw + S::kUs + (chunk & 1) * COLS * DT_PITCH;
+      float* o_s = dt_raw + S::kOs + (chunk & 1) * DC_TOKENS * (COLS + 4);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      unsigned a[4][3][4];                               // W and G q: tile of 16 rows, piece
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
+      for (int m = 0; m < 4; ++m)
 #pragma unroll
-          for (int e = 0; e < kWide; ++e) {
-            const float4 y = *reinterpret_cast<const float4*>(s_s + (k + kk) * COLS + e * 16 + cols);
+        for (int p = 0; p < 3; ++p) piece(chunk, m * 3 + p, a[m][p]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float v = kk == 0 ? x[i].x : kk == 1 ? x[i].y : kk == 2 ? x[i].z : x[i].w;
-              acc[i][4 * e] = fmaf(v, y.x, acc[i][4 * e]);
-              acc[i][4 * e + 1] = fmaf(v, y.y, acc[i][4 * e + 1]);
-              acc[i][4 * e + 2] = fmaf(v, y.z, acc[i][4 * e + 2]);
-              acc[i][4 * e + 3] = fmaf(v, y.w, acc[i][4 * e + 3]);
-            }
+      for (int e = 0; e < kHalves; ++e) {
+        unsigned b[2][3][2];                             // S as second operand, columns 0 .. 7 and 8 .. 15 of the half
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) xm_cut(s[e][j][2 * i], s[e][j][2 * i + 1], b[i][0][j], b[i][1][j], b[i][2][j]);
+        float d[4][2][4] = {};
+        xm_products(d, a, b);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            // columns in eights change places where two rows of one bank would meet
+            const int at = (warp * 64 + m * 16 + g) * 16 + ((i * 8) ^ ((g >> 1 & 1) * 8)) + 2 * c;
+            *reinterpret_cast<float2*>(part_s + at) = make_float2(d[m][i][0], d[m][i][1]);
+            *reinterpret_cast<float2*>(part_s + at + 8 * 16) = make_float2(d[m][i][2], d[m][i][3]);
           }
-      }
-      float* to = part_s + (warp * 2 * DC_TOKENS + group) * COLS + cols;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const int row = threadIdx.x >> 2, q = (threadIdx.x & 3) * 4;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int e = 0; e < kWide; ++e)
-          *reinterpret_cast<float4*>(to + i * 8 * COLS + e * 16) =
-              make_float4(acc[i][4 * e], acc[i][4 * e + 1], acc[i][4 * e + 2], acc[i][4 * e + 3]);
-    }
-    __syncthreads();
-    // kRows rows (of W for the first half of the threads, of G q for the second) of four columns a thread
-    const int t = (threadIdx.x & 127) / (COLS / 4), cols = threadIdx.x % (COLS / 4) * 4;
-    float4 sum[kRows];
-#pragma unroll
-    for (int e = 0; e < kRows; ++e) {
-      sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 v = *reinterpret_cast<const float4*>(
-            part_s + ((i * 2 + !owner) * DC_TOKENS + t + e * (DC_TOKENS / kRows)) * COLS + cols);
-        sum[e].x += v.x; sum[e].y += v.y; sum[e].z += v.z; sum[e].w += v.w;
-      }
-      if (owner) {
-        const int at = (t + e * (DC_TOKENS / kRows)) * COLS + cols;
-        const float4 v = *reinterpret_cast<const float4*>(stage + kDsU + at);
-        *reinterpret_cast<float4*>(u_s + at) = make_float4(v.x - sum[e].x, v.y - sum[e].y, v.z - sum[e].z, v.w - sum[e].w);
-      }
-    }
-    __syncthreads();
-    if (!owner) {
-      // what comes behind a row's own token is left out, not added with weight 0: an infinity or a NaN there is not this row's
-      constexpr int kApart = DC_TOKENS / kRows;
-      const float* m_row = stage + kDsM + t * kDcPairs;
-#pragma unroll
-      for (int s = 0; s < DC_TOKENS; s += 4) {
-        float4 x[kRows];
-#pragma unroll
-        for (int e = 0; e < kRows; ++e)
-          if (s < (e + 1) * kApart) x[e] = *reinterpret_cast<const float4*>(m_row + e * kApart * kDcPairs + s);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 u = *reinterpret_cast<const float4*>(u_s + (s + i) * COLS + cols);
-#pragma unroll
-          for (int e = 0; e < kRows; ++e)
-            if (s + i < (e + 1) * kApart && (s + i <= e * kApart || s + i <= t + e * kApart))
-              dc_add(sum[e], i == 0 ? x[e].x : i == 1 ? x[e].y : i == 2 ? x[e].z : x[e].w, u);
+        for (int w = 0; w < 8; ++w) {
+          const float4 v = *reinterpret_cast<const float4*>(part_s + (w * 64 + row) * 16 + (q ^ ((row >> 1 & 1) * 8)));
+          sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
+        if (row < DC_TOKENS) {
+          const float4 v = *reinterpret_cast<const float4*>(stage + kDtU + row * COLS + e * 16 + q);
+          float* to = u_s + (e * 16 + q) * DT_PITCH + row;
+          to[0] = v.x - sum.x; to[DT_PITCH] = v.y - sum.y; to[2 * DT_PITCH] = v.z - sum.z; to[3 * DT_PITCH] = v.w - sum.w;
+        } else {
+          *reinterpret_cast<float4*>(o_s + (row - DC_TOKENS) * (COLS + 4) + e * 16 + q) = sum;
+        }
+        if (e + 1 < kHalves) asm volatile("bar.sync 1, 256;" ::: "memory");
       }
-#pragma unroll
-      for (int e = 0; e < kRows; ++e) {
-        const int token = c * DC_TOKENS + t + e * (DC_TOKENS / kRows);
-        if (token < n)
-          *reinterpret_cast<float4*>(o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + cols) = sum[e];
-      }
-    } else {
+      __syncthreads();                                   // U and G q S are in place, and the next stage
       // the matrix moves on by the chunk
+      float2 decay[2];
 #pragma unroll
-      for (int i = 0; i < kOwn; ++i) {
-        const float g = stage[kDsG + row + i];
-        S[i] = make_float4(S[i].x * g, S[i].y * g, S[i].z * g, S[i].w * g);
+      for (int j = 0; j < 2; ++j) decay[j] = *reinterpret_cast<const float2*>(stage + kDtG + warp * 16 + j * 8 + 2 * c);
+      float more[kHalves][2][4] = {};
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        unsigned k[2][3][2];                             // keys of 16 tokens: [eight channels][piece]
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          unsigned v[4];
+          piece(chunk, 12 + t * 3 + p, v);
+          k[0][p][0] = v[0]; k[0][p][1] = v[1]; k[1][p][0] = v[2]; k[1][p][1] = v[3];
+        }
+        unsigned u[kHalves][3][4];                       // U transposed: columns g, g + 8 of tokens 2 c, + 1 and 8 behind
+#pragma unroll
+        for (int e = 0; e < kHalves; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 v = *reinterpret_cast<const float2*>(u_s + (e * 16 + g + (i & 1) * 8) * DT_PITCH + t * 16 + 2 * c + (i >> 1) * 8);
+            xm_cut(v.x, v.y, u[e][0][i], u[e][1][i], u[e][2][i]);
+          }
+        xm_products(more, u, k);
       }
-#pragma unroll 8
-      for (int s = 0; s < DC_TOKENS; ++s) {
-        const float4 u = *reinterpret_cast<const float4*>(u_s + s * COLS + own);
+      fetch(chunk + 2);
 #pragma unroll
-        for (int e = 0; e < kOwn; e += 4) {
-          const float4 k = *reinterpret_cast<const float4*>(stage + kDsK + s * DC_DIM + row + e);
-          dc_add(S[e], k.x, u); dc_add(S[e + 1], k.y, u); dc_add(S[e + 2], k.z, u); dc_add(S[e + 3], k.w, u);
+      for (int e = 0; e < kHalves; ++e)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(i & 1 ? decay[j].y : decay[j].x, s[e][j][i], more[e][j][i]);
+    }
+#pragma unroll
+    for (int e = 0; e < kHalves; ++e)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+          *reinterpret_cast<float2*>(mine + (e * 16 + i * 4) * DC_DIM + j * 8) = *reinterpret_cast<const float2*>(&s[e][j][i]);
+  } else {
+    const int id = threadIdx.x - 256;
+    auto fetch = [&](int chunk) {                        // M, G_31 and U0
+      if (chunk < chunks) {
+        const float* src = base + (size_t)chunk * heads * record;
+        float* to = dt_raw + chunk % 3 * S::kStage;
+        auto copy = [&](float* dst, const float* from) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(from) : "memory");
+        };
+#pragma unroll
+        for (int i = id; i < DC_TOKENS * DC_TOKENS / 4; i += DT_HELPERS) copy(to + i / 8 * kDcPairs + i % 8 * 4, src + kDcM + i * 4);
+        if (id < DC_DIM / 4) copy(to + kDtG + id * 4, src + kDcG + id * 4);
+#pragma unroll
+        for (int i = id; i < DC_TOKENS * COLS / 4; i += DT_HELPERS)
+          copy(to + kDtU + i * 4, src + kDcU + i / (COLS / 4) * vdim + col0 + i % (COLS / 4) * 4);
+      }
+    };
+    const int t = id >> 2, col = id & 3;                 // of G q S + M U: a row, columns col + 4 i
+    auto outputs = [&](int chunk) {
+      const float* m_row = dt_raw + chunk % 3 * S::kStage + t * kDcPairs;
+      const float* u_s = dt_raw + S::kUs + (chunk & 1) * COLS * DT_PITCH + col * DT_PITCH;
+      const float* o_s = dt_raw + S::kOs + (chunk & 1) * DC_TOKENS * (COLS + 4) + t * (COLS + 4) + col;
+      float sum[COLS / 4];
+#pragma unroll
+      for (int i = 0; i < COLS / 4; ++i) sum[i] = o_s[4 * i];
+#pragma unroll
+      for (int s0 = 0; s0 < DC_TOKENS; s0 += 4) {
+        if (s0 > t) break;
+        const float4 m = *reinterpret_cast<const float4*>(m_row + s0);
+#pragma unroll
+        for (int i = 0; i < COLS / 4; ++i) {
+          const float4 u = *reinterpret_cast<const float4*>(u_s + 4 * i * DT_PITCH + s0);
+          sum[i] = fmaf(m.x, u.x, sum[i]);
+          if (s0 + 1 <= t) sum[i] = fmaf(m.y, u.y, sum[i]);
+          if (s0 + 2 <= t) sum[i] = fmaf(m.z, u.z, sum[i]);
+          if (s0 + 3 <= t) sum[i] = fmaf(m.w, u.w, sum[i]);
         }
       }
+      const int token = chunk * DC_TOKENS + t;
+      if (token < n) {
+        float* to = o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + col;
 #pragma unroll
-      for (int i = 0; i < kOwn; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * COLS + own) = S[i];
+        for (int i = 0; i < COLS / 4; ++i) to[4 * i] = sum[i];
+      }
+    };
+    fetch(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      fetch(chunk + 1);                                  // three stages: what the one before the last held is read by now
+      if (chunk > 0) outputs(chunk - 1);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
     }
-  }
-  if (owner) {
-#pragma unroll
-    for (int e = 0; e < kOwn; e += 4) {
-      const float4* v = S + e;
-      *reinterpret_cast<float4*>(mine + e) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-      *reinterpret_cast<float4*>(mine + DC_DIM + e) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-      *reinterpret_cast<float4*>(mine + 2 * DC_DIM + e) = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
-      *reinterpret_cast<float4*>(mine + 3 * DC_DIM + e) = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
-    }
+    outputs(chunks - 1);
   }
 }
 
@@ -639,11 +688,11 @@ TOKB200_API int tokb200_delta_chunk_prepare(const void* proj, int proj_dtype, in
 template <int COLS>
 static int dc_scan(const float* records, int heads, int vdim, float* state, long long state_stride, const int* q_start,
                    const int* state_slot, int n_requests, float* o_out, cudaStream_t stream) {
-  constexpr int bytes = dc_scan_floats<COLS>() * (int)sizeof(float);
+  constexpr int bytes = DtShape<COLS>::kSmem;
   static bool done[64] = {};
   const int status = dc_allow(delta_chunk_scan_kernel<COLS>, bytes, done);
   if (status != TOKB200_OK) return status;
-  return launch_dependent(delta_chunk_scan_kernel<COLS>, dim3(vdim / COLS, heads, n_requests), dim3(DC_SCAN_THREADS),
+  return launch_dependent(delta_chunk_scan_kernel<COLS>, dim3(vdim / COLS, heads, n_requests), dim3(DT_THREADS),
                           (size_t)bytes, stream, records, heads, vdim, state, state_stride, q_start, state_slot, o_out);
 }
 
@@ -656,8 +705,8 @@ TOKB200_API int tokb200_delta_chunk_scan(const float* records, int heads, int di
     return TOKB200_BAD_SIZE;
   if ((((uintptr_t)records | (uintptr_t)state | (uintptr_t)o_out) & 15) || state_stride % 4) return TOKB200_BAD_ALIGNMENT;
   // Wide blocks do a column's work in less time but are half as many: taken where narrow ones would need a second turn on
-  // 148 SMs (us, narrow / wide: 16 heads of one request of 2,048 tokens 254 / 353, of four of 512 260 / 228, 32 heads of one
-  // of 1,024 257 / 227).
+  // 148 SMs (us of both kernels, narrow / wide: 16 heads of one request of 2,048 tokens 212 / 296, of sixteen of 128 223 /
+  // 206, of one of 512 and 63 single ones 306 / 264, of eight of 512 371 / 371).
   const bool wide = columns ? columns == 32 : (long long)vdim / DC_COLS * heads * n_requests > 148;
   if (columns && columns != 16 && columns != 32) return TOKB200_BAD_SIZE;
   if (wide && vdim % 32 == 0)

@@ -6,30 +6,39 @@
 //     S32 = G_31 S0 + sum_s (a_{s+1} .. a_31 dt_s) B_s x_s^T
 // (products of decays only, never quotients: nothing can overflow).
 //
-//   ssd_chunk_prepare   a block a (chunk, group): C_t . B_s once for all heads of the group, then a head a warp: steps,
-//                       decays, M, G and the weights of the state's sum as one record
-//   ssd_chunk_scan      a block a (32 columns of a head's matrix, request): the chunks one after another.  The 32 rows of C
-//                       meet the columns in 8 x 8 register tiles, lanes cut over 16 half warps; then half of the threads
-//                       move the matrix on (8 x 4 of it each, in registers) while the others finish the chunk's rows.  The
-//                       next chunk's B, C, x and record are on their way (cp.async) meanwhile
+//   ssd_chunk_prepare   a block a (chunk, group): C_t . B_s once for all heads of the group, and C and B in pieces; then a
+//                       head a warp: steps, decays, M, G and the weights of the state's sum as one record
+//   ssd_chunk_scan      a block a (32 columns of a head's matrix, request): the chunks one after another, the products with
+//                       the matrix on the tensor cores with their operands in exact pieces (exact_mma.cuh).  A warp has 16
+//                       channels of the matrix: the rows of C times them, whose sums over the warps meet in shared memory,
+//                       then the matrix moves on; four more warps bring the next chunk, cut its weighted x and finish the
+//                       rows of the one before
 //
-// The scan is bound by reads of shared memory (counters: the pipe that brings them back busy 66 % of the time, the FMA pipe
-// 44 %; a tile of R x C costs R + C cycles of the 128 bytes a cycle that come back, and R C / 4
-// of the multiply-adds): hence the large tiles.  Measured (heads of 64 x 128, us, token by token / here): 64 heads, a prompt
-// of 2,048 tokens 307 / 214, two of 1,905 and 1,096 412 / 312; with tiles of 4 x 4 it was 301 and 441.
+// The tensor pipe is busy 41 % of a block's time (counters), the pipe of shared memory 60 %: two warps a scheduler, each
+// a chain of reads, cuts, products and sums.  Measured (heads of 64 x 128, us of both kernels, token by token / multiply-adds
+// in chunks / here): 64 heads, a prompt of 2,048 tokens 392 / 213 / 149, two of 1,905 and 1,096 611 / 311 / 210; 16 heads,
+// 2,048 126 / 198 / 125, four of 1,200 235 / 135 / 97.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).
 #include "common.cuh"
+#include "exact_mma.cuh"
 
 #define SC_TOKENS 32
 #define SC_DIM 128                        // lanes of B and C, zeros behind the model's own
 #define SC_THREADS 256
+#define SC_SCAN_THREADS 384
 #define SC_COLS 32                        // columns of a scan block
 constexpr int kScStride = SC_DIM + 4;     // of rows that several lanes read at once, 16 bytes each
 constexpr int kScPairs = SC_TOKENS + 4;   // of M's rows
 // a record, in floats: M (32 x 32), G (32), the weights of the state's sum (32)
 constexpr int kScG = SC_TOKENS * SC_TOKENS, kScR = kScG + SC_TOKENS, kScRecord = kScR + SC_TOKENS;
+// in front of a chunk's records, a group each: its C, then its B, as pieces in the order in which a lane of a product takes
+// them ([16 channels][tile][piece][lane] of 16 bytes, see exact_mma.cuh); in floats
+constexpr int kScB = 8 * 2 * 3 * 128, kScPieces = 2 * kScB;
+__host__ __device__ static inline size_t sc_place(int heads, int groups) {
+  return (size_t)groups * kScPieces + (size_t)heads * kScRecord;
+}
 
 __device__ __forceinline__ void sc_copy16(float* dst, const float* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
@@ -84,10 +93,31 @@ ssd_chunk_prepare_kernel(const float* __restrict__ xbc, int channels, const T* _
     for (int i = 0; i < 4; ++i) cb_s[t * kScPairs + s0 + 8 * i] = (dot[i].x + dot[i].y) + (dot[i].z + dot[i].w);
   }
   __syncthreads();
+  float* at_place = records + (size_t)place * sc_place(heads, groups);
+  {
+    const int row = lane >> 2, pair = (lane & 3) * 2;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      unsigned p[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (e < 2) {                      // 16 rows of C, 16 channels
+          const float2 v = *reinterpret_cast<const float2*>(c_s + (e * 16 + row + (i & 1) * 8) * kScStride + warp * 16 + pair + (i >> 1) * 8);
+          xm_cut(v.x, v.y, p[0][i], p[1][i], p[2][i]);
+        } else {                          // 16 tokens of B, twice eight channels
+          const float* v = b_s + ((e - 2) * 16 + pair + (i & 1) * 8) * kScStride + warp * 16 + (i >> 1) * 8 + row;
+          xm_cut(v[0], v[kScStride], p[0][i], p[1][i], p[2][i]);
+        }
+      }
+      uint4* to = reinterpret_cast<uint4*>(at_place + (size_t)g * kScPieces + (e < 2 ? 0 : kScB)) + (warp * 2 + (e & 1)) * 3 * 32 + lane;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) to[q * 32] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    }
+  }
   const int share = heads / groups;
   for (int j = warp; j < share; j += SC_THREADS / 32) {
     const int h = g * share + j;
-    float* rec = records + ((size_t)place * heads + h) * kScRecord;
+    float* rec = at_place + (size_t)groups * kScPieces + (size_t)h * kScRecord;
     float dt = 0.f, keep = 1.f;           // this lane's token
     if (lane < n_here) {
       const float v = to_float(raw[(size_t)(t0 + lane) * raw_ld + h]) + dt_bias[h];
@@ -113,203 +143,225 @@ ssd_chunk_prepare_kernel(const float* __restrict__ xbc, int channels, const T* _
   }
 }
 
-// a stage, in floats: C (32 x 132), B (32 x 128), M (32 x 36), G and the weights (32 each), x (32 x 32)
-constexpr int kSsB = SC_TOKENS * kScStride, kSsM = kSsB + SC_TOKENS * SC_DIM, kSsG = kSsM + SC_TOKENS * kScPairs,
-              kSsR = kSsG + SC_TOKENS, kSsX = kSsR + SC_TOKENS, kSsStage = kSsX + SC_TOKENS * SC_COLS;
-// behind the two stages: the columns of S [128][32], the eight partial sums [8][32][32], the weighted x [32][32]
-constexpr int kSsBytes = (2 * kSsStage + SC_DIM * SC_COLS + 8 * SC_TOKENS * SC_COLS + SC_TOKENS * SC_COLS) * 4;
-
-template <bool V> struct sc_bool { static constexpr bool value = V; };
-
 __device__ __forceinline__ void sc_add(float4& a, float v, const float4& b) {
   a.x = fmaf(v, b.x, a.x); a.y = fmaf(v, b.y, a.y); a.z = fmaf(v, b.z, a.z); a.w = fmaf(v, b.w, a.w);
 }
 
-__global__ void __launch_bounds__(SC_THREADS, 1)
+// a stage, in bytes: the weighted x as pieces ([half of the columns][16 tokens][piece][lane] of 16 bytes), then x (32 x 32),
+// M (32 x 36) and G (32) as floats
+constexpr int kSsX = 4 * 3 * 512, kSsM = kSsX + SC_TOKENS * SC_COLS * 4, kSsG = kSsM + SC_TOKENS * kScPairs * 4,
+              kSsStage = kSsG + SC_TOKENS * 4;
+// behind the three stages: the eight partial sums of C S [8][32][32] of two chunks
+constexpr int kSsPart = 3 * kSsStage, kSsRing = kSsPart + 2 * 8 * SC_TOKENS * SC_COLS * 4 /* two chunks' pieces */,
+              kSsBytes = kSsRing + 2 * kScPieces * 4;
+
+__global__ void __launch_bounds__(SC_SCAN_THREADS, 1)
 ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* __restrict__ records,
                       const float* __restrict__ skip, int heads, int groups, int P, int N, float* __restrict__ state,
                       long long state_stride, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                       float* __restrict__ y_out) {
-  extern __shared__ __align__(16) float ss_raw[];
-  float* s_s = ss_raw + 2 * kSsStage;
-  float* part_s = s_s + SC_DIM * SC_COLS;
-  float* u_s = part_s + 8 * SC_TOKENS * SC_COLS;
+  extern __shared__ __align__(16) unsigned char ss_raw[];
   const int r = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * SC_COLS;
   const int first = q_start[r], n = q_start[r + 1] - first;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp's number through a shuffle: the compiler sees that the roles do not diverge
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int g = lane >> 2, c = lane & 3;                 // of a product's layout: row (or column) and pair
   pdl_wait();
   pdl_launch();
   if (n <= 0) return;
   const int chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
-  const float* base = records + ((size_t)(first / SC_TOKENS + r) * heads + h) * kScRecord;
-  const int g = h / (heads / groups);
-  const float* b_in = xbc + (size_t)heads * P + (size_t)g * N;
-  const float* c_in = b_in + (size_t)groups * N;
-  // t and c4: of the 32 x 32 numbers of x, of its weighted copy and of M, four neighbours a thread
-  const int t = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;
-  auto fetch = [&](int c) {
-    if (c < chunks) {
-      float* dst = ss_raw + (c & 1) * kSsStage;
-      const int t0 = c * SC_TOKENS, tb = threadIdx.x / (SC_DIM / 4), l = threadIdx.x % (SC_DIM / 4) * 4;
-#pragma unroll
-      for (int i = 0; i < SC_TOKENS; i += SC_THREADS / (SC_DIM / 4)) {
-        const bool in = t0 + tb + i < n && l < N;
-        const size_t at = in ? (size_t)(first + t0 + tb + i) * channels + l : 0;
-        sc_copy16(dst + (tb + i) * kScStride + l, c_in + at, in);
-        sc_copy16(dst + kSsB + (tb + i) * SC_DIM + l, b_in + at, in);
-      }
-      const float* rec = base + (size_t)c * heads * kScRecord;
-      sc_copy16(dst + kSsM + t * kScPairs + c4, rec + threadIdx.x * 4, true);
-      if (threadIdx.x < 16) sc_copy16(dst + kSsG + threadIdx.x * 4, rec + kScG + threadIdx.x * 4, true);
-      const bool in = t0 + t < n;
-      sc_copy16(dst + kSsX + threadIdx.x * 4, xbc + (in ? (size_t)(first + t0 + t) * channels + (size_t)h * P + col0 + c4 : 0), in);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  static_assert(SC_THREADS * 4 == SC_TOKENS * SC_TOKENS && SC_TOKENS == SC_COLS, "a copy a thread");
-  fetch(0);
-  // threads 0 .. 127: rows row .. + 7 of columns c4 .. + 3 of the matrix
-  const bool owner = threadIdx.x < 128;
-  const int row = t * 8;
-  float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * P + col0 + c4) * N + row;
-  float4 S[8];                                           // a row's four columns each
-  if (owner) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float4 v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        v[j] = row + 4 * e < N ? *reinterpret_cast<const float4*>(mine + (size_t)j * N + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
-      S[4 * e] = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-      S[4 * e + 1] = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-      S[4 * e + 2] = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
-      S[4 * e + 3] = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * SC_COLS + c4) = S[i];
-  }
-  const float d = skip[h];
+  const size_t place = sc_place(heads, groups);
+  const float* here = records + (size_t)(first / SC_TOKENS + r) * place;
 
-  for (int c = 0; c < chunks; ++c) {
-    const float* stage = ss_raw + (c & 1) * kSsStage;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                     // the chunk and the matrix are in place
-    fetch(c + 1);                                        // into the stage that the chunk before has left
-    float zero;
-    {
-      const float w = stage[kSsR + t];
-      const float4 x = *reinterpret_cast<const float4*>(stage + kSsX + threadIdx.x * 4);
-      *reinterpret_cast<float4*>(u_s + threadIdx.x * 4) = make_float4(w * x.x, w * x.y, w * x.z, w * x.w);
-      zero = fmaf(x.x, 0.f, x.y * 0.f) + fmaf(x.z, 0.f, x.w * 0.f);      // a NaN where one of them is no number
-    }
-    {
-      // the rows of C times the columns, lanes k0 .. k0 + 7 a half warp: rows group + 4 i, columns cols .. + 3 and
-      // cols + 16 .. + 19
-      const int k0 = warp * 16 + (lane >> 4) * 8, group = (lane >> 2) & 3, cols = (lane & 3) * 4;
-      const float* x_s = stage + group * kScStride;
-      float acc[8][8];
+  if (warp < 8) {
+    // ---- channels 16 w .. + 15 of the columns of S, transposed, as results and second operands of products lie ----
+    const float* pieces = here + (size_t)(h / (heads / groups)) * kScPieces;
+    const int channel = warp * 16 + 2 * c;
+    float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * P + col0 + g) * N + channel;
+    float s[2][2][4];                                    // columns g and g + 8 of a half, channels 8 j + 2 c, + 1
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+    for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int k = k0; k < k0 + 8; k += 4) {
-        float4 x[8];
+        for (int i = 0; i < 4; i += 2)
+          *reinterpret_cast<float2*>(&s[e][j][i]) =
+              channel + 8 * j < N ? *reinterpret_cast<const float2*>(mine + (size_t)(e * 16 + i * 4) * N + j * 8) : make_float2(0.f, 0.f);
+    // The pieces of C and B that a lane takes are its own alone: copied two chunks ahead to places of shared memory that no
+    // other thread touches.
+    const unsigned ring = (unsigned)__cvta_generic_to_shared(ss_raw + kSsRing) + (warp * 12 * 32 + lane) * 16;
+    auto fetch = [&](int chunk) {
+      if (chunk < chunks) {
+        const float* src = pieces + (size_t)chunk * place + lane * 4;
+        const unsigned to = ring + (chunk & 1) * kScPieces * 4;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(x_s + i * 4 * kScStride + k);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const float4 lo = *reinterpret_cast<const float4*>(s_s + (k + kk) * SC_COLS + cols);
-          const float4 hi = *reinterpret_cast<const float4*>(s_s + (k + kk) * SC_COLS + 16 + cols);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float v = kk == 0 ? x[i].x : kk == 1 ? x[i].y : kk == 2 ? x[i].z : x[i].w;
-            acc[i][0] = fmaf(v, lo.x, acc[i][0]); acc[i][1] = fmaf(v, lo.y, acc[i][1]);
-            acc[i][2] = fmaf(v, lo.z, acc[i][2]); acc[i][3] = fmaf(v, lo.w, acc[i][3]);
-            acc[i][4] = fmaf(v, hi.x, acc[i][4]); acc[i][5] = fmaf(v, hi.y, acc[i][5]);
-            acc[i][6] = fmaf(v, hi.z, acc[i][6]); acc[i][7] = fmaf(v, hi.w, acc[i][7]);
-          }
+        for (int i = 0; i < 12; ++i) {
+          const float* from = src + (i < 6 ? 0 : kScB) + (warp * 6 + i % 6) * 128;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * 512), "l"(from) : "memory");
         }
       }
-      const bool upper = lane & 16;                      // the half warps' sums meet: the upper one keeps i = 4 .. 7
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto piece = [&](int chunk, int i, unsigned (&v)[4]) {
+      asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                   : "r"(ring + (chunk & 1) * kScPieces * 4 + i * 512) : "memory");
+    };
+    fetch(0);
+    fetch(1);
+    __syncthreads();                                     // the first stage is in place
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      const unsigned char* stage = ss_raw + chunk % 3 * kSsStage;
+      float* part_s = reinterpret_cast<float*>(ss_raw + kSsPart) + (chunk & 1) * 8 * SC_TOKENS * SC_COLS;
+      // the rows of C times the columns, over this warp's channels
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      unsigned a[2][3][4];                               // C: tile of 16 rows, piece
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float v[8];
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          v[j] = (upper ? acc[i + 4][j] : acc[i][j]) + __shfl_xor_sync(0xffffffffu, upper ? acc[i][j] : acc[i + 4][j], 16);
-        float* to = part_s + (warp * SC_TOKENS + group + 4 * i + (upper ? 16 : 0)) * SC_COLS + cols;
-        *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4*>(to + 16) = make_float4(v[4], v[5], v[6], v[7]);
-      }
-    }
-    const bool wild = __syncthreads_or(!(zero == 0.f));      // the chunk's x holds infinities or NaN
-    if (owner) {
+        for (int p = 0; p < 3; ++p) piece(chunk, m * 3 + p, a[m][p]);
+      unsigned b[4][3][2];                               // eight columns each
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          xm_cut(s[e >> 1][j][2 * (e & 1)], s[e >> 1][j][2 * (e & 1) + 1], b[e][0][j], b[e][1][j], b[e][2][j]);
+      float d[2][4][4] = {};
+      xm_products(d, a, b);
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          // columns in eights change places so that the rows of a store lie on different banks
+          const int row = m * 16 + g, at = (warp * SC_TOKENS + row) * SC_COLS + ((e ^ (row & 3)) * 8) + 2 * c;
+          *reinterpret_cast<float2*>(part_s + at) = make_float2(d[m][e][0], d[m][e][1]);
+          *reinterpret_cast<float2*>(part_s + at + 8 * SC_COLS) = make_float2(d[m][e][2], d[m][e][3]);
+        }
       // the matrix moves on by the chunk
-      const float all = stage[kSsG + SC_TOKENS - 1];
+      const float all = *reinterpret_cast<const float*>(stage + kSsG + (SC_TOKENS - 1) * 4);
+      const uint4* u_s = reinterpret_cast<const uint4*>(stage) + lane;
+      float more[2][2][4] = {};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) S[i] = make_float4(S[i].x * all, S[i].y * all, S[i].z * all, S[i].w * all);
-#pragma unroll 8
-      for (int s = 0; s < SC_TOKENS; ++s) {
-        const float4 lo = *reinterpret_cast<const float4*>(stage + kSsB + s * SC_DIM + row);
-        const float4 hi = *reinterpret_cast<const float4*>(stage + kSsB + s * SC_DIM + row + 4);
-        const float4 u = *reinterpret_cast<const float4*>(u_s + s * SC_COLS + c4);
-        sc_add(S[0], lo.x, u); sc_add(S[1], lo.y, u); sc_add(S[2], lo.z, u); sc_add(S[3], lo.w, u);
-        sc_add(S[4], hi.x, u); sc_add(S[5], hi.y, u); sc_add(S[6], hi.z, u); sc_add(S[7], hi.w, u);
+      for (int t = 0; t < 2; ++t) {
+        unsigned u[2][3][4], k[2][3][2];                 // B of 16 tokens: [eight channels][piece]
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          unsigned v[4];
+          piece(chunk, 6 + t * 3 + p, v);
+          k[0][p][0] = v[0]; k[0][p][1] = v[1]; k[1][p][0] = v[2]; k[1][p][1] = v[3];
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(u[e][p]) = u_s[((e * 2 + t) * 3 + p) * 32];
+        xm_products(more, u, k);
       }
+      fetch(chunk + 2);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(s_s + (row + i) * SC_COLS + c4) = S[i];
-    } else {
-      // rows t - 16 and t, four columns of each
-      const int at[2] = {t - 16, t};
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(all, s[e][j][i], more[e][j][i]);
+      __syncthreads();                                   // the partial sums and the next stage are in place
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+          if (channel + 8 * j < N)
+            *reinterpret_cast<float2*>(mine + (size_t)(e * 16 + i * 4) * N + j * 8) = *reinterpret_cast<const float2*>(&s[e][j][i]);
+  } else {
+    const int w = warp - 8, id = threadIdx.x - 256;
+    const float* base = here + (size_t)groups * kScPieces + (size_t)h * kScRecord;
+    const float* x_in = xbc + (size_t)h * P + col0;
+    const float d = skip[h];
+    const int t = id >> 3, c4 = (id & 7) * 4;            // of x, M and the outputs: rows t and t + 16, four columns
+    float uu[8], weight[4];                              // columns g, g + 8 of half w / 2, tokens 16 (w % 2) + 2 c, + 1 and 8 behind
+    auto load = [&](int chunk) {
+      const float* rec = base + (size_t)chunk * place;
+      const size_t at0 = (size_t)(first + chunk * SC_TOKENS) * channels;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = (w & 1) * 16 + 2 * c + (i & 1) + (i >> 2) * 8, col = (w >> 1) * 16 + g + (i >> 1 & 1) * 8;
+        uu[i] = chunk * SC_TOKENS + row < n ? x_in[at0 + (size_t)row * channels + col] : 0.f;
+        if (!(i & 2)) weight[(i & 1) + (i >> 2) * 2] = rec[kScR + row];       // used a chunk later, as is x
+      }
+    };
+    auto put = [&](int chunk) {
+      unsigned char* stage = ss_raw + chunk % 3 * kSsStage;
+      const float* rec = base + (size_t)chunk * place;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int row = t + 16 * e;
+        const bool in = chunk * SC_TOKENS + row < n;
+        sc_copy16(reinterpret_cast<float*>(stage + kSsX + (row * SC_COLS + c4) * 4),
+                  x_in + (in ? (size_t)(first + chunk * SC_TOKENS + row) * channels + c4 : 0), in);
+        sc_copy16(reinterpret_cast<float*>(stage + kSsM + (row * kScPairs + c4) * 4), rec + row * SC_TOKENS + c4, true);
+      }
+      if (id < SC_TOKENS / 4) sc_copy16(reinterpret_cast<float*>(stage + kSsG + id * 16), rec + kScG + id * 4, true);
+      unsigned p[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        xm_cut(weight[i & 2] * uu[2 * i], weight[(i & 2) + 1] * uu[2 * i + 1], p[0][i], p[1][i], p[2][i]);
+      uint4* to = reinterpret_cast<uint4*>(stage) + w * 3 * 32 + lane;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) to[q * 32] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+    };
+    auto outputs = [&](int chunk) {
+      const unsigned char* stage = ss_raw + chunk % 3 * kSsStage;
+      const float* part_s = reinterpret_cast<const float*>(ss_raw + kSsPart) + (chunk & 1) * 8 * SC_TOKENS * SC_COLS;
+      const float* m_row = reinterpret_cast<const float*>(stage + kSsM) + t * kScPairs;
+      const float4* x_s = reinterpret_cast<const float4*>(stage + kSsX) + (id & 7);
       float4 sum[2], acc[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         sum[e] = acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float4 v = *reinterpret_cast<const float4*>(part_s + (i * SC_TOKENS + at[e]) * SC_COLS + c4);
+          const float4 v = *reinterpret_cast<const float4*>(part_s + (i * SC_TOKENS + t + 16 * e) * SC_COLS + (c4 ^ ((t & 3) * 8)));
           sum[e].x += v.x; sum[e].y += v.y; sum[e].z += v.z; sum[e].w += v.w;
         }
       }
-      // M is 0 behind a row's own token; where an infinity or a NaN stands there it is left out, not added with weight 0
-      auto rows = [&](auto all) {
+      // what comes behind a row's own token is left out, not added with weight 0: an infinity or a NaN there is not this row's
 #pragma unroll
-        for (int s = 0; s < SC_TOKENS; s += 4) {
-          float4 m[2];
+      for (int s0 = 0; s0 < SC_TOKENS; s0 += 4) {
+        float4 m[2];
 #pragma unroll
-          for (int e = 0; e < 2; ++e) m[e] = *reinterpret_cast<const float4*>(stage + kSsM + at[e] * kScPairs + s);
+        for (int e = 0; e < 2; ++e) m[e] = *reinterpret_cast<const float4*>(m_row + 16 * e * kScPairs + s0);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 x = *reinterpret_cast<const float4*>(stage + kSsX + (s + i) * SC_COLS + c4);
+        for (int i = 0; i < 4; ++i) {
+          const float4 v = x_s[(s0 + i) * 8];
 #pragma unroll
-            for (int e = 0; e < 2; ++e)
-              if (decltype(all)::value || s + i <= at[e])
-                sc_add(acc[e], i == 0 ? m[e].x : i == 1 ? m[e].y : i == 2 ? m[e].z : m[e].w, x);
-          }
+          for (int e = 0; e < 2; ++e)
+            if (s0 + i <= 16 * e || (s0 + i < 16 * e + 16 && s0 + i <= t + 16 * e))
+              sc_add(acc[e], i == 0 ? m[e].x : i == 1 ? m[e].y : i == 2 ? m[e].z : m[e].w, v);
         }
-      };
-      if (wild) rows(sc_bool<false>());
-      else rows(sc_bool<true>());
+      }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int token = c * SC_TOKENS + at[e];
-        sc_add(acc[e], d, *reinterpret_cast<const float4*>(stage + kSsX + at[e] * SC_COLS + c4));
-        sc_add(acc[e], stage[kSsG + at[e]], sum[e]);
+        const int row = t + 16 * e, token = chunk * SC_TOKENS + row;
+        sc_add(acc[e], d, x_s[row * 8]);
+        sc_add(acc[e], *reinterpret_cast<const float*>(stage + kSsG + row * 4), sum[e]);
         if (token < n) *reinterpret_cast<float4*>(y_out + ((size_t)(first + token) * heads + h) * P + col0 + c4) = acc[e];
       }
-    }
-  }
-  if (owner) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (row + 4 * e < N) {
-        const float4* v = S + 4 * e;
-        *reinterpret_cast<float4*>(mine + 4 * e) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-        *reinterpret_cast<float4*>(mine + (size_t)N + 4 * e) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-        *reinterpret_cast<float4*>(mine + (size_t)2 * N + 4 * e) = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
-        *reinterpret_cast<float4*>(mine + (size_t)3 * N + 4 * e) = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
+    };
+    load(0);
+    put(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (chunks > 1) load(1);
+    __syncthreads();
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      if (chunk + 1 < chunks) {                          // three stages: what the one before the last held is read by now
+        put(chunk + 1);
+        if (chunk + 2 < chunks) load(chunk + 2);
       }
+      if (chunk > 0) outputs(chunk - 1);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+    }
+    outputs(chunks - 1);
   }
 }
 
@@ -320,8 +372,8 @@ TOKB200_API int tokb200_ssd_chunks_supported(int P, int N) {
 }
 
 // Floats of the records of a step.
-TOKB200_API long long tokb200_ssd_chunk_floats(int n_rows, int n_requests, int heads) {
-  return ((long long)n_rows / SC_TOKENS + n_requests) * heads * kScRecord;
+TOKB200_API long long tokb200_ssd_chunk_floats(int n_rows, int n_requests, int heads, int groups) {
+  return ((long long)n_rows / SC_TOKENS + n_requests) * (long long)sc_place(heads, groups);
 }
 
 TOKB200_API int tokb200_ssd_chunks(const float* xbc, int channels, const void* proj, int proj_dtype, int ld, int dt_at,
@@ -351,7 +403,7 @@ TOKB200_API int tokb200_ssd_chunks(const float* xbc, int channels, const void* p
                               (const __nv_bfloat16*)proj + dt_at, ld, dt_bias, a_log, heads, groups, P, N, q_start, n_requests,
                               records);
   if (status != TOKB200_OK) return status;
-  return launch_dependent(ssd_chunk_scan_kernel, dim3(P / SC_COLS, heads, n_requests), dim3(SC_THREADS),
+  return launch_dependent(ssd_chunk_scan_kernel, dim3(P / SC_COLS, heads, n_requests), dim3(SC_SCAN_THREADS),
                           (size_t)kSsBytes, stream, xbc, channels, records, skip, heads, groups, P, N, state, stride, q_start,
                           state_slot, y);
 }

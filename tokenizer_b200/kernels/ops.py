@@ -1797,7 +1797,7 @@ def ssd_chunks(xbc: torch.Tensor, proj: torch.Tensor, dt_at: int, dt_bias, a_log
         raise ValueError("ssd_chunks: sizes of the inputs, the state or the output disagree")
     lib = _lib("ssd_chunks")
     lib.tokb200_ssd_chunk_floats.restype = ctypes.c_longlong
-    records = torch.empty(lib.tokb200_ssd_chunk_floats(_i(n), _i(requests), _i(heads)), dtype=torch.float32, device=xbc.device)
+    records = torch.empty(lib.tokb200_ssd_chunk_floats(_i(n), _i(requests), _i(heads), _i(groups)), dtype=torch.float32, device=xbc.device)
     _check(lib.tokb200_ssd_chunks(
         _ptr(xbc), _i(xbc.shape[1]), _sliced_ptr(proj), _i(_tag(proj)), _i(_ld(proj)), _i(dt_at), _ptr(dt_bias), _ptr(a_log),
         _ptr(skip), _i(heads), _i(groups), _i(vdim), _i(n_state), _ptr(state), _ll(state.shape[1]), _ptr(q_start),
