@@ -124,9 +124,16 @@ __device__ __forceinline__ float mc_before(const McArgs& a, const McChunk& m, in
 }
 
 __device__ __forceinline__ void mc_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the sums of the pieces, the smallest first
+__device__ __forceinline__ void mc_sum(float (&to)[2][4], const float (&part)[3][2][4]) {
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) to[n][e] = (part[2][n][e] + part[1][n][e]) + part[0][n][e];
 }
 __device__ __forceinline__ void mc_ldmatrix(unsigned (&r)[4], const __nv_bfloat16* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -259,17 +266,18 @@ __global__ void __launch_bounds__(MC_STATE_THREADS) mlstm_chunk_states_kernel(co
 #pragma unroll
       for (int p = 0; p < 3; ++p) mc_ldmatrix_trans(b[k][p], mc_b_trans(k_s + p * MC_L * MC_PITCH, n * 16, k * 16, lane));
     for (int r = 0; r < dv; ++r) {
-      float acc[2][4] = {};
+      float part[3][2][4] = {}, acc[2][4];               // a sum a piece: each product waits only for its own sum's last
 #pragma unroll
       for (int k = 0; k < MC_L / 16; ++k) {
         unsigned v[4];
         mc_ldmatrix_trans(v, mc_a_trans(v_s, r * 16, k * 16, lane));
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
-          mc_mma(acc[0], v, b[k][p][0], b[k][p][1]);
-          mc_mma(acc[1], v, b[k][p][2], b[k][p][3]);
+          mc_mma(part[p][0], v, b[k][p][0], b[k][p][1]);
+          mc_mma(part[p][1], v, b[k][p][2], b[k][p][3]);
         }
       }
+      mc_sum(acc, part);
       const int g = lane >> 2, q = lane & 3;
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -424,17 +432,20 @@ __global__ void __launch_bounds__(MC_OUT_THREADS, 2) mlstm_chunk_outputs_kernel(
     if (j + 1 < first_half) fetch_columns(j + 1);
     __syncthreads();
     if (j < my_tiles) {
+      float part[3][2][4] = {};                         // a sum a piece: each product waits only for its own sum's last
+#pragma unroll 2
       for (int k = 0; k < dk; ++k) {
-        unsigned aq[4];
+        unsigned aq[4], b[3][4];
         mc_ldmatrix(aq, mc_a(q_s, rt * 16, k * 16, lane));
 #pragma unroll
+        for (int p = 0; p < 3; ++p) mc_ldmatrix(b[p], mc_b(S_s + p * 32 * MC_PITCH, half * 16, k * 16, lane));
+#pragma unroll
         for (int p = 0; p < 3; ++p) {
-          unsigned b[4];
-          mc_ldmatrix(b, mc_b(S_s + p * 32 * MC_PITCH, half * 16, k * 16, lane));
-          mc_mma(acc[j][0], aq, b[0], b[1]);
-          mc_mma(acc[j][1], aq, b[2], b[3]);
+          mc_mma(part[p][0], aq, b[p][0], b[p][1]);
+          mc_mma(part[p][1], aq, b[p][2], b[p][3]);
         }
       }
+      mc_sum(acc[j], part);
     }
   }
   // ---- n_0 . q: four threads a token ----
@@ -459,13 +470,24 @@ __global__ void __launch_bounds__(MC_OUT_THREADS, 2) mlstm_chunk_outputs_kernel(
   // ---- the chunk's own keys, 16 at a time, up to this warp's rows ----
   float own_lo = 0.f, own_hi = 0.f;
   for (int st = 0; st <= rt; ++st) {
-    float score[2][4] = {};
-    for (int k = 0; k < dk; ++k) {
+    float score[2][4] = {}, odd[2][4] = {};
+    for (int k = 0; k < dk; k += 2) {
       unsigned aq[4], b[4];
       mc_ldmatrix(aq, mc_a(q_s, rt * 16, k * 16, lane));
       mc_ldmatrix(b, mc_b(k_s, st * 16, k * 16, lane));
       mc_mma(score[0], aq, b[0], b[1]);
       mc_mma(score[1], aq, b[2], b[3]);
+      if (k + 1 < dk) {
+        mc_ldmatrix(aq, mc_a(q_s, rt * 16, k * 16 + 16, lane));
+        mc_ldmatrix(b, mc_b(k_s, st * 16, k * 16 + 16, lane));
+        mc_mma(odd[0], aq, b[0], b[1]);
+        mc_mma(odd[1], aq, b[2], b[3]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      score[0][e] += odd[0][e];
+      score[1][e] += odd[1][e];
     }
     unsigned w[3][4];
 #pragma unroll
@@ -486,17 +508,18 @@ __global__ void __launch_bounds__(MC_OUT_THREADS, 2) mlstm_chunk_outputs_kernel(
         w[p][2 * n + 1] = mc_two(c2[p], c3[p]);
       }
     }
+    unsigned b[MC_OUT_TILES][4];
 #pragma unroll
-    for (int j = 0; j < MC_OUT_TILES; ++j) {
-      if (j >= my_tiles) break;
-      unsigned b[4];
-      mc_ldmatrix_trans(b, mc_b_trans(v_s, (my_first + j) * 16, st * 16, lane));
+    for (int j = 0; j < MC_OUT_TILES; ++j)
+      if (j < my_tiles) mc_ldmatrix_trans(b[j], mc_b_trans(v_s, (my_first + j) * 16, st * 16, lane));
 #pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        mc_mma(acc[j][0], w[p], b[0], b[1]);
-        mc_mma(acc[j][1], w[p], b[2], b[3]);
-      }
-    }
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+      for (int j = 0; j < MC_OUT_TILES; ++j)
+        if (j < my_tiles) {
+          mc_mma(acc[j][0], w[p], b[j][0], b[j][1]);
+          mc_mma(acc[j][1], w[p], b[j][2], b[j][3]);
+        }
   }
   own_lo += __shfl_xor_sync(0xffffffffu, own_lo, 1);
   own_lo += __shfl_xor_sync(0xffffffffu, own_lo, 2);
