@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   float* a_s = r_s + 16 * kDcStride;                    // [32][36]
   float* m_s = a_s + DC_TOKENS * kDcPairs;              // [32][36]
   float* beta_s = m_s + DC_TOKENS * kDcPairs;           // [32]
+  float* v_s = beta_s + DC_TOKENS;                      // [32][132]
   const int place = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the request whose chunks lie around this place: the last one that begins at or before it
@@ -121,34 +122,61 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
 
   const int l = threadIdx.x & (DC_DIM - 1), half = threadIdx.x / DC_DIM;
   // ---- convolution and silu, a channel a thread: threads 0 .. 127 take q and the first half of k's tokens, the others v
-  // (kept in registers) and the second half; all inputs are asked for before the first is used ----
-  float col[DC_TOKENS], key[DC_TOKENS / 2], pre[DC_TOKENS / 2];
+  // and the second half.  A thread brings its own channels' inputs to where their results will lie (32-bit ones as copies
+  // that it does not wait for one by one) and walks over them; short loops: the block runs this code once, and what it
+  // waited for most was the code itself ----
   const int a_lanes = half ? a.vdim : a.dim;
   const int a_ch = half ? 2 * a.groups * a.dim + h * a.vdim + l : group * a.dim + l, k_ch = (a.groups + group) * a.dim + l;
   const int k0 = half * (DC_TOKENS / 2);
+  float* a_to = (half ? v_s : q_s) + l;
   // an input `back` places before the portion's start is the kept one that many from the end
   auto input = [&](int ch, int at) {
     return at >= 0 ? to_float(proj[(size_t)(start + at) * a.ld + a.qkv_at + ch]) : kept[(size_t)(a.taps - 1 + at) * channels + ch];
   };
+  auto bring = [&](float* to, const auto* from, int ld, int n, bool on) {
+#pragma unroll 8
+    for (int t = 0; t < n; ++t) {
+      const bool in = on && t < n_here;
+      if constexpr (sizeof(*from) == 4) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to + t * kDcStride)),
+                     "l"(from + (in ? (size_t)t * ld : 0)), "r"(in ? 4 : 0) : "memory");
+      } else {
+        to[t * kDcStride] = in ? to_float(from[(size_t)t * ld]) : 0.f;
+      }
+    }
+  };
+  bring(a_to, proj + (size_t)t0 * a.ld + a.qkv_at + (l < a_lanes ? a_ch : 0), a.ld, DC_TOKENS, l < a_lanes);
+  {
+    const T* from = proj + (size_t)t0 * a.ld + a.qkv_at + (l < a.dim ? k_ch : 0);
+#pragma unroll 8
+    for (int t = k0; t < k0 + DC_TOKENS / 2; ++t) {
+      const bool in = l < a.dim && t < n_here;
+      if constexpr (sizeof(T) == 4) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(k_s + t * kDcStride + l)),
+                     "l"(from + (in ? (size_t)t * a.ld : 0)), "r"(in ? 4 : 0) : "memory");
+      } else {
+        k_s[t * kDcStride + l] = in ? to_float(from[(size_t)t * a.ld]) : 0.f;
+      }
+    }
+  }
+  float pre[4];
   if (BY_CHANNEL) {
-    const float* raw = static_cast<const float*>(a.decay) + a.decay_at + h * a.dim + l;
-#pragma unroll
-    for (int i = 0; i < DC_TOKENS / 2; ++i)
-      pre[i] = half + 2 * i < n_here && l < a.dim ? raw[(size_t)(t0 + half + 2 * i) * a.decay_ld] : 0.f;
+    const float* raw = static_cast<const float*>(a.decay) + a.decay_at + (l < a.dim ? h * a.dim + l : 0);
+#pragma unroll 8
+    for (int t = half; t < DC_TOKENS; t += 2) {
+      const bool in = l < a.dim && t < n_here;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(g_s + t * kDcStride + l)),
+                   "l"(raw + (in ? (size_t)(t0 + t) * a.decay_ld : 0)), "r"(in ? 4 : 0) : "memory");
+    }
   } else {
     const T* raw = static_cast<const T*>(a.decay) + a.decay_at + h;
 #pragma unroll
     for (int i = 0; i < 4; ++i) pre[i] = warp + 8 * i < n_here ? to_float(raw[(size_t)(t0 + warp + 8 * i) * a.decay_ld]) : 0.f;
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
   auto silu = [](float v) { return v * dc_sigmoid(v); };
   if (a.taps == 4) {
-    const T* a_in = proj + a.qkv_at + a_ch;
-    const T* k_in = proj + a.qkv_at + k_ch;
-    float ax[3], kx[3], aw[4], kw[4];
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) col[t] = t < n_here && l < a_lanes ? to_float(a_in[(size_t)(t0 + t) * a.ld]) : 0.f;
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS / 2; ++t) key[t] = k0 + t < n_here && l < a.dim ? to_float(k_in[(size_t)(t0 + k0 + t) * a.ld]) : 0.f;
+    float aw[4], kw[4], ax[3], kx[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       ax[j] = l < a_lanes ? input(a_ch, at0 - 3 + j) : 0.f;
@@ -159,44 +187,38 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
       aw[j] = l < a_lanes ? a.conv_w[(size_t)a_ch * 4 + j] : 0.f;
       kw[j] = l < a.dim ? a.conv_w[(size_t)k_ch * 4 + j] : 0.f;
     }
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) {
-      const float x = col[t], v = fmaf(aw[3], x, fmaf(aw[2], ax[2], fmaf(aw[1], ax[1], aw[0] * ax[0])));
-      col[t] = t < n_here ? silu(v) : 0.f;
-      ax[0] = ax[1]; ax[1] = ax[2]; ax[2] = x;
-    }
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS / 2; ++t) {
-      const float x = key[t], v = fmaf(kw[3], x, fmaf(kw[2], kx[2], fmaf(kw[1], kx[1], kw[0] * kx[0])));
-      key[t] = k0 + t < n_here ? silu(v) : 0.f;
-      kx[0] = kx[1]; kx[1] = kx[2]; kx[2] = x;
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    auto walk = [&](float* at, int n, int from, const float (&w)[4], float (&before)[3]) {
+#pragma unroll 4
+      for (int t = 0; t < n; ++t) {
+        const float x = at[t * kDcStride], v = fmaf(w[3], x, fmaf(w[2], before[2], fmaf(w[1], before[1], w[0] * before[0])));
+        at[t * kDcStride] = from + t < n_here ? silu(v) : 0.f;
+        before[0] = before[1]; before[1] = before[2]; before[2] = x;
+      }
+    };
+    walk(a_to, DC_TOKENS, 0, aw, ax);
+    walk(k_s + k0 * kDcStride + l, DC_TOKENS / 2, k0, kw, kx);
   } else {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     auto sum = [&](int ch, int t) {
       float v = 0.f;
       for (int j = 0; j < a.taps; ++j) v = fmaf(a.conv_w[(size_t)ch * a.taps + j], input(ch, at0 + t - (a.taps - 1 - j)), v);
       return silu(v);
     };
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) col[t] = t < n_here && l < a_lanes ? sum(a_ch, t) : 0.f;
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS / 2; ++t) key[t] = k0 + t < n_here && l < a.dim ? sum(k_ch, k0 + t) : 0.f;
+#pragma unroll 1
+    for (int t = 0; t < DC_TOKENS; ++t) a_to[t * kDcStride] = t < n_here && l < a_lanes ? sum(a_ch, t) : 0.f;
+#pragma unroll 1
+    for (int t = k0; t < k0 + DC_TOKENS / 2; ++t) k_s[t * kDcStride + l] = t < n_here && l < a.dim ? sum(k_ch, t) : 0.f;
   }
-  if (!half) {
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) q_s[t * kDcStride + l] = col[t];
-  }
-#pragma unroll
-  for (int t = 0; t < DC_TOKENS / 2; ++t) k_s[(k0 + t) * kDcStride + l] = key[t];
   // ---- decays and beta; A and M start as zeros ----
   {
     const float rate = expf(a.a_log[h]);
     if (BY_CHANNEL) {
       const float shift = l < a.dim ? a.dt_bias[h * a.dim + l] : 0.f;
-#pragma unroll
-      for (int i = 0; i < DC_TOKENS / 2; ++i) {
-        const int t = half + 2 * i;
-        g_s[t * kDcStride + l] = t < n_here && l < a.dim ? expf(-rate * dc_softplus(pre[i] + shift)) : 1.f;
+#pragma unroll 2
+      for (int t = half; t < DC_TOKENS; t += 2) {
+        float* at = g_s + t * kDcStride + l;
+        *at = t < n_here && l < a.dim ? expf(-rate * dc_softplus(*at + shift)) : 1.f;
       }
     } else {
 #pragma unroll
@@ -324,13 +346,8 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   }
   __syncthreads();
   // ---- (I + A) W = beta G k and (I + A) U0 = beta v, a column of both a thread of the first half (a row of A is read
-  // once for the two); the second half writes the scaled queries and keys and M meanwhile ----
-  if (half) {
-#pragma unroll
-    for (int t = 0; t < DC_TOKENS; ++t) l_s[t * kDcStride + l] = col[t];
-  }
-  __syncthreads();
-  float other[DC_TOKENS];
+  // once for the two); the second half scales the queries and keys and writes M meanwhile ----
+  float col[DC_TOKENS], other[DC_TOKENS];
   if (!half) {
     float upto = 1.f;
 #pragma unroll
@@ -338,7 +355,7 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
       const float beta = beta_s[t];
       upto *= g_s[t * kDcStride + l];
       col[t] = beta * (upto * k_s[t * kDcStride + l]);
-      other[t] = beta * l_s[t * kDcStride + l];
+      other[t] = beta * v_s[t * kDcStride + l];
     }
   }
   __syncthreads();                                       // the keys' rows are read
@@ -406,7 +423,7 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
     for (int q = 0; q < 3; ++q) to[q * 32] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
   }
 }
-constexpr int kDcPrepareSmem = (4 * DC_TOKENS * kDcStride + 16 * kDcStride + 2 * DC_TOKENS * kDcPairs + DC_TOKENS) * 4;
+constexpr int kDcPrepareSmem = (5 * DC_TOKENS * kDcStride + 16 * kDcStride + 2 * DC_TOKENS * kDcPairs + DC_TOKENS) * 4;
 
 // ---- the chunks one after another --------------------------------------------------------------------------------
 // The products run on the tensor cores with their operands in exact pieces (exact_mma.cuh).
