@@ -90,7 +90,9 @@ class bound_stream:
         return False
 
 
-_i, _f, _ll = ctypes.c_int, ctypes.c_float, ctypes.c_longlong
+# a Python integer is passed as a C int as it is (a c_int object each would cost a tenth of a microsecond, a layer passes
+# more than a hundred)
+_i, _f, _ll = int, ctypes.c_float, ctypes.c_longlong
 
 
 class ScratchSpace:
@@ -166,8 +168,14 @@ def _load(source: str, defines=()):
     return lib
 
 
+_libraries = {}             # name -> loaded library that knows the error word
+
+
 def _lib(name):
-    return _load(name + ".cu")
+    lib = _libraries.get(name)
+    if lib is None:
+        lib = _libraries[name] = _load(name + ".cu")
+    return lib
 
 
 def error_code() -> int:

@@ -127,11 +127,11 @@ def linear_bf16(a: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         ops.linear_stream(a, weight, bias, out)
         return out
-    if out_dtype == torch.bfloat16 and use_tcgen05(M, N, K) and use_pair(M, N, K):
+    if out_dtype == torch.bfloat16 and use_pair(M, N, K) and use_tcgen05(M, N, K):
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         ops.gemm_tcgen05_pair(a, weight, bias, out, ops.PAIR_PLAIN)
         return out
-    if partials_ok and bias is None and use_tcgen05(M, N, K) and use_pair_halves(M, N, K):
+    if partials_ok and bias is None and use_pair_halves(M, N, K) and use_tcgen05(M, N, K):
         out = torch.empty((2, M, N), dtype=torch.float32, device=a.device)
         ops.gemm_tcgen05_pair(a, weight, None, out, ops.PAIR_PARTIALS)
         return out
