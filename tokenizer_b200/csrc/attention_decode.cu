@@ -548,7 +548,13 @@ TOKB200_API int tokb200_decode_attention(
     }
     const double per_pass = 2.0 * HEAD_DIM / 64.0;
     double best = 1e30;
-    for (int c = DEC_MIN_CHUNK; c <= 4096; c += DEC_BLOCK_KEYS) {
+    // Where the (row, kv head) pairs alone fill the device, a row may also stay whole beyond 4,096 keys: no piece starts, none
+    // is merged (64 rows over 8,192 keys, 4 kv heads of size 128, us at the best piece of up to 4,096 keys / whole: rows of one
+    // length 210 / 183, from 8,192 down to 2,048 148 / 115, these shuffled 145 / 143; with 2 kv heads, 128 pairs, 73 / 87).
+    // Up to some 8,192: a lone long row among short ones is then one block's chain of 34 passes at most (tables reach a page
+    // or two further than the rows they were made for).
+    const int longest = pairs >= have ? 8192 + 512 : 4096;
+    for (int c = DEC_MIN_CHUNK; c <= longest; c += DEC_BLOCK_KEYS) {
       int chunk = c;
       while ((reach + chunk - 1) / chunk > DEC_MAX_SPLITS) chunk <<= 1;
       const long long pieces = (reach + chunk - 1) / chunk;
