@@ -501,6 +501,32 @@ TOKB200_API long long tokb200_decode_attention_scratch_floats(int n_rows, int nh
 
 TOKB200_API int tokb200_decode_attention_head_dim() { return HEAD_DIM; }
 
+// Clusters of `size` blocks that the device holds at once (asked once a size; all that fit by count where it cannot be asked).
+static long long clusters_at_once(int size, size_t smem) {
+  static long long known[DEC_CLUSTER_MAX + 1] = {};
+  if (!known[size]) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(size, 1, 1);
+    config.blockDim = dim3(DEC_THREADS);
+    config.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = size;
+    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute(decode_attention_kernel<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, decode_attention_kernel<true, true, false>, &config) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 1 << 30;
+    }
+    known[size] = n;
+  }
+  return known[size];
+}
+
 // `counters` holds n_rows * nkv ints, zero before the first launch; every launch
 // leaves them zero again.  `rows` (optional, n_rows ints): the batch rows to serve, -1 for none;
 // without it the launch serves rows 0 .. n_rows - 1.
@@ -581,7 +607,11 @@ TOKB200_API int tokb200_decode_attention(
   // pieces than the grid stays until its siblings are done, which costs nothing in a single wave
   // and a quarter of the device's block slots in a long run of uneven rows (64 rows of 4,900 to
   // 8,192 keys, head size 128: 227 us with clusters, 172 us through scratch memory)
-  const bool cluster = clusters_allowed && most <= DEC_CLUSTER_MAX && pairs * most <= slots;
+  // ... which clusters are only as far as they fit the device's groups of multiprocessors: 16 clusters of 8 blocks are 128
+  // blocks, and 148 multiprocessors do not hold them (4 rows of 2,000 keys, 4 kv heads of size 128: 15.4 us in two waves of
+  // clusters, 9.8 through scratch memory)
+  const bool cluster = clusters_allowed && most <= DEC_CLUSTER_MAX && pairs * most <= slots &&
+                       (most == 1 || pairs <= clusters_at_once((int)most, smem));
   // pieces of up to two passes: the first tiles before the wait (see EARLY)
   const bool early = min_chunk <= 2 * DEC_BLOCK_KEYS;
   // one pool read as keys and as values, while a warp has two staging buffers (see ALIAS)
