@@ -125,3 +125,37 @@ def test_a_token_changes_nothing_before_it(by_channel, columns, value, at):
         if column >= 2 * dim:                                 # a value's column meets no other
             others = [c for c in range(heads * vdim) if c != column - 2 * dim]
             assert torch.equal(got[:, others], want[:, others])
+
+
+@pytest.mark.parametrize("by_channel", [False, True])
+@pytest.mark.parametrize("taps", [4, 2])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_inputs_off_16_bytes(by_channel, taps, shift):
+    """Copies of four channels or of one bring the same inputs: the same bits wherever the rows begin."""
+    o = ops()
+    groups, heads, dim, vdim, n = 1, 2, 72, 32, 75
+    channels = 2 * dim + heads * vdim
+    g = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    conv_w, a_log, dt_bias = rnd(channels, taps), rnd(heads), rnd(heads * (dim if by_channel else 1))
+    proj, rates = rnd(n, channels + 2 * heads), rnd(n, heads * dim)
+    first = rnd(1, heads * vdim * 128 + (taps - 1) * channels)
+    first[:, :heads * vdim * 128].view(-1, 128)[:, dim:] = 0
+    q_start = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+
+    def moved(t, by):                                  # the same rows, `by` floats behind an aligned place
+        room = torch.empty(t.numel() + 4, device=DEV)
+        room[by:by + t.numel()] = t.reshape(-1)
+        return room[by:by + t.numel()].view(t.shape)
+
+    def run(by_proj, by_rates):
+        p, d = moved(proj, by_proj), moved(rates, by_rates)
+        out, state = torch.empty(n, heads * vdim, device=DEV), first.clone()
+        o.delta_chunks(p, 0, channels, d if by_channel else p, 0 if by_channel else channels + heads, by_channel, groups,
+                       heads, dim, vdim, taps, conv_w, a_log, dt_bias, state, heads * vdim * 128, q_start,
+                       torch.zeros(1, dtype=torch.int32, device=DEV), out)
+        return out, state
+    want = run(0, 0)
+    for moves in ((shift, 0), (0, shift), (shift, shift)):
+        for got, ref in zip(run(*moves), want):
+            assert torch.equal(got, ref)

@@ -15,18 +15,18 @@
 //                         halves of 32, 16 or 8 tokens are plain products of rows that were decayed to and from the
 //                         middle; inside four the decays are multiplied in key by key
 //   delta_chunk_scan      a block a (16 or 32 columns of a head's matrix, request): the chunks one after another.  The 64
-//                         x 128 rows of W and G q meet the columns in 8 x 4 or 8 x 8 register tiles, k cut over the eight
-//                         warps; the next chunk's record is on its way (cp.async) while this one is worked through
+//                         x 128 rows of W and G q meet the columns on the tensor cores (mma.sync), every 32-bit value as
+//                         three bfloat16 pieces that add up to it; the next chunk's pieces are on their way (cp.async, each
+//                         thread its own) while this one is worked through
 //
-// The scan is bound by reads of shared memory (counters: the pipe that brings them back busy 62 % of the time, the FMA
-// pipe 36 %): a register tile of R x C costs R + C cycles of the 128 bytes a cycle that come back, and R C / 4 of the
-// multiply-adds.  So tiles are as large as the threads allow, a row of A is read once for two columns, and half of a scan
-// block's threads own the whole matrix (4 x 4 or 8 x 4 of it each).  The prepare kernel waits for instructions most (more
-// than a quarter of its warps' time: a block runs its long unrolled code once), then for registers and shared memory; that
-// pipe is busy 36 % there.  Measured (16 heads of
-// 128 x 128, both kernels and the kept inputs between them, us; before: tiles of 4 x 4, pairs eight tokens at a time): a
-// prompt of 2,048 tokens 294 -> 254 with one decay a head and 328 -> 272 with one a channel, four prompts of 5,100 in all
-// 763 -> 537, eight of 256 316 -> 247.
+// The scan is one chain: a chunk's products need the matrix that the chunk before left.  Counters at 2,048 tokens: shared
+// memory's pipe busy 53 % of the time, the tensor cores 30 %; with FMA register tiles that pipe was busy 62 % and the scan of
+// 16 heads took 162 us where it now takes 111.  The prepare kernel is bound by latency, not by a pipe (instructions issue 39 %
+// of the time, two blocks of eight warps an SM by shared memory): loops that keep its code small made it slower (88.7 -> 100
+// us), loads and exponentials side by side faster (105 -> 94 us by head at 2,048, 239 -> 221 by
+// channel over four prompts).  Measured
+// (16 heads of 128 x 128, both kernels and the kept inputs between them, us; in front the FMA tiles): a prompt of 2,048
+// tokens 254 -> 200 with one decay a head and 272 -> 212 with one a channel, four prompts of 5,100 in all 537 -> 479.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).
@@ -62,6 +62,7 @@ struct DeltaChunkArgs {
   float* records;
   float q_scale;
   int groups, heads, dim, vdim, taps, conv_off, n_requests;
+  int quads;                 // 32-bit rows whose pieces of four channels lie on 16 bytes
 };
 
 // N sums of every lane over LANES neighbouring lanes, all N together: lanes give away the half of their sums that the
@@ -122,9 +123,9 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
 
   const int l = threadIdx.x & (DC_DIM - 1), half = threadIdx.x / DC_DIM;
   // ---- convolution and silu, a channel a thread: threads 0 .. 127 take q and the first half of k's tokens, the others v
-  // and the second half.  A thread brings its own channels' inputs to where their results will lie (32-bit ones as copies
-  // that it does not wait for one by one) and walks over them; short loops: the block runs this code once, and what it
-  // waited for most was the code itself ----
+  // and the second half.  The inputs come to where the results will lie, four channels a copy where they lie on 16 bytes; a
+  // thread then takes eight tokens at a time, all read before the first is written, so that eight chains of exponential and
+  // quotient run side by side (one by one a token took 195 cycles, a quarter of the block's time) ----
   const int a_lanes = half ? a.vdim : a.dim;
   const int a_ch = half ? 2 * a.groups * a.dim + h * a.vdim + l : group * a.dim + l, k_ch = (a.groups + group) * a.dim + l;
   const int k0 = half * (DC_TOKENS / 2);
@@ -133,42 +134,47 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   auto input = [&](int ch, int at) {
     return at >= 0 ? to_float(proj[(size_t)(start + at) * a.ld + a.qkv_at + ch]) : kept[(size_t)(a.taps - 1 + at) * channels + ch];
   };
-  auto bring = [&](float* to, const auto* from, int ld, int n, bool on) {
-#pragma unroll 8
-    for (int t = 0; t < n; ++t) {
-      const bool in = on && t < n_here;
-      if constexpr (sizeof(*from) == 4) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to + t * kDcStride)),
-                     "l"(from + (in ? (size_t)t * ld : 0)), "r"(in ? 4 : 0) : "memory");
+  if constexpr (sizeof(T) == 4) {
+    auto copy = [](float* to, const float* from, bool in, auto bytes) {
+      constexpr int n = decltype(bytes)::value;
+      if constexpr (n == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+                     "r"(in ? 16 : 0) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+                     "r"(in ? 4 : 0) : "memory");
+    };
+    auto bring = [&](float* to, const float* from, int ld, int lanes) {       // 32 rows
+      if (a.quads) {
+#pragma unroll
+        for (int t = warp; t < DC_TOKENS; t += DC_PREPARE_THREADS / 32) {
+          const bool in = lane * 4 < lanes && t < n_here;
+          copy(to + t * kDcStride + lane * 4, from + (in ? (size_t)t * ld + lane * 4 : 0), in, dc_int<16>());
+        }
       } else {
-        to[t * kDcStride] = in ? to_float(from[(size_t)t * ld]) : 0.f;
-      }
-    }
-  };
-  bring(a_to, proj + (size_t)t0 * a.ld + a.qkv_at + (l < a_lanes ? a_ch : 0), a.ld, DC_TOKENS, l < a_lanes);
-  {
-    const T* from = proj + (size_t)t0 * a.ld + a.qkv_at + (l < a.dim ? k_ch : 0);
 #pragma unroll 8
-    for (int t = k0; t < k0 + DC_TOKENS / 2; ++t) {
-      const bool in = l < a.dim && t < n_here;
-      if constexpr (sizeof(T) == 4) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(k_s + t * kDcStride + l)),
-                     "l"(from + (in ? (size_t)t * a.ld : 0)), "r"(in ? 4 : 0) : "memory");
-      } else {
-        k_s[t * kDcStride + l] = in ? to_float(from[(size_t)t * a.ld]) : 0.f;
+        for (int t = half; t < DC_TOKENS; t += 2) {
+          const bool in = l < lanes && t < n_here;
+          copy(to + t * kDcStride + l, from + (in ? (size_t)t * ld + l : 0), in, dc_int<4>());
+        }
       }
-    }
+    };
+    const float* row = proj + (size_t)t0 * a.ld + a.qkv_at;
+    bring(q_s, row + group * a.dim, a.ld, a.dim);
+    bring(k_s, row + (a.groups + group) * a.dim, a.ld, a.dim);
+    bring(v_s, row + 2 * a.groups * a.dim + h * a.vdim, a.ld, a.vdim);
+    if (BY_CHANNEL)
+      bring(g_s, static_cast<const float*>(a.decay) + (size_t)t0 * a.decay_ld + a.decay_at + h * a.dim, a.decay_ld, a.dim);
+  } else {
+#pragma unroll 8
+    for (int t = 0; t < DC_TOKENS; ++t)
+      a_to[t * kDcStride] = l < a_lanes && t < n_here ? to_float(proj[(size_t)(t0 + t) * a.ld + a.qkv_at + a_ch]) : 0.f;
+#pragma unroll 8
+    for (int t = k0; t < k0 + DC_TOKENS / 2; ++t)
+      k_s[t * kDcStride + l] = l < a.dim && t < n_here ? to_float(proj[(size_t)(t0 + t) * a.ld + a.qkv_at + k_ch]) : 0.f;
   }
   float pre[4];
-  if (BY_CHANNEL) {
-    const float* raw = static_cast<const float*>(a.decay) + a.decay_at + (l < a.dim ? h * a.dim + l : 0);
-#pragma unroll 8
-    for (int t = half; t < DC_TOKENS; t += 2) {
-      const bool in = l < a.dim && t < n_here;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(g_s + t * kDcStride + l)),
-                   "l"(raw + (in ? (size_t)(t0 + t) * a.decay_ld : 0)), "r"(in ? 4 : 0) : "memory");
-    }
-  } else {
+  if (!BY_CHANNEL) {
     const T* raw = static_cast<const T*>(a.decay) + a.decay_at + h;
 #pragma unroll
     for (int i = 0; i < 4; ++i) pre[i] = warp + 8 * i < n_here ? to_float(raw[(size_t)(t0 + warp + 8 * i) * a.decay_ld]) : 0.f;
@@ -188,18 +194,34 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
       kw[j] = l < a.dim ? a.conv_w[(size_t)k_ch * 4 + j] : 0.f;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    auto walk = [&](float* at, int n, int from, const float (&w)[4], float (&before)[3]) {
-#pragma unroll 4
-      for (int t = 0; t < n; ++t) {
-        const float x = at[t * kDcStride], v = fmaf(w[3], x, fmaf(w[2], before[2], fmaf(w[1], before[1], w[0] * before[0])));
-        at[t * kDcStride] = from + t < n_here ? silu(v) : 0.f;
-        before[0] = before[1]; before[1] = before[2]; before[2] = x;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 0; i < 6; ++i) {                        // four times eight tokens of q or v, twice of k
+      const bool of_k = i >= 4;
+      const int from = of_k ? k0 + (i - 4) * 8 : i * 8;
+      float* at = (of_k ? k_s + l : a_to) + from * kDcStride;
+      if (i == 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) aw[j] = kw[j];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) ax[j] = kx[j];
       }
-    };
-    walk(a_to, DC_TOKENS, 0, aw, ax);
-    walk(k_s + k0 * kDcStride + l, DC_TOKENS / 2, k0, kw, kx);
+      float x[11];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) x[j] = ax[j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[3 + j] = at[j * kDcStride];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) ax[j] = x[8 + j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        x[j] = silu(fmaf(aw[3], x[3 + j], fmaf(aw[2], x[2 + j], fmaf(aw[1], x[1 + j], aw[0] * x[j]))));
+#pragma unroll
+      for (int j = 0; j < 8; ++j) at[j * kDcStride] = from + j < n_here ? x[j] : 0.f;
+    }
   } else {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
     auto sum = [&](int ch, int t) {
       float v = 0.f;
       for (int j = 0; j < a.taps; ++j) v = fmaf(a.conv_w[(size_t)ch * a.taps + j], input(ch, at0 + t - (a.taps - 1 - j)), v);
@@ -215,10 +237,16 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
     const float rate = expf(a.a_log[h]);
     if (BY_CHANNEL) {
       const float shift = l < a.dim ? a.dt_bias[h * a.dim + l] : 0.f;
-#pragma unroll 2
-      for (int t = half; t < DC_TOKENS; t += 2) {
-        float* at = g_s + t * kDcStride + l;
-        *at = t < n_here && l < a.dim ? expf(-rate * dc_softplus(*at + shift)) : 1.f;
+#pragma unroll 1
+      for (int i = half; i < DC_TOKENS; i += 16) {       // eight at a time, side by side as above
+        float* at = g_s + i * kDcStride + l;
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = at[2 * j * kDcStride];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = expf(-rate * dc_softplus(x[j] + shift));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) at[2 * j * kDcStride] = i + 2 * j < n_here && l < a.dim ? x[j] : 1.f;
       }
     } else {
 #pragma unroll
@@ -234,14 +262,26 @@ __global__ void __launch_bounds__(DC_PREPARE_THREADS, 2) delta_chunk_prepare_ker
   }
   __syncthreads();
   // ---- unit vectors: a warp a row, four lanes of it a thread ----
+  {
+    constexpr int kRows = 2 * DC_TOKENS / (DC_PREPARE_THREADS / 32);
+    float4 v[kRows];
+    float sum[kRows];
+    auto at = [&](int i) {                               // four rows of q, four of k
+      return reinterpret_cast<float4*>((i < kRows / 2 ? q_s : k_s) + (i % (kRows / 2) * 8 + warp) * kDcStride) + lane;
+    };
 #pragma unroll
-  for (int i = 0; i < 2 * DC_TOKENS; i += DC_PREPARE_THREADS / 32) {
-    const bool of_k = i >= DC_TOKENS;
-    float4* at = reinterpret_cast<float4*>((of_k ? k_s : q_s) + (i % DC_TOKENS + warp) * kDcStride) + lane;
-    float4 v = *at;
-    const float unit = 1.0f / sqrtf(warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w) + 1e-6f) * (of_k ? 1.f : a.q_scale);
-    v.x *= unit; v.y *= unit; v.z *= unit; v.w *= unit;
-    *at = v;
+    for (int i = 0; i < kRows; ++i) v[i] = *at(i);
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) sum[i] = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const float unit = 1.0f / sqrtf(sum[i] + 1e-6f) * (i < kRows / 2 ? a.q_scale : 1.f);
+      *at(i) = make_float4(v[i].x * unit, v[i].y * unit, v[i].z * unit, v[i].w * unit);
+    }
   }
   __syncthreads();
   // ---- A and M: pairs whose tokens a block of 2 w tokens' middle parts, w = 16, 8, 4, as products of rows that were
@@ -694,7 +734,9 @@ TOKB200_API int tokb200_delta_chunk_prepare(const void* proj, int proj_dtype, in
   if (((uintptr_t)records & 15)) return TOKB200_BAD_ALIGNMENT;
   const DeltaChunkArgs args = {proj, ld, qkv_at, b_at, decay, decay_ld, decay_at, conv_w, a_log, dt_bias, state,
                                state_stride, q_start, state_slot, records, 1.0f / sqrtf((float)dim), groups, heads, dim,
-                               vdim, taps, conv_off, n_requests};
+                               vdim, taps, conv_off, n_requests,
+                               (dim | vdim | ld | qkv_at | (by_channel ? decay_ld | decay_at : 0)) % 4 == 0 &&
+                                   (((uintptr_t)proj | (by_channel ? (uintptr_t)decay : 0)) & 15) == 0};
   const dim3 grid(n_rows / DC_TOKENS + n_requests, heads);
   if (by_channel) return proj_dtype == TOKB200_F32 ? dc_prepare<float, true>(args, grid, stream) : TOKB200_BAD_DTYPE;
   if (proj_dtype == TOKB200_F32) return dc_prepare<float, false>(args, grid, stream);
