@@ -1347,3 +1347,49 @@ def test_layer_small_m(M, hidden, inner, nh, nkv, d, page, window, lengths):
         assert err <= 2e-2 * scale + 1e-4, f"feed-forward off by {err} of {scale}"
     assert o.layer_small_m_splits(33, hidden, inner, nh, nkv, d) == (0, 0)
     assert o.layer_small_m_splits(4, 100, inner, nh, nkv, d) == (0, 0)
+
+
+@pytest.mark.parametrize("n,inner", [(3, 172), (1, 303100), (1, 303104), (777, 1028), (5000, 2432)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_pytorch_tanh"])
+def test_gate_of_32_bit_rows_on_and_off_16_bytes(n, inner, activation):
+    """Four elements a thread and one give the same bits, the last row and column included."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(n)
+    room = torch.randn(n * 2 * inner + 4, device=DEV, generator=g) * 4
+    on = room[:n * 2 * inner].view(n, 2 * inner)
+    moved = torch.empty_like(room)
+    off = moved[1:1 + n * 2 * inner].view(n, 2 * inner).copy_(on)
+    got, want = torch.full((n, inner), 9.0, device=DEV), torch.full((n, inner), 9.0, device=DEV)
+    o.silu_gate(on, got, activation)
+    o.silu_gate(off, want, activation)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 3, 130])
+@pytest.mark.parametrize("nh,nkv,d,pools", [(14, 2, 64, True), (3, 1, 24, True), (4, 4, 8, True), (2, 1, 128, False)])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_rope_store_of_32_bit_rows_on_and_off_16_bytes(n, nh, nkv, d, pools, with_bias):
+    """Four lanes and their partners a thread against one pair a thread; idle rows write nothing to the pools."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(n)
+    width = (nh + 2 * nkv) * d
+    room = torch.randn(n * width + 4, device=DEV, generator=g)
+    on = room[:n * width].view(n, width)
+    off = torch.empty_like(room)[1:1 + n * width].view(n, width).copy_(on)
+    bias = torch.randn(width, device=DEV, generator=g) if with_bias else None
+    pos = torch.randint(0, 64, (n,), device=DEV, generator=g, dtype=torch.int32)
+    slot = torch.randperm(n, device=DEV, generator=g).int()
+    slot[n // 2] = -1
+    angle = torch.rand(64, d // 2, device=DEV, generator=g) * 6
+    results = []
+    for qkv in (on, off):
+        q_out = torch.full((n, nh * d), 9.0, device=DEV)
+        k_pool, v_pool = torch.full((n, nkv, d), 9.0, device=DEV), torch.full((n, nkv, d), 9.0, device=DEV)
+        o.rope_store(qkv, bias, pos, slot if pools else None, angle.cos(), angle.sin(), q_out, k_pool if pools else None,
+                     v_pool if pools else None, nh, nkv, d, d)
+        results.append((q_out, k_pool, v_pool))
+    (q, k, v), (q2, k2, v2) = results
+    assert torch.equal(v, v2)
+    top = 2 * float(on.abs().max() + (bias.abs().max() if with_bias else 0))
+    for got, want in ((q, q2), (k, k2)):                 # two products of which either may be fused: an ulp of each
+        assert float((got - want).abs().max()) <= top * 2.0 ** -23

@@ -486,6 +486,55 @@ __global__ void rope_store_bf16x8_kernel(const __nv_bfloat16* __restrict__ qkv, 
   *reinterpret_cast<uint4*>(dst + j + half) = ob;
 }
 
+// The same in 32 bits where the whole head is rotated and pieces of four lanes lie on 16 bytes: a thread takes four lanes of
+// a head and their partners.  Bound by latency
+// for few rows and by memory for many; us, this / a pair of lanes a thread and a block a token: 777 rows of (14 + 4) x 64 2.4 /
+// 4.0, 2,048 of (28 + 8) x 128 9.6 / 18.5, one row 1.5 / 2.2.
+__global__ void rope_store_f32x4_kernel(const float* __restrict__ qkv, const float* __restrict__ bias, const int* __restrict__ pos,
+                                        const int* __restrict__ slot, const float* __restrict__ cos_t,
+                                        const float* __restrict__ sin_t, float* __restrict__ q_out, float* __restrict__ k_pool,
+                                        float* __restrict__ v_pool, int n_tokens, int nh, int nkv, int d) {
+  const int heads = nh + 2 * nkv, half = d / 2, per_head = d / 8, per_token = heads * per_head;
+  const size_t item = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = (int)(item / per_token), rest = (int)(item % per_token);
+  const int head = rest / per_head, j = (rest % per_head) * 4;
+  pdl_wait();
+  pdl_launch();
+  if (t >= n_tokens) return;
+  auto four = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+  const float* src = qkv + ((size_t)t * heads + head) * d + j;
+  float4 a = four(src), b = four(src + half);
+  if (bias) {
+    const float4 ba = four(bias + head * d + j), bb = four(bias + head * d + j + half);
+    a.x += ba.x; a.y += ba.y; a.z += ba.z; a.w += ba.w;
+    b.x += bb.x; b.y += bb.y; b.z += bb.z; b.w += bb.w;
+  }
+  float* dst;
+  if (head < nh) {
+    dst = q_out + ((size_t)t * nh + head) * d;
+  } else {
+    const int s = slot ? slot[t] : -1;
+    const bool is_key = head < nh + nkv;
+    float* pool = is_key ? k_pool : v_pool;
+    if (s < 0 || !pool) return;
+    dst = pool + ((size_t)s * nkv + (head - nh - (is_key ? 0 : nkv))) * d;
+  }
+  if (head < nh + nkv) {
+    const float4 c = four(cos_t + (size_t)pos[t] * half + j), sn = four(sin_t + (size_t)pos[t] * half + j);
+    auto turn = [](float& va, float& vb, float c, float sn) {
+      const float ra = va * c - vb * sn, rb = vb * c + va * sn;
+      va = ra;
+      vb = rb;
+    };
+    turn(a.x, b.x, c.x, sn.x);
+    turn(a.y, b.y, c.y, sn.y);
+    turn(a.z, b.z, c.z, sn.z);
+    turn(a.w, b.w, c.w, sn.w);
+  }
+  *reinterpret_cast<float4*>(dst + j) = a;
+  *reinterpret_cast<float4*>(dst + j + half) = b;
+}
+
 // The same from float32 partial sums [S, T, heads d] of a product that was cut along k: the
 // pieces are added in index order, then bias, rotation and the cache write as above.
 __global__ void rope_store_partials_kernel(const float* __restrict__ parts, int n_partials, size_t stride,
@@ -584,6 +633,14 @@ TOKB200_API int tokb200_rope_store(const void* qkv, const float* bias, const int
                             (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool,
                             n_tokens, nh, nkv, d);
   }
+  if (dtype == TOKB200_F32 && rotary == d && d % 8 == 0 &&
+      (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)bias |
+        (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0) {
+    const size_t total = (size_t)n_tokens * (nh + 2 * nkv) * (d / 8);
+    return launch_dependent(rope_store_f32x4_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream,
+                            (const float*)qkv, bias, pos, slot, cos_t, sin_t, (float*)q_out, (float*)k_pool, (float*)v_pool,
+                            n_tokens, nh, nkv, d);
+  }
   const int items = (nh + 2 * nkv) * (d / 2);
   int threads = items < 256 ? ((items + 31) / 32) * 32 : 256;
   if (dtype == TOKB200_F32)
@@ -641,6 +698,24 @@ __global__ void silu_gate_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu,
   }
 }
 
+// 32-bit rows whose width is a multiple of 4, on 16 bytes: four elements a thread, all of the grid's threads busy whatever
+// the width.  Bound by memory (777 rows of 4,864: 45 MB that lie in L2); us, this / an element a thread: 777 rows of 4,864 6.3 /
+// 15.7, 2,048 of 8,960 32 / 75.
+__global__ void silu_gate_f32x4_kernel(const float* __restrict__ gu, float* __restrict__ out, int inner, int n_rows, int act) {
+  const unsigned per_row = inner / 4;
+  const size_t total = (size_t)n_rows * per_row;
+  pdl_wait();
+  pdl_launch();
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t t = i / per_row, c = (i - t * per_row) * 4;
+    const float4 g = *reinterpret_cast<const float4*>(gu + t * 2 * inner + c);
+    const float4 u = *reinterpret_cast<const float4*>(gu + t * 2 * inner + inner + c);
+    *reinterpret_cast<float4*>(out + t * inner + c) =
+        make_float4(gate_activation(act, g.x) * u.x, gate_activation(act, g.y) * u.y, gate_activation(act, g.z) * u.z,
+                    gate_activation(act, g.w) * u.w);
+  }
+}
+
 // the same for the interleaved layout of the gated kernels: for every 128 outputs,
 // 128 gate values followed by their 128 up values
 __global__ void silu_gate_interleaved_kernel(const __nv_bfloat16* __restrict__ gu,
@@ -689,6 +764,15 @@ TOKB200_API int tokb200_silu_gate(const void* gu, void* out, int dtype, int n_to
     const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     return launch_dependent(silu_gate_bf16x8_kernel, dim3(blocks), dim3(256), 0, stream,
                             (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, inner, n_tokens, act);
+  }
+  // four elements a thread once that still gives every SM 512 threads: 64 rows of 4,864 take 1.7 us either way, eight 1.6
+  // against 1.2 with an element a thread
+  if (dtype == TOKB200_F32 && inner % 4 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0 &&
+      (long long)n_tokens * (inner / 4) >= 148 * 512) {
+    const size_t total = (size_t)n_tokens * (inner / 4);
+    const int blocks = (int)((total + 255) / 256 < 148 * 64 ? (total + 255) / 256 : 148 * 64);
+    return launch_dependent(silu_gate_f32x4_kernel, dim3(blocks), dim3(256), 0, stream, (const float*)gu, (float*)out, inner,
+                            n_tokens, act);
   }
   // grid.y is limited to 65535 rows; tile rows over several launches beyond it
   for (int row0 = 0; row0 < n_tokens; row0 += 65535) {
