@@ -1393,3 +1393,55 @@ def test_rope_store_of_32_bit_rows_on_and_off_16_bytes(n, nh, nkv, d, pools, wit
     top = 2 * float(on.abs().max() + (bias.abs().max() if with_bias else 0))
     for got, want in ((q, q2), (k, k2)):                 # two products of which either may be fused: an ulp of each
         assert float((got - want).abs().max()) <= top * 2.0 ** -23
+
+
+@pytest.mark.parametrize("M", [1, 17, 31, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(1, 8), (127, 72), (129, 640), (260, 1096), (148 * 128 + 1, 64), (300 * 128, 200)])
+def test_gemm_tcgen05_up_to_64_rows(M, N, K):
+    """The weight's rows as the product's M: tiles cut by N and K, one unit a block and several, rows past M untouched."""
+    o = ops()
+    a = rnd(M, K, seed=71, dtype=torch.bfloat16)
+    w = rnd(N, K, seed=72, dtype=torch.bfloat16, scale=0.1)
+    want = a.double().cpu() @ w.double().cpu().t()
+    size = a.double().cpu().abs() @ w.double().cpu().abs().t()
+    # sums in 32 bits over k (a 2^-23 of the products' sizes at each of K / 16 steps), a last rounding to 16
+    slack = size * (K / 16 + 2) * 2.0 ** -23
+    for bias in (None, rnd(N, seed=73)):
+        ref = want + (bias.double().cpu() if bias is not None else 0)
+        for dtype in (torch.bfloat16, torch.float32):
+            room = torch.full((M + 1, N), 7.0, dtype=dtype, device=DEV)
+            o.gemm_tcgen05(a, w, bias, room[:M])
+            o.gemm_tcgen05_check()
+            bound = slack + ref.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23)
+            assert bool(((room[:M].double().cpu() - ref).abs() <= bound).all())
+            assert bool((room[M:] == 7.0).all())
+    if N % 4 == 0:
+        blocks = -(-K // 64)
+        for splits in {s for s in (2, 3, blocks) if s <= blocks and (s - 1) * -(-blocks // s) < blocks}:
+            parts = torch.full((splits, M, N), 9.0, device=DEV)
+            o.gemm_tcgen05_partials(a, w, parts)
+            o.gemm_tcgen05_check()
+            assert bool(((parts.double().sum(0).cpu() - want).abs() <= slack).all())
+
+
+@pytest.mark.parametrize("M", [17, 32, 33, 64])
+@pytest.mark.parametrize("inner,K", [(128, 8), (384, 328), (148 * 64 + 128, 704)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_pytorch_tanh"])
+def test_gated_product_up_to_64_rows(M, inner, K, activation):
+    """Gate and up rows of a unit come from two places of the weight and meet in 32 bits; rows past M untouched."""
+    o = ops()
+    inner = inner // 128 * 128
+    x = rnd(M, K, seed=74, dtype=torch.bfloat16)
+    gate, up = (rnd(inner, K, seed=s, dtype=torch.bfloat16, scale=0.2) for s in (75, 76))
+    room = torch.full((M + 1, inner), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.gated_linear(x, o.interleave_gate_up(gate, up), room[:M], activation)
+    o.gemm_tcgen05_check()
+    xd, gd, ud = x.double().cpu(), gate.double().cpu(), up.double().cpu()
+    g, u = xd @ gd.t(), xd @ ud.t()
+    act = torch.nn.functional.silu if activation == "silu" else lambda t: torch.nn.functional.gelu(t, approximate="tanh")
+    want = act(g) * u
+    # 32-bit sums (as above), through an activation whose slope stays below 1.2, one rounding to 16 bits
+    eps = (K / 16 + 4) * 2.0 ** -23
+    slack = 1.2 * eps * ((xd.abs() @ gd.abs().t()) * u.abs() + (xd.abs() @ ud.abs().t()) * (g.abs() + 1))
+    assert bool(((room[:M].double().cpu() - want).abs() <= slack + want.abs() * 2.0 ** -8 + 1e-7).all())
+    assert bool((room[M:] == 7.0).all())

@@ -731,6 +731,186 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
   }
 }
 
+// ----------------------------------------------------------------------------
+// Up to 64 rows (a batch being decoded): the weight's rows are the product's M and the batch its N, so that a stage of 64 of
+// k is 16 KB of weight and 8 KB of batch.  Bound by the
+// weight's way from memory; with the batch's rows as M, half of a tile of 128 was zeros that cost as much shared memory as the
+// weight, and a tile's output was staged in 64 KB more, so that 64 KB of weight were on their way an SM where it is 144 now.
+// Measured (64 rows, weights from memory, us, this / rows as M / the vendor library): 4,608 x 3,584 in 4 pieces of k 9.1 /
+// 10.9 / 8.9, 3,584 x 18,944 in 5 27 / 31 / 31, 37,888 x 3,584 48 / 50 / 49 (floor 42), 896 x 896 in 7 3.5 / 4.7 / 3.3, 151,936
+// x 896 52 / 70 / 50.  GATED (64 rows; in front of it the product as 16 bits and the activation's own kernel): 37,888 x 3,584
+// 48.0 with the activation in it; 17 rows, against the ring kernel's gated form: 9,728 x 896 6.7 / 8.8, 17,920 x 1,536 11.5 /
+// 16.7.  A layer of 64 rows over long contexts 244 -> 232.
+// A unit of work is 128 weight rows and a piece of k; its sums come back with a weight row a lane, 32 neighbouring columns of
+// the output a warp, and are stored from registers.
+// ----------------------------------------------------------------------------
+template <int NT, bool GATED> struct TcFewSmem {
+  static constexpr int kWBytes = TC_BLOCK_M * TC_BLOCK_K * 2, kXBytes = NT * TC_BLOCK_K * 2;
+  static constexpr int kStage = kWBytes + kXBytes;
+  static constexpr int kSwap = GATED ? 2 * NT * 64 * 4 : 0;      // a unit's gate and up sums
+  static constexpr int kStages = (NT == 64 ? 9 : 11) - (GATED ? 1 : 0);
+  static constexpr int kTotal = kStages * kStage + kSwap + 1024 /* alignment slack */ + 256 /* barriers */;
+  static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
+};
+
+template <int NT, bool OUT_F32, bool GATED>
+__global__ void __launch_bounds__(TC_THREADS)
+gemm_tcgen05_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                        const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int k_splits,
+                        int activation) {
+  using S = TcFewSmem<NT, GATED>;
+  constexpr int STAGES = S::kStages;
+  extern __shared__ unsigned char tc_raw[];
+  unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~(uintptr_t)1023);
+  float* swap = reinterpret_cast<float*>(tiles + STAGES * S::kStage);        // GATED: [2][NT][64]
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(tiles + STAGES * S::kStage + S::kSwap);
+  unsigned long long* empty = full + STAGES;
+  unsigned long long* acc_full = empty + STAGES;         // [2]
+  unsigned long long* acc_empty = acc_full + 2;          // [2]
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_empty + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_tiles = (N + TC_BLOCK_M - 1) / TC_BLOCK_M, k_blocks = (K + TC_BLOCK_K - 1) / TC_BLOCK_K;
+  const int per = (k_blocks + k_splits - 1) / k_splits, units = n_tiles * k_splits;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(tc_smem(tmem_slot)), "r"((unsigned)(2 * NT)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem_base = *tmem_slot;
+  // GATED: 64 gate rows, then the up rows of the same outputs, of the blocks of 128 and 128 of the interleaved weight
+  auto load_w = [&](unsigned char* stage, unsigned long long* bar, int kb, int tile) {
+    if (GATED) {
+      const int row = tile / 2 * 256 + tile % 2 * 64;
+      tma_load_2d(stage, &map_w, bar, kb * TC_BLOCK_K, row);
+      tma_load_2d(stage + S::kWBytes / 2, &map_w, bar, kb * TC_BLOCK_K, row + 128);
+    } else {
+      tma_load_2d(stage, &map_w, bar, kb * TC_BLOCK_K, tile * TC_BLOCK_M);
+    }
+  };
+  // the weight, which no kernel of the step writes, is on its way before the predecessor has ended
+  int early = 0;
+  if (warp == 0 && lane == 0) {
+    const int kb0 = blockIdx.x / n_tiles * per;
+    early = min(STAGES, min(k_blocks, kb0 + per) - kb0);
+    for (int s = 0; s < early; ++s) {
+      mbar_expect_tx(&full[s], S::kStage);
+      load_w(tiles + s * S::kStage, &full[s], kb0 + s, blockIdx.x % n_tiles);
+    }
+  }
+  pdl_wait();
+  pdl_launch();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+        const int kb0 = unit / n_tiles * per, kb1 = min(k_blocks, kb0 + per);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          unsigned char* stage = tiles + s * S::kStage;
+          if (it >= early) {
+            if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
+            mbar_expect_tx(&full[s], S::kStage);
+            load_w(stage, &full[s], kb, unit % n_tiles);
+          }
+          tma_load_2d(stage + S::kWBytes, &map_x, &full[s], kb * TC_BLOCK_K, 0);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) | ((unsigned)(TC_BLOCK_M >> 4) << 24);
+      int it = 0, round = 0;
+      bool ok = true;
+      for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x, ++round) {
+        const int kb0 = unit / n_tiles * per, kb1 = min(k_blocks, kb0 + per), buf = round & 1;
+        if (!mbar_wait(&acc_empty[buf], ((round >> 1) & 1) ^ 1)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&full[s], (it / STAGES) & 1)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const unsigned char* stage = tiles + s * S::kStage;
+          const unsigned long long w_desc = umma_desc(stage), x_desc = umma_desc(stage + S::kWBytes);
+#pragma unroll
+          for (int k = 0; k < TC_BLOCK_K / TC_UMMA_K; ++k)
+            umma_bf16(tmem_base + (unsigned)(buf * NT), w_desc + 2 * k, x_desc + 2 * k, idesc, ((kb - kb0) | k) != 0);
+          umma_commit(&empty[s]);
+        }
+        umma_commit(&acc_full[buf]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    int round = 0;
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++round) {
+      const int n = unit % n_tiles * TC_BLOCK_M + quarter * 32 + lane, buf = round & 1;
+      bool ok = mbar_wait(&acc_full[buf], (round >> 1) & 1);
+      if (GATED) {                       // the four warps go on or give up together; the sums of the unit before have been read
+        unsigned all;
+        asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, 1, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                     : "=r"(all) : "r"((unsigned)ok) : "memory");
+        ok = all != 0;
+      }
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      unsigned v[NT / 32][32];
+#pragma unroll
+      for (int c = 0; c < NT / 32; ++c)
+        tmem_load_32_async(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * NT + c * 32), v[c]);
+      tmem_wait_loads();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      if constexpr (GATED) {
+        // through shared memory, so that a thread gets the gate and up sums of two neighbouring outputs.  The loop is kept a
+        // loop: unrolled, the activations were code that a unit's warps fetched cold (64 rows of 37,888 x 3,584 52 us)
+#pragma unroll
+        for (int m = 0; m < NT; ++m)
+          swap[(quarter / 2 * NT + m) * 64 + (quarter & 1) * 32 + lane] = __uint_as_float(v[m / 32][m % 32]);
+        epilogue_barrier();
+        __nv_bfloat16* to = static_cast<__nv_bfloat16*>(out) + (size_t)unit * 64 + lane * 2;
+#pragma unroll 2
+        for (int m = quarter; m < M; m += 4) {
+          const float2 g = *reinterpret_cast<const float2*>(swap + m * 64 + lane * 2);
+          const float2 u = *reinterpret_cast<const float2*>(swap + (NT + m) * 64 + lane * 2);
+          *reinterpret_cast<__nv_bfloat162*>(to + (size_t)m * (N / 2)) =
+              __floats2bfloat162_rn(gate_activation(activation, g.x) * u.x, gate_activation(activation, g.y) * u.y);
+        }
+        continue;
+      }
+      if (n >= N) continue;
+      const float shift = bias ? bias[n] : 0.f;
+      const size_t first = (size_t)(unit / n_tiles) * M * N + n;
+#pragma unroll
+      for (int m = 0; m < NT; ++m) {
+        if (m >= M) break;
+        const float sum = __uint_as_float(v[m / 32][m % 32]) + shift;
+        if (OUT_F32) static_cast<float*>(out)[first + (size_t)m * N] = sum;
+        else static_cast<__nv_bfloat16*>(out)[first + (size_t)m * N] = __float2bfloat16_rn(sum);
+      }
+    }
+  }
+  // ---- common exit: everybody arrives, then tensor memory is given back ----
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((unsigned)(2 * NT)) : "memory");
+  }
+}
+
+
 // ---- host side ----------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -875,6 +1055,32 @@ static int launch_tc(const void* x, const void* w, const float* bias, void* out,
                           (size_t)S::kTotal, stream, map_x, map_w, bias, out, out_is_f32, M, N, K);
 }
 
+// `k_splits` > 1: 32-bit partial sums [k_splits, M, N]
+template <int NT, bool OUT_F32, bool GATED = false>
+static int launch_tc_few(const void* x, const void* w, const float* bias, void* out, int M, int N, int K, int k_splits,
+                         cudaStream_t stream, int activation = TOKB200_ACT_NONE) {
+  using S = TcFewSmem<NT, GATED>;
+  CUtensorMap map_x, map_w;
+  int status = make_map(&map_x, x, M, K, NT);
+  if (status == TOKB200_OK) status = make_map(&map_w, w, N, K, GATED ? TC_BLOCK_M / 2 : TC_BLOCK_M);
+  if (status != TOKB200_OK) return status;
+  static bool configured[64] = {};
+  static int sm_count[64] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return TOKB200_BAD_SIZE;
+  auto kernel = gemm_tcgen05_few_kernel<NT, OUT_F32, GATED>;
+  if (!configured[device]) {
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
+    if (err != cudaSuccess) return (int)err;
+    err = cudaDeviceGetAttribute(&sm_count[device], cudaDevAttrMultiProcessorCount, device);
+    if (err != cudaSuccess) return (int)err;
+    configured[device] = true;
+  }
+  const int units = (N + TC_BLOCK_M - 1) / TC_BLOCK_M * k_splits;
+  return launch_dependent(kernel, dim3(units < sm_count[device] ? units : sm_count[device]), dim3(TC_THREADS), (size_t)S::kTotal,
+                          stream, map_x, map_w, bias, out, M, N, K, k_splits, activation);
+}
+
 // 1 when some launch since the last call recorded a wait that ran out; clears the flag.
 TOKB200_API int tokb200_gemm_tcgen05_error(void) {
   int flag = 0, zero = 0;
@@ -894,8 +1100,16 @@ TOKB200_API int tokb200_gemm_tcgen05(const void* x, const void* w, const float* 
   // block_n + 1000 asks for the persistent kernel (TMA-stored output): the output's
   // row pitch must then be a multiple of 16 bytes
   if (activation != TOKB200_ACT_NONE &&                  // the persistent kernel's bfloat16 epilogue alone applies one
-      (block_n < 1000 || out_is_f32 || activation < 0 || activation >= TOKB200_ACT_COUNT))
+      (block_n < 1000 || block_n == 2000 || out_is_f32 || activation < 0 || activation >= TOKB200_ACT_COUNT))
     return TOKB200_BAD_SIZE;
+  if (block_n == 2000) {                                 // up to 64 rows
+    if (M > 64) return TOKB200_BAD_SIZE;
+    if (M <= 32)
+      return out_is_f32 ? launch_tc_few<32, true>(x, w, bias, out, M, N, K, 1, stream)
+                        : launch_tc_few<32, false>(x, w, bias, out, M, N, K, 1, stream);
+    return out_is_f32 ? launch_tc_few<64, true>(x, w, bias, out, M, N, K, 1, stream)
+                      : launch_tc_few<64, false>(x, w, bias, out, M, N, K, 1, stream);
+  }
   if (block_n >= 1000) {
     if ((out_is_f32 ? N % 4 : N % 8) != 0) return TOKB200_BAD_SIZE;
     switch (block_n - 1000) {
@@ -928,6 +1142,8 @@ TOKB200_API int tokb200_gemm_tcgen05_partials(const void* x, const void* w, void
   if ((k_splits - 1) * per >= k_blocks) return TOKB200_BAD_SIZE;        // an empty piece
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) return TOKB200_BAD_ALIGNMENT;
   if (M > 128 * 65535) return TOKB200_BAD_SIZE;
+  if (M <= 32) return launch_tc_few<32, true>(x, w, nullptr, out, M, N, K, k_splits, stream);
+  if (M <= 64) return launch_tc_few<64, true>(x, w, nullptr, out, M, N, K, k_splits, stream);
   return launch_tc_persistent<128, 4, true>(x, w, nullptr, out, M, N, K, stream, k_splits);
 }
 
@@ -998,6 +1214,8 @@ TOKB200_API int tokb200_gemm_tcgen05_gated(const void* x, const void* w, void* o
   if (K <= 0 || K % 8 || N % 256 || activation < 0 || activation >= TOKB200_ACT_COUNT) return TOKB200_BAD_SIZE;
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) return TOKB200_BAD_ALIGNMENT;
   if (M > 128 * 65535) return TOKB200_BAD_SIZE;
+  if (M <= 32) return launch_tc_few<32, false, true>(x, w, nullptr, out, M, N, K, 1, stream, activation);
+  if (M <= 64) return launch_tc_few<64, false, true>(x, w, nullptr, out, M, N, K, 1, stream, activation);
   return launch_tc_persistent<256, 3, false, true>(x, w, nullptr, out, M, N, K, stream, 1, nullptr, activation);
 }
 

@@ -664,6 +664,8 @@ def gemm_tcgen05(a, w, bias, out, block_n: int = 0, activation: Optional[str] = 
         raise ValueError(f"gemm_tcgen05: K = {K} must be a multiple of 8")
     if tuple(out.shape) != (M, N) or out.dtype not in (torch.bfloat16, torch.float32):
         raise ValueError("gemm_tcgen05: out is [M,N] bfloat16 or float32")
+    if not block_n and M <= 64 and activation is None:
+        block_n = 2000          # the weight's rows as the product's M: faster at every size (see the kernel)
     if not block_n:
         pitch_ok = N % (4 if out.dtype == torch.float32 else 8) == 0
         if pitch_ok and (M * N >= 128 * 128 * 32 or activation is not None):
@@ -764,18 +766,6 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
     elif M <= SMALL_M_ROWS:
         _check(_lib("linear_small_m").tokb200_linear_small_m_gated(
             _ptr(x), _ptr(w), _ptr(out), _i(M), _i(N), _i(K), act, _stream()), "gated_linear")
-    elif M <= RING_MAX_ROWS and _RING and (M <= 24 or N * K <= 9_000_000) and linear_ring_supported(M, N, K, 1, True):
-        # 17 to 32 rows: the ring kernel where it leads a tensor-core tile that is mostly padding
-        # followed by the activation's own kernel (us in a captured chain, hidden 896: 11.3 -> 9.0
-        # at 17 rows, 13.3 -> 10.6 at 32; hidden 1,536: 24.3 -> 17.5 at 17 rows, but 18.8 -> 20.6 at 32)
-        linear_ring_gated(x, w, out, activation)
-    elif M <= 64:
-        # too few rows to fill the 256-wide gated tiles over the SMs: the plain tensor-core
-        # product over the same (interleaved) weight, then the activation on its output
-        gu = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-        gemm_tcgen05(x, w, None, gu)
-        _check(_lib("elementwise").tokb200_silu_gate_interleaved(
-            _ptr(gu), _ptr(out), _i(M), _i(N // 2), act, _stream()), "silu_gate_interleaved")
     elif M >= 256 and _PAIR:
         # two tiles of rows and more: pairs of CTAs on tiles of 256 rows, each loading half of the
         # weight tile (a sixth fewer cycles than lone CTAs at 2,048 rows)
@@ -783,6 +773,8 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
             _ptr(x), _ptr(w), None, _ptr(out), _i(PAIR_GATED), _i(M), _i(N), _i(K), _i(1), act, _stream()),
             "gated_linear")
     else:
+        # up to 64 rows the entry has the weight's rows as the product's M (us at 17 and 32 rows, against the ring kernel:
+        # 9,728 x 896 6.8 / 8.8 and 7.2 / 10.1, 17,920 x 1,536 11.5 / 16.7 and 11.9 / 19.7)
         _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_gated(
             _ptr(x), _ptr(w), _ptr(out), _i(M), _i(N), _i(K), act, _stream()), "gated_linear")
 
