@@ -53,6 +53,23 @@ __device__ __forceinline__ void rs_load4(const float* in, int col, const float* 
   }
 }
 
+// sine and cosine of frequency i at position p, times the magnitude
+__device__ __forceinline__ void rs_angle(int p, int i, const float* inv_freq, const double* inv_freq64, float magnitude,
+                                         float& sine, float& cosine) {
+  float angle;
+  if (inv_freq64 != nullptr) {       // the product and its reduction to one turn in 64-bit: good to 1e-7 at any position
+    double a = (double)p * inv_freq64[i];
+    a -= 6.283185307179586476925 * rint(a * 0.15915494309189533577);
+    angle = (float)a;
+  } else {
+    angle = (float)p * inv_freq[i];
+  }
+  float sn, cs;
+  sincosf(angle, &sn, &cs);
+  sine = sn * magnitude;
+  cosine = cs * magnitude;
+}
+
 template <typename TI, typename T>
 __global__ void qkv_rotate_store_kernel(const TI* __restrict__ proj, int ld, int at, const float* __restrict__ bias,
                                         const float* __restrict__ inv_freq,
@@ -76,18 +93,7 @@ __global__ void qkv_rotate_store_kernel(const TI* __restrict__ proj, int ld, int
   const int p = pos[t];
   const int where = slot ? slot[t] : -1;
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    float angle;
-    if (inv_freq64 != nullptr) {       // the product and its reduction to one turn in 64-bit: good to 1e-7 at any position
-      double a = (double)p * inv_freq64[i];
-      a -= 6.283185307179586476925 * rint(a * 0.15915494309189533577);
-      angle = (float)a;
-    } else {
-      angle = (float)p * inv_freq[i];
-    }
-    float sn, cs;
-    sincosf(angle, &sn, &cs);
-    sine[i] = sn * magnitude;
-    cosine[i] = cs * magnitude;
+    rs_angle(p, i, inv_freq, inv_freq64, magnitude, sine[i], cosine[i]);
   }
   pdl_wait();
   pdl_launch();
@@ -247,6 +253,92 @@ __global__ void qkv_rotate_store_kernel(const TI* __restrict__ proj, int ld, int
   }
 }
 
+// The same from 32-bit products of many tokens without norms, where heads have as many lanes as rows (eights, all on 16 bytes):
+// a block RS_TOKENS tokens, a thread four lanes and their mates.
+// Bound by memory from some 4,000 tokens on.  A block a token had its chain of position, angles and barrier for four and a half
+// heads a warp, and read each head twice for its halves' mates; four tokens give every thread one angle and nine pieces, whose
+// loads are asked for three at a time.  us, this / a block a token, half form, 32-bit to 16: 8,192 tokens of (28 + 8) x 128 43.9 /
+// 76.4 (5.1 TB/s), of (14 + 4) x 64 12.4 / 35.9, 2,048 of (16 + 32) x 128 17.2 / 20.3.
+#define RS_TOKENS 4
+#define RS_MANY (148 * 8)        // tokens from which on that is the faster one (us, this / a block a token, interleaved, (28 + 8) x 128:
+                                 // 600 tokens 7.4 / 5.8, 1,200 9.2 / 9.6; half form 7.0 / 7.2 and 8.7 / 11.8)
+template <typename T>
+__global__ void __launch_bounds__(256) qkv_rotate_store8_kernel(
+    const float* __restrict__ proj, int ld, int at, const float* __restrict__ bias, const float* __restrict__ inv_freq,
+    const double* __restrict__ inv_freq64, int rot_dims, const int* __restrict__ pos, const int* __restrict__ slot,
+    const int* __restrict__ row_req, T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool, int n_rows, int heads,
+    int kv_heads, int dim, const float* __restrict__ temp, int half_layout, float magnitude, int v_col) {
+  extern __shared__ float shared[];                      // cosines of the tokens' frequencies, then their sines
+  __shared__ int where_s[RS_TOKENS];                     // a token's cache slot, -1: none; -2: an idle row
+  const int half = rot_dims >> 1, t0 = blockIdx.x * RS_TOKENS;
+  float *cosine = shared, *sine = shared + RS_TOKENS * half;
+  for (int i = threadIdx.x; i < RS_TOKENS * half; i += blockDim.x) {
+    const int t = t0 + i / half, f = i % half;
+    if (t >= n_rows) break;
+    rs_angle(pos[t], f, inv_freq, inv_freq64, magnitude, sine[i], cosine[i]);
+  }
+  if (threadIdx.x < RS_TOKENS) {
+    const int t = t0 + threadIdx.x;
+    where_s[threadIdx.x] = t >= n_rows || row_req[t] < 0 ? -2 : slot ? max(slot[t], -1) : -1;
+  }
+  pdl_wait();
+  pdl_launch();
+  __syncthreads();
+  const int per_head = dim / 8, per_token = (heads + 2 * kv_heads) * per_head;
+#pragma unroll 3
+  for (int i = threadIdx.x; i < RS_TOKENS * per_token; i += 256) {
+    const int token = i / per_token, rest = i - token * per_token, head = rest / per_head, quad = (rest - head * per_head) * 4;
+    // the half form: a quad of the rotated lanes and its mates, or two of the lanes behind them
+    const bool turned = !half_layout || quad < half;
+    const int l = turned ? quad : quad + half, apart = !half_layout ? dim >> 1 : turned ? half : (dim >> 1) - half;
+    const int where = where_s[token], t = t0 + token;
+    if (where == -2 || (head >= heads && where < 0)) continue;
+    const bool value = head >= heads + kv_heads;
+    const float* in = proj + (size_t)t * ld + at;
+    const int col = value ? v_col + (head - heads - kv_heads) * dim + l : head * dim + l;
+    float a[4], b[4];
+    rs_load4(in, col, bias, nullptr, 0, 1.f, a);
+    rs_load4(in, col + apart, bias, nullptr, 0, 1.f, b);
+    if (!value) {
+      const float *c = cosine + token * half, *s = sine + token * half;
+      if (half_layout) {
+        if (turned) {
+          const float4 c4 = *reinterpret_cast<const float4*>(c + l), s4 = *reinterpret_cast<const float4*>(s + l);
+          const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float x = a[j], y = b[j];
+            a[j] = x * cs[j] - y * sn[j];
+            b[j] = y * cs[j] + x * sn[j];
+          }
+        }
+      } else {
+        auto turn = [&](float (&v)[4], int lane) {
+          if (lane >= rot_dims) return;
+          const float2 cs = *reinterpret_cast<const float2*>(c + lane / 2), sn = *reinterpret_cast<const float2*>(s + lane / 2);
+          const float v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
+          v[0] = v0 * cs.x - v1 * sn.x;
+          v[1] = v1 * cs.x + v0 * sn.x;
+          v[2] = v2 * cs.y - v3 * sn.y;
+          v[3] = v3 * cs.y + v2 * sn.y;
+        };
+        turn(a, l);
+        turn(b, l + apart);
+      }
+      if (head < heads && temp != nullptr) {
+        const float heat = temp[head];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { a[j] *= heat; b[j] *= heat; }
+      }
+    }
+    T* dst = (head < heads ? q_out + ((size_t)t * heads + head) * dim
+                           : (value ? v_pool + ((size_t)where * kv_heads + (head - heads - kv_heads)) * dim
+                                    : k_pool + ((size_t)where * kv_heads + (head - heads)) * dim)) + l;
+    rs_store4(dst, a);
+    rs_store4(dst + apart, b);
+  }
+}
+
 TOKB200_API int tokb200_qkv_rotate_store(const void* proj, int proj_dtype, int ld, int at, const float* bias,
                                          const float* inv_freq, const double* inv_freq64, int rot_dims,
                                          const int* pos, const int* slot,
@@ -270,6 +362,22 @@ TOKB200_API int tokb200_qkv_rotate_store(const void* proj, int proj_dtype, int l
   if (heads <= 0 || kv_heads < 0 || dim <= 0 || vdim <= 0 || row < dim || row < vdim || rot_dims < 0 ||
       rot_dims % 2 || rot_dims > dim || (head_norm && magnitude != 1.0f) || (rot_dims > 0 && inv_freq == nullptr && inv_freq64 == nullptr))
     return TOKB200_BAD_SIZE;
+  const int aligned = quads && row == dim && vdim == dim && dim % 8 == 0;
+  if (aligned && q_gain == nullptr && k_gain == nullptr && !head_norm && n_rows >= RS_MANY &&
+      (out_dtype == TOKB200_F32 || out_dtype == TOKB200_BF16)) {
+    const size_t tables = (size_t)RS_TOKENS * rot_dims * sizeof(float);
+    if (tables <= 40000) {
+      const dim3 grid((n_rows + RS_TOKENS - 1) / RS_TOKENS);
+      if (out_dtype == TOKB200_F32)
+        return launch_dependent(qkv_rotate_store8_kernel<float>, grid, dim3(256), tables, stream, (const float*)proj, ld, at, bias,
+                                inv_freq, inv_freq64, rot_dims, pos, slot, row_req, (float*)q_out, (float*)k_pool, (float*)v_pool,
+                                n_rows, heads, kv_heads, dim, temp, half_layout, magnitude, v_col);
+      return launch_dependent(qkv_rotate_store8_kernel<__nv_bfloat16>, grid, dim3(256), tables, stream, (const float*)proj, ld, at,
+                              bias, inv_freq, inv_freq64, rot_dims, pos, slot, row_req, (__nv_bfloat16*)q_out,
+                              (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, n_rows, heads, kv_heads, dim, temp, half_layout,
+                              magnitude, v_col);
+    }
+  }
 #define LAUNCH(TI, T)                                                                                         \
   return launch_dependent(qkv_rotate_store_kernel<TI, T>, dim3(n_rows), dim3(256), smem, stream,              \
                           (const TI*)proj, ld, at, bias, inv_freq, inv_freq64, rot_dims, pos, slot, row_req,  \
