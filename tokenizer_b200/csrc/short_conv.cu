@@ -117,6 +117,27 @@ __device__ __forceinline__ float4 conv_row4(const float (&wt)[4][TAPS], const fl
   return make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
+// The weights of four channels.  Four taps that lie on 16 bytes come a channel a load: lane for lane 64 bytes apart, sixteen
+// loads of one weight were 256 lines of L1 a warp, beside 76 of the run's
+// inputs and outputs (us, this / that, 4,352 channels: 1 row 2.8 / 2.9, 64 3.6 / 4.8, 500 10.3 / 21.0, 8,192 64 / 71).
+template <int TAPS>
+__device__ __forceinline__ void conv_weights(const float* __restrict__ w, int c, float (&wt)[4][TAPS]) {
+  if constexpr (TAPS == 4) {
+    if (((uintptr_t)w & 15) == 0) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const float4 four = *reinterpret_cast<const float4*>(w + (size_t)(c + v) * 4);
+        wt[v][0] = four.x; wt[v][1] = four.y; wt[v][2] = four.z; wt[v][3] = four.w;
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) wt[v][j] = w[(size_t)(c + v) * TAPS + j];
+}
+
 // A block covers ROWS consecutive rows of the step.  A run that lies inside one request's portion, at least
 // TAPS - 1 rows behind its start, takes the straight path: the run's inputs and the TAPS - 1 rows in front of it
 // are asked for at once, before anything is waited for, every input is loaded once and the window moves through
@@ -143,14 +164,11 @@ short_conv_tile_kernel(const TI* __restrict__ x, int ld, int at, int channels, c
     for (int i = 0; i < ROWS; ++i) in[i] = conv_load_raw(x + (size_t)(t0 + i) * ld + at + c);
 #pragma unroll
     for (int k = 0; k < TAPS - 1; ++k) ahead[k] = conv_load_raw(x + (size_t)(t0 - (TAPS - 1 - k)) * ld + at + c);
+    conv_weights<TAPS>(w, c, wt);
+    const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int r = row_req[t0];
     const int begin = r >= 0 ? q_start[r] : 0, end = r >= 0 ? q_start[r + 1] : 0;
     if (r >= 0 && begin + TAPS - 1 <= t0 && t0 + ROWS <= end) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) wt[v][j] = w[(size_t)(c + v) * TAPS + j];
-      const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int k = 0; k < TAPS - 1; ++k) win[k] = conv_unpack(ahead[k]);
 #pragma unroll
@@ -164,10 +182,7 @@ short_conv_tile_kernel(const TI* __restrict__ x, int ld, int at, int channels, c
       return;
     }
   }
-#pragma unroll
-  for (int v = 0; v < 4; ++v)
-#pragma unroll
-    for (int j = 0; j < TAPS; ++j) wt[v][j] = w[(size_t)(c + v) * TAPS + j];
+  conv_weights<TAPS>(w, c, wt);
   const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
   for (int t = t0; t < t0 + ROWS && t < n_rows; ++t) {
@@ -228,8 +243,10 @@ TOKB200_API int tokb200_short_conv(const void* x, int x_dtype, int ld, int at, i
   if (taps >= 2 && taps <= 4 && channels % 4 == 0 && at % 4 == 0 && ld % 4 == 0 && off % 4 == 0 && stride % 4 == 0 &&
       ((uintptr_t)x % (4 * x_size)) == 0 && ((uintptr_t)y % (4 * y_size)) == 0 &&
       (((uintptr_t)state | (uintptr_t)bias) & 15) == 0) {
-    // many rows: runs of 8 rows a thread; few (a decoding step): a row a thread, so that the blocks are many
-    const int rows = n_rows >= 1024 ? 8 : 1;
+    // much work: runs of 8 rows a thread; little (a decoding step, a short prompt): a row a thread, so that the blocks are many.
+    // us, a row / 8 rows, 32-bit: 4,352 channels 300 rows 7.1 / 7.7, 500 10.3 / 8.9; 2,304 channels 500 rows 6.4 / 7.5, 700 8.3 /
+    // 8.6, 1,000 10.8 / 8.9; 1,024 channels 1,000 rows 6.0 / 7.2
+    const int rows = (shift ? n_rows >= 1024 : (long long)n_rows * channels >= 1500000) ? 8 : 1;
     const int threads = channels / 4 >= 128 ? 128 : (channels / 4 + 31) / 32 * 32;
     const dim3 grid((n_rows + rows - 1) / rows, (channels / 4 + threads - 1) / threads);
 #define TILE(TAPS, ROWS, TI, TO)                                                                                     \
