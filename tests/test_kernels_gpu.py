@@ -1445,3 +1445,26 @@ def test_gated_product_up_to_64_rows(M, inner, K, activation):
     slack = 1.2 * eps * ((xd.abs() @ gd.abs().t()) * u.abs() + (xd.abs() @ ud.abs().t()) * (g.abs() + 1))
     assert bool(((room[:M].double().cpu() - want).abs() <= slack + want.abs() * 2.0 ** -8 + 1e-7).all())
     assert bool((room[M:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M", [8, 9, 16, 17])
+def test_large_weights_on_both_sides_of_nine_rows(M):
+    """A weight of 13 million elements: the ring kernel's rows and the tensor cores' give the same product."""
+    from tokenizer_b200.parts import gemm_bf16
+    o = ops()
+    inner, K = 6656, 1024
+    x = rnd(M, K, seed=77, dtype=torch.bfloat16)
+    gate, up = (rnd(inner, K, seed=s, dtype=torch.bfloat16, scale=0.2) for s in (78, 79))
+    out = torch.full((M, inner), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.gated_linear(x, o.interleave_gate_up(gate, up), out)
+    xd = x.double().cpu()
+    g, u = xd @ gate.double().cpu().t(), xd @ up.double().cpu().t()
+    want = torch.nn.functional.silu(g) * u
+    assert bool(((out.double().cpu() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-3).all())      # one rounding, and 32-bit sums
+    w = rnd(1024, 13312, seed=80, dtype=torch.bfloat16, scale=0.1)
+    a = rnd(M, 13312, seed=81, dtype=torch.bfloat16)
+    got = gemm_bf16.linear_bf16(a, w, None, torch.bfloat16, partials_ok=True)
+    total = got.double().sum(0) if got.dim() == 3 else got.double()
+    want = a.double().cpu() @ w.double().cpu().t()
+    assert float((total.cpu() - want).abs().max()) <= float(want.abs().max()) * (2.0 ** -8 if got.dim() == 2 else 2.0 ** -16)
+    o.gemm_tcgen05_check()

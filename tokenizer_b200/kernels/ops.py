@@ -761,7 +761,12 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
         raise ValueError("gated_linear is the bfloat16 kernel")
     if not gated_linear_supported(K, N) or w.shape[1] != K or tuple(out.shape) != (M, N // 2):
         raise ValueError("gated_linear: K a multiple of 8, N of 256, out [M, N/2]")
-    if M <= SMALL_M_ROWS and _RING and N * K >= RING_ELEMENTS and linear_ring_supported(M, N, K, 1, True):
+    if M <= SMALL_M_ROWS and N * K >= RING_ELEMENTS and M > RING_ROWS:
+        # a large weight and nine rows or more (us at 16 rows, this / the ring kernel: 17,920 x 1,536 11.3 / 13.6, 37,888 x 3,584
+        # 44 / 50; at 8 11.1 / 11.6 and 43.7 / 43.6)
+        _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_gated(
+            _ptr(x), _ptr(w), _ptr(out), _i(M), _i(N), _i(K), act, _stream()), "gated_linear")
+    elif M <= SMALL_M_ROWS and _RING and N * K >= RING_ELEMENTS and linear_ring_supported(M, N, K, 1, True):
         linear_ring_gated(x, w, out, activation)
     elif M <= SMALL_M_ROWS:
         _check(_lib("linear_small_m").tokb200_linear_small_m_gated(
@@ -1025,6 +1030,7 @@ def layer_small_m_check(d: int) -> None:
 # ---- few rows, a large weight: one block a multiprocessor streams it through rings in shared memory ----
 RING_ELEMENTS = 13_000_000     # from this many weight elements on (26 MB) the ring kernel leads the one with plain loads
 RING_MAX_ROWS = 32
+RING_ROWS = 8                   # rows up to which the ring kernel is at least level with the tensor cores on such a weight
 _RING = os.environ.get("TOKB200_RING", "1") != "0"     # TOKB200_RING=0: large weights on linear_small_m too
 _ring_plans = {}
 

@@ -136,12 +136,14 @@ def linear_bf16(a: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         ops.gemm_tcgen05_pair(a, weight, None, out, ops.PAIR_PARTIALS)
         return out
     tiles_cut = 1
-    if partials_ok and bias is None and M > ops.SMALL_M_ROWS and use_tcgen05(M, N, K, cut_along_k=True):
+    tensor_rows = ops.RING_ROWS if N * K >= ops.RING_ELEMENTS else ops.SMALL_M_ROWS
+    if partials_ok and bias is None and M > tensor_rows and use_tcgen05(M, N, K, cut_along_k=True):
         tiles_cut = choose_tile_k_splits(M, N, K)
     if tiles_cut > 1:
         # few output tiles (a narrow matrix, a few dozen rows): pieces of k over all SMs.  From 17 rows on this leads the ring
         # kernel (us, this / ring: 896 x 896 2.5 / 3.2 at 17 rows, 2.6 / 3.9 at 32; 896 x 4,864 4.5 / 4.9 and 4.7 / 5.3;
-        # 2,048 x 8,192 8.5 / 13.1 and 8.7 / 13.7), and the kernel of plain loads (3.4 to 17.5 at 17 rows)
+        # 2,048 x 8,192 8.5 / 13.1 and 8.7 / 13.7), and the kernel of plain loads (3.4 to 17.5 at 17 rows); of large
+        # weights from 9 rows on (16 rows: 3,584 x 18,944 24.3 / 28.9, 2,048 x 8,192 8.4 / 9.9; 8: 24.1 / 23.6, 8.4 / 8.5)
         out = torch.empty((tiles_cut, M, N), dtype=torch.float32, device=a.device)
         ops.gemm_tcgen05_partials(a, weight, out)
         return out
