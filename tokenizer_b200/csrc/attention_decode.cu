@@ -13,7 +13,7 @@
 //
 // A row's visible keys lo..pos are cut into n_splits pieces of `chunk` keys; chunk is
 // min_chunk * 2^k, the smallest that needs at most MAX_SPLITS pieces.  The launcher picks
-// min_chunk (256 .. 2048) for the launch as a whole from the number of (row, kv head) pairs
+// min_chunk (256 .. 4,096, to 8,704 where the pairs alone fill the device) for the launch as a whole from the number of (row, kv head) pairs
 // and the table's reach: with few pairs, short pieces on many blocks win (a block's time is
 // a chain of dependent loads per pass); with many pairs, long pieces win (fewer blocks than
 // the device holds at once cost no second wave, and fewer pieces cost less merging).  The

@@ -1,4 +1,5 @@
-// True 32-bit matrix product for the check path: C[M,N] = A[M,K] W[N,K]^T (+ bias),
+// True 32-bit matrix product C[M,N] = A[M,K] W[N,K]^T (+ bias) where K is below 768, no multiple of 4 or the operands do not
+// lie on 16 bytes (the others go to the tensor cores in exact pieces, gemm_f32_tcgen05.cu, whose error is the smaller one there):
 // plain FMA in float, no tensor cores and no reduced-precision mode.  Each output
 // element sums its K products in index order, so a row's result does not depend
 // on how many other rows are in the batch, nor on the tile the element falls into.

@@ -1,6 +1,6 @@
 """The matrix product y = a W^T (+ bias) behind every projection.
 
-float32: the framework's own FMA kernel, true 32-bit.  bfloat16: operands in
+float32: the framework's own kernels, true 32-bit (on the tensor cores in exact pieces from 768 of k on, multiply-adds below).  bfloat16: operands in
 bfloat16, accumulation in 32-bit; the result is bfloat16 or, where asked
 (logits), float32.
 """

@@ -125,12 +125,14 @@ DELTA_CHUNKS_HEADS = 8
 
 def _chunks_pay(q_lens, heads: int, chain: float, work: float) -> bool:
     """Whether chunks of 32 tokens are the faster form of a delta rule for portions of these lengths.  Chunks cost 0.22 us
-    a chunk and head whatever is in it (a lone token too); their chain, some 2.6 us a chunk of the longest portion, is a
-    quarter of the one token by token and never decides.  Token by token a step takes `chain` us a token of its longest
+    a chunk and head whatever is in it (a lone token too); their chain, some 1.7 us a chunk of the longest portion, is a
+    sixth of the one token by token and never decides.  Token by token a step takes `chain` us a token of its longest
     portion, or `work` us a token and head once the device is full.  Fitted to heads of 128 x 128, one decay a head / one a
-    channel, us token by token -> in chunks, 16 heads: 2,048 tokens 772 -> 254 / 558 -> 272; 512 and 15 single ones 231 ->
-    114 / 199 -> 124; 512 and 63 single ones 248 -> 309 / 171 -> 320 (not taken); 128 x 4 and 8 x 28 154 -> 185 / 116 -> 195
-    (not taken); eight of 512 with one a channel 494 -> 441.  Values of fewer lanes make both forms cheaper, and the choice
+    channel, us token by token -> in chunks, 16 heads: 2,048 tokens 772 -> 200 / 558 -> 212; 512 and 15 single ones 231 ->
+    114 / 199 -> 124; 512 and 63 single ones 248 -> 263 / 171 -> 275 (not taken); 128 x 4 and 8 x 28 154 -> 185 / 116 -> 195
+    (not taken); eight of 512 with one a channel 494 -> 441.  (Figures of
+    more portions than one were taken with the scans on multiply-adds, which are up to a third slower: where chunks are taken
+    they still lead by more.)  Values of fewer lanes make both forms cheaper, and the choice
     stays right: a layer of 16 heads of 128 x 16, us, eight of 512 394 -> 282 / 470 -> 312, sixteen of 128 174 -> 167 / 223
     -> 186, one of 128 73 -> 48 / 56 -> 54; of 128 x 64 sixteen of 128 295 -> 227 / 236 -> 245, which `_full_turns` is for."""
     chunks = sum((n + 31) // 32 for n in q_lens)
