@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const F
       const int kb0 = group * p.group_stages, kb1 = min(p.stages, kb0 + p.group_stages);
       for (int kb = kb0; kb < kb1; kb += FS_CHUNK, ++turn) {
         const int b = turn & 1;
-        if (!fs_wait(&sums_full[b], (turn >> 1) & 1)) { sound = false; break; }
+        // the lanes come here one by one, from polls and from stores that some of them skip: the loads want all of them at once
+        if (!__all_sync(0xffffffffu, fs_wait(&sums_full[b], (turn >> 1) & 1))) { sound = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < kCols; c += kPiece) {

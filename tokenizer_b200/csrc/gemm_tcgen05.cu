@@ -198,6 +198,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll 1
       for (int c0 = 0; c0 < BLOCK_N; c0 += 32) {
         unsigned v[32];
+        __syncwarp();                    // behind rows and columns that some lanes skip
         tmem_load_32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
         const int col0 = n0 + c0;
         if (row < M && col0 < N) {
@@ -855,7 +856,10 @@ gemm_tcgen05_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     int round = 0;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++round) {
       const int n = unit % n_tiles * TC_BLOCK_M + quarter * 32 + lane, buf = round & 1;
+      // the lanes come here one by one, from polls and from stores that some of them skip: the loads want all of them at once
       bool ok = mbar_wait(&acc_full[buf], (round >> 1) & 1);
+      __syncwarp();
+      if (!GATED) ok = __all_sync(0xffffffffu, ok);
       if (GATED) {                       // the four warps go on or give up together; the sums of the unit before have been read
         unsigned all;
         asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, 1, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
