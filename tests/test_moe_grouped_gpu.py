@@ -74,3 +74,61 @@ def test_a_layer_gives_the_same_either_way():
     parts = torch.cat([p.float() if p.dim() == 2 else p.sum(0) for p in parts])
     # three roundings to bfloat16 on one way, two on the other
     assert float((whole - parts).norm() / parts.norm()) < 6e-3
+
+
+@pytest.mark.parametrize("score", ["sigmoid", "softmax", "softmax_of_chosen"])
+@pytest.mark.parametrize("experts,groups,keep", [(64, 1, 1), (40, 1, 1), (64, 8, 4)])
+@pytest.mark.parametrize("tokens", [5, 600])
+def test_a_token_of_nan_takes_no_more_experts(score, experts, groups, keep, tokens):
+    """Rows that are all NaN, or whose scores are NaN for one expert, choose `top` experts like any other; the others choose as
+    they do without them."""
+    o = ops()
+    if groups > 1 and score == "softmax_of_chosen":
+        pytest.skip("that score knows no groups")
+    top, hidden = 3, 128
+    g = torch.Generator(device=DEV).manual_seed(experts)
+    h, router = torch.randn(tokens, hidden, generator=g, device=DEV), torch.randn(experts, hidden, generator=g, device=DEV)
+
+    def route(h, router):
+        share = torch.full((tokens, experts), 9.0, device=DEV)
+        o.moe_route(h, router, experts, top, None, share, score=score, groups=groups, keep=keep)
+        return share
+    clean = route(h, router)
+    assert bool(((clean != 0).sum(1) == top).all())
+    bad = h.clone()
+    bad[1::3] = float("nan")
+    share = route(bad, router)
+    assert bool(((share != 0).sum(1) <= top).all())
+    healthy = [t for t in range(tokens) if t % 3 != 1]
+    assert torch.equal(share[healthy], clean[healthy])
+    if score != "softmax_of_chosen":                      # which passes a NaN by
+        assert bool(share[1::3].isnan().any(1).all())
+        worn = router.clone()
+        worn[7, 3] = float("nan")
+        share = route(h, worn)
+        assert bool(((share != 0).sum(1) <= top).all())
+
+
+def test_tokens_of_nan_leave_the_others_alone():
+    """A request of NaN rows in a routed layer's step: every other row's output is what it is without them, bit for bit."""
+    from tokenizer_b200.config import PartSpec
+    from tokenizer_b200.parts import Runtime, build_part, part_class
+    from tokenizer_b200.weights import WeightStore
+    o = ops()
+    experts, top, ff, hidden, tokens = 64, 1, 512, 512, 2000
+    spec = PartSpec("routed_mlp", dict(experts=experts, top=top, expert_inner=ff, hidden_size=hidden, activation="silu",
+                                       score="sigmoid"), "mlp")
+    g = torch.Generator(device=DEV).manual_seed(6)
+    weights = {t.name: (torch.randn(tuple(t.shape), generator=g, device=DEV) / t.shape[1] ** 0.5).bfloat16()
+               for t in part_class("feed_forward", "routed_mlp").tensors(spec)}
+    layer = build_part("feed_forward", spec, WeightStore(weights), Runtime(torch.device(DEV), torch.bfloat16))
+    assert o.moe_grouped_pays(tokens, experts, top, ff, 0, hidden)
+    h = torch.randn(tokens, hidden, generator=g, device=DEV).bfloat16()
+    want = layer.forward(h)
+    bad = h.clone()
+    bad[300:1500] = float("nan")
+    got = layer.forward(bad)
+    healthy = torch.ones(tokens, dtype=torch.bool, device=DEV)
+    healthy[300:1500] = False
+    assert torch.equal(got[healthy], want[healthy])
+    assert bool(got[~healthy].isnan().all())

@@ -31,13 +31,17 @@ enum : int { MOE_SHARED_NONE = 0, MOE_SHARED_GATED = 1, MOE_SHARED_ONE = 2 };
 
 #define MOE_MAX_EXPERTS 1024
 
-// the largest value and, among equals, the lowest index over a warp's lanes (index -1: nothing to offer)
+// Whether v comes in front of value: the larger one, a NaN in front of every number (so that all lanes of a warp agree on
+// one choice whatever the scores hold: a token whose scores are NaN takes `top` experts like any other, not every lane its own).
+__device__ __forceinline__ bool moe_above(float v, float value) { return v > value || (v != v && value == value); }
+
+// the first by `moe_above` and, among equals, the lowest index over a warp's lanes (index -1: nothing to offer)
 __device__ __forceinline__ void moe_warp_best(float& value, int& index) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float v = __shfl_xor_sync(0xffffffffu, value, o);
     const int i = __shfl_xor_sync(0xffffffffu, index, o);
-    if (i >= 0 && (index < 0 || v > value || (v == value && i < index))) {
+    if (i >= 0 && (index < 0 || moe_above(v, value) || (!moe_above(value, v) && i < index))) {
       value = v;
       index = i;
     }
@@ -65,7 +69,7 @@ __device__ __forceinline__ void moe_choose(const float* z, const float* choice, 
       int best = -1;
       float value = -INFINITY;
       for (int g = lane; g < groups; g += 32)
-        if (!open[g] && (best < 0 || group_worth[g] > value)) { best = g; value = group_worth[g]; }
+        if (!open[g] && (best < 0 || moe_above(group_worth[g], value))) { best = g; value = group_worth[g]; }
       moe_warp_best(value, best);
       if (best >= 0 && best % 32 == lane) open[best] = 1;
     }
@@ -78,7 +82,7 @@ __device__ __forceinline__ void moe_choose(const float* z, const float* choice, 
     int best = -1;
     float value = -INFINITY;
     for (int e = lane, i = 0; e < experts; e += 32, ++i)
-      if (!((taken >> i) & 1u) && (keep == groups || open[e / size]) && (best < 0 || choice[e] > value)) {
+      if (!((taken >> i) & 1u) && (keep == groups || open[e / size]) && (best < 0 || moe_above(choice[e], value))) {
         best = e;
         value = choice[e];
       }
