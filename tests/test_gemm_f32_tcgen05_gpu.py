@@ -60,3 +60,24 @@ def test_small_numbers_keep_their_bits():
     o.gemm_f32_tcgen05(a, w, None, out)
     want = a.double() @ w.double().t()
     assert float((out.double() - want).abs().max()) <= 20 * 2.0 ** -24 * float((a.double().abs() @ w.double().abs().t()).max())
+
+
+@pytest.mark.parametrize("K", [768, 2000])
+def test_products_just_below_the_largest_number(K):
+    """The first pieces of two numbers are rounded up: their product, or a sum of such products, may lie above the largest
+    number where the numbers' own does not."""
+    o = ops()
+    M, N = 20, 130
+    a, w = torch.zeros(M, K, device=DEV), torch.zeros(N, K, device=DEV)
+    a[:, 5], w[:, 5] = 1.999 * 2.0 ** 63, 2.0 ** 64                      # 1.999 is 2 in sixteen bits
+    a[3, 6], w[:, 6] = -1.999 * 2.0 ** 63, 2.0 ** 63                     # half of it off again
+    w[7, 5], w[7, 6] = -1.9999 * 2.0 ** 63, 0.0
+    w[9, 5] = 2.0 ** 66                                                  # truly above
+    want = a.double() @ w.double().t()
+    for tile in range(5):
+        for split in (False, True):
+            got = torch.empty(M, N, device=DEV)
+            o.gemm_f32_tcgen05(a, w, None, got, tile=tile, split=split)
+            columns = [n for n in range(N) if n != 9]
+            assert bool(torch.isfinite(got[:, columns]).all()) and bool(got[:, 9].isinf().all())
+            assert float(((got[:, columns].double() - want[:, columns]) / want[:, columns]).abs().max()) < 1e-6

@@ -28,9 +28,10 @@
 // things that counted: a row's 32 bytes in one load (140 -> 128 us at 9,728 x 896) and loads of the output in front of
 // the adds to it, eight at a time (the drain alone took 47 us of 148).
 //
-// An operand that is an infinity, a NaN or rounds to an infinity in 16 bits has no such pieces (its last one is a NaN):
-// outputs that come out as a NaN are computed anew by a chain of multiply-adds.  Numbers below 2^-109 keep an absolute error
-// of 2^-133.  Every wait on an mbarrier is bounded.
+// An operand that is an infinity, a NaN or rounds to an infinity in 16 bits has no such pieces (its last one is a NaN), and a
+// product just below the largest number may lie above it in its first pieces: outputs that come out as no finite number are
+// computed anew by a chain of multiply-adds.  Numbers below 2^-109 keep an absolute error of 2^-133.  Every wait on an mbarrier is
+// bounded.
 #include "common.cuh"
 
 #define FS_K 64
@@ -239,14 +240,14 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_tcgen05_kernel(const F
         for (int j = 0; j < 8; ++j) {
           if (m0 + c + j >= p.M) continue;
           const float v = acc[c + j];
-          if (v == v) out[(size_t)(c + j) * p.N] = first ? v + shift : (before[j] + v) + shift;
+          if (v - v == 0.f) out[(size_t)(c + j) * p.N] = first ? v + shift : (before[j] + v) + shift;
           else odd = true;
         }
       }
-      if (odd) {                       // an operand without pieces, or a true NaN
+      if (odd) {                       // an operand without pieces, a product of pieces beyond the largest number, or truly no finite one
         unsigned long long which = 0;
 #pragma unroll
-        for (int j = 0; j < kCols; ++j) which |= (unsigned long long)(m0 + j < p.M && acc[j] != acc[j]) << j;
+        for (int j = 0; j < kCols; ++j) which |= (unsigned long long)(m0 + j < p.M && !(acc[j] - acc[j] == 0.f)) << j;
 #pragma unroll 1
         for (int j = 0; j < kCols; ++j) {
           if (!(which >> j & 1)) continue;
