@@ -81,3 +81,33 @@ def test_products_just_below_the_largest_number(K):
             columns = [n for n in range(N) if n != 9]
             assert bool(torch.isfinite(got[:, columns]).all()) and bool(got[:, 9].isinf().all())
             assert float(((got[:, columns].double() - want[:, columns]) / want[:, columns]).abs().max()) < 1e-6
+
+
+@pytest.mark.parametrize("K", [768, 772, 896, 1024])
+@pytest.mark.parametrize("M,N", [(1, 300), (65, 257)])
+def test_numbers_of_one_sign(K, M, N):
+    """What the tensor core cuts off instead of rounding adds up where all products have one sign: from 768 of k on it is still
+    closer to 64 bits than a chain of multiply-adds."""
+    o = ops()
+    a, w = rnd(M, K, seed=21).abs(), rnd(N, K, seed=22).abs()
+    got, chain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    o.gemm_f32_tcgen05(a, w, None, got)
+    o.gemm_f32(a, w, None, chain, form=0)
+    want = a.double() @ w.double().t()
+    assert float((got.double() - want).norm()) <= float((chain.double() - want).norm())
+
+
+@pytest.mark.parametrize("M", [1, 7, 100])
+def test_where_the_tensor_cores_take_over(M):
+    """By k and the operands' place alone, whatever the rows: 768 of k on 16 bytes and more."""
+    o = ops()
+    for K, off, tensor in ((764, 0, False), (768, 0, True), (770, 0, False), (772, 0, True), (768, 1, False)):
+        room = rnd(M * K + 4, seed=23)
+        a, w = room[off:off + M * K].view(M, K), rnd(90, K, seed=24)
+        got, own, chain = (torch.empty(M, 90, device=DEV) for _ in range(3))
+        o.gemm_f32(a, w, None, got)
+        o.gemm_f32(a, w, None, chain, form=0)
+        if tensor:
+            o.gemm_f32_tcgen05(a, w, None, own)
+        assert torch.equal(got, own if tensor else chain)
+        assert not tensor or not torch.equal(own, chain)
