@@ -159,3 +159,88 @@ def test_inputs_off_16_bytes(by_channel, taps, shift):
     for moves in ((shift, 0), (0, shift), (shift, shift)):
         for got, ref in zip(run(*moves), want):
             assert torch.equal(got, ref)
+
+
+def in_chunks(q, k, v, beta, g, S):
+    """One head by the chunks' own sums in 64 bits (q scaled): S [dim, vdim] moves on; the rows' outputs."""
+    out, n = torch.empty(q.shape[0], v.shape[1], dtype=torch.float64), q.shape[0]
+    for t0 in range(0, n, 32):
+        m = min(32, n - t0)
+        qc, kc, vc, bc, gc = (x[t0:t0 + m] for x in (q, k, v, beta, g))
+        G = torch.cumprod(gc, 0)
+        between = torch.zeros(m, m, q.shape[1], dtype=torch.float64)
+        for s in range(m):
+            between[s, s] = 1.0
+            for t in range(s + 1, m):
+                between[t, s] = between[t - 1, s] * gc[t]
+        A = bc[:, None] * torch.einsum("tc,sc,tsc->ts", kc, kc, between).tril(-1)
+        M = torch.einsum("tc,sc,tsc->ts", qc, kc, between)
+        solve = lambda r: torch.linalg.solve_triangular(A + torch.eye(m, dtype=torch.float64), r, upper=False, unitriangular=True)
+        W, U0 = solve(bc[:, None] * G * kc), solve(bc[:, None] * vc)
+        U = U0 - W @ S
+        for t in range(m):
+            out[t0 + t] = (G[t] * qc[t]) @ S + sum(M[t, s] * U[s] for s in range(t + 1))
+        S = G[-1][:, None] * S + sum((between[m - 1, s] * kc[s])[:, None] * U[s][None, :] for s in range(m))
+    return out, S
+
+
+@pytest.mark.parametrize("by_channel,columns", [(False, 16), (False, 32), (True, 16), (True, 32)])
+@pytest.mark.parametrize("where", ["matrix", "large matrix", "values", "large values"])
+@pytest.mark.parametrize("n", [20, 70])
+def test_numbers_without_pieces(by_channel, columns, where, n):
+    """Infinities, and numbers that round to one in 16 bits, in the matrix or in the values: outputs and matrix hold numbers,
+    infinities (with their signs) and NaN where the same sums in 64 bits do, and other columns what they hold without them."""
+    o = ops()
+    groups, heads, dim, vdim, inf = 1, 2, 128, 32, float("inf")
+    channels, off = 2 * dim + heads * vdim, heads * vdim * 128
+    gen = torch.Generator().manual_seed(19)
+    rnd = lambda *s: torch.randn(*s, generator=gen)
+    conv_w, a_log = torch.ones(channels, 1), rnd(heads) * 0.3
+    dt_bias = rnd(heads * (dim if by_channel else 1)) - 3.0
+    proj = rnd(n, channels + 2 * heads)
+    decay = rnd(n, heads * dim) if by_channel else proj
+    S = rnd(heads, dim, vdim)
+    bad_S, bad_proj, touched = S.clone(), proj.clone(), [5, vdim + 30]       # columns of the two heads side by side
+    if where == "matrix":
+        bad_S[0, 3, 5], bad_S[1, 127, 30] = inf, -inf
+    elif where == "large matrix":
+        bad_S[0, 3, 5], bad_S[1, 127, 30] = 3.4e38, -3.395e38
+    else:                                         # silu keeps a large number and an infinity above zero
+        bad_proj[11, 2 * dim + 5] = bad_proj[17, 2 * dim + vdim + 30] = inf if where == "values" else 3.4e38
+
+    def run(S, proj):
+        state, out = S.transpose(1, 2).reshape(1, -1).to(DEV), torch.empty(n, heads * vdim, device=DEV)
+        p = proj.to(DEV)
+        o.delta_chunks(p, 0, channels, decay.to(DEV) if by_channel else p, 0 if by_channel else channels + heads, by_channel,
+                       groups, heads, dim, vdim, 1, conv_w.to(DEV), a_log.to(DEV), dt_bias.to(DEV), state, off,
+                       torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV), out,
+                       columns=columns)
+        return out.cpu(), state.cpu().view(heads, vdim, 128).transpose(1, 2)
+    clean, clean_S = run(S, proj)
+    got, got_S = run(bad_S, bad_proj)
+    others = [c for c in range(heads * vdim) if c not in touched]
+    assert torch.equal(got[:, others], clean[:, others])
+    flat, flat_clean = (x.permute(1, 0, 2).reshape(dim, -1) for x in (got_S, clean_S))
+    assert torch.equal(flat[:, others], flat_clean[:, others])
+    x = bad_proj[:, :channels].double()
+    y = torch.where(x.isinf(), x, x * torch.sigmoid(x))
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+    beta = torch.sigmoid(proj[:, channels:channels + heads].double())
+    width = heads * (dim if by_channel else 1)
+    at = 0 if by_channel else channels + heads
+    soft = torch.nn.functional.softplus(decay[:, at:at + width].double() + dt_bias.double())
+    rate = torch.exp(a_log.double())
+    for h, column in ((0, 5), (1, 30)):
+        g = torch.exp(-rate[h] * (soft[:, h * dim:(h + 1) * dim] if by_channel else soft[:, h:h + 1].expand(n, dim)))
+        want, want_S = in_chunks(unit(y[:, :dim]) * dim ** -0.5, unit(y[:, dim:2 * dim]),
+                                 y[:, 2 * dim + h * vdim:2 * dim + (h + 1) * vdim], beta[:, h], g, bad_S[h].double())
+        for mine, ref in ((got[:, h * vdim + column], want[:, column]), (got_S[h][:, column], want_S[:, column])):
+            ref = ref.float()
+            assert torch.equal(mine.isnan(), ref.isnan()) and torch.equal(mine.isinf(), ref.isinf())
+            assert torch.equal(mine[mine.isinf()], ref[ref.isinf()])
+            fine = ref.isfinite()
+            if bool(fine.any()):
+                size = float(ref[fine].abs().max())
+                assert float((mine[fine] - ref[fine]).abs().max()) <= 1e-4 * max(1.0, size)
+        if where[:5] == "large":
+            assert bool(got[:, h * vdim + column].isfinite().all())

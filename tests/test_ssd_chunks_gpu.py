@@ -86,3 +86,73 @@ def test_a_token_changes_nothing_before_it(value, at):
         if column == 3:                                       # a column of x meets no other
             others = [c for c in range(inner) if c != 3]
             assert torch.equal(got[:, others], want[:, others])
+
+
+def in_chunks(xbc, dt_in, dt_bias, a_log, skip, heads, groups, vdim, n_state, S):
+    """One request by the chunks' own sums in 64 bits: S [heads, n_state, vdim] moves on in place; the rows' outputs."""
+    n, inner, share = xbc.shape[0], heads * vdim, heads // groups
+    xbc = xbc.double()
+    dt = torch.nn.functional.softplus(dt_in.double() + dt_bias.double())
+    keep = torch.exp(-torch.exp(a_log.double()) * dt)
+    out = torch.empty(n, heads, vdim, dtype=torch.float64)
+    for t0 in range(0, n, 32):
+        rows = slice(t0, min(n, t0 + 32))
+        for h in range(heads):
+            g = h // share
+            x = xbc[rows, h * vdim:(h + 1) * vdim]
+            b = xbc[rows, inner + g * n_state:inner + (g + 1) * n_state]
+            c = xbc[rows, inner + (groups + g) * n_state:inner + (groups + g + 1) * n_state]
+            a, d, m = keep[rows, h], dt[rows, h], x.shape[0]
+            decay = [[float(torch.prod(a[s + 1:t + 1])) for s in range(m)] for t in range(m)]
+            for t in range(m):
+                v = sum(decay[t][s] * (c[t] @ b[s]) * d[s] * x[s] for s in range(t + 1))
+                out[t0 + t, h] = v + skip[h].double() * x[t] + torch.prod(a[:t + 1]) * (c[t] @ S[h])
+            S[h] = torch.prod(a) * S[h] + sum(b[s][:, None] * (decay[m - 1][s] * d[s] * x[s])[None, :] for s in range(m))
+    return out.reshape(n, inner)
+
+
+@pytest.mark.parametrize("where", ["matrix", "x", "B", "C", "large matrix", "large x", "large product"])
+@pytest.mark.parametrize("n", [20, 70])
+def test_numbers_without_pieces(where, n):
+    """Infinities, and numbers that round to one in 16 bits, in the matrix or in what comes in: outputs and matrix hold numbers,
+    infinities (with their signs) and NaN where the same sums in 64 bits do."""
+    from tokenizer_b200.kernels import ops as o
+    heads, groups, vdim, n_state = 2, 1, 64, 100
+    inner, inf = heads * vdim, float("inf")
+    g = torch.Generator().manual_seed(17)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    dt_bias, a_log, skip, S = rnd(heads) - 5.0, rnd(heads) * 0.3, rnd(heads), rnd(heads, n_state, vdim)
+    xbc, proj = rnd(n, inner + 2 * n_state), rnd(n, heads)
+    if where == "matrix":
+        S[0, 3, 5], S[1, 99, 63] = inf, -inf
+    elif where == "x":
+        xbc[6, 5], xbc[18, vdim + 40] = inf, -inf
+    elif where == "B":
+        xbc[9, inner + 50] = inf
+    elif where == "C":
+        xbc[9, inner + n_state + 50] = -inf
+    elif where == "large matrix":                   # one lane of it alone meets C, at an eighth
+        xbc[:, inner + n_state + 3] *= 2.0 ** -4
+        S[0, 3, 5], S[1, 3, 63] = 3.4e38, -3.395e38
+    elif where == "large x":
+        xbc[:, inner:] *= 2.0 ** -4
+        skip *= 2.0 ** -3
+        xbc[6, 5], xbc[18, vdim + 40] = 3.4e38, -3.395e38
+    else:                                           # below the largest number by the numbers, above it by their first pieces
+        xbc[:, inner + n_state:] = 0
+        xbc[0, inner + n_state + 3], S[0, 3, 5], dt_bias[0], skip[0] = 2.0, 1.999 * 2.0 ** 126, -30.0, 0.0
+    state = S.transpose(1, 2).reshape(1, -1).to(DEV)
+    y = torch.empty(n, inner, device=DEV)
+    o.ssd_chunks(xbc.to(DEV), proj.to(DEV), 0, dt_bias.to(DEV), a_log.to(DEV), skip.to(DEV), heads, groups, vdim, n_state, state,
+                 torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV), y)
+    want_S = S.double()
+    want = in_chunks(xbc, proj, dt_bias, a_log, skip, heads, groups, vdim, n_state, want_S)
+    assert where[:5] != "large" or bool(want.isfinite().all())
+    for got, ref in ((y.cpu(), want), (state.cpu().view(heads, vdim, n_state).transpose(1, 2), want_S)):
+        ref32 = ref.float()
+        assert torch.equal(got.isnan(), ref32.isnan()) and torch.equal(got.isinf(), ref32.isinf())
+        assert torch.equal(got[got.isinf()], ref32[ref32.isinf()])
+        fine = ref32.isfinite()
+        size = ref[fine].abs().reshape(-1)
+        # what meets a large number is as large, the rest as above: an element's error against its own size or that of its row
+        assert bool(((got[fine].double() - ref[fine]).abs().reshape(-1) <= 1e-4 * size + 1e-4 * (1.0 + size)).all())

@@ -491,6 +491,62 @@ template <int COLS> struct DtShape {
   static constexpr int kSmem = kRing * 4 + 2 * kDtPieces;
 };
 
+// A number of a record's pieces: they add up to it (a NaN where it is one; W, G q and K hold no infinities, their rows being
+// products of decays, of unit vectors and of what the substitution makes of them).
+__device__ __forceinline__ float dt_whole(const float* tile, int lane, int i) {       // tile: [piece][lane][8]
+  const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(tile) + lane * 8 + i;
+  return (__bfloat162float(p[0]) + __bfloat162float(p[256])) + __bfloat162float(p[512]);
+}
+// The same portion in plain multiply-adds, all threads of the block, for numbers that have no pieces (an infinity in the matrix
+// or in U, numbers that round to one in 16 bits, and what then comes of them): slow, and replaces nothing but what the pieces
+// left as no finite number.  `mine`: the block's columns of the matrix in memory, as they were before the portion; what lies
+// behind the portion's last token, or behind a row's own, takes no part.  s_s: [128][COLS] floats, behind it the matrix as the
+// pieces left it, of that form, and U [32][COLS].
+template <int COLS>
+__device__ __noinline__ void dt_scan_plain(float* s_s, const float* __restrict__ rec, size_t record_ld, int n, int vdim, int col0,
+                                           float* __restrict__ mine, float* __restrict__ o_out, size_t o_ld) {
+  const float* end_s = s_s + DC_DIM * COLS;
+  float* u_s = s_s + 2 * DC_DIM * COLS;
+  for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS) s_s[i] = mine[(size_t)(i % COLS) * DC_DIM + i / COLS];
+  __syncthreads();
+  for (int t0 = 0; t0 < n; t0 += DC_TOKENS, rec += record_ld) {
+    const int here = min(DC_TOKENS, n - t0);
+    auto product = [&](int row, int c) {                 // a row of W (0 .. 31) or G q (32 .. 63) times a column
+      const int lane = (row & 7) * 4, high = row >> 3 & 1;
+      float sum = 0.f;
+      for (int k = 0; k < DC_DIM; ++k)
+        sum = fmaf(dt_whole(rec + (k / 16 * 4 + row / 16) * 384, lane + (k & 7) / 2, ((k >> 3 & 1) * 2 + high) * 2 + (k & 1)),
+                   s_s[k * COLS + c], sum);
+      return sum;
+    };
+    for (int i = threadIdx.x; i < here * COLS; i += DT_THREADS) {
+      const int t = i / COLS, c = i % COLS;
+      u_s[i] = rec[kDcU + t * vdim + col0 + c] - product(t, c);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < here * COLS; i += DT_THREADS) {
+      const int t = i / COLS, c = i % COLS;
+      float* to = o_out + (size_t)(t0 + t) * o_ld + c;
+      if (*to - *to == 0.f) continue;
+      float sum = product(DC_TOKENS + t, c);
+      for (int s = 0; s <= t; ++s) sum = fmaf(rec[kDcM + t * DC_TOKENS + s], u_s[s * COLS + c], sum);
+      *to = sum;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS) {
+      const int k = i / COLS, c = i % COLS;
+      float more = 0.f;
+      for (int t = 0; t < here; ++t)
+        more = fmaf(dt_whole(rec + kDcK + (k / 16 * 2 + t / 16) * 384, (k & 7) * 4 + (t & 7) / 2,
+                             ((k >> 3 & 1) * 2 + (t >> 3 & 1)) * 2 + (t & 1)), u_s[t * COLS + c], more);
+      s_s[i] = fmaf(rec[kDcG + k], s_s[i], more);
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS)
+    mine[(size_t)(i % COLS) * DC_DIM + i / COLS] = end_s[i] - end_s[i] == 0.f ? end_s[i] : s_s[i];
+}
+
 template <int COLS>
 __global__ void __launch_bounds__(DT_THREADS, 1)
 delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, float* __restrict__ state,
@@ -511,6 +567,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
   const int chunks = (n + DC_TOKENS - 1) / DC_TOKENS;
   const size_t record = (size_t)(kDcU + DC_TOKENS * vdim);
   const float* base = records + ((size_t)(first / DC_TOKENS + r) * heads + h) * record;
+  bool wild;                                             // a result of the pieces is no finite number
 
   if (warp < 8) {
     float* mine = state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0 + g) * DC_DIM + warp * 16 + 2 * c;
@@ -622,15 +679,30 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
 #pragma unroll
           for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(i & 1 ? decay[j].y : decay[j].x, s[e][j][i], more[e][j][i]);
     }
+    float zero = 0.f;                                    // a NaN where one of them is no finite number, which then stays so
+#pragma unroll
+    for (int e = 0; e < kHalves; ++e)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) zero = fmaf(s[e][j][i], 0.f, zero);
+    wild = __syncthreads_or(!(zero == 0.f));
 #pragma unroll
     for (int e = 0; e < kHalves; ++e)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int i = 0; i < 4; i += 2)
-          *reinterpret_cast<float2*>(mine + (e * 16 + i * 4) * DC_DIM + j * 8) = *reinterpret_cast<const float2*>(&s[e][j][i]);
+          if (wild) {
+            float* to = dt_raw + (DC_DIM + warp * 16 + 2 * c + 8 * j) * COLS + e * 16 + i * 4 + g;
+            to[0] = s[e][j][i];
+            to[COLS] = s[e][j][i + 1];
+          } else {
+            *reinterpret_cast<float2*>(mine + (e * 16 + i * 4) * DC_DIM + j * 8) = *reinterpret_cast<const float2*>(&s[e][j][i]);
+          }
   } else {
     const int id = threadIdx.x - 256;
+    float zero = 0.f;                                    // as above, of the outputs
     auto fetch = [&](int chunk) {                        // M, G_31 and U0
       if (chunk < chunks) {
         const float* src = base + (size_t)chunk * heads * record;
@@ -671,7 +743,10 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
       if (token < n) {
         float* to = o_out + ((size_t)(first + token) * heads + h) * vdim + col0 + col;
 #pragma unroll
-        for (int i = 0; i < COLS / 4; ++i) to[4 * i] = sum[i];
+        for (int i = 0; i < COLS / 4; ++i) {
+          to[4 * i] = sum[i];
+          zero = fmaf(sum[i], 0.f, zero);
+        }
       }
     };
     fetch(0);
@@ -684,7 +759,12 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
       __syncthreads();
     }
     outputs(chunks - 1);
+    wild = __syncthreads_or(!(zero == 0.f));
   }
+  if (wild)
+    dt_scan_plain<COLS>(dt_raw, base, heads * record, n, vdim, col0,
+                        state + (size_t)state_slot[r] * state_stride + ((size_t)h * vdim + col0) * DC_DIM,
+                        o_out + ((size_t)first * heads + h) * vdim + col0, (size_t)heads * vdim);
 }
 
 // ---- launchers ---------------------------------------------------------------------------------------------------

@@ -2,7 +2,8 @@
 // them exactly (8 + 8 + 8 bits and signs), and the six products of pieces that reach 2^-24 of the whole are added up in
 // 32-bit, the smallest first.  The tensor core cuts a sum's low bits off instead of rounding: leave it a few dozen terms and
 // add its sums to others in plain 32-bit.  A number that is an infinity, a NaN or rounds to an infinity in 16 bits has a NaN
-// among its pieces: what it takes part in comes out as a NaN.
+// among its pieces, and a product just below the largest number may lie above it in its first pieces: what comes of them is no
+// finite number, and whoever uses this computes it anew from the numbers themselves.
 #pragma once
 #include "common.cuh"
 

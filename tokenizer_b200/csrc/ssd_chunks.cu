@@ -155,6 +155,42 @@ constexpr int kSsX = 4 * 3 * 512, kSsM = kSsX + SC_TOKENS * SC_COLS * 4, kSsG = 
 constexpr int kSsPart = 3 * kSsStage, kSsRing = kSsPart + 2 * 8 * SC_TOKENS * SC_COLS * 4 /* two chunks' pieces */,
               kSsBytes = kSsRing + 2 * kScPieces * 4;
 
+// The same portion in plain multiply-adds, all threads of the block, for numbers that have no pieces (an infinity in the matrix,
+// in B, C or x, numbers that round to one in 16 bits, and what then comes of them): slow, and replaces nothing but what the pieces
+// left as no finite number.  `mine`: the block's columns of the matrix in memory, as they were before the portion; end_s: as the
+// pieces left them ([128][32], as s_s); what lies behind the portion's last token, or behind a row's own, takes no part.
+__device__ __noinline__ void sc_scan_plain(float* s_s, const float* end_s, const float* __restrict__ x_in, const float* __restrict__ b_in,
+                                           const float* __restrict__ c_in, int channels, const float* __restrict__ rec, size_t place,
+                                           float d, int n, int N, float* __restrict__ mine, float* __restrict__ y_out, size_t y_ld) {
+  for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS) s_s[i] = mine[(size_t)(i % SC_COLS) * N + i / SC_COLS];
+  __syncthreads();
+  for (int t0 = 0; t0 < n; t0 += SC_TOKENS, rec += place) {
+    const int here = min(SC_TOKENS, n - t0);
+    const float* x = x_in + (size_t)t0 * channels;
+    for (int i = threadIdx.x; i < here * SC_COLS; i += SC_SCAN_THREADS) {
+      const int t = i / SC_COLS, c = i % SC_COLS;
+      float* to = y_out + (size_t)(t0 + t) * y_ld + c;
+      if (*to - *to == 0.f) continue;
+      float sum = 0.f, acc = 0.f;
+      for (int l = 0; l < N; ++l) sum = fmaf(c_in[(size_t)(t0 + t) * channels + l], s_s[l * SC_COLS + c], sum);
+      for (int s = 0; s <= t; ++s) acc = fmaf(rec[t * SC_TOKENS + s], x[(size_t)s * channels + c], acc);
+      acc = fmaf(d, x[(size_t)t * channels + c], acc);
+      *to = fmaf(rec[kScG + t], sum, acc);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS) {
+      const int l = i / SC_COLS, c = i % SC_COLS;
+      float v = rec[kScG + SC_TOKENS - 1] * s_s[i];
+      for (int s = 0; s < here; ++s)
+        v = fmaf(b_in[(size_t)(t0 + s) * channels + l], rec[kScR + s] * x[(size_t)s * channels + c], v);
+      s_s[i] = v;
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS)
+    mine[(size_t)(i % SC_COLS) * N + i / SC_COLS] = end_s[i] - end_s[i] == 0.f ? end_s[i] : s_s[i];
+}
+
 __global__ void __launch_bounds__(SC_SCAN_THREADS, 1)
 ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* __restrict__ records,
                       const float* __restrict__ skip, int heads, int groups, int P, int N, float* __restrict__ state,
@@ -172,6 +208,9 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
   const int chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
   const size_t place = sc_place(heads, groups);
   const float* here = records + (size_t)(first / SC_TOKENS + r) * place;
+  const float* base = here + (size_t)groups * kScPieces + (size_t)h * kScRecord;
+  bool wild;                                             // a result of the pieces is no finite number
+  float* end_s = reinterpret_cast<float*>(ss_raw) + SC_DIM * SC_COLS;      // then the matrix as the pieces left it
 
   if (warp < 8) {
     // ---- channels 16 w .. + 15 of the columns of S, transposed, as results and second operands of products lie ----
@@ -264,17 +303,30 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
           for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(all, s[e][j][i], more[e][j][i]);
       __syncthreads();                                   // the partial sums and the next stage are in place
     }
+    float zero = 0.f;                                    // a NaN where one of them is no finite number, which then stays so
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) zero = fmaf(s[e][j][i], 0.f, zero);
+    wild = __syncthreads_or(!(zero == 0.f));
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int i = 0; i < 4; i += 2)
-          if (channel + 8 * j < N)
+          if (wild) {
+            float* to = end_s + (channel + 8 * j) * SC_COLS + e * 16 + i * 4 + g;
+            to[0] = s[e][j][i];
+            to[SC_COLS] = s[e][j][i + 1];
+          } else if (channel + 8 * j < N) {
             *reinterpret_cast<float2*>(mine + (size_t)(e * 16 + i * 4) * N + j * 8) = *reinterpret_cast<const float2*>(&s[e][j][i]);
+          }
   } else {
     const int w = warp - 8, id = threadIdx.x - 256;
-    const float* base = here + (size_t)groups * kScPieces + (size_t)h * kScRecord;
+    float zero = 0.f;                                    // as above, of the outputs
     const float* x_in = xbc + (size_t)h * P + col0;
     const float d = skip[h];
     const int t = id >> 3, c4 = (id & 7) * 4;            // of x, M and the outputs: rows t and t + 16, four columns
@@ -344,7 +396,10 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
         const int row = t + 16 * e, token = chunk * SC_TOKENS + row;
         sc_add(acc[e], d, x_s[row * 8]);
         sc_add(acc[e], *reinterpret_cast<const float*>(stage + kSsG + row * 4), sum[e]);
-        if (token < n) *reinterpret_cast<float4*>(y_out + ((size_t)(first + token) * heads + h) * P + col0 + c4) = acc[e];
+        if (token < n) {
+          *reinterpret_cast<float4*>(y_out + ((size_t)(first + token) * heads + h) * P + col0 + c4) = acc[e];
+          zero = fmaf(acc[e].x, 0.f, fmaf(acc[e].y, 0.f, fmaf(acc[e].z, 0.f, fmaf(acc[e].w, 0.f, zero))));
+        }
       }
     };
     load(0);
@@ -362,6 +417,14 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
       __syncthreads();
     }
     outputs(chunks - 1);
+    wild = __syncthreads_or(!(zero == 0.f));
+  }
+  if (wild) {
+    const float* x_in = xbc + (size_t)first * channels;
+    const float* b_in = x_in + (size_t)heads * P + (size_t)(h / (heads / groups)) * N;
+    sc_scan_plain(reinterpret_cast<float*>(ss_raw), end_s, x_in + (size_t)h * P + col0, b_in, b_in + (size_t)groups * N, channels, base, place,
+                  skip[h], n, N, state + (size_t)state_slot[r] * state_stride + ((size_t)h * P + col0) * N,
+                  y_out + ((size_t)first * heads + h) * P + col0, (size_t)heads * P);
   }
 }
 
