@@ -3,6 +3,10 @@ ask for are ones the kernels accept (no empty piece, whole 64-element blocks), a
 within the bounds their comments state.  Pure arithmetic: runs without a GPU."""
 import itertools
 
+import pytest
+
+torch = pytest.importorskip("torch")
+
 from tokenizer_b200.parts import gemm_bf16 as rules
 
 ROWS = [1, 7, 16, 17, 33, 64, 100, 128, 129, 256, 300, 512, 777, 1024, 1536, 2048, 3000, 4096, 9000]
@@ -61,3 +65,12 @@ def test_the_sizes_the_rules_were_measured_at():
     assert rules.use_pair(4096, 896, 4864) and not rules.use_pair_halves(4096, 896, 4864)
     assert not rules.use_pair(1, 22528, 2048) and not rules.use_pair(128, 22528, 2048) and rules.use_pair(256, 22528, 2048)
     assert not rules.use_pair(2048, 896, 896) and not rules.use_pair_halves(2048, 1152, 896)
+
+
+def test_what_is_no_integer_is_refused():
+    """A float or a text that reaches a launcher as a size is an error, never another size."""
+    from tokenizer_b200.kernels import ops
+    for bad in (3.7, 4.0, "12", None):
+        with pytest.raises(TypeError):
+            ops._i(bad)
+    assert [ops._i(v) for v in (3, True, -1)] == [3, 1, -1]

@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import operator
 import os
 from typing import Optional
 
@@ -90,9 +91,9 @@ class bound_stream:
         return False
 
 
-# a Python integer is passed as a C int as it is (a c_int object each would cost a tenth of a microsecond, a layer passes
-# more than a hundred)
-_i, _f, _ll = int, ctypes.c_float, ctypes.c_longlong
+# an integer is passed as a C int as it is (a c_int object each would cost a tenth of a microsecond, a layer passes more than a
+# hundred); what is none, a float or a text, is a TypeError as it is for c_int
+_i, _f, _ll = operator.index, ctypes.c_float, ctypes.c_longlong
 
 
 class ScratchSpace:
