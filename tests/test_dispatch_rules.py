@@ -67,6 +67,38 @@ def test_the_sizes_the_rules_were_measured_at():
     assert not rules.use_pair(2048, 896, 896) and not rules.use_pair_halves(2048, 1152, 896)
 
 
+class Launches:
+    """Stands for the libraries: notes the launchers that are called, answers every one of them with success."""
+
+    def __init__(self, monkeypatch):
+        from tokenizer_b200.kernels import ops
+        self.names = []
+        monkeypatch.setattr(ops, "_lib", lambda name: self)
+        monkeypatch.setattr(ops, "_ptr", lambda t: None)
+        monkeypatch.setattr(ops, "_stream", lambda: None)
+        monkeypatch.setattr(ops, "linear_ring_supported", lambda M, N, K, k_splits=1, gated=False: M <= ops.RING_MAX_ROWS)
+
+    def __getattr__(self, name):
+        return lambda *args: self.names.append(name.replace("tokb200_", "")) or 0
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("on", [True, False])
+def test_large_weights_of_few_rows(monkeypatch, M, on):
+    """On rings up to 8 rows and on the tensor cores from 9 on; with the switch off on the kernel of small weights throughout."""
+    from tokenizer_b200.kernels import ops
+    launches = Launches(monkeypatch)
+    monkeypatch.setattr(ops, "_RING", on)
+    empty = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="meta")
+    ops.gated_linear(empty(M, 1536), empty(17920, 1536), empty(M, 8960))
+    rules.linear_bf16(empty(M, 13312), empty(1024, 13312), None, torch.bfloat16, partials_ok=True)
+    rules.linear_bf16(empty(M, 3584), empty(4608, 3584), torch.empty(4608, device="meta"), torch.bfloat16)
+    want = ["linear_small_m_gated", "linear_small_m", "linear_small_m"] if not on else \
+        ["linear_ring_gated", "linear_ring", "linear_ring"] if M <= 8 else \
+        ["gemm_tcgen05_gated", "gemm_tcgen05_partials", "linear_ring"]
+    assert launches.names == want
+
+
 def test_what_is_no_integer_is_refused():
     """A float or a text that reaches a launcher as a size is an error, never another size."""
     from tokenizer_b200.kernels import ops

@@ -762,7 +762,7 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
         raise ValueError("gated_linear is the bfloat16 kernel")
     if not gated_linear_supported(K, N) or w.shape[1] != K or tuple(out.shape) != (M, N // 2):
         raise ValueError("gated_linear: K a multiple of 8, N of 256, out [M, N/2]")
-    if M <= SMALL_M_ROWS and N * K >= RING_ELEMENTS and M > RING_ROWS:
+    if _RING and RING_ROWS < M <= SMALL_M_ROWS and N * K >= RING_ELEMENTS:
         # a large weight and nine rows or more (us at 16 rows, this / the ring kernel: 17,920 x 1,536 11.3 / 13.6, 37,888 x 3,584
         # 44 / 50; at 8 11.1 / 11.6 and 43.7 / 43.6)
         _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_gated(
@@ -1032,7 +1032,8 @@ def layer_small_m_check(d: int) -> None:
 RING_ELEMENTS = 13_000_000     # from this many weight elements on (26 MB) the ring kernel leads the one with plain loads
 RING_MAX_ROWS = 32
 RING_ROWS = 8                   # rows up to which the ring kernel is at least level with the tensor cores on such a weight
-_RING = os.environ.get("TOKB200_RING", "1") != "0"     # TOKB200_RING=0: large weights on linear_small_m too
+# TOKB200_RING=0: large weights of few rows on linear_small_m like small ones, neither on rings nor (9 to 16 rows) on the tensor cores
+_RING = os.environ.get("TOKB200_RING", "1") != "0"
 _ring_plans = {}
 
 

@@ -136,7 +136,7 @@ def linear_bf16(a: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         ops.gemm_tcgen05_pair(a, weight, None, out, ops.PAIR_PARTIALS)
         return out
     tiles_cut = 1
-    tensor_rows = ops.RING_ROWS if N * K >= ops.RING_ELEMENTS else ops.SMALL_M_ROWS
+    tensor_rows = ops.RING_ROWS if ops._RING and N * K >= ops.RING_ELEMENTS else ops.SMALL_M_ROWS
     if partials_ok and bias is None and M > tensor_rows and use_tcgen05(M, N, K, cut_along_k=True):
         tiles_cut = choose_tile_k_splits(M, N, K)
     if tiles_cut > 1:
