@@ -82,7 +82,7 @@ __global__ void qkv_rotate_store_kernel(const TI* __restrict__ proj, int ld, int
                                         int half_layout, int head_norm, float head_eps, int quads, float magnitude, int v_col) {
   // shared memory: a token's cosines and sines, one pair a frequency (every head turns by the same
   // angles), then the heads' inverse root mean squares (with `head_norm`)
-  extern __shared__ float shared[];
+  extern __shared__ __align__(16) float shared[];
   __shared__ float scratch[33];
   const int half = rot_dims >> 1;
   float* cosine = shared;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256) qkv_rotate_store8_kernel(
     const double* __restrict__ inv_freq64, int rot_dims, const int* __restrict__ pos, const int* __restrict__ slot,
     const int* __restrict__ row_req, T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool, int n_rows, int heads,
     int kv_heads, int dim, const float* __restrict__ temp, int half_layout, float magnitude, int v_col) {
-  extern __shared__ float shared[];                      // cosines of the tokens' frequencies, then their sines
+  extern __shared__ __align__(16) float shared[];                      // cosines of the tokens' frequencies, then their sines
   __shared__ int where_s[RS_TOKENS];                     // a token's cache slot, -1: none; -2: an idle row
   const int half = rot_dims >> 1, t0 = blockIdx.x * RS_TOKENS;
   float *cosine = shared, *sine = shared + RS_TOKENS * half;
