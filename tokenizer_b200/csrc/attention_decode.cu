@@ -28,6 +28,7 @@
 //
 // HEAD_DIM is a compile-time size (a multiple of 16, at most 256), given with
 // -DHEAD_DIM=...; the library is built per head size at first use.
+#include <atomic>
 #include "common.cuh"
 
 #ifndef HEAD_DIM
@@ -501,10 +502,16 @@ TOKB200_API long long tokb200_decode_attention_scratch_floats(int n_rows, int nh
 
 TOKB200_API int tokb200_decode_attention_head_dim() { return HEAD_DIM; }
 
-// Clusters of `size` blocks that the device holds at once (asked once a size; all that fit by count where it cannot be asked).
-static long long clusters_at_once(int size, size_t smem) {
-  static long long known[DEC_CLUSTER_MAX + 1] = {};
-  if (!known[size]) {
+// Clusters of `size` blocks of this kernel that the current device holds at once (all that fit by count where it cannot be
+// asked).  `which` numbers the kernels; an answer is kept by device, kernel and size with the shared memory that it is for, which
+// follows the head group.
+template <typename K>
+static long long clusters_at_once(K* kernel, int which, int size, size_t smem) {
+  static std::atomic<unsigned long long> known[64][4][DEC_CLUSTER_MAX + 1];      // shared memory << 32 | clusters
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1 << 30;
+  unsigned long long kept = known[device][which][size].load(std::memory_order_relaxed);
+  if (!kept || kept >> 32 != smem) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(size, 1, 1);
     config.blockDim = dim3(DEC_THREADS);
@@ -515,16 +522,16 @@ static long long clusters_at_once(int size, size_t smem) {
     attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
     config.attrs = attribute;
     config.numAttrs = 1;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(decode_attention_kernel<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, decode_attention_kernel<true, true, false>, &config) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &config) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = 1 << 30;
     }
-    known[size] = n;
+    kept = (unsigned long long)smem << 32 | (unsigned)n;
+    known[device][which][size].store(kept, std::memory_order_relaxed);
   }
-  return known[size];
+  return (long long)(kept & 0xffffffffu);
 }
 
 // `counters` holds n_rows * nkv ints, zero before the first launch; every launch
@@ -610,19 +617,20 @@ TOKB200_API int tokb200_decode_attention(
   // ... which clusters are only as far as they fit the device's groups of multiprocessors: 16 clusters of 8 blocks are 128
   // blocks, and 148 multiprocessors do not hold them (4 rows of 2,000 keys, 4 kv heads of size 128: 15.4 us in two waves of
   // clusters, 9.8 through scratch memory)
-  const bool cluster = clusters_allowed && most <= DEC_CLUSTER_MAX && pairs * most <= slots &&
-                       (most == 1 || pairs <= clusters_at_once((int)most, smem));
   // pieces of up to two passes: the first tiles before the wait (see EARLY)
   const bool early = min_chunk <= 2 * DEC_BLOCK_KEYS;
   // one pool read as keys and as values, while a warp has two staging buffers (see ALIAS)
   const bool alias = k_pool == v_pool && kVBuffers == 2;
+  const auto in_clusters = alias ? (early ? decode_attention_kernel<true, true, true> : decode_attention_kernel<true, false, true>)
+                                 : (early ? decode_attention_kernel<true, true, false> : decode_attention_kernel<true, false, false>);
+  const bool cluster = clusters_allowed && most <= DEC_CLUSTER_MAX && pairs * most <= slots &&
+                       (most == 1 || pairs <= clusters_at_once(in_clusters, 2 * alias + early, (int)most, smem));
   void (*kernel)(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*, __nv_bfloat16*, const int*,
                  int, const int*, const int*, int, int, int, int, int, int, float, float*, int*, int, const int*,
                  const float*, float) =
-      alias ? (early ? (cluster ? decode_attention_kernel<true, true, true> : decode_attention_kernel<false, true, true>)
-                     : (cluster ? decode_attention_kernel<true, false, true> : decode_attention_kernel<false, false, true>))
-            : (early ? (cluster ? decode_attention_kernel<true, true, false> : decode_attention_kernel<false, true, false>)
-                     : (cluster ? decode_attention_kernel<true, false, false> : decode_attention_kernel<false, false, false>));
+      cluster ? in_clusters
+              : alias ? (early ? decode_attention_kernel<false, true, true> : decode_attention_kernel<false, false, true>)
+                      : (early ? decode_attention_kernel<false, true, false> : decode_attention_kernel<false, false, false>);
   if (smem > 48 * 1024) {   // the larger shared memory is granted per device, once
     static bool configured[64][8] = {};
     int device = 0;
