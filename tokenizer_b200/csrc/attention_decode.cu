@@ -13,8 +13,9 @@
 //
 // A row's visible keys lo..pos are cut into n_splits pieces of `chunk` keys; chunk is
 // min_chunk * 2^k, the smallest that needs at most MAX_SPLITS pieces.  The launcher picks
-// min_chunk (256 .. 4,096, to 8,704 where the pairs alone fill the device) for the launch as a whole from the number of (row, kv head) pairs
-// and the table's reach: with few pairs, short pieces on many blocks win (a block's time is
+// min_chunk (256 .. 4,096) for the launch as a whole from the number of (row, kv head) pairs
+// and the table's reach, and where the pairs alone fill the device a long one beside it (to 8,704), which is
+// taken when the rows are of like length (see the launcher): with few pairs, short pieces on many blocks win (a block's time is
 // a chain of dependent loads per pass); with many pairs, long pieces win (fewer blocks than
 // the device holds at once cost no second wave, and fewer pieces cost less merging).  The
 // cut thus changes with the batch, which changes the order of the 32-bit merge, nothing else.  The eight warps of a block take tiles of 32 keys in turn, each with its
@@ -41,6 +42,7 @@
 #define DEC_TILE 32            // keys a warp takes per pass
 #define DEC_BLOCK_KEYS (DEC_WARPS * DEC_TILE)   // keys a block takes per pass
 #define DEC_MIN_CHUNK 256      // one pass of a block's warps: the shortest piece a launch may choose
+#define DEC_MOST_CHUNK 4096    // the longest, but for long pieces of rows of like length
 
 static_assert(HEAD_DIM % 16 == 0 && HEAD_DIM >= 16 && HEAD_DIM <= 256, "head size");
 constexpr int kSteps32 = HEAD_DIM / 32;              // steps of 32 lanes: one 16-byte load, two mma
@@ -119,8 +121,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
                         const int* __restrict__ block_table, int table_stride,
                         const int* __restrict__ row_req, const int* __restrict__ pos, int nh,
                         int nkv, int page, int window, int key_chunk, int keep_first, float scale,
-                        float* __restrict__ scratch, int* __restrict__ counters, int min_chunk,
-                        const int* __restrict__ rows, const float* __restrict__ sink, float softcap) {
+                        float* __restrict__ scratch, int* __restrict__ counters, int min_chunk, int long_chunk, int long_pieces,
+                        const int* __restrict__ even, const int* __restrict__ rows, const float* __restrict__ sink, float softcap) {
   extern __shared__ __align__(16) unsigned char dec_smem[];
   __shared__ int is_last;
   // The rows' requests, positions and block tables were written before the predecessor (the
@@ -128,10 +130,24 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
   // runs; q, keys and values only after the wait.
   // `rows` (optional): the batch rows this launch serves, one per z (-1: none); scratch and
   // counters are indexed by z, q, out, positions and requests by the row
-  const int split = blockIdx.x, kvh = blockIdx.y, z = blockIdx.z;
-  const int row = rows ? rows[z] : z;
-  const int r = row < 0 ? -1 : row_req[row];
-  const int p = r < 0 ? 0 : pos[row];
+  int split = blockIdx.x, kvh = blockIdx.y, z = blockIdx.z;
+  auto request_of = [&](int row) { return row < 0 ? -1 : row_req[row]; };
+  auto position_of = [&](int row) { return row < 0 ? 0 : pos[row]; };
+  int row = rows ? rows[z] : z, r = request_of(row), p = position_of(row);
+  if (HEAD_DIM == 128 && !CLUSTER && long_chunk > 0 && *even) {
+    // the grid is made for the short pieces: of the long ones the blocks with work come first, the others find none
+    const long long block = blockIdx.x + (long long)gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const long long pair = block / long_pieces;
+    const bool on = pair < (long long)gridDim.y * gridDim.z;
+    split = (int)(block % long_pieces);
+    kvh = on ? (int)(pair % gridDim.y) : 0;
+    z = on ? (int)(pair / gridDim.y) : 0;
+    row = !on ? -1 : rows ? rows[z] : z;
+    r = request_of(row);
+    p = position_of(row);
+    min_chunk = long_chunk;
+  }
+  if (r < 0) p = 0;
   const int lo = first_key_with_kept(first_visible_key(p, window, key_chunk), keep_first);
   const int kept = kept_first_keys(lo, keep_first);
   const int n_keys = p - lo + 1 + kept;
@@ -536,12 +552,12 @@ static long long clusters_at_once(K* kernel, int which, int size, size_t smem) {
 
 // `counters` holds n_rows * nkv ints, zero before the first launch; every launch
 // leaves them zero again.  `rows` (optional, n_rows ints): the batch rows to serve, -1 for none;
-// without it the launch serves rows 0 .. n_rows - 1.
+// without it the launch serves rows 0 .. n_rows - 1.  `even` (optional, one int): whether the rows are of like length.
 TOKB200_API int tokb200_decode_attention(
     const void* q, const void* k_pool, const void* v_pool, void* out, const int* block_table,
     int table_stride, const int* row_req, const int* pos, int n_rows, int nh, int nkv, int d,
     int page, int window, int key_chunk, int keep_first, float scale, float* scratch, int* counters, const int* rows,
-    const float* sink, float softcap, cudaStream_t stream) {
+    const int* even, const float* sink, float softcap, cudaStream_t stream) {
   if (n_rows <= 0) return TOKB200_OK;
   if (d != HEAD_DIM || nh <= 0 || nkv <= 0 || nh % nkv || nh / nkv > DEC_MAX_GROUP || page <= 0 || keep_first < 0 ||
       nkv > 65535 || n_rows > 65535)
@@ -566,7 +582,7 @@ TOKB200_API int tokb200_decode_attention(
   // (768 blocks, 5.2 waves of 148) against 266 us in pieces of 2,048 (1,024 blocks, 6.9 waves).
   static int slots = 0;      // blocks the device holds at once
   const long long pairs = (long long)n_rows * nkv;
-  int min_chunk = DEC_MIN_CHUNK;
+  int min_chunk = DEC_MIN_CHUNK, long_chunk = 0;
   {
     int& have = slots;
     if (!have) {
@@ -581,21 +597,29 @@ TOKB200_API int tokb200_decode_attention(
     }
     const double per_pass = 2.0 * HEAD_DIM / 64.0;
     double best = 1e30;
-    // Where the (row, kv head) pairs alone fill the device, a row may also stay whole beyond 4,096 keys: no piece starts, none
-    // is merged (64 rows over 8,192 keys, 4 kv heads of size 128, us at the best piece of up to 4,096 keys / whole: rows of one
-    // length 210 / 183, from 8,192 down to 2,048 148 / 115, these shuffled 145 / 143; with 2 kv heads, 128 pairs, 73 / 87).
-    // Up to some 8,192: a lone long row among short ones is then one block's chain of 34 passes at most (tables reach a page
-    // or two further than the rows they were made for).
-    const int longest = pairs >= have ? 8192 + 512 : 4096;
-    for (int c = DEC_MIN_CHUNK; c <= longest; c += DEC_BLOCK_KEYS) {
-      int chunk = c;
-      while ((reach + chunk - 1) / chunk > DEC_MAX_SPLITS) chunk <<= 1;
-      const long long pieces = (reach + chunk - 1) / chunk;
-      const long long passes = ((reach < chunk ? reach : chunk) + DEC_BLOCK_KEYS - 1) / DEC_BLOCK_KEYS;
-      const long long waves = (pairs * pieces + have - 1) / have;
-      const double t = (double)waves * (3.0 + per_pass * (double)passes + (pieces > 1 ? 3.0 : 0.0));
-      if (t < best - 1e-9) { best = t; min_chunk = c; }
-    }
+    auto consider = [&](int from, int to, int& chosen) {
+      for (int c = from; c <= to; c += DEC_BLOCK_KEYS) {
+        int chunk = c;
+        while ((reach + chunk - 1) / chunk > DEC_MAX_SPLITS) chunk <<= 1;
+        const long long pieces = (reach + chunk - 1) / chunk;
+        const long long passes = ((reach < chunk ? reach : chunk) + DEC_BLOCK_KEYS - 1) / DEC_BLOCK_KEYS;
+        const long long waves = (pairs * pieces + have - 1) / have;
+        const double t = (double)waves * (3.0 + per_pass * (double)passes + (pieces > 1 ? 3.0 : 0.0));
+        if (t < best - 1e-9) { best = t; chosen = c; }
+      }
+    };
+    consider(DEC_MIN_CHUNK, DEC_MOST_CHUNK, min_chunk);
+    // Where the (row, kv head) pairs alone fill the device, a row may also stay whole beyond 4,096 keys (or be cut into longer
+    // pieces): no piece starts, none is merged.  That pays while the rows are of like length, which the caller says with `even`
+    // (a word on the device, so that a captured launch can follow it; nullptr: never), and longest first; a lone long row among
+    // short ones would be one block's chain of 32 passes.
+    // us, pieces of up to 4,096 keys / whole rows whatever their lengths / this: 64 rows, 4 kv heads of size 128, 8,192 keys
+    // each 205 / 182 / 182, from 8,192 down to 2,048 in that order 142 / 112 / 113, these shuffled 142 / 144 / 113, one of 8,192
+    // among rows of 512 27 to 42 / 69 to 78 / 27; 8 kv heads, shuffled 253 / 243 / 235, one among rows of 512 46 to 68 / 49 to 79
+    // / 46; 100 rows of 2 kv heads, 4,096 to 8,192 keys 132 / 130 / 130, to 12,000 176 / 184 / 182 (the worst of some hundred
+    // sets).  Heads of size 64 and 256 gained from no order but a falling one (64 rows, 8 kv heads of 64, shuffled 132 / 136; 4 of
+    // 256 459 / 531) and keep short pieces.
+    if (HEAD_DIM == 128 && even && pairs >= have) consider(DEC_MOST_CHUNK + DEC_BLOCK_KEYS, 8192 + 512, long_chunk);
   }
   // no row has more pieces than this (a row a little shorter than the reach may be cut finer
   // than the reach itself would be: its pieces are counted from min_chunk, not from the
@@ -603,6 +627,7 @@ TOKB200_API int tokb200_decode_attention(
   long long most = (reach + min_chunk - 1) / min_chunk;
   if (most > DEC_MAX_SPLITS) most = DEC_MAX_SPLITS;
   if (most < 1) most = 1;
+  const int long_pieces = long_chunk ? (int)((reach + long_chunk - 1) / long_chunk < DEC_MAX_SPLITS ? (reach + long_chunk - 1) / long_chunk : DEC_MAX_SPLITS) : 1;
   // up to DEC_CLUSTER_MAX pieces: one cluster a (row, kv head), pieces merged through
   // distributed shared memory; more: scratch memory and the last block.  TOKB200_DECODE_MERGE
   // = scratch always takes the second way.
@@ -623,10 +648,10 @@ TOKB200_API int tokb200_decode_attention(
   const bool alias = k_pool == v_pool && kVBuffers == 2;
   const auto in_clusters = alias ? (early ? decode_attention_kernel<true, true, true> : decode_attention_kernel<true, false, true>)
                                  : (early ? decode_attention_kernel<true, true, false> : decode_attention_kernel<true, false, false>);
-  const bool cluster = clusters_allowed && most <= DEC_CLUSTER_MAX && pairs * most <= slots &&
+  const bool cluster = clusters_allowed && !long_chunk && most <= DEC_CLUSTER_MAX && pairs * most <= slots &&
                        (most == 1 || pairs <= clusters_at_once(in_clusters, 2 * alias + early, (int)most, smem));
   void (*kernel)(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*, __nv_bfloat16*, const int*,
-                 int, const int*, const int*, int, int, int, int, int, int, float, float*, int*, int, const int*,
+                 int, const int*, const int*, int, int, int, int, int, int, float, float*, int*, int, int, int, const int*, const int*,
                  const float*, float) =
       cluster ? in_clusters
               : alias ? (early ? decode_attention_kernel<false, true, true> : decode_attention_kernel<false, false, true>)
@@ -647,7 +672,7 @@ TOKB200_API int tokb200_decode_attention(
                             (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
                             (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, block_table,
                             table_stride, row_req, pos, nh, nkv, page, window, key_chunk, keep_first, scale, scratch,
-                            counters, min_chunk, rows, sink, softcap);
+                            counters, min_chunk, long_chunk, long_pieces, even, rows, sink, softcap);
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = dim3(DEC_THREADS);
@@ -669,6 +694,6 @@ TOKB200_API int tokb200_decode_attention(
   cudaError_t err = cudaLaunchKernelEx(&config, kernel, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool,
                                        (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, block_table,
                                        table_stride, row_req, pos, nh, nkv, page, window, key_chunk, keep_first, scale, scratch,
-                                       counters, min_chunk, rows, sink, softcap);
+                                       counters, min_chunk, long_chunk, long_pieces, even, rows, sink, softcap);
   return err == cudaSuccess ? TOKB200_OK : (int)err;
 }

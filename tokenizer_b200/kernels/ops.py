@@ -466,12 +466,14 @@ def decode_attention_supported(nh: int, nkv: int, d: int) -> bool:
 
 def decode_attention(q, k_pool, v_pool, out, block_table, row_req, pos, nh, nkv, d, page, window,
                      scale, rows: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
-                     chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0) -> None:
+                     chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0,
+                     even: Optional[torch.Tensor] = None) -> None:
     """Attention for rows of one token each (bfloat16): keys are split over
     blocks and merged; the scratch for the pieces is kept per (device, rows,
     heads, head size) and reused by every layer, which run one after another.  With `rows`
     (int32, -1 for none) only those rows of the batch are served: the single-token rows of a
-    step that also brings portions of prompts, which go to the kernels for portions."""
+    step that also brings portions of prompts, which go to the kernels for portions.  `even` (int32, one word on the
+    device): not zero while the rows are of like length, so that long ones may stay whole (None: never)."""
     if q.dtype != torch.bfloat16:
         raise ValueError("decode_attention is the bfloat16 kernel")
     if not decode_attention_supported(nh, nkv, d):
@@ -489,7 +491,7 @@ def decode_attention(q, k_pool, v_pool, out, block_table, row_req, pos, nh, nkv,
         _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
         _i(block_table.shape[1]), _ptr(row_req), _ptr(pos), _i(n_rows), _i(nh), _i(nkv), _i(d),
         _i(page), _i(-1 if window is None else int(window)), _i(0 if chunk is None else int(chunk)), _i(int(keep_first)), _f(scale), _ptr(scratch),
-        _ptr(counters), _ptr(rows), _sink(sink, nh), _f(softcap or 0.0), _stream()), "decode_attention")
+        _ptr(counters), _ptr(rows), _ptr(even), _sink(sink, nh), _f(softcap or 0.0), _stream()), "decode_attention")
 
 
 _stream_plans = {}

@@ -115,6 +115,28 @@ class SingleRows(BatchAnnotation):
         return (len(out) if made else 0) if padded else made
 
 
+class RowsByLength(BatchAnnotation):
+    """Of a step of single tokens: whether the rows are of like length (one word, 1 where their keys are on the average
+    `EVEN` of the longest row's or more), and behind three words of nothing the rows' indices, the longest row first, -1
+    where there is none: int32 [4 + requests]."""
+
+    key = "rows_by_length"
+    EVEN = 0.6
+
+    def capacity(self, n_tokens, n_requests):
+        return 4 + n_requests
+
+    def fill(self, out, first_rows, counts, starts, padded):
+        n = len(counts)
+        out[4:] = -1
+        if not n or int(counts.max()) > 1:
+            return 0
+        order = np.argsort(-starts, kind="stable")
+        out[4:4 + n] = first_rows[order]
+        out[0] = int(starts.sum()) + n >= self.EVEN * n * (int(starts[order[0]]) + 1)
+        return (len(out) - 4) if padded else n
+
+
 # the tiles of the two prompt kernels: 64 rows (mma.sync) and 128 rows (tcgen05), for all
 # requests and for those alone that bring more than one token
 _TILES = RowTiles(ops.PREFILL_TILE_ROWS)
@@ -122,6 +144,7 @@ _WIDE_TILES = RowTiles(ops.WIDE_TILE_ROWS)
 _LONG_TILES = RowTiles(ops.PREFILL_TILE_ROWS, long_only=True)
 _LONG_WIDE_TILES = RowTiles(ops.WIDE_TILE_ROWS, long_only=True)
 _SINGLES = SingleRows()
+_BY_LENGTH = RowsByLength()
 # TOKB200_MIXED=tiles sends the single-token rows of a mixed step through the kernels for portions
 _SPLIT_MIXED = os.environ.get("TOKB200_MIXED", "split") != "tiles"
 # portions from this length on go to the tcgen05 kernel (shorter ones would leave most of a
@@ -156,7 +179,7 @@ class PagedAttention:
     softcap = None      # c: a score s counts as c * tanh(s / c)
 
     def batch_annotations(self):
-        return [_TILES, _WIDE_TILES, _LONG_TILES, _LONG_WIDE_TILES, _SINGLES]
+        return [_TILES, _WIDE_TILES, _LONG_TILES, _LONG_WIDE_TILES, _SINGLES, _BY_LENGTH]
 
     def shape_key(self, q_lens):
         """Which attention kernel a step of these portion lengths gets (part of the key under
@@ -187,6 +210,16 @@ class PagedAttention:
             reach <= _NEAR and self.nh * ctx.n_tokens * min(reach, _WIDE_ALWAYS - 1) <= _NEAR_WORK and \
             ops.prefill_attention_supported(self.nh, self.nkv, self.d)
 
+    def _by_length(self, ctx, group):
+        """A decoding step's rows by length and the word that says whether they are alike, where the launch may leave long rows
+        whole: heads of 128 lanes, keys beyond 4,096 in reach, rows that fill the device (None, None elsewhere: the order
+        is a lookup more on the way to a row's first key).  By the step's shape alone, as a captured launch must."""
+        if self.d != 128 or self.nkv * ctx.n_tokens < gemm_bf16.sm_count() or \
+                group.block_table.shape[1] * group.page_size <= 4096:
+            return None, None
+        words, count = ctx.views.get(_BY_LENGTH.key, (None, 0))
+        return (words[4:4 + count], words[:1]) if count == ctx.n_tokens else (None, None)
+
     def attend(self, q, out, ctx, group, cache):
         """Choose the kernel by precision and by the shape of the batch.  A group that keeps one
         row a token (`cache.v_pool` None) is read as keys and as values: the values are then the
@@ -196,10 +229,11 @@ class PagedAttention:
         sink = self.sink
         if q.dtype == torch.bfloat16 and ctx.max_q_len == 1 and \
                 ops.decode_attention_supported(self.nh, self.nkv, self.d):
+            rows, even = self._by_length(ctx, group)
             ops.decode_attention(
                 q, k_pool, v_pool, out, group.block_table, ctx.row_req, ctx.pos,
-                self.nh, self.nkv, self.d, group.page_size, self.window, self.scale, sink=sink, chunk=self.chunk, softcap=self.softcap,
-                keep_first=self.keep_first)
+                self.nh, self.nkv, self.d, group.page_size, self.window, self.scale, rows=rows, sink=sink, chunk=self.chunk,
+                softcap=self.softcap, keep_first=self.keep_first, even=even)
             return
         wide, tiles = ctx.views.get(_WIDE_TILES.key), ctx.views.get(_TILES.key)
         singles = ctx.views.get(_SINGLES.key)
