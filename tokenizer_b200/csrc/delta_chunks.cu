@@ -499,43 +499,51 @@ __device__ __forceinline__ float dt_whole(const float* tile, int lane, int i) { 
 }
 // The same portion in plain multiply-adds, all threads of the block, for numbers that have no pieces (an infinity in the matrix
 // or in U, numbers that round to one in 16 bits, and what then comes of them): slow, and replaces nothing but what the pieces
-// left as no finite number.  `mine`: the block's columns of the matrix in memory, as they were before the portion; what lies
+// left as no finite number.  Inlined in small loops: a call, which is never made, cost the fast walk 2 to 4 %.  `mine`: the block's columns of the matrix in memory, as they were before the portion; what lies
 // behind the portion's last token, or behind a row's own, takes no part.  s_s: [128][COLS] floats, behind it the matrix as the
 // pieces left it, of that form, and U [32][COLS].
 template <int COLS>
-__device__ __noinline__ void dt_scan_plain(float* s_s, const float* __restrict__ rec, size_t record_ld, int n, int vdim, int col0,
+__device__ __forceinline__ void dt_scan_plain(float* s_s, const float* __restrict__ rec, size_t record_ld, int n, int vdim, int col0,
                                            float* __restrict__ mine, float* __restrict__ o_out, size_t o_ld) {
   const float* end_s = s_s + DC_DIM * COLS;
   float* u_s = s_s + 2 * DC_DIM * COLS;
+#pragma unroll 1
   for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS) s_s[i] = mine[(size_t)(i % COLS) * DC_DIM + i / COLS];
   __syncthreads();
+#pragma unroll 1
   for (int t0 = 0; t0 < n; t0 += DC_TOKENS, rec += record_ld) {
     const int here = min(DC_TOKENS, n - t0);
     auto product = [&](int row, int c) {                 // a row of W (0 .. 31) or G q (32 .. 63) times a column
       const int lane = (row & 7) * 4, high = row >> 3 & 1;
       float sum = 0.f;
+#pragma unroll 1
       for (int k = 0; k < DC_DIM; ++k)
         sum = fmaf(dt_whole(rec + (k / 16 * 4 + row / 16) * 384, lane + (k & 7) / 2, ((k >> 3 & 1) * 2 + high) * 2 + (k & 1)),
                    s_s[k * COLS + c], sum);
       return sum;
     };
+#pragma unroll 1
     for (int i = threadIdx.x; i < here * COLS; i += DT_THREADS) {
       const int t = i / COLS, c = i % COLS;
       u_s[i] = rec[kDcU + t * vdim + col0 + c] - product(t, c);
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = threadIdx.x; i < here * COLS; i += DT_THREADS) {
       const int t = i / COLS, c = i % COLS;
       float* to = o_out + (size_t)(t0 + t) * o_ld + c;
       if (*to - *to == 0.f) continue;
       float sum = product(DC_TOKENS + t, c);
+#pragma unroll 1
       for (int s = 0; s <= t; ++s) sum = fmaf(rec[kDcM + t * DC_TOKENS + s], u_s[s * COLS + c], sum);
       *to = sum;
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS) {
       const int k = i / COLS, c = i % COLS;
       float more = 0.f;
+#pragma unroll 1
       for (int t = 0; t < here; ++t)
         more = fmaf(dt_whole(rec + kDcK + (k / 16 * 2 + t / 16) * 384, (k & 7) * 4 + (t & 7) / 2,
                              ((k >> 3 & 1) * 2 + (t >> 3 & 1)) * 2 + (t & 1)), u_s[t * COLS + c], more);
@@ -543,6 +551,7 @@ __device__ __noinline__ void dt_scan_plain(float* s_s, const float* __restrict__
     }
     __syncthreads();
   }
+#pragma unroll 1
   for (int i = threadIdx.x; i < DC_DIM * COLS; i += DT_THREADS)
     mine[(size_t)(i % COLS) * DC_DIM + i / COLS] = end_s[i] - end_s[i] == 0.f ? end_s[i] : s_s[i];
 }

@@ -158,35 +158,44 @@ constexpr int kSsPart = 3 * kSsStage, kSsRing = kSsPart + 2 * 8 * SC_TOKENS * SC
 // The same portion in plain multiply-adds, all threads of the block, for numbers that have no pieces (an infinity in the matrix,
 // in B, C or x, numbers that round to one in 16 bits, and what then comes of them): slow, and replaces nothing but what the pieces
 // left as no finite number.  `mine`: the block's columns of the matrix in memory, as they were before the portion; end_s: as the
-// pieces left them ([128][32], as s_s); what lies behind the portion's last token, or behind a row's own, takes no part.
-__device__ __noinline__ void sc_scan_plain(float* s_s, const float* end_s, const float* __restrict__ x_in, const float* __restrict__ b_in,
+// pieces left them ([128][32], as s_s); what lies behind the portion's last token, or behind a row's own, takes no part.  Inlined
+// in small loops: a call, which is never made, cost the fast walk 2 to 4 %.
+__device__ __forceinline__ void sc_scan_plain(float* s_s, const float* end_s, const float* __restrict__ x_in, const float* __restrict__ b_in,
                                            const float* __restrict__ c_in, int channels, const float* __restrict__ rec, size_t place,
                                            float d, int n, int N, float* __restrict__ mine, float* __restrict__ y_out, size_t y_ld) {
+#pragma unroll 1
   for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS) s_s[i] = mine[(size_t)(i % SC_COLS) * N + i / SC_COLS];
   __syncthreads();
+#pragma unroll 1
   for (int t0 = 0; t0 < n; t0 += SC_TOKENS, rec += place) {
     const int here = min(SC_TOKENS, n - t0);
     const float* x = x_in + (size_t)t0 * channels;
+#pragma unroll 1
     for (int i = threadIdx.x; i < here * SC_COLS; i += SC_SCAN_THREADS) {
       const int t = i / SC_COLS, c = i % SC_COLS;
       float* to = y_out + (size_t)(t0 + t) * y_ld + c;
       if (*to - *to == 0.f) continue;
       float sum = 0.f, acc = 0.f;
+#pragma unroll 1
       for (int l = 0; l < N; ++l) sum = fmaf(c_in[(size_t)(t0 + t) * channels + l], s_s[l * SC_COLS + c], sum);
+#pragma unroll 1
       for (int s = 0; s <= t; ++s) acc = fmaf(rec[t * SC_TOKENS + s], x[(size_t)s * channels + c], acc);
       acc = fmaf(d, x[(size_t)t * channels + c], acc);
       *to = fmaf(rec[kScG + t], sum, acc);
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS) {
       const int l = i / SC_COLS, c = i % SC_COLS;
       float v = rec[kScG + SC_TOKENS - 1] * s_s[i];
+#pragma unroll 1
       for (int s = 0; s < here; ++s)
         v = fmaf(b_in[(size_t)(t0 + s) * channels + l], rec[kScR + s] * x[(size_t)s * channels + c], v);
       s_s[i] = v;
     }
     __syncthreads();
   }
+#pragma unroll 1
   for (int i = threadIdx.x; i < N * SC_COLS; i += SC_SCAN_THREADS)
     mine[(size_t)(i % SC_COLS) * N + i / SC_COLS] = end_s[i] - end_s[i] == 0.f ? end_s[i] : s_s[i];
 }
