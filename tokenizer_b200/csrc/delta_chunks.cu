@@ -627,14 +627,16 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 2; ++j) xm_cut(s[e][j][2 * i], s[e][j][2 * i + 1], b[i][0][j], b[i][1][j], b[i][2][j]);
-        float d[4][2][4] = {};
-        xm_products(d, a, b);
+        float d[4][2][4] = {}, low[4][2][4] = {};
+        xm_products(d, low, a, b);
 #pragma unroll
         for (int m = 0; m < 4; ++m)
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             // columns in eights change places where two rows of one bank would meet
             const int at = (warp * 64 + m * 16 + g) * 16 + ((i * 8) ^ ((g >> 1 & 1) * 8)) + 2 * c;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) d[m][i][j] += low[m][i][j];
             *reinterpret_cast<float2*>(part_s + at) = make_float2(d[m][i][0], d[m][i][1]);
             *reinterpret_cast<float2*>(part_s + at + 8 * 16) = make_float2(d[m][i][2], d[m][i][3]);
           }
@@ -660,7 +662,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
       float2 decay[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) decay[j] = *reinterpret_cast<const float2*>(stage + kDtG + warp * 16 + j * 8 + 2 * c);
-      float more[kHalves][2][4] = {};
+      float more[kHalves][2][4] = {}, low[kHalves][2][4] = {};
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         unsigned k[2][3][2];                             // keys of 16 tokens: [eight channels][piece]
@@ -678,7 +680,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
             const float2 v = *reinterpret_cast<const float2*>(u_s + (e * 16 + g + (i & 1) * 8) * DT_PITCH + t * 16 + 2 * c + (i >> 1) * 8);
             xm_cut(v.x, v.y, u[e][0][i], u[e][1][i], u[e][2][i]);
           }
-        xm_products(more, u, k);
+        xm_products(more, low, u, k);
       }
       fetch(chunk + 2);
 #pragma unroll
@@ -686,7 +688,7 @@ delta_chunk_scan_kernel(const float* __restrict__ records, int heads, int vdim, 
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(i & 1 ? decay[j].y : decay[j].x, s[e][j][i], more[e][j][i]);
+          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(i & 1 ? decay[j].y : decay[j].x, s[e][j][i], more[e][j][i] + low[e][j][i]);
     }
     float zero = 0.f;                                    // a NaN where one of them is no finite number, which then stays so
 #pragma unroll

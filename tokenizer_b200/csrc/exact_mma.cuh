@@ -24,15 +24,17 @@ __device__ __forceinline__ void xm_mma(float (&d)[4], const unsigned (&a)[4], un
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// d[m][n] += a[m] b[n] for operands in pieces ([piece][registers]).  The sums of one term are issued together: each waits for
-// its own sum of the term before, some 20 cycles.
+// large[m][n] + small[m][n] += a[m] b[n] for operands in pieces ([piece][registers]): the products of first pieces in a sum of
+// their own, so that what they cut off is their own low bits alone and not those of the five others' sum, which is added to them
+// in plain 32-bit.  The sums of one term are issued together: each waits for its own sum of the term before, some 20 cycles.
 template <int M, int N>
-__device__ __forceinline__ void xm_products(float (&d)[M][N][4], const unsigned (&a)[M][3][4], const unsigned (&b)[N][3][2]) {
-  constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+__device__ __forceinline__ void xm_products(float (&large)[M][N][4], float (&small)[M][N][4], const unsigned (&a)[M][3][4],
+                                            const unsigned (&b)[N][3][2]) {
+  constexpr int kA[6] = {2, 0, 0, 1, 1, 0}, kB[6] = {0, 2, 0, 1, 0, 1};
 #pragma unroll
   for (int e = 0; e < 6; ++e)
 #pragma unroll
     for (int m = 0; m < M; ++m)
 #pragma unroll
-      for (int n = 0; n < N; ++n) xm_mma(d[m][n], a[m][kA[e]], b[n][kB[e]][0], b[n][kB[e]][1]);
+      for (int n = 0; n < N; ++n) xm_mma(e == 2 ? large[m][n] : small[m][n], a[m][kA[e]], b[n][kB[e]][0], b[n][kB[e]][1]);
 }

@@ -273,21 +273,23 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
 #pragma unroll
         for (int j = 0; j < 2; ++j)
           xm_cut(s[e >> 1][j][2 * (e & 1)], s[e >> 1][j][2 * (e & 1) + 1], b[e][0][j], b[e][1][j], b[e][2][j]);
-      float d[2][4][4] = {};
-      xm_products(d, a, b);
+      float d[2][4][4] = {}, low[2][4][4] = {};
+      xm_products(d, low, a, b);
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           // columns in eights change places so that the rows of a store lie on different banks
           const int row = m * 16 + g, at = (warp * SC_TOKENS + row) * SC_COLS + ((e ^ (row & 3)) * 8) + 2 * c;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[m][e][i] += low[m][e][i];
           *reinterpret_cast<float2*>(part_s + at) = make_float2(d[m][e][0], d[m][e][1]);
           *reinterpret_cast<float2*>(part_s + at + 8 * SC_COLS) = make_float2(d[m][e][2], d[m][e][3]);
         }
       // the matrix moves on by the chunk
       const float all = *reinterpret_cast<const float*>(stage + kSsG + (SC_TOKENS - 1) * 4);
       const uint4* u_s = reinterpret_cast<const uint4*>(stage) + lane;
-      float more[2][2][4] = {};
+      float more[2][2][4] = {}, low_more[2][2][4] = {};
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         unsigned u[2][3][4], k[2][3][2];                 // B of 16 tokens: [eight channels][piece]
@@ -301,7 +303,7 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(u[e][p]) = u_s[((e * 2 + t) * 3 + p) * 32];
-        xm_products(more, u, k);
+        xm_products(more, low_more, u, k);
       }
       fetch(chunk + 2);
 #pragma unroll
@@ -309,7 +311,7 @@ ssd_chunk_scan_kernel(const float* __restrict__ xbc, int channels, const float* 
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(all, s[e][j][i], more[e][j][i]);
+          for (int i = 0; i < 4; ++i) s[e][j][i] = fmaf(all, s[e][j][i], more[e][j][i] + low_more[e][j][i]);
       __syncthreads();                                   // the partial sums and the next stage are in place
     }
     float zero = 0.f;                                    // a NaN where one of them is no finite number, which then stays so
