@@ -6,7 +6,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from tokenizer_b200.parts import attention, recurrent
+from tokenizer_b200.parts import attention, part_class, recurrent
 
 
 def delta(kind, heads, chunked=True):
@@ -26,14 +26,27 @@ def test_delta_rules(q_lens, by_head, by_channel):
             assert (delta(kind, 16).shape_key(q_lens) == "delta_chunks") is want
 
 
-@pytest.mark.parametrize("heads,q_lens,want", [
-    (64, [2048], True), (64, [1905, 1096], True), (64, [128], True), (64, [127], False), (128, [255], False), (128, [1024], True),
-    (32, [2048], False), (48, [1024], True), (64, [512] * 4, False), (64, [2048] + [1] * 15, False), (64, [400, 1, 1, 1], True),
-    (64, [1], False)])
-def test_state_space_rule(heads, q_lens, want):
-    part = delta(recurrent.Mamba2, heads)
-    part.vdim = 64
-    assert part._in_chunks(q_lens) is want and (part.shape_key(q_lens) == "ssm_chunks") is want
+@pytest.mark.parametrize("heads,groups,q_lens,want", [
+    (64, 8, [2048], True), (64, 8, [1905, 1096], True), (64, 8, [128], True), (64, 8, [127], False), (64, 8, [1], False),
+    (64, 8, [], False), (128, 8, [255], True), (128, 8, [128], True), (48, 1, [1024], True), (32, 1, [2048], True),
+    (24, 1, [2048], False), (16, 1, [2048], False), (16, 1, [1905, 1096], True), (16, 1, [128, 128], True),
+    (64, 8, [622, 357, 1021], True), (64, 8, [512] * 4, True), (64, 8, [1200] * 4, True), (64, 8, [128] * 16, True),
+    (64, 8, [64] * 16, False), (64, 8, [100] * 8, False), (64, 8, [2048] + [1] * 15, True), (64, 8, [1024, 600] + [1] * 20, True),
+    (64, 8, [400, 1, 1, 1], True), (64, 8, [128, 1, 1, 1], True), (64, 8, [300] + [1] * 31, False), (64, 8, [1024] + [1] * 63, False),
+    (64, 8, [256] * 4 + [1] * 60, False), (128, 8, [512] + [1] * 31, False), (64, 8, [130] * 16 + [2] * 16, False),
+    (32, 1, [140] * 16 + [2] * 10, False),
+    # B and C in pieces for every head or two: while the blocks fill one or two turns
+    (64, 64, [2048], True), (64, 64, [1905, 1096], True), (64, 64, [512] * 4, False), (64, 64, [128] * 8, False),
+    (64, 32, [128] * 4, False), (64, 16, [512] * 4, True), (32, 32, [128] * 3, False), (16, 16, [1905, 1096], False)])
+def test_state_space_rule(heads, groups, q_lens, want):
+    part = delta(part_class("mixer", "mamba2"), heads)
+    part.vdim, part.groups = 64, groups
+    assert part._in_chunks(q_lens) is want
+    part.chunked = False
+    assert not part._in_chunks(q_lens)
+    part.chunked = True
+    if q_lens:
+        assert (part.shape_key(q_lens) == "ssm_chunks") is want
 
 
 @pytest.mark.parametrize("longest,tokens,reach,d,want", [

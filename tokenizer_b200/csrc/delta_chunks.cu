@@ -499,9 +499,10 @@ __device__ __forceinline__ float dt_whole(const float* tile, int lane, int i) { 
 }
 // The same portion in plain multiply-adds, all threads of the block, for numbers that have no pieces (an infinity in the matrix
 // or in U, numbers that round to one in 16 bits, and what then comes of them): slow, and replaces nothing but what the pieces
-// left as no finite number.  Inlined in small loops: a call, which is never made, cost the fast walk 2 to 4 %.  `mine`: the block's columns of the matrix in memory, as they were before the portion; what lies
-// behind the portion's last token, or behind a row's own, takes no part.  s_s: [128][COLS] floats, behind it the matrix as the
-// pieces left it, of that form, and U [32][COLS].
+// left as no finite number.  Inlined in small loops: a call, which is never made, cost the fast walk 2
+// to 4 %.  `mine`: the block's columns of the matrix in memory, as they were before the portion; what lies behind the portion's
+// last token, or behind a row's own, takes no part.  s_s: [128][COLS] floats, behind it the matrix as the pieces left it, of that
+// form, and U [32][COLS].
 template <int COLS>
 __device__ __forceinline__ void dt_scan_plain(float* s_s, const float* __restrict__ rec, size_t record_ld, int n, int vdim, int col0,
                                            float* __restrict__ mine, float* __restrict__ o_out, size_t o_ld) {

@@ -468,145 +468,29 @@ class Mamba2:
         return CacheNeed(state=StateNeed((self.state_floats,)))
 
     def _in_chunks(self, q_lens) -> bool:
-        """Chunks of 32 tokens are cut over blocks of 32 columns, one a multiprocessor at a time, and are the faster form
-        where portions of length bring blocks enough; the token-by-token form cuts finer, which counts for few columns, and
-        a portion of a few tokens costs a block its start.  us token by token / in chunks, heads of 64 x 128, both kernels:
-        64 heads, 2,048 tokens 392 / 149, two prompts of 1,905 and 1,096 611 / 210, four of 1,200 487 / 331, eight of 128
-        98 / 87, sixteen of 64 100 / 104, one of 300 and 31 single ones 98 / 141; 16 heads (32 blocks a prompt), 2,048
-        tokens 126 / 125, 4,000 227 / 237, 1,905 and 1,096 178 / 121, four of 1,200 235 / 97."""
-        if not self.chunked or max(q_lens, default=0) < SSD_CHUNKS_FROM:
-            return False
-        blocks = self.heads * self.vdim // 32 * sum(n >= SSD_CHUNKS_FROM // 2 for n in q_lens)
-        return blocks >= 64 and sum((n + 31) // 32 for n in q_lens) >= 3 * len(q_lens)
-
-    def shape_key(self, q_lens):                                             # the kernels' choice
-        return "channel_delta1" if max(q_lens) == 1 else "delta_chunks" if self._in_chunks(q_lens) else "channel_delta"
-
-    def cache_need(self):
-        return CacheNeed(state=StateNeed((self.state_floats,)))
-
-    def streamed_weights(self):
-        return [self.inputs.weight, self.second.weight, self.out.weight]
-
-    def _second_products(self, proj):
-        """The decay's and the gate's pre-activations, float32 [T, heads * (dim + vdim)]."""
-        low = self.runtime.empty(proj.shape[0], self.ra + self.rg)
-        ops.take_columns(proj, self.low_at, low)
-        return self.second.forward(low, out_dtype=torch.float32)
-
-    def forward(self, h, ctx, cache):
-        n, heads = ctx.n_tokens, self.heads
-        proj = self.inputs.forward(h, out_dtype=torch.float32)
-        y = self.runtime.empty(n, heads * self.vdim)
-        if ctx.max_q_len == 1 and _ONE_KERNEL_STEP:
-            # every request brings one token: one kernel behind the input product (a decoding step is bound by
-            # its launches)
-            shift = heads == self.groups
-            pre = self._second_products(proj) if n > CHANNEL_STEP_ROWS else None
-            ops.cdr_step(proj, 0, self.b_at, self.low_at, self.ra, self.rg, self.second.weight, pre, self.groups, heads,
-                         self.dim, self.vdim, self.taps, self.conv_w, self.a_log, self.dt_bias, self.gain, self.eps,
-                         cache.state, self.conv_off, ctx.row_req, ctx.state_slot, shift, y)
-            if not shift:
-                ops.short_conv_state(proj, 0, self.channels, self.taps, cache.state, self.conv_off, ctx.q_start,
-                                     ctx.state_slot)
-            return self.out.forward(y, partials_ok=True)
-        pre = self._second_products(proj)
-        o = torch.empty((n, heads * self.vdim), dtype=torch.float32, device=proj.device)
-        if self._in_chunks(ctx.q_lens):
-            ops.delta_chunks(proj, 0, self.b_at, pre, 0, True, self.groups, heads, self.dim, self.vdim, self.taps,
-                             self.conv_w, self.a_log, self.dt_bias, cache.state, self.conv_off, ctx.q_start,
-                             ctx.state_slot, o)
-            ops.gdn_out_norm(o, pre, heads * self.dim, self.gain, 1.0, self.eps, y, heads, self.vdim, ctx.row_req,
-                             gate_kind="sigmoid")
-            return self.out.forward(y, partials_ok=True)
-        records = ops.cdr_records(n, ctx.q_start.shape[0] - 1, heads, self.dim, self.vdim, proj.device)
-        ops.cdr_prepare(proj, 0, self.b_at, pre, self.groups, heads, self.dim, self.vdim, self.taps, self.conv_w, self.a_log,
-                        self.dt_bias, cache.state, self.conv_off, ctx.q_start, ctx.state_slot, records)
-        ops.short_conv_state(proj, 0, self.channels, self.taps, cache.state, self.conv_off, ctx.q_start, ctx.state_slot)
-        ops.cdr_scan(records, heads, self.dim, self.vdim, cache.state, ctx.q_start, ctx.state_slot, o)
-        ops.gdn_out_norm(o, pre, heads * self.dim, self.gain, 1.0, self.eps, y, heads, self.vdim, ctx.row_req,
-                         gate_kind="sigmoid")
-        return self.out.forward(y, partials_ok=True)
-
-
-# A step whose longest portion has this many tokens may run the state-space recurrence in chunks
-SSD_CHUNKS_FROM = 128
-
-
-class Mamba2:
-    """The selective state-space mixer with a scalar decay a head (Mamba-2).  With inner = heads * vdim,
-    N = `state` lanes and G = `groups`: the input product W_in h is [z: inner | x: inner | B: G N | C: G N |
-    dt: heads].  x, B and C together pass a short causal convolution over time, channel by channel
-    (`.conv` [channels, taps], bias `.conv.b`, the last tap on the current token, zeros before a sequence's
-    start), and silu.  dt = softplus(dt + `.dt_bias`).  Per head (head h reads the B and C of group
-    h // (heads / G)) a matrix S (N x vdim) from zero:
-        S <- exp(-exp(A_log) dt) S + dt B x^T;   y = S^T C + D x.
-    y, heads side by side, times silu(z), is divided by its root mean square inside each of `norm_groups`
-    equal parts of the row (`eps` inside the root), multiplied by `.norm` and goes through `.o`.
-
-    The input product is written in float32; the convolution, dt, the decay, the recurrence, its state, the
-    gate and the norm are 32-bit whatever the products' precision (`csrc/short_conv.cu`, `csrc/mamba2.cu`).
-    Per request it keeps, in one state slot, the heads' matrices ([heads, vdim, N]) and behind them the
-    convolution's last taps - 1 inputs."""
-
-    graph_safe = True    # launches depend on device-side metadata alone
-
-    @staticmethod
-    def tensors(spec):
-        p, x = spec.params, spec.prefix
-        hidden, heads, vdim, n, groups, taps = p["hidden_size"], p["heads"], p["vdim"], p["state"], p["groups"], p["conv"]
-        inner, channels = heads * vdim, heads * vdim + 2 * groups * n
-        return [TensorSpec(x + ".in", (2 * inner + 2 * groups * n + heads, hidden)),
-                TensorSpec(x + ".conv", (channels, taps), "normal", 0.5), TensorSpec(x + ".conv.b", (channels,), "normal", 0.1),
-                TensorSpec(x + ".dt_bias", (heads,), "normal", 0.5), TensorSpec(x + ".A_log", (heads,), "normal", 0.5),
-                TensorSpec(x + ".D", (heads,), "one_plus_normal", 0.2), TensorSpec(x + ".norm", (inner,), "one_plus_normal"),
-                TensorSpec(x + ".o", (hidden, inner))]
-
-    def __init__(self, spec, store, runtime):
-        p, x = spec.params, spec.prefix
-        self.runtime = runtime
-        self.hidden = int(p["hidden_size"])
-        self.heads, self.vdim, self.n, self.groups = int(p["heads"]), int(p["vdim"]), int(p["state"]), int(p["groups"])
-        self.taps, self.norm_groups, self.eps = int(p["conv"]), int(p["norm_groups"]), float(p["eps"])
-        self.inner = self.heads * self.vdim
-        self.channels = self.inner + 2 * self.groups * self.n
-        if self.groups <= 0 or self.heads % self.groups:
-            raise ConfigError(f"{self.heads} heads do not divide into {self.groups} groups")
-        if self.norm_groups <= 0 or self.inner % self.norm_groups:
-            raise ConfigError(f"{self.inner} lanes do not divide into {self.norm_groups} parts for the norm")
-        if not 1 <= self.n <= ops.MAMBA2_MAX_STATE or not 1 <= self.taps <= 16:
-            raise ConfigError(f"the state-space recurrence takes states of up to {ops.MAMBA2_MAX_STATE} lanes and "
-                              f"convolutions of up to 16 taps; found {self.n} and {self.taps}")
-        self.inputs = Linear(runtime.matrix(stacked_rows([store.get(x + ".in")])))
-        self.conv_w = runtime.vector(store.get(x + ".conv"))
-        self.conv_b = runtime.vector(store.get(x + ".conv.b"))
-        self.dt_bias = runtime.vector(store.get(x + ".dt_bias"))
-        self.a_log = runtime.vector(store.get(x + ".A_log"))
-        self.skip = runtime.vector(store.get(x + ".D"))
-        self.gain = runtime.vector(store.get(x + ".norm"))
-        self.out = Linear(runtime.matrix(store.get(x + ".o")))
-        # a slot: [heads, vdim, N] and behind it [taps - 1, channels], in whole 4s of floats
-        self.conv_off = self.heads * self.vdim * self.n
-        self.state_floats = -(-(self.conv_off + (self.taps - 1) * self.channels) // 4) * 4
-        # a float32 model keeps the token-by-token form, as with the delta rules, and so does who asks for its segments
-        self.chunked = runtime.dtype == torch.bfloat16 and ops.ssd_chunks_supported(self.vdim, self.n) and \
-            "TOKB200_M2_SEGMENTS" not in os.environ
-
-    def cache_need(self):
-        return CacheNeed(state=StateNeed((self.state_floats,)))
-
-    def _in_chunks(self, q_lens) -> bool:
-        """Chunks of 32 tokens are cut over blocks of 32 columns, one a multiprocessor at a time, and are the faster form
-        where portions of length fill one or two turns of them; the token-by-token form cuts finer (few columns) and packs
-        better (many).  us token by token / in chunks, heads of 64 x 128: 64 heads, 2,048 tokens 307 / 214, two prompts of
-        1,905 and 1,096 412 / 312, 128 tokens 32 / 24, 40 tokens 13 / 18; 48 heads, 1,024 tokens 128 / 111; 32 heads, 2,048
-        tokens 175 / 203; 128 heads, 1,024 tokens 247 / 210, 128 tokens 44 / 52; 64 heads, four of 512 215 / 220."""
-        if not self.chunked or max(q_lens, default=0) < SSD_CHUNKS_FROM:
+        """Chunks of 32 tokens are cut over blocks of 32 columns, one a multiprocessor at a time, and are the faster form where
+        portions of length bring blocks enough; the token-by-token form cuts finer, which counts for few columns, and a
+        portion of a few tokens costs a block its start.  us a layer, token by token / in chunks, 64 heads of 64 x 128 in 8
+        groups: 2,048 tokens 477 / 298, 128 65 / 52, three of 622, 357 and 1,021 567 / 301, four of 1,200 834 / 675, sixteen of
+        128 346 / 320, 1,024, 600 and 20 single ones 545 / 316, 700 and 29 single ones a third of it 456 / 409 (not taken), 300 and
+        31 158 / 205, sixteen of 130 and sixteen of 2 384 / 422; 32 heads in one group 2,048 238 / 195, sixteen of 140 and ten of 2
+        183 / 197; 24 heads (48 blocks) 185 / 182; 16 heads (32) 150 / 172, two of 1,905
+        and 1,096 (64) 202 / 184; 128 heads, 128 tokens 117 / 102.  Where B and C are cut into pieces for few heads a group only
+        while the blocks fill one or two turns (64 heads in 64 groups, 2,048 791 / 634, three of 128 158 / 155, four of 1,200
+        1,424 / 1,443, eight of 128 323 / 353)."""
+        longest = max(q_lens, default=0)
+        if not self.chunked or longest < SSD_CHUNKS_FROM:
             return False
         columns = self.heads * self.vdim // 32
         blocks = columns * sum(n >= SSD_CHUNKS_FROM // 2 for n in q_lens)
-        return 96 <= blocks <= 296 and max(q_lens) >= SSD_CHUNKS_FROM * (1 if blocks <= 148 else 2) and \
-            columns * len(q_lens) <= 592                              # portions of a few tokens take turns, too
+        if 4 * self.groups > self.heads and \
+                not (96 <= blocks <= 296 and longest >= SSD_CHUNKS_FROM * (1 if blocks <= 148 else 2)):
+            return False
+        # more than three chunks a portion (four, where none is long), or so few portions that those of a few tokens take turns
+        # with no others
+        chunks = sum((n + 31) // 32 for n in q_lens)
+        return blocks >= 64 and (chunks > 3 * len(q_lens) and (longest >= 256 or chunks >= 4 * len(q_lens)) or
+                                 columns * len(q_lens) <= 592)
 
     def shape_key(self, q_lens):                                             # the kernels' choice
         return "ssm1" if max(q_lens) == 1 else "ssm_chunks" if self._in_chunks(q_lens) else "ssm"
