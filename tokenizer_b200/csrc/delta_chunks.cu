@@ -22,11 +22,13 @@
 // The scan is one chain: a chunk's products need the matrix that the chunk before left.  Counters at 2,048 tokens: shared
 // memory's pipe busy 53 % of the time, the tensor cores 30 %; with FMA register tiles that pipe was busy 62 % and the scan of
 // 16 heads took 162 us where it now takes 111.  The prepare kernel is bound by latency, not by a pipe (instructions issue 39 %
-// of the time, two blocks of eight warps an SM by shared memory): loops that keep its code small made it slower (88.7 -> 100
-// us), loads and exponentials side by side faster (105 -> 94 us by head at 2,048, 239 -> 221 by
-// channel over four prompts).  Measured
+// of the time, two blocks of eight warps an SM by shared memory): short loops over copied inputs for the convolution
+// and the decays, eight tokens' loads and exponentials side by side, made it faster (105 -> 94 us by head at 2,048, 239 -> 221 by
+// channel over four prompts); half of all its code in loops, tried on an earlier form of it, slower (88.7 -> 100 us).  Measured
 // (16 heads of 128 x 128, both kernels and the kept inputs between them, us; in front the FMA tiles): a prompt of 2,048
-// tokens 254 -> 200 with one decay a head and 272 -> 212 with one a channel, four prompts of 5,100 in all 537 -> 479.
+// tokens 254 -> 197 with one decay a head and 272 -> 209 with one a channel, four prompts of 5,100 in all 537 -> 479.  Error
+// against 64 bits (2-norm, 2,048 tokens at memories of tens to hundreds), outputs and 32-bit states, FMA tiles / here: 1.89e-7 /
+// 1.85e-7 and 2.03e-7 / 1.85e-7, by channel 1.94e-7 / 1.87e-7 and 2.55e-7 / 2.33e-7.  A record takes 95 KB at 128 values.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).

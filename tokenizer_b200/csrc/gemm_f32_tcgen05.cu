@@ -20,7 +20,11 @@
 // `gemm_f32_sum_kernel` adds in the same order, which gives the same bits.
 //
 // Measured (one B200, us, this / the kernel of multiply-adds): 777 rows of 1,152 x 896 21 / 71, 896 x 896 16 / 57, 9,728 x 896
-// 104 / 343 (131 TFLOP/s), 896 x 4,864 56 / 291; one row of the same 9.6 / 9.0, 9.6 / 9.0, 14.4 / 15.0, 12.9 / 39.9.  Error
+// 104 / 343 (131 TFLOP/s), 896 x 4,864 56 / 291; one row of the same 9.6 / 9.0, 9.6 / 9.0, 14.0 / 14.9, 13.1 / 39.8,
+// and of the vocabulary's 151,936 x 896 137 / 118 (to four rows; 8 rows 141 / 217, 16 147 / 214), of 17,920 x 1,536 30.5 / 28.6, 37,888
+// x 3,584 125 / 123: few rows of a wide weight wait for the converters, which have one stage of 32 KB an SM on its way.  A whole
+// step of one row gains (24 layers of the first four and the vocabulary 1,250 / 1,870), and a row must meet the same kernel
+// in every batch, so the line is drawn by k alone.  Error
 // against 64 bits (2-norm, normal numbers) 2.1e-7 / 5.3e-7 at k = 896, 2.2e-7 / 1.25e-6 at 4,864; from k = 768 on it is the
 // smaller one for numbers of one sign too (896: 3.2e-7 / 4.4e-7; 512: 3.8e-7 / 3.5e-7), which is where `ops.gemm_f32` draws
 // the line.  A stage of 80 rows takes 1,270 ns: the products alone 745, the cutting alone 735 (both bound by shared memory,

@@ -16,8 +16,10 @@
 //
 // The tensor pipe is busy 41 % of a block's time (counters), the pipe of shared memory 60 %: two warps a scheduler, each
 // a chain of reads, cuts, products and sums.  Measured (heads of 64 x 128, us of both kernels, token by token / multiply-adds
-// in chunks / here): 64 heads, a prompt of 2,048 tokens 392 / 213 / 149, two of 1,905 and 1,096 611 / 311 / 210; 16 heads,
-// 2,048 126 / 198 / 125, four of 1,200 235 / 135 / 97.
+// in chunks / here): 64 heads, a prompt of 2,048 tokens 392 / 213 / 149, two of 1,905 and 1,096 611 / 311 / 214; 16 heads,
+// 2,048 126 / 198 / 125, four of 1,200 235 / 135 / 97.  Error against 64 bits (2-norm, memories of tens to hundreds of tokens),
+// outputs and 32-bit states, multiply-adds in chunks / here: two prompts, 64 heads 1.43e-7 / 1.44e-7 and 1.66e-7 / 1.46e-7, 2,048
+// tokens, 16 heads 1.38e-7 / 1.36e-7 and 1.77e-7 / 1.51e-7.  A chunk's records take 4.3 KB a head and 49 KB a group.
 //
 // A request's chunks are counted from its portion's first row; the record of chunk c of request r lies at place
 // q_start[r] / 32 + r + c (no two the same, and known without a pass over the other requests).

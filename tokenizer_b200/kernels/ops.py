@@ -1033,7 +1033,8 @@ def layer_small_m_check(d: int) -> None:
 # ---- few rows, a large weight: one block a multiprocessor streams it through rings in shared memory ----
 RING_ELEMENTS = 13_000_000     # from this many weight elements on (26 MB) the ring kernel leads the one with plain loads
 RING_MAX_ROWS = 32
-RING_ROWS = 8                   # rows up to which the ring kernel is at least level with the tensor cores on such a weight
+RING_ROWS = 8                   # rows up to which the ring kernel is at least level with the tensor cores on such a weight (gated
+                                # products, and partial sums; a finished product of 9 to 16 rows stays on the ring)
 # TOKB200_RING=0: large weights of few rows on linear_small_m like small ones, neither on rings nor (9 to 16 rows) on the tensor cores
 _RING = os.environ.get("TOKB200_RING", "1") != "0"
 _ring_plans = {}
@@ -1069,7 +1070,7 @@ def linear_ring_splits(M: int, N: int, K: int, sms: int) -> int:
 
 
 def linear_ring(x, w, bias, out, k_splits: int = 1, activation: Optional[str] = None) -> None:
-    """out = act(x @ w.T (+ bias)) (`activation` None: no act) for up to 16 rows and a large weight (bfloat16 in; out [M,N]
+    """out = act(x @ w.T (+ bias)) (`activation` None: no act) for up to 32 rows and a large weight (bfloat16 in; out [M,N]
     bfloat16/float32, or float32 partial sums [k_splits, M, N] without bias)."""
     M, K = x.shape
     N = w.shape[0]
@@ -1088,7 +1089,8 @@ def linear_ring(x, w, bias, out, k_splits: int = 1, activation: Optional[str] = 
 
 
 def linear_ring_gated(x, w, out, activation: str = "silu") -> None:
-    """out[M, N/2] = act(x Wg^T) * (x Wu^T) for w from `interleave_gate_up`, up to 16 rows, a large weight."""
+    """out[M, N/2] = act(x Wg^T) * (x Wu^T) for w from `interleave_gate_up`, up to 32 rows, a large weight (`gated_linear` comes
+    here with up to RING_ROWS; beyond, the tensor cores lead)."""
     M, K = x.shape
     N = w.shape[0]
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or \
