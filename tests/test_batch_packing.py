@@ -104,19 +104,22 @@ def test_what_a_step_may_not_bring():
 
 
 def test_rows_by_length():
-    """The longest row first, -1 behind the last, and whether the rows are alike; nothing of a step that brings portions."""
+    """The longest row first, -1 behind the last, and whether the rows are alike."""
     from tokenizer_b200.parts.attention import RowsByLength
     note = RowsByLength()
 
     def fill(starts, counts=None, capacity=8, padded=True):
+        capacity = max(capacity, len(starts))
         counts = np.ones(len(starts), dtype=np.int32) if counts is None else np.asarray(counts, dtype=np.int32)
         first = np.concatenate(([0], np.cumsum(counts)[:-1])).astype(np.int32)
         out = np.zeros(note.capacity(capacity, capacity), dtype=np.int32)
         made = note.fill(out, first, counts, np.asarray(starts, dtype=np.int32), padded)
         return made, int(out[0]), out[4:].tolist()
-    assert fill([5, 9, 9, 7]) == (8, 1, [1, 2, 3, 0, -1, -1, -1, -1])
-    assert fill([5, 9, 9, 7], padded=False)[0] == 4
-    assert fill([99, 39, 39, 62])[1] == 1 and fill([99, 39, 39, 58])[1] == 0          # 60 % of 4 x 100 keys, and below
-    assert fill([0, 0])[1] == 1
-    assert fill([5, 9], counts=[1, 3]) == (0, 0, [-1] * 8)
-    assert fill([]) == (0, 0, [-1] * 8)
+    many = [5, 9, 9, 7, 8, 8, 8, 8, 8, 8]
+    assert fill(many, capacity=12) == (12, 1, [1, 2, 4, 5, 6, 7, 8, 9, 3, 0, -1, -1])
+    assert fill(many, padded=False)[0] == 10
+    assert fill([99] + [54] * 8 + [59])[1] == 1 and fill([99] + [54] * 8 + [58])[1] == 0      # 60 % of 10 x 100 keys, and below
+    assert fill([0] * 10)[1] == 1
+    assert fill([5, 9, 9, 7]) == (8, 0, [0, 1, 2, 3, -1, -1, -1, -1])                         # few rows: as they come
+    assert fill([5] * 10, counts=[1] * 9 + [3])[1] == 0
+    assert fill([]) == (8, 0, [-1] * 8)

@@ -118,22 +118,25 @@ class SingleRows(BatchAnnotation):
 class RowsByLength(BatchAnnotation):
     """Of a step of single tokens: whether the rows are of like length (one word, 1 where their keys are on the average
     `EVEN` of the longest row's or more), and behind three words of nothing the rows' indices, the longest row first, -1
-    where there is none: int32 [4 + requests]."""
+    where there is none: int32 [4 + requests].  Steps of a few rows, which fill no device, keep their order (packing is on
+    the way of a small step)."""
 
     key = "rows_by_length"
     EVEN = 0.6
+    FEW = 10
 
     def capacity(self, n_tokens, n_requests):
         return 4 + n_requests
 
     def fill(self, out, first_rows, counts, starts, padded):
         n = len(counts)
-        out[4:] = -1
-        if not n or int(counts.max()) > 1:
-            return 0
-        order = np.argsort(-starts, kind="stable")
-        out[4:4 + n] = first_rows[order]
-        out[0] = int(starts.sum()) + n >= self.EVEN * n * (int(starts[order[0]]) + 1)
+        out[4 + n:] = -1
+        if n < self.FEW:
+            out[4:4 + n] = first_rows
+        elif int(counts.max()) == 1:
+            order = np.argsort(-starts, kind="stable")
+            out[4:4 + n] = first_rows[order]
+            out[0] = int(starts.sum()) + n >= self.EVEN * n * (int(starts[order[0]]) + 1)
         return (len(out) - 4) if padded else n
 
 
@@ -218,7 +221,7 @@ class PagedAttention:
                 group.block_table.shape[1] * group.page_size <= 4096:
             return None, None
         words, count = ctx.views.get(_BY_LENGTH.key, (None, 0))
-        return (words[4:4 + count], words[:1]) if count == ctx.n_tokens else (None, None)
+        return (words[4:4 + count], words[:1]) if count == ctx.n_tokens else (None, None)      # a row a request
 
     def attend(self, q, out, ctx, group, cache):
         """Choose the kernel by precision and by the shape of the batch.  A group that keeps one
