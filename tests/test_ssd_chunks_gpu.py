@@ -161,8 +161,8 @@ def test_numbers_without_pieces(where, n):
 @pytest.mark.parametrize("heads,groups,lengths", [(16, 1, [2048]), (64, 8, [1905, 1096]), (64, 8, [300])])
 def test_error_of_outputs_and_states(heads, groups, lengths):
     """Pieces on the tensor cores against plain multiply-adds token by token, both against 64 bits, at memories of tens to
-    hundreds of tokens: 1.02 to 1.12 times its error in the outputs, up to 1.00 times in the matrix (measured; with one sum for all products
-    of pieces 1.10 to 1.24 and 1.10 to 1.13)."""
+    hundreds of tokens: measured 1.11 to 1.13 times its error in the outputs and 0.95 to 1.03 times in the matrix (with one sum
+    for all products of pieces 1.18 to 1.25 and 1.06 to 1.18)."""
     from tokenizer_b200.kernels import ops as o
     vdim, n_state, rows = 64, 128, sum(lengths)
     inner, share = heads * vdim, heads // groups
@@ -192,4 +192,4 @@ def test_error_of_outputs_and_states(heads, groups, lengths):
         states.append(S.reshape(-1))
     want = (want.reshape(rows, -1), torch.stack(states))
     chunks, tokens = ([float((got.double() - ref).norm() / ref.norm()) for got, ref in zip(pair, want)] for pair in found)
-    assert chunks[0] <= 1.2 * tokens[0] and chunks[1] <= 1.07 * tokens[1]
+    assert chunks[0] <= 1.16 * tokens[0] and chunks[1] <= 1.05 * tokens[1]
