@@ -164,11 +164,11 @@ short_conv_tile_kernel(const TI* __restrict__ x, int ld, int at, int channels, c
     for (int i = 0; i < ROWS; ++i) in[i] = conv_load_raw(x + (size_t)(t0 + i) * ld + at + c);
 #pragma unroll
     for (int k = 0; k < TAPS - 1; ++k) ahead[k] = conv_load_raw(x + (size_t)(t0 - (TAPS - 1 - k)) * ld + at + c);
-    conv_weights<TAPS>(w, c, wt);
-    const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int r = row_req[t0];
     const int begin = r >= 0 ? q_start[r] : 0, end = r >= 0 ? q_start[r + 1] : 0;
     if (r >= 0 && begin + TAPS - 1 <= t0 && t0 + ROWS <= end) {
+      conv_weights<TAPS>(w, c, wt);
+      const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int k = 0; k < TAPS - 1; ++k) win[k] = conv_unpack(ahead[k]);
 #pragma unroll
