@@ -76,10 +76,14 @@ class Launches:
         monkeypatch.setattr(ops, "_lib", lambda name: self)
         monkeypatch.setattr(ops, "_ptr", lambda t: None)
         monkeypatch.setattr(ops, "_stream", lambda: None)
-        monkeypatch.setattr(ops, "linear_ring_supported", lambda M, N, K, k_splits=1, gated=False: M <= ops.RING_MAX_ROWS)
+        monkeypatch.setattr(ops, "linear_ring_supported", lambda M, N, K, k_splits=1, gated=False:
+                            M <= ops.RING_MAX_ROWS and K // k_splits <= (4096 if M <= 16 else 1536))
 
     def __getattr__(self, name):
         return lambda *args: self.names.append(name.replace("tokb200_", "")) or 0
+
+
+BF16 = dict(dtype=torch.bfloat16, device="meta")
 
 
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
@@ -89,14 +93,40 @@ def test_large_weights_of_few_rows(monkeypatch, M, on):
     from tokenizer_b200.kernels import ops
     launches = Launches(monkeypatch)
     monkeypatch.setattr(ops, "_RING", on)
-    empty = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="meta")
-    ops.gated_linear(empty(M, 1536), empty(17920, 1536), empty(M, 8960))
-    rules.linear_bf16(empty(M, 13312), empty(1024, 13312), None, torch.bfloat16, partials_ok=True)
-    rules.linear_bf16(empty(M, 3584), empty(4608, 3584), torch.empty(4608, device="meta"), torch.bfloat16)
+    ops.gated_linear(torch.empty(M, 1536, **BF16), torch.empty(17920, 1536, **BF16), torch.empty(M, 8960, **BF16))
+    rules.linear_bf16(torch.empty(M, 8192, **BF16), torch.empty(2048, 8192, **BF16), None, torch.bfloat16, partials_ok=True)
+    rules.linear_bf16(torch.empty(M, 3584, **BF16), torch.empty(4608, 3584, **BF16), torch.empty(4608, device="meta"),
+                      torch.bfloat16)
     want = ["linear_small_m_gated", "linear_small_m", "linear_small_m"] if not on else \
         ["linear_ring_gated", "linear_ring", "linear_ring"] if M <= 8 else \
         ["gemm_tcgen05_gated", "gemm_tcgen05_partials", "linear_ring"]
     assert launches.names == want
+
+
+@pytest.mark.parametrize("M,N,K,want", [
+    # tiles that fill their turns of 148, that do not, and k so short that it does not matter
+    (9, 37888, 3584, "gemm_tcgen05"), (16, 28672, 2048, "gemm_tcgen05"), (9, 14336, 2048, "gemm_tcgen05"),
+    (9, 8192, 4096, "linear_ring"), (16, 11264, 2048, "linear_ring"), (9, 20480, 3584, "linear_ring"), (9, 40960, 2560, "linear_ring"),
+    (9, 20480, 896, "gemm_tcgen05"), (16, 22528, 1024, "gemm_tcgen05"), (9, 20480, 1024, "linear_ring"),
+    # k beyond the ring kernel's
+    (9, 4096, 5120, "linear_small_m"), (16, 8192, 5120, "linear_small_m"), (9, 11264, 5120, "gemm_tcgen05"),
+    # a small weight: never; 17 to 32 rows: the ring where tiles are few
+    (16, 9728, 896, "linear_small_m"), (17, 1024, 1024, "linear_ring"), (32, 4096, 1536, "linear_ring"),
+    (17, 9728, 896, "gemm_tcgen05"), (33, 1024, 1024, "gemm_tcgen05"), (24, 4096, 2048, "gemm_tcgen05")])
+def test_gated_products_of_few_rows(monkeypatch, M, N, K, want):
+    from tokenizer_b200.kernels import ops
+    launches = Launches(monkeypatch)
+    ops.gated_linear(torch.empty(M, K, **BF16), torch.empty(N, K, **BF16), torch.empty(M, N // 2, **BF16))
+    assert launches.names == [want + "_gated"]
+
+
+@pytest.mark.parametrize("M,N,K,want", [
+    (9, 1024, 13312, "linear_ring"), (16, 1024, 13312, "linear_ring"), (17, 1024, 13312, "gemm_tcgen05_partials"),
+    (9, 1536, 8960, "gemm_tcgen05_partials"), (9, 4096, 12288, "gemm_tcgen05_partials"), (8, 4096, 12288, "linear_ring")])
+def test_partial_sums_of_few_rows(monkeypatch, M, N, K, want):
+    launches = Launches(monkeypatch)
+    rules.linear_bf16(torch.empty(M, K, **BF16), torch.empty(N, K, **BF16), None, torch.bfloat16, partials_ok=True)
+    assert launches.names == [want]
 
 
 def test_what_is_no_integer_is_refused():

@@ -754,6 +754,19 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
         .reshape(2 * inner, k).contiguous()
 
 
+def few_rows_on_tensor_cores(units: int, k: int, ring: bool) -> bool:
+    """Whether nine to sixteen rows of a large gated weight go to the tensor cores, whose units of work are its tiles of 128
+    rows: where they fill their turns of 148 multiprocessors to three quarters (us at 9 rows, ring / tensor cores: 17,920 x 1,536,
+    140 units 14.5 / 13.0, 37,888 x 3,584, 296 47 / 44, 28,672 x 2,048, 224 25.2 / 24.2; 8,192 x 4,096, 64 17 / 21, 20,480 x 3,584, 160
+    29 / 37, 40,960 x 3,584, 320 53 / 57) or k is short (20,480 x 896 11.8 / 10.9, 22,528 x 1,024, 176 13.5 / 13.3, 20,480 x 1,024, 160
+    12.4 / 13.8).  A weight that the ring kernel does not take (k above 4,096) falls to `linear_small_m` else, which leads
+    up to 64 units alone (x 5,120, 64 18.5 / 25.7, 88 34 / 26, 160 52 / 52)."""
+    if not ring:
+        return units > 64
+    idle = -(-units // 148) * 148 / units
+    return k < 1024 or idle <= (1.7 if k < 1536 else 1.34)
+
+
 def gated_linear(x, w, out, activation: str = "silu") -> None:
     """out[M, N/2] = act(x Wg^T) * (x Wu^T) for w from `interleave_gate_up`; the activation
     is an epilogue parameter of whichever kernel the row count selects."""
@@ -764,12 +777,15 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
         raise ValueError("gated_linear is the bfloat16 kernel")
     if not gated_linear_supported(K, N) or w.shape[1] != K or tuple(out.shape) != (M, N // 2):
         raise ValueError("gated_linear: K a multiple of 8, N of 256, out [M, N/2]")
-    if _RING and RING_ROWS < M <= SMALL_M_ROWS and N * K >= RING_ELEMENTS:
-        # a large weight and nine rows or more (us at 16 rows, this / the ring kernel: 17,920 x 1,536 11.3 / 13.6, 37,888 x 3,584
-        # 44 / 50; at 8 11.1 / 11.6 and 43.7 / 43.6)
+    large = _RING and M <= SMALL_M_ROWS and N * K >= RING_ELEMENTS
+    ring = (large or (_RING and SMALL_M_ROWS < M <= RING_MAX_ROWS and N <= 5120)) and linear_ring_supported(M, N, K, 1, True)
+    if large and M > RING_ROWS and few_rows_on_tensor_cores(N // 128, K, ring):
         _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_gated(
             _ptr(x), _ptr(w), _ptr(out), _i(M), _i(N), _i(K), act, _stream()), "gated_linear")
-    elif M <= SMALL_M_ROWS and _RING and N * K >= RING_ELEMENTS and linear_ring_supported(M, N, K, 1, True):
+    elif ring:
+        # a large weight, or 17 to 32 rows of one whose 40 tiles of 128 and fewer leave most of the tensor cores idle (us at 17 / 32
+        # rows, this / tensor cores: 1,024 x 1,024 3.6 / 6.9 and 4.3 / 7.5, 4,096 x 1,536 6.8 / 9.1 and 8.3 / 9.6; 5,632 x 1,024 6.9 / 7.3
+        # and 7.9 / 7.7)
         linear_ring_gated(x, w, out, activation)
     elif M <= SMALL_M_ROWS:
         _check(_lib("linear_small_m").tokb200_linear_small_m_gated(
@@ -781,7 +797,7 @@ def gated_linear(x, w, out, activation: str = "silu") -> None:
             _ptr(x), _ptr(w), None, _ptr(out), _i(PAIR_GATED), _i(M), _i(N), _i(K), _i(1), act, _stream()),
             "gated_linear")
     else:
-        # up to 64 rows the entry has the weight's rows as the product's M (us at 17 and 32 rows, against the ring kernel:
+        # up to 64 rows the entry has the weight's rows as the product's M (us at 17 and 32 rows, this / the ring kernel:
         # 9,728 x 896 6.8 / 8.8 and 7.2 / 10.1, 17,920 x 1,536 11.5 / 16.7 and 11.9 / 19.7)
         _check(_lib("gemm_tcgen05").tokb200_gemm_tcgen05_gated(
             _ptr(x), _ptr(w), _ptr(out), _i(M), _i(N), _i(K), act, _stream()), "gated_linear")

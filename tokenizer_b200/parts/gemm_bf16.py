@@ -139,6 +139,10 @@ def linear_bf16(a: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     tensor_rows = ops.RING_ROWS if ops._RING and N * K >= ops.RING_ELEMENTS else ops.SMALL_M_ROWS
     if partials_ok and bias is None and M > tensor_rows and use_tcgen05(M, N, K, cut_along_k=True):
         tiles_cut = choose_tile_k_splits(M, N, K)
+        if M <= ops.SMALL_M_ROWS and -(-N // 128) * tiles_cut < 96:
+            # a narrow weight, in eight pieces still few units of work (us at 9 / 16 rows, ring / tensor cores: 1,024 x 13,312, 64 units
+            # 8.5 / 10.1 and 9.2 / 10.2; 1,536 x 8,960, 96 7.8 / 7.8 and 8.2 / 8.1; 2,048 x 8,192, 128 10.3 / 9.4 and 10.8 / 9.4)
+            tiles_cut = 1
     if tiles_cut > 1:
         # few output tiles (a narrow matrix, a few dozen rows): pieces of k over all SMs.  From 17 rows on this leads the ring
         # kernel (us, this / ring: 896 x 896 2.5 / 3.2 at 17 rows, 2.6 / 3.9 at 32; 896 x 4,864 4.5 / 4.9 and 4.7 / 5.3;
